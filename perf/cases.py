@@ -212,7 +212,7 @@ def tolerance(case):
     """Four times the largest error of the calls against the same recurrence (and layer) in 64-bit arithmetic, over the
     listed cases and a few drawn ones; measured (2-norm, largest): decode 1.7e-3, 3.9e-3 in bf16 (the rounding of o)
     and 2.1e-4, 4.9e-4 in f16; the chunkwise forms 2.9e-3, 2.1e-2 in bf16 (their erase and query operands are bf16);
-    float32 2.7e-7, 1.7e-6; the layer 5.5e-3, 4.3e-2 for prompts and 4.1e-3, 1.7e-2 for one token (its projections
+    float32 2.8e-7, 2.1e-6; the layer 5.5e-3, 4.3e-2 for prompts and 4.1e-3, 1.7e-2 for one token (its projections
     are rounded to bf16)."""
     kind = case["kind"]
     if kind == "layer_prefill":
@@ -220,7 +220,7 @@ def tolerance(case):
     if kind == "layer_step":
         return {"rel": 1.6e-2, "max": 7e-2}
     if case["dtype"] == "f32":
-        return {"rel": 1.1e-6, "max": 7e-6}
+        return {"rel": 1.1e-6, "max": 8e-6}
     if case["dtype"] == "f16":
         return {"rel": 9e-4, "max": 2e-3}
     return {"rel": 7e-3, "max": 1.6e-2} if kind == "decode" else {"rel": 1.2e-2, "max": 8e-2}
