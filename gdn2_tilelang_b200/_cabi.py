@@ -39,6 +39,7 @@ SIGNATURES = {
     "gdn2_prefill_scan_segments": (_int, [_i64] * 5 + [_int, _int]),
     "gdn2_prefill_scan_launches": (_int, [_i64] * 5 + [_int, _int]),
     "gdn2_prefill_scan_part": (_int, [_vp, _sz, _vp, _vp, _vp] + [_i64] * 7 + [_int, _int, _int, _vp]),
+    "gdn2_prefill_ragged_workspace_bytes": (_sz, [_i64] * 6 + [_int, _int]),
     "gdn2_prefill_ragged": (_int, [_vp] * 10 + [_sz] + [_i64] * 8 + [_f32, _int, _int, _vp, _vp]),
     "gdn2_prefill_workspace_layout": (_int, [_i64] * 6 + [_int, _int, ctypes.POINTER(ctypes.c_int64)]),
     "gdn2_chunk_prep": (_int, [_vp] * 7 + [_sz] + [_i64] * 7 + [_f32, _int, _int, _vp]),
@@ -246,7 +247,8 @@ class NativeKernels:
     # -- prefill in one call ---------------------------------------------------------------
     def prefill_ragged(self, q, k, v, g, b, w, scale: float, initial_state=None):
         """``gdn2_prefill`` as ONE library call (``gdn2_prefill_ragged``): chunk-local stage and scan on the whole
-        chunks, decode on the ragged tail, the tail beside the scan's correction pass when the scan is cut.
+        chunks, decode on the ragged tail, the tail beside the scan's correction pass when the scan is cut; the SIMT
+        family takes the tail as one more chunk.
         Returns ``(o, final_state)`` or ``None`` when this form does not apply (fewer than 64 tokens; a problem
         whose two stages the host overlaps segment by segment) and the caller composes the stages itself."""
         _require_cuda(q, k, v, g, b, w, initial_state)
@@ -265,7 +267,7 @@ class NativeKernels:
         in_bs = views[0][1]
         q, k, v, g, b, w = (t for t, _ in views)
         dev = q.device
-        nbytes = self.lib.gdn2_prefill_workspace_bytes(B, n_full, H, HK, DK, DV, code, p)
+        nbytes = self.lib.gdn2_prefill_ragged_workspace_bytes(B, S, H, HK, DK, DV, code, p)
         if nbytes == 0:
             raise GDN2KernelError(
                 f"no kernel for DK={DK}, DV={DV}, dtype={q.dtype} (SIMT family: DK<=128, DK%8==0, DV%4==0)")
@@ -284,7 +286,7 @@ class NativeKernels:
                 None if side is None else side.cuda_stream, main.cuda_stream)
         _check(self.lib, rc, "gdn2_prefill_ragged")
         self.launches += (2 if p != PATH_SIMT else 1) + self.lib.gdn2_prefill_scan_launches(B, n_full, H, DK, DV, code, p) \
-            + (1 if S > n_full else 0)
+            + (1 if S > n_full and p != PATH_SIMT else 0)
         return o, final_state
 
     # -- chunkwise forward -----------------------------------------------------------------

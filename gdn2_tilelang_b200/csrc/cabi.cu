@@ -259,6 +259,17 @@ int prefill_scan_impl(const void* workspace, size_t workspace_bytes, const float
 }
 }  // namespace
 
+size_t gdn2_prefill_ragged_workspace_bytes(int64_t B, int64_t S, int64_t H, int64_t HK, int64_t DK, int64_t DV, int dtype,
+                                           int path) {
+  if (S <= 0) return 0;
+  const int64_t n_full = S / kChunk * kChunk, up = (S + kChunk - 1) / kChunk * kChunk;
+  int p;
+  bool seg;
+  if (resolve_path(DK, DV, dtype, path, &p, &seg) != GDN2_OK) return 0;
+  // the exact family takes the ragged tail as one more chunk with neutral rows; the tensor-core family decodes it
+  return gdn2_prefill_workspace_bytes(B, n_full && p == GDN2_PATH_SIMT ? up : n_full, H, HK, DK, DV, dtype, path);
+}
+
 int gdn2_prefill_ragged(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
                         const float* initial_state, void* o, float* final_state, void* workspace, size_t workspace_bytes,
                         int64_t B, int64_t S, int64_t H, int64_t HK, int64_t DK, int64_t DV, int64_t in_batch_stride,
@@ -271,6 +282,26 @@ int gdn2_prefill_ragged(const void* q, const void* k, const void* v, const float
   const size_t esz = dtype == GDN2_F32 ? 4 : 2;
   cudaStream_t st = static_cast<cudaStream_t>(stream), side = static_cast<cudaStream_t>(side_stream);
   int rc = GDN2_OK;
+  if (n_full && n_tail && workspace) {
+    // Exact family: the tail is one more chunk whose missing rows have k = q = v = 0 and no decay: one more step of the
+    // scan's chain (a few us) where the token-by-token decode takes up to 63. A workspace sized for the whole chunks only
+    // keeps the decode.
+    int p;
+    bool seg;
+    const int64_t up = n_full + kChunk;
+    if (check_prefill_shape(B, up, H, HK, DK, DV, dtype) == GDN2_OK && resolve_path(DK, DV, dtype, path, &p, &seg) == GDN2_OK &&
+        p == GDN2_PATH_SIMT) {
+      const WsLayout L = layout_for(B, up, H, HK, DK, DV, p, seg);
+      if (workspace_bytes >= L.total) {
+        if (!aligned16(workspace) || !aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(g) || !aligned16(b) || !aligned16(w))
+          return GDN2_ERR_MISALIGNED;
+        const WsPtrs P = ws_pointers(workspace, L);
+        rc = launch_prep_simt(q, k, v, g, b, w, L, P, (int)B, (int)S, (int)H, (int)HK, in_batch_stride, scale, dtype, false, st);
+        if (rc != GDN2_OK) return rc;
+        return launch_scan_simt(L, P, initial_state, o, final_state, nullptr, (int)B, (int)S, (int)H, o_batch_stride, dtype, st);
+      }
+    }
+  }
   if (n_full) {
     if (!workspace) return GDN2_ERR_NULL_POINTER;
     rc = gdn2_chunk_prep(q, k, v, g, b, w, workspace, workspace_bytes, B, n_full, H, HK, DK, DV, in_batch_stride, scale,

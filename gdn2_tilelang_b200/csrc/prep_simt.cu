@@ -2,14 +2,21 @@
 // of 8), any DV (multiple of 4), fp32 arithmetic throughout. One 256-thread block per
 // (chunk, batch*head).
 //
-// Every entry of the two intra-chunk matrices is evaluated with the exact pairwise decay
-//     sum_c x_r[c] * k_s[c] * exp2(G_r[c] - G_s[c]),   r >= s   (exponent <= 0 by construction)
-// which is the form the reference uses only for its diagonal sub-blocks (intra_diag_kernel,
-// gdn2/forward.py:220-235 of the reference project); using it everywhere makes this family safe
-// for arbitrarily fast decay without any reference-row factorisation. The inverse (I + Tm)^-1 is
-// built column by column with forward substitution (solve_kernel, gdn2/forward.py:424-434), then
-// W = Ai E, U = Ai (w*v), KG and Qg follow wy_kernel (gdn2/forward.py:512-533) and the query
-// scaling of prefill_scan_kernel (gdn2/inference.py:461).
+// The two intra-chunk matrices are sums over channels of x_r * k_s * exp2(G_r - G_s), r >= s (exponent <= 0 by
+// construction), evaluated in 4 x 4 tiles of (r, s). On a tile of the diagonal every pair has its own exponential
+// (the form the reference uses for its diagonal sub-blocks, intra_diag_kernel, gdn2/forward.py:220-235 of the
+// reference project). Below it the decay is split at the tile's first row, exp2(G_r - G_ref) * exp2(G_ref - G_s):
+// both exponents are <= 0 whatever the inputs, so nothing can overflow and a factor flushes to zero only where the
+// product is below 2^-126; 7 exponentials per channel stand for the tile's 16. The inverse (I + Tm)^-1 is built by
+// 16 x 16 blocks (solve_kernel, gdn2/forward.py:424-434, substitutes column by column), then W = Ai E, U = Ai (w*v),
+// KG and Qg follow wy_kernel (gdn2/forward.py:512-533) and the query scaling of prefill_scan_kernel
+// (gdn2/inference.py:461).
+//
+// What bounds it: a call of this family has few chunk-heads (hundreds), so a block's own chain of phases sets the
+// time. Hence eight lanes per tile and register tiles of 4 x 4 in every product; one pair per warp and a
+// substitution over all 64 rows by one thread per column set the
+// pace before. Measured with the scan (scan_simt.cu), B = 2, S = 1000, 8 heads of 64, float32: the call took 501 us,
+// now 80.
 //
 // This family also serves as the exact path for chunks the tensor-core family flags as decaying
 // too fast for its factorised diagonal blocks (`only_flagged`).
@@ -19,9 +26,45 @@ namespace gdn2 {
 
 namespace {
 
+constexpr int LT = kChunk + 4;        // floats per row of the transposed 64 x 64 matrices
+__host__ __device__ inline int row_stride(int DK) { return DK + 4; }   // floats per token row: 16-byte aligned, rows 4 banks apart
+
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));   // what exp2f is made of; here it need not be inlined with range checks
+  return y;
+}
+__device__ __forceinline__ float4 load4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
+  const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
+  return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
+                     __uint_as_float(u.y & 0xffff0000u));
+}
+__device__ __forceinline__ float4 load4(const __half* p) {
+  const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
+  const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+template <typename T> struct alignas(4 * sizeof(T)) Pack4 { T x[4]; };
+template <typename T> __device__ __forceinline__ void store4(T* p, T a, T b, T c, T d) {
+  *reinterpret_cast<Pack4<T>*>(p) = Pack4<T>{{a, b, c, d}};
+}
+__device__ __forceinline__ float4 mul4(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
+
+// acc[i][j] += a_i * b_j
+__device__ __forceinline__ void outer4(float (&acc)[4][4], float4 a, float4 b) {
+  const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+  }
+}
 
 // The whole chunk-local stage for chunk n of (batch, KEY head) bk, by one 256-thread block: everything that depends
-// on q, k, b, g once, then U = Ai (w*v) for each of the H / HK value heads that share the key head.
+// on q, k, b, g once, then U = Ai (w*v) for each of the H / HK value heads that share the key head. `S` tokens per
+// batch entry, NC = ceil(S / 64): the rows past the end count as tokens with k = q = v = 0 and no decay, which leave
+// the state alone.
 template <typename TIn, typename TW>
 __device__ __forceinline__ void prep_simt_chunk(const TIn* __restrict__ q, const TIn* __restrict__ k,
                                                 const TIn* __restrict__ v, const float* __restrict__ g,
@@ -32,100 +75,238 @@ __device__ __forceinline__ void prep_simt_chunk(const TIn* __restrict__ q, const
   using WT = WsTraits<TW>;
   using TV = typename WT::TV;
   constexpr int E = WT::E;
-  const int DK = L.DK, DV = L.DV;
-  const int NC = S / BS;
+  const int DK = L.DK, DV = L.DV, LD = row_stride(L.DK);
+  const int NC = (S + BS - 1) / BS;
   const int ib = bk / HK, ihk = bk % HK;
   const int64_t ch = (int64_t)bk * NC + n;
   const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
+  const int rows = min(BS, S - n * BS);
 
-  extern __shared__ float sm[];
-  float* Gs = sm;                    // [BS][DK] cumulative log2 decay
-  float* ks = Gs + BS * DK;          // [BS][DK] k
-  float* es = ks + BS * DK;          // [BS][DK] b*k, later E = b*k*gamma
-  float* qs = es + BS * DK;          // [BS][DK] q, later the w*v tiles
-  float* Tm = qs + BS * DK;          // [BS][BS] strictly lower
-  float* Aq = Tm + BS * BS;          // [BS][BS] lower incl. diagonal (scaled)
-  float* Ai = Aq + BS * BS;          // [BS][BS] (I + Tm)^-1
+  extern __shared__ __align__(16) float sm[];
+  float* Gs = sm;                    // [BS][LD] cumulative log2 decay
+  float* ks = Gs + BS * LD;          // [BS][LD] k
+  float* es = ks + BS * LD;          // [BS][LD] b*k, later E = b*k*gamma
+  float* qs = es + BS * LD;          // [BS][LD] q, later the w*v tiles
+  float* TT = qs + BS * LD;          // [BS][LT] Tm transposed (row s, column r; strictly s < r), later N
+  float* AT = TT + BS * LT;          // [BS][LT] (I + Tm)^-1 transposed; before that, partial sums of the decay
 
-  const size_t tok0 = ((size_t)ib * in_bs + (size_t)n * BS) * HK + ihk;   // token index of row 0 (stride HK per row)
-  for (int idx = tid; idx < BS * DK; idx += 256) {
-    const int t = idx / DK, c = idx % DK;
-    const size_t gi = (tok0 + (size_t)t * HK) * DK + c;
-    const float kk = to_f32(k[gi]);
-    ks[idx] = kk;
-    qs[idx] = to_f32(q[gi]);
-    es[idx] = to_f32(b[gi]) * kk;
-    Gs[idx] = g[gi];
-  }
-  for (int idx = tid; idx < BS * BS; idx += 256) { Tm[idx] = 0.f; Aq[idx] = 0.f; Ai[idx] = 0.f; }
-  __syncthreads();
-  if (tid < DK) {
-    float run = 0.f;
-    for (int t = 0; t < BS; ++t) { run += Gs[t * DK + tid]; Gs[t * DK + tid] = run * kLog2e; }
-  }
-  __syncthreads();
-
-  // pairwise matrices: warp `wid` takes rows {wid+8j, 63-(wid+8j)}, 65 pairs per row pair
-  for (int j = 0; j < 4; ++j) {
-    for (int half = 0; half < 2; ++half) {
-      const int r = half ? (BS - 1 - (wid + 8 * j)) : (wid + 8 * j);
-      for (int s = 0; s <= r; ++s) {
-        float aq = 0.f, ae = 0.f;
-        for (int c = lane; c < DK; c += 32) {
-          const float kd = ks[s * DK + c] * exp2f(Gs[r * DK + c] - Gs[s * DK + c]);
-          aq = fmaf(qs[r * DK + c], kd, aq);
-          ae = fmaf(es[r * DK + c], kd, ae);
-        }
-#pragma unroll
-        for (int off = 16; off; off >>= 1) {
-          aq += __shfl_xor_sync(0xffffffffu, aq, off);
-          ae += __shfl_xor_sync(0xffffffffu, ae, off);
-        }
-        if (lane == 0) {
-          Aq[r * BS + s] = aq * scale;
-          if (s < r) Tm[r * BS + s] = ae;
-        }
-      }
-    }
-  }
-  __syncthreads();
-
-  // inverse by columns: thread j solves (I + Tm) x = e_j
-  if (tid < BS) {
-    const int j = tid;
-    Ai[j * BS + j] = 1.f;
-    for (int r = j + 1; r < BS; ++r) {
-      float acc = 0.f;
-      for (int s = j; s < r; ++s) acc = fmaf(Tm[r * BS + s], Ai[s * BS + j], acc);
-      Ai[r * BS + j] = -acc;
-    }
-  }
-  // outputs that need only G, q, k: Aqk image, Qg rows, KG^T image, gamma_last; E in place
   TW* wq = reinterpret_cast<TW*>(P.wq + (size_t)ch * L.wq_bytes);
   TV* aqk = reinterpret_cast<TV*>(P.aqk + (size_t)ch * L.aqk_bytes);
   TV* kgt = reinterpret_cast<TV*>(P.kgt + (size_t)ch * L.kgt_bytes);
-  float* gl = P.gl + (size_t)ch * DK;
-  for (int idx = tid; idx < BS * BS; idx += 256) {
-    const int r = idx / BS, s = idx % BS;
-    aqk[kc_index<E>(r, s, BS)] = WT::kg_store(Aq[idx]);
+
+  const size_t tok0 = ((size_t)ib * in_bs + (size_t)n * BS) * HK + ihk;   // token index of row 0 (stride HK per row)
+  const int nq = DK / 4;                                                  // channel quads
+#pragma unroll 4
+  for (int idx = tid; idx < BS * nq; idx += 256) {
+    const int t = idx / nq, c = 4 * (idx % nq);
+    const size_t gi = (tok0 + (size_t)t * HK) * DK + c;
+    float4 kk = make_float4(0.f, 0.f, 0.f, 0.f), qq = kk, bb = kk, gg = kk;
+    if (t < rows) { kk = load4(k + gi); qq = load4(q + gi); bb = load4(b + gi); gg = load4(g + gi); }
+    *reinterpret_cast<float4*>(&ks[t * LD + c]) = kk;
+    *reinterpret_cast<float4*>(&qs[t * LD + c]) = qq;
+    *reinterpret_cast<float4*>(&es[t * LD + c]) = mul4(bb, kk);
+    *reinterpret_cast<float4*>(&Gs[t * LD + c]) = gg;
   }
-  for (int idx = tid; idx < BS * DK; idx += 256) {
-    const int t = idx / DK, c = idx % DK;
-    const float G = Gs[idx];
-    const float gam = exp2f(G);
-    wq[kc_index<E>(BS + t, c, 2 * BS)] = from_f32<TW>(scale * qs[idx] * gam);
-    kgt[kc_index<E>(c, t, DK)] = WT::kg_store(ks[idx] * exp2f(Gs[(BS - 1) * DK + c] - G));
-    es[idx] *= gam;
+  __syncthreads();
+  // cumulative decay: four runs of 16 tokens per channel, then the totals of the runs before
+  for (int it = tid; it < 4 * DK; it += 256) {
+    const int c = it % DK, sg = it / DK;
+    float run = 0.f;
+#pragma unroll
+    for (int t = 0; t < 16; ++t) { run += Gs[(16 * sg + t) * LD + c]; Gs[(16 * sg + t) * LD + c] = run; }
+    AT[sg * DK + c] = run;
   }
-  if (tid < DK) gl[tid] = exp2f(Gs[(BS - 1) * DK + tid]);
+  __syncthreads();
+  for (int it = tid; it < 4 * DK; it += 256) {
+    const int c = it % DK, sg = it / DK;
+    float base = 0.f;
+    for (int x = 0; x < sg; ++x) base += AT[x * DK + c];
+#pragma unroll
+    for (int t = 0; t < 16; ++t) Gs[(16 * sg + t) * LD + c] = (Gs[(16 * sg + t) * LD + c] + base) * kLog2e;
+  }
+  // the part of the Aqk image above the diagonal tiles
+  for (int idx = tid; idx < BS * (BS / 4); idx += 256) {
+    const int r = idx % BS, sq = idx / BS;
+    if (sq > r / 4) store4(aqk + kc_index<E>(r, 4 * sq, BS), WT::kg_store(0.f), WT::kg_store(0.f), WT::kg_store(0.f), WT::kg_store(0.f));
+  }
   __syncthreads();
 
-  // W = Ai E
-  for (int idx = tid; idx < BS * DK; idx += 256) {
-    const int r = idx / DK, c = idx % DK;
-    float acc = 0.f;
-    for (int s = 0; s <= r; ++s) acc = fmaf(Ai[r * BS + s], es[s * DK + c], acc);
-    wq[kc_index<E>(r, c, 2 * BS)] = from_f32<TW>(acc);
+  // The two matrices: 120 tiles below the diagonal, then the 16 on it; eight lanes per tile share its channels.
+  const int l8 = lane & 7;
+  for (int grp = wid; grp < 34; grp += 8) {
+    const int p = 4 * grp + (lane >> 3);
+    float val[32];                                        // [0, 16): q side, [16, 32): erase side; 4 * (r - r0) + (s - s0)
+#pragma unroll
+    for (int x = 0; x < 32; ++x) val[x] = 0.f;
+    int rt, st;
+    if (grp < 30) {
+      rt = (int)((1.f + sqrtf(8.f * p + 1.f)) * 0.5f);    // largest rt with rt (rt - 1) / 2 <= p
+      if (rt * (rt - 1) / 2 > p) --rt;
+      if ((rt + 1) * rt / 2 <= p) ++rt;
+      st = p - rt * (rt - 1) / 2;
+      for (int u = l8; u < DK / 2; u += 8) {
+        const int o_r = 4 * rt * LD + 2 * u, o_s = 4 * st * LD + 2 * u;
+        const float2 gref = *reinterpret_cast<const float2*>(&Gs[o_r]);
+        float2 kf[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 gj = *reinterpret_cast<const float2*>(&Gs[o_s + j * LD]), kj = *reinterpret_cast<const float2*>(&ks[o_s + j * LD]);
+          kf[j] = make_float2(kj.x * ex2(gref.x - gj.x), kj.y * ex2(gref.y - gj.y));
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float2 qi = *reinterpret_cast<const float2*>(&qs[o_r + i * LD]), ei = *reinterpret_cast<const float2*>(&es[o_r + i * LD]);
+          if (i > 0) {
+            const float2 gi = *reinterpret_cast<const float2*>(&Gs[o_r + i * LD]);
+            const float ax = ex2(gi.x - gref.x), ay = ex2(gi.y - gref.y);
+            qi.x *= ax; qi.y *= ay; ei.x *= ax; ei.y *= ay;
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            val[4 * i + j] = fmaf(qi.x, kf[j].x, fmaf(qi.y, kf[j].y, val[4 * i + j]));
+            val[16 + 4 * i + j] = fmaf(ei.x, kf[j].x, fmaf(ei.y, kf[j].y, val[16 + 4 * i + j]));
+          }
+        }
+      }
+    } else {
+      rt = st = p - 120;
+      for (int u = l8; u < DK / 2; u += 8) {
+        const int o_r = 4 * rt * LD + 2 * u;
+        float2 gg[4], kk[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          gg[i] = *reinterpret_cast<const float2*>(&Gs[o_r + i * LD]); kk[i] = *reinterpret_cast<const float2*>(&ks[o_r + i * LD]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 qi = *reinterpret_cast<const float2*>(&qs[o_r + i * LD]), ei = *reinterpret_cast<const float2*>(&es[o_r + i * LD]);
+#pragma unroll
+          for (int j = 0; j <= i; ++j) {
+            float2 kd = kk[j];
+            if (j < i) { kd.x *= ex2(gg[i].x - gg[j].x); kd.y *= ex2(gg[i].y - gg[j].y); }
+            val[4 * i + j] = fmaf(qi.x, kd.x, fmaf(qi.y, kd.y, val[4 * i + j]));
+            if (j < i) val[16 + 4 * i + j] = fmaf(ei.x, kd.x, fmaf(ei.y, kd.y, val[16 + 4 * i + j]));
+          }
+        }
+      }
+    }
+    // sum over the eight lanes; each step halves what a lane keeps: bit 2 chooses the matrix, bits 1 and 0 the row
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      const int half = 16 >> m, bit = 4 >> m;
+      const bool up = (lane & bit) != 0;
+#pragma unroll
+      for (int x = 0; x < half; ++x) {
+        const float send = up ? val[x] : val[x + half], keep = up ? val[x + half] : val[x];
+        val[x] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+      }
+    }
+    const int r = 4 * rt + (lane & 3), s0 = 4 * st;
+    if (lane & 4) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) TT[(s0 + j) * LT + r] = val[j];
+    } else {
+      store4(aqk + kc_index<E>(r, s0, BS), WT::kg_store(val[0] * scale), WT::kg_store(val[1] * scale),
+             WT::kg_store(val[2] * scale), WT::kg_store(val[3] * scale));
+    }
+  }
+  __syncthreads();
+
+  // (I + Tm)^-1 by 16 x 16 blocks, everything transposed (a row of AT is a column of the inverse):
+  //   X_ii = D_i = (I + T_ii)^-1;   N_ik = D_i T_ik;   X_ij = - sum_{k=j}^{i-1} N_ik X_kj
+  if (tid < BS) {
+    const int i = tid >> 4, j = tid & 15;
+    const float* tb = TT + 16 * i * LT + 16 * i;          // T_ii[r][s] = tb[s * LT + r]
+    float x[16];
+#pragma unroll
+    for (int r = 0; r < 16; ++r) x[r] = r == j ? 1.f : 0.f;
+#pragma unroll
+    for (int s_ = 0; s_ < 15; ++s_) {
+#pragma unroll
+      for (int r4 = (s_ + 1) / 4; r4 < 4; ++r4) {
+        const float4 t4 = *reinterpret_cast<const float4*>(&tb[s_ * LT + 4 * r4]);
+        const float tv[4] = {t4.x, t4.y, t4.z, t4.w};
+#pragma unroll
+        for (int y = 0; y < 4; ++y)
+          if (4 * r4 + y > s_) x[4 * r4 + y] = fmaf(-tv[y], x[s_], x[4 * r4 + y]);
+      }
+    }
+#pragma unroll
+    for (int r4 = 0; r4 < 4; ++r4)
+      *reinterpret_cast<float4*>(&AT[tid * LT + 16 * i + 4 * r4]) = make_float4(x[4 * r4], x[4 * r4 + 1], x[4 * r4 + 2], x[4 * r4 + 3]);
+  } else {
+    // meanwhile the other six warps: gamma_last, the query rows Qg and KG^T, which need G, q, k only
+    const int z = tid - BS, nz = 256 - BS;
+    const float* glast = Gs + (BS - 1) * LD;
+    for (int idx = z; idx < BS * nq; idx += nz) {          // tokens fastest: 16-byte pieces in a row
+      const int t = idx % BS, c = 4 * (idx / BS);
+      const float4 G = *reinterpret_cast<const float4*>(&Gs[t * LD + c]), qq = *reinterpret_cast<const float4*>(&qs[t * LD + c]);
+      store4(wq + kc_index<E>(BS + t, c, 2 * BS), from_f32<TW>(scale * qq.x * ex2(G.x)), from_f32<TW>(scale * qq.y * ex2(G.y)),
+             from_f32<TW>(scale * qq.z * ex2(G.z)), from_f32<TW>(scale * qq.w * ex2(G.w)));
+    }
+    for (int idx = z; idx < (BS / 4) * DK; idx += nz) {
+      const int c = idx % DK, t = 4 * (idx / DK);
+      float kg[4];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) kg[x] = ks[(t + x) * LD + c] * ex2(glast[c] - Gs[(t + x) * LD + c]);
+      store4(kgt + kc_index<E>(c, t, DK), WT::kg_store(kg[0]), WT::kg_store(kg[1]), WT::kg_store(kg[2]), WT::kg_store(kg[3]));
+    }
+    float* gl = P.gl + (size_t)ch * DK;
+    for (int c = z; c < DK; c += nz) gl[c] = ex2(glast[c]);
+  }
+  __syncthreads();
+  for (int pass = 0; pass < 2; ++pass) {                   // N^T in place over T^T: 6 blocks x 16 rows t x 4 row quads
+    const int it = tid + 256 * pass;
+    if (it < 384) {                                        // whole warps
+      const int blk = it >> 6, t = (it >> 2) & 15, r4 = 4 * (it & 3);
+      const int bi = blk < 1 ? 1 : blk < 3 ? 2 : 3, bkk = blk < 1 ? 0 : blk < 3 ? blk - 1 : blk - 3;
+      float* trow = TT + (16 * bkk + t) * LT + 16 * bi;
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        const float4 d = *reinterpret_cast<const float4*>(&AT[(16 * bi + u) * LT + 16 * bi + r4]);
+        const float tv = trow[u];
+        a.x = fmaf(d.x, tv, a.x); a.y = fmaf(d.y, tv, a.y); a.z = fmaf(d.z, tv, a.z); a.w = fmaf(d.w, tv, a.w);
+      }
+      __syncwarp();                                        // the four lanes of a row have read it
+      *reinterpret_cast<float4*>(&trow[r4]) = a;
+    }
+  }
+  // E = b k gamma in place (needed from here on)
+  for (int idx = tid; idx < BS * nq; idx += 256) {
+    const int t = idx / nq, c = 4 * (idx % nq);
+    const float4 G = *reinterpret_cast<const float4*>(&Gs[t * LD + c]);
+    float4* ep = reinterpret_cast<float4*>(&es[t * LD + c]);
+    *ep = mul4(*ep, make_float4(ex2(G.x), ex2(G.y), ex2(G.z), ex2(G.w)));
+  }
+  __syncthreads();
+  for (int d = 1; d < 4; ++d) {
+    if (tid < 64 * (4 - d)) {
+      const int bj = tid >> 6, c = (tid >> 2) & 15, r4 = 4 * (tid & 3), bi = bj + d;
+      float* xcol = AT + (16 * bj + c) * LT;
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 16
+      for (int t = 16 * bj; t < 16 * bi; ++t) {
+        const float4 nn = *reinterpret_cast<const float4*>(&TT[t * LT + 16 * bi + r4]);
+        const float xv = xcol[t];
+        a.x = fmaf(-nn.x, xv, a.x); a.y = fmaf(-nn.y, xv, a.y); a.z = fmaf(-nn.z, xv, a.z); a.w = fmaf(-nn.w, xv, a.w);
+      }
+      *reinterpret_cast<float4*>(&xcol[16 * bi + r4]) = a;
+    }
+    __syncthreads();
+  }
+
+  // W = Ai E: one thread per 4 tokens x 4 channels; row quad rq needs the source tokens up to its own only
+  for (int idx = tid; idx < 16 * nq; idx += 256) {
+    const int rq = idx / nq, c = 4 * (idx % nq);
+    float acc[4][4] = {};
+#pragma unroll 4
+    for (int s_ = 0; s_ < 4 * rq + 4; ++s_)
+      outer4(acc, *reinterpret_cast<const float4*>(&AT[s_ * LT + 4 * rq]), *reinterpret_cast<const float4*>(&es[s_ * LD + c]));
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      store4(wq + kc_index<E>(4 * rq + i, c, 2 * BS), from_f32<TW>(acc[i][0]), from_f32<TW>(acc[i][1]), from_f32<TW>(acc[i][2]),
+             from_f32<TW>(acc[i][3]));
   }
   // U = Ai (w*v) for every value head of this key head, value columns in tiles of DK
   const int rep = H / HK;
@@ -134,26 +315,32 @@ __device__ __forceinline__ void prep_simt_chunk(const TIn* __restrict__ q, const
     const size_t tok0v = ((size_t)ib * in_bs + (size_t)n * BS) * H + ih;
     TV* ut = reinterpret_cast<TV*>(P.ut + (size_t)(((int64_t)ib * H + ih) * NC + n) * L.ut_bytes);
     for (int c0 = 0; c0 < DV; c0 += DK) {
-      const int cw = min(DK, DV - c0);
-      __syncthreads();
-      for (int idx = tid; idx < BS * cw; idx += 256) {
-        const int t = idx / cw, c = idx % cw;
+      const int cwq = min(DK, DV - c0) / 4;
+      if (hr + c0 > 0) __syncthreads();                    // the previous tile has been read (the query rows long since)
+#pragma unroll 4
+      for (int idx = tid; idx < BS * cwq; idx += 256) {
+        const int t = idx / cwq, c = 4 * (idx % cwq);
         const size_t gi = (tok0v + (size_t)t * H) * DV + c0 + c;
-        qs[t * DK + c] = to_f32(w[gi]) * to_f32(v[gi]);
+        *reinterpret_cast<float4*>(&qs[t * LD + c]) = t < rows ? mul4(load4(w + gi), load4(v + gi)) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
       __syncthreads();
-      for (int idx = tid; idx < BS * cw; idx += 256) {
-        const int r = idx / cw, c = idx % cw;
-        float acc = 0.f;
-        for (int s = 0; s <= r; ++s) acc = fmaf(Ai[r * BS + s], qs[s * DK + c], acc);
-        ut[kc_index<E>(c0 + c, r, DV)] = WT::u_store(acc);
+      for (int idx = tid; idx < 16 * cwq; idx += 256) {
+        const int rq = idx / cwq, c = 4 * (idx % cwq);
+        float acc[4][4] = {};
+#pragma unroll 4
+        for (int s_ = 0; s_ < 4 * rq + 4; ++s_)
+          outer4(acc, *reinterpret_cast<const float4*>(&AT[s_ * LT + 4 * rq]), *reinterpret_cast<const float4*>(&qs[s_ * LD + c]));
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          store4(ut + kc_index<E>(c0 + c + j, 4 * rq, DV), WT::u_store(acc[0][j]), WT::u_store(acc[1][j]), WT::u_store(acc[2][j]),
+                 WT::u_store(acc[3][j]));
       }
     }
   }
 }
 
 template <typename TIn, typename TW>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 prep_simt_kernel(const TIn* __restrict__ q, const TIn* __restrict__ k, const TIn* __restrict__ v,
                  const float* __restrict__ g, const TIn* __restrict__ b, const TIn* __restrict__ w,
                  WsLayout L, WsPtrs P, int S, int H, int HK, int64_t in_bs, float scale) {
@@ -163,7 +350,7 @@ prep_simt_kernel(const TIn* __restrict__ q, const TIn* __restrict__ k, const TIn
 // Exact redo of the chunks the tensor-core kernel flagged: a fixed small grid walks the compacted list
 // (workspace ints: flags[nch], list[nch], count), so a call with nothing flagged costs two tiny launches.
 template <typename TIn, typename TW>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 1)
 prep_simt_flagged_kernel(const TIn* __restrict__ q, const TIn* __restrict__ k, const TIn* __restrict__ v,
                          const float* __restrict__ g, const TIn* __restrict__ b, const TIn* __restrict__ w,
                          WsLayout L, WsPtrs P, int S, int H, int HK, int64_t in_bs, float scale) {
@@ -181,7 +368,7 @@ template <typename TIn, typename TW>
 int launch_typed(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
                  const WsLayout& L, const WsPtrs& P, int B, int S, int H, int HK, int64_t in_bs, float scale,
                  bool only_flagged, cudaStream_t st) {
-  const size_t smem = ((size_t)4 * kChunk * L.DK + 3 * kChunk * kChunk) * sizeof(float);
+  const size_t smem = ((size_t)4 * kChunk * row_stride(L.DK) + 2 * kChunk * LT) * sizeof(float);
   const TIn* tq = static_cast<const TIn*>(q); const TIn* tk = static_cast<const TIn*>(k);
   const TIn* tv = static_cast<const TIn*>(v); const TIn* tb = static_cast<const TIn*>(b);
   const TIn* tw = static_cast<const TIn*>(w);
@@ -194,7 +381,7 @@ int launch_typed(const void* q, const void* k, const void* v, const float* g, co
   } else {
     auto kern = prep_simt_kernel<TIn, TW>;
     GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
-    dim3 grid(S / kChunk, B * HK);
+    dim3 grid((S + kChunk - 1) / kChunk, B * HK);
     kern<<<grid, 256, smem, st>>>(tq, tk, tv, g, tb, tw, L, P, S, H, HK, in_bs, scale);
   }
   GDN2_CUDA_TRY(cudaGetLastError());

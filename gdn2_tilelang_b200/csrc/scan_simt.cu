@@ -1,22 +1,27 @@
 // Sequential state scan fused with the output, SIMT (CUDA-core) family, and the chunk-parallel
 // output from stored chunk states. fp32 arithmetic; any DK <= 128, any DV.
 //
-// Scan: one 256-thread block per (32-column value tile, batch*head), sequential over chunks, the
-// [DK x 32] state tile resident in shared memory. Per chunk (prefill_scan_kernel,
-// gdn2/inference.py:446-475 of the reference project):
+// Scan: one 256-thread block per (value tile, batch*head), sequential over chunks. Per chunk
+// (prefill_scan_kernel, gdn2/inference.py:446-475 of the reference project):
 //     Un = U - W S ;  o = Qg S + tril(Aqk) Un ;  S <- diag(gamma_C) S + KG^T Un
 // Optionally the state entering each chunk is stored (state_kernel, gdn2/forward.py:617-620).
+// What bounds it: the chunk-to-chunk chain, since a call of this family has few (batch, head) pairs. The value
+// columns never meet, so a head is spread over tiles of 8 of them while SMs are free (16 and 32 beyond that: the
+// records are read once per tile). The records arrive by bulk copies in the layout they are stored in, each one
+// refilled for the next chunk as soon as its last reader is through, and the two halves of the block form the output
+// rows and the new state at the same time: two barriers per chunk. Measured
+// with the chunk-local stage (prep_simt.cu), B = 2, S = 1000, 8 heads of 64, float32: the call took 501 us, now 80.
 //
 // Output: one block per (value tile, chunk, batch*head) doing the first two lines from a stored
 // chunk state (output_kernel, gdn2/forward.py:710-725).
 #include "common.cuh"
+#include "tc_utils.cuh"
 
 namespace gdn2 {
 
 namespace {
 
-constexpr int NV = 32;   // value columns per block
-
+constexpr int NV = 32;   // value columns per block of the output kernel
 
 struct ScanSmem {
   float *Ws, *Qs, *As, *Ks, *Us, *Un, *St, *gl;
@@ -96,53 +101,193 @@ __device__ __forceinline__ void un_and_output(ScanSmem& s, int DK, int DV, int l
   }
 }
 
-template <typename TOut, typename TW>
-__global__ void __launch_bounds__(256)
-scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __restrict__ o,
-                 float* __restrict__ sT, float* __restrict__ hs, int S, int H, int64_t o_bs) {
-  const int DK = L.DK, DV = L.DV, NC = S / kChunk;
-  const int bh = blockIdx.y, ib = bh / H, ih = bh % H;
-  const int lo = blockIdx.x * NV;
-  const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-  extern __shared__ float sm[];
-  ScanSmem s(sm, DK);
-  const bool col_ok = lo + lane < DV;
+// packed fp32 pairs: two FMAs per instruction
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(*reinterpret_cast<unsigned long long*>(&d))
+      : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
+        "l"(*reinterpret_cast<unsigned long long*>(&c)));
+  return d;
+}
 
-  for (int idx = tid; idx < DK * NV; idx += 256) {
-    const int c = idx / NV, d = lo + idx % NV;
-    s.St[idx] = (s0 != nullptr && d < DV) ? s0[((size_t)bh * DK + c) * DV + d] : 0.f;
+enum : uint32_t { kWaitSimtWq = 0x200000u, kWaitSimtUt = 0x400000u, kWaitSimtAqk = 0x800000u, kWaitSimtKgt = 0x1000000u };
+
+// Shared memory of the scan: the chunk's records as stored (fp32 images), the state tile and Un, value columns inside.
+template <int NVT> struct ScanTile {
+  float *wq, *aqk, *kgt, *ut, *gl, *St, *Un;
+  __device__ ScanTile(float* base, int DK) {
+    wq = base;                          // [DK/4][128 rows][4]
+    kgt = wq + 2 * kChunk * DK;         // [64/4][DK][4]
+    aqk = kgt + kChunk * DK;            // [64/4][64 r][4]
+    ut = aqk + kChunk * kChunk;         // [64/4][NVT][4]
+    gl = ut + kChunk * NVT;             // [DK]
+    St = gl + DK;                       // [DK][NVT]
+    Un = St + DK * NVT;                 // [64][NVT]
   }
+  static size_t bytes(int DK) {
+    return ((size_t)3 * kChunk * DK + kChunk * kChunk + 2 * kChunk * NVT + DK + (size_t)DK * NVT) * sizeof(float);
+  }
+};
+
+// S tokens per batch entry, NC = ceil(S / 64): the rows past the end are not written (the chunk-local stage has made
+// them neutral). Threads: tid & 127 = row of the W | Qg image, tid >> 7 = half of the tile's columns. The W rows' threads
+// go on to the state update (row & 63 = key channel, two of them when DK > 64), the Qg rows' threads to the output.
+template <typename TOut, int NVT>
+__global__ void __launch_bounds__(256, 1)
+scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __restrict__ o,
+                 float* __restrict__ sT, float* __restrict__ hs, int S, int H, int64_t o_bs, uint32_t* status) {
+  constexpr int CT = NVT / 2;                             // columns per thread
+  const int DK = L.DK, DV = L.DV, NC = (S + kChunk - 1) / kChunk;
+  const int bh = blockIdx.x, ib = bh / H, ih = bh % H;
+  const int lo = blockIdx.y * NVT, nv = min(NVT, DV - lo);
+  const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
+  const int row = tid & 127, col0 = (tid >> 7) * CT;
+  const bool is_q = row >= kChunk;
+  extern __shared__ __align__(128) float sm[];
+  ScanTile<NVT> s(sm, DK);
+  __shared__ uint64_t bar_wq, bar_ut, bar_aqk, bar_kgt;
+  __shared__ int abort_flag;
+
   const int64_t bk = (int64_t)ib * (H / L.rep) + ih / L.rep;       // (batch, key head) whose records this value head reads
+  const char* g_wq = P.wq + (size_t)(bk * NC) * L.wq_bytes;
+  const char* g_aqk = P.aqk + (size_t)(bk * NC) * L.aqk_bytes;
+  const char* g_kgt = P.kgt + (size_t)(bk * NC) * L.kgt_bytes;
+  const char* g_ut = P.ut + (size_t)((int64_t)bh * NC) * L.ut_bytes + (size_t)lo * 16;
+  const float* g_gl = P.gl + (size_t)(bk * NC) * DK;
+
+  // copies of chunk n, issued by the first warp (the 16 column pieces of U by its first 16 lanes)
+  auto load_wq_ut = [&](int n) {
+    if (lane == 0) {
+      tc::mbar_expect_tx(&bar_wq, (uint32_t)L.wq_bytes);
+      tc::bulk_g2s(s.wq, g_wq + (size_t)n * L.wq_bytes, (uint32_t)L.wq_bytes, &bar_wq);
+      tc::mbar_expect_tx(&bar_ut, (uint32_t)(16 * nv * 16));
+    }
+    __syncwarp();
+    if (lane < 16)
+      tc::bulk_g2s(s.ut + lane * NVT * 4, g_ut + (size_t)n * L.ut_bytes + (size_t)lane * DV * 16, (uint32_t)(nv * 16), &bar_ut);
+  };
+  auto load_aqk_kgt = [&](int n) {
+    if (lane == 0) {
+      tc::mbar_expect_tx(&bar_kgt, (uint32_t)L.kgt_bytes + (uint32_t)L.gl_bytes);
+      tc::bulk_g2s(s.kgt, g_kgt + (size_t)n * L.kgt_bytes, (uint32_t)L.kgt_bytes, &bar_kgt);
+      tc::bulk_g2s(s.gl, g_gl + (size_t)n * DK, (uint32_t)L.gl_bytes, &bar_kgt);
+      tc::mbar_expect_tx(&bar_aqk, (uint32_t)L.aqk_bytes);
+      tc::bulk_g2s(s.aqk, g_aqk + (size_t)n * L.aqk_bytes, (uint32_t)L.aqk_bytes, &bar_aqk);
+    }
+  };
+
+  if (tid == 0) {
+    tc::mbar_init(&bar_wq, 1); tc::mbar_init(&bar_ut, 1); tc::mbar_init(&bar_aqk, 1); tc::mbar_init(&bar_kgt, 1);
+    abort_flag = 0;
+    tc::mbar_init_fence();
+  }
+  for (int idx = tid; idx < DK * NVT; idx += 256) {
+    const int c = idx / NVT, d = idx % NVT;
+    s.St[idx] = (s0 != nullptr && d < nv) ? s0[((size_t)bh * DK + c) * DV + lo + d] : 0.f;
+  }
+  if (nv < NVT)                                            // columns past DV: no copy brings them
+    for (int idx = tid; idx < kChunk * NVT; idx += 256) s.ut[idx] = 0.f;
+  tc::fence_async_smem();
+  __syncthreads();
+  if (wid == 0) { load_wq_ut(0); load_aqk_kgt(0); }
+
+  float2 acc[CT / 2];
   for (int n = 0; n < NC; ++n) {
-    const int64_t ch = bk * NC + n;
-    __syncthreads();
-    load_chunk_operands<TW>(L, P, ch, (int64_t)bh * NC + n, lo, s, true);
+    const uint32_t ph = n & 1;
     if (hs != nullptr) {
-      float* hp = hs + (((size_t)ib * NC + n) * H + ih) * DK * DV;
-      for (int idx = tid; idx < DK * NV; idx += 256) {
-        const int c = idx / NV, d = lo + idx % NV;
-        if (d < DV) hp[(size_t)c * DV + d] = s.St[idx];
+      float* hp = hs + (((size_t)ib * NC + n) * H + ih) * DK * DV + lo;
+      for (int idx = tid; idx < DK * NVT; idx += 256) {
+        const int c = idx / NVT, d = idx % NVT;
+        if (d < nv) hp[(size_t)c * DV + d] = s.St[idx];
       }
     }
-    __syncthreads();
-    TOut* o_rows = o + (((size_t)ib * o_bs + (size_t)n * kChunk) * H + ih) * DV;
-    un_and_output<TOut>(s, DK, DV, lo, o_rows, (size_t)H * DV);
-    __syncthreads();
-    // state update: warp `wid` owns key rows wid, wid+8, ...
-    for (int c = wid; c < DK; c += 8) {
-      float acc = s.gl[c] * s.St[c * NV + lane];
-      for (int t = 0; t < kChunk; ++t) acc = fmaf(s.Ks[t * DK + c], s.Un[t * NV + lane], acc);
-      s.St[c * NV + lane] = acc;
+    // ---- row of W S or Qg S
+#pragma unroll
+    for (int x = 0; x < CT / 2; ++x) acc[x] = make_float2(0.f, 0.f);
+    tc::mbar_wait(&bar_wq, ph, &abort_flag, status, kWaitSimtWq);
+    const float4* wrow = reinterpret_cast<const float4*>(s.wq) + row;
+#pragma unroll 4
+    for (int c4 = 0; c4 < DK / 4; ++c4) {
+      const float4 w4 = wrow[c4 * 2 * kChunk];
+      const float wv[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+      for (int y = 0; y < 4; ++y) {
+        const float2* st = reinterpret_cast<const float2*>(&s.St[(4 * c4 + y) * NVT + col0]);
+#pragma unroll
+        for (int x = 0; x < CT / 2; ++x) acc[x] = ffma2(make_float2(wv[y], wv[y]), st[x], acc[x]);
+      }
     }
+    tc::mbar_wait(&bar_ut, ph, &abort_flag, status, kWaitSimtUt);
+    if (!is_q) {
+      const float* u = s.ut + ((row >> 2) * NVT + col0) * 4 + (row & 3);
+      float2* un = reinterpret_cast<float2*>(&s.Un[row * NVT + col0]);
+#pragma unroll
+      for (int x = 0; x < CT / 2; ++x) un[x] = make_float2(u[8 * x] - acc[x].x, u[8 * x + 4] - acc[x].y);
+    }
+    __syncthreads();                                       // Un complete; the state and W | Qg have been read
+    if (wid == 0 && n + 1 < NC && !abort_flag) load_wq_ut(n + 1);
+
+    if (is_q) {
+      // ---- o = Qg S + tril(Aqk) Un: source tokens up to the warp's last row (Aqk is zero above the diagonal)
+      const int r = row - kChunk;
+      tc::mbar_wait(&bar_aqk, ph, &abort_flag, status, kWaitSimtAqk);
+      const float4* arow = reinterpret_cast<const float4*>(s.aqk) + r;
+      const int tq = ((r & ~31) + 32) / 4;
+#pragma unroll 4
+      for (int t4 = 0; t4 < tq; ++t4) {
+        const float4 a4 = arow[t4 * kChunk];
+        const float av[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+          const float2* un = reinterpret_cast<const float2*>(&s.Un[(4 * t4 + y) * NVT + col0]);
+#pragma unroll
+          for (int x = 0; x < CT / 2; ++x) acc[x] = ffma2(make_float2(av[y], av[y]), un[x], acc[x]);
+        }
+      }
+      const int t = n * kChunk + r;
+      if (t < S) {
+        TOut* op = o + (((size_t)ib * o_bs + t) * H + ih) * DV + lo + col0;
+#pragma unroll
+        for (int x = 0; x < CT / 2; ++x) {
+          if (col0 + 2 * x < nv) {                         // nv is a multiple of 4
+            op[2 * x] = from_f32<TOut>(acc[x].x); op[2 * x + 1] = from_f32<TOut>(acc[x].y);
+          }
+        }
+      }
+    } else {
+      // ---- S <- gamma_C S + KG^T Un, this thread's channel(s)
+      tc::mbar_wait(&bar_kgt, ph, &abort_flag, status, kWaitSimtKgt);
+      for (int c = row; c < DK; c += kChunk) {
+        float2* st = reinterpret_cast<float2*>(&s.St[c * NVT + col0]);
+        const float gm = s.gl[c];
+#pragma unroll
+        for (int x = 0; x < CT / 2; ++x) { acc[x] = st[x]; acc[x].x *= gm; acc[x].y *= gm; }
+        const float4* krow = reinterpret_cast<const float4*>(s.kgt) + c;
+#pragma unroll 4
+        for (int t4 = 0; t4 < kChunk / 4; ++t4) {
+          const float4 k4 = krow[t4 * DK];
+          const float kv[4] = {k4.x, k4.y, k4.z, k4.w};
+#pragma unroll
+          for (int y = 0; y < 4; ++y) {
+            const float2* un = reinterpret_cast<const float2*>(&s.Un[(4 * t4 + y) * NVT + col0]);
+#pragma unroll
+            for (int x = 0; x < CT / 2; ++x) acc[x] = ffma2(make_float2(kv[y], kv[y]), un[x], acc[x]);
+          }
+        }
+#pragma unroll
+        for (int x = 0; x < CT / 2; ++x) st[x] = acc[x];
+      }
+    }
+    __syncthreads();                                       // the new state is complete; Un, Aqk and KG have been read
+    if (wid == 0 && n + 1 < NC && !abort_flag) load_aqk_kgt(n + 1);
   }
-  __syncthreads();
   if (sT != nullptr) {
-    for (int idx = tid; idx < DK * NV; idx += 256) {
-      const int c = idx / NV, d = lo + idx % NV;
-      if (d < DV) sT[((size_t)bh * DK + c) * DV + d] = s.St[idx];
+    for (int idx = tid; idx < DK * NVT; idx += 256) {
+      const int c = idx / NVT, d = idx % NVT;
+      if (d < nv) sT[((size_t)bh * DK + c) * DV + lo + d] = s.St[idx];
     }
   }
-  (void)col_ok;
 }
 
 template <typename TOut, typename TW>
@@ -166,16 +311,22 @@ output_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ hs, TOut* __r
   un_and_output<TOut>(s, DK, DV, lo, o_rows, (size_t)H * DV);
 }
 
-template <typename TOut, typename TW>
+template <typename TOut>
 int launch_scan_typed(const WsLayout& L, const WsPtrs& P, const float* s0, void* o, float* sT, float* hs,
                       int B, int S, int H, int64_t o_bs, cudaStream_t st) {
-  const size_t smem = ScanSmem::bytes(L.DK);
-  auto kern = scan_simt_kernel<TOut, TW>;
-  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
-  dim3 grid((L.DV + NV - 1) / NV, B * H);
-  kern<<<grid, 256, smem, st>>>(L, P, s0, static_cast<TOut*>(o), sT, hs, S, H, o_bs);
-  GDN2_CUDA_TRY(cudaGetLastError());
-  return GDN2_OK;
+  const int BH = B * H, sms = device_sm_count();
+  auto launch = [&](auto kern, int nvt, size_t smem) -> int {
+    GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
+    kern<<<dim3(BH, (L.DV + nvt - 1) / nvt), 256, smem, st>>>(L, P, s0, static_cast<TOut*>(o), sT, hs, S, H, o_bs,
+                                                              device_status_word());
+    GDN2_CUDA_TRY(cudaGetLastError());
+    return GDN2_OK;
+  };
+  // the narrowest tile whose blocks all run at once (two per SM while the records of DK <= 64 leave room)
+  const int64_t room = L.DK <= 64 ? 2 * sms : sms;
+  if ((int64_t)BH * ((L.DV + 7) / 8) <= room) return launch(scan_simt_kernel<TOut, 8>, 8, ScanTile<8>::bytes(L.DK));
+  if ((int64_t)BH * ((L.DV + 15) / 16) <= room) return launch(scan_simt_kernel<TOut, 16>, 16, ScanTile<16>::bytes(L.DK));
+  return launch(scan_simt_kernel<TOut, 32>, 32, ScanTile<32>::bytes(L.DK));
 }
 
 template <typename TOut, typename TW>
@@ -196,9 +347,9 @@ int launch_scan_simt(const WsLayout& L, const WsPtrs& P, const float* s0, void* 
                      int B, int S, int H, int64_t o_bs, int dtype, cudaStream_t st) {
   if (L.esz != 4) return GDN2_ERR_UNSUPPORTED;   // 16-bit records belong to the tensor-core family's kernels
   switch (dtype) {
-    case GDN2_F32: return launch_scan_typed<float, float>(L, P, s0, o, sT, hs, B, S, H, o_bs, st);
-    case GDN2_BF16: return launch_scan_typed<__nv_bfloat16, float>(L, P, s0, o, sT, hs, B, S, H, o_bs, st);
-    case GDN2_F16: return launch_scan_typed<__half, float>(L, P, s0, o, sT, hs, B, S, H, o_bs, st);
+    case GDN2_F32: return launch_scan_typed<float>(L, P, s0, o, sT, hs, B, S, H, o_bs, st);
+    case GDN2_BF16: return launch_scan_typed<__nv_bfloat16>(L, P, s0, o, sT, hs, B, S, H, o_bs, st);
+    case GDN2_F16: return launch_scan_typed<__half>(L, P, s0, o, sT, hs, B, S, H, o_bs, st);
     default: return GDN2_ERR_BAD_DTYPE;
   }
 }

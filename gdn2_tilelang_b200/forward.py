@@ -35,7 +35,7 @@ def chunk_gdn2_fwd(q, k, v, g, b, w, scale, initial_state=None, output_final_sta
     K = _cabi.kernels()
     g = g.float()
     if out is None:
-        o = torch.empty(B, S, H, DV, dtype=v.dtype, device=q.device)
+        o = None
     else:
         if tuple(out.shape) != (B, S, H, DV) or out.dtype != v.dtype or out.stride(3) != 1 or out.stride(2) != DV \
                 or out.stride(1) != H * DV or (B > 1 and out.stride(0) % (H * DV)):
@@ -45,6 +45,13 @@ def chunk_gdn2_fwd(q, k, v, g, b, w, scale, initial_state=None, output_final_sta
     state, hs = initial_state, None
     if state is not None and state.shape != (B, H, DK, DV):
         raise ValueError(f"initial_state must have shape {(B, H, DK, DV)}, got {tuple(state.shape)}")
+    if n_full and out is None and not return_chunk_states:
+        res = K.prefill_ragged(q, k, v, g, b, w, scale, state)      # the whole call in the library, where it applies
+        if res is not None:
+            K.maybe_check_device_status(q.device)
+            return res[0], (res[1] if output_final_state else None)
+    if o is None:
+        o = torch.empty(B, S, H, DV, dtype=v.dtype, device=q.device)
     def tail(st):                                     # the ragged tail through the decode kernel, state in place
         K.decode(*(t[:, n_full:] for t in (q, k, v, g, b, w)), st, scale, out=o[:, n_full:])
 

@@ -170,13 +170,16 @@ int gdn2_prefill_scan_part(const void* workspace, size_t workspace_bytes, const 
  * gdn2_chunk_prep + gdn2_prefill_scan on the floor(S/64)*64 leading tokens and gdn2_decode on the ragged tail
  * (S need not be a multiple of 64), the state chained through final_state (written even without a tail; must not be
  * initial_state unless S < 64).
- *   workspace     gdn2_prefill_workspace_bytes(B, floor(S/64)*64, ...) bytes; NULL is accepted when S < 64
+ *   workspace     gdn2_prefill_workspace_bytes(B, floor(S/64)*64, ...) bytes; NULL is accepted when S < 64. With
+ *                 gdn2_prefill_ragged_workspace_bytes bytes the SIMT family takes the tail as one more chunk
  *   side_stream   NULL, or a second stream of the same device: when the scan is cut into segments the tail's decode,
  *                 which needs only the final state, runs there beside the scan's correction pass; `stream` is ordered
  *                 after it when the call returns
  * Results are those of the three calls made one after the other. No counterpart in the reference as ONE function:
  * its gdn2_prefill is the same sequence in Python.
  */
+size_t gdn2_prefill_ragged_workspace_bytes(int64_t B, int64_t S, int64_t H, int64_t HK, int64_t DK, int64_t DV, int dtype,
+                                           int path);
 int gdn2_prefill_ragged(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
                         const float* initial_state, void* o, float* final_state, void* workspace, size_t workspace_bytes,
                         int64_t B, int64_t S, int64_t H, int64_t HK, int64_t DK, int64_t DV, int64_t in_batch_stride,
