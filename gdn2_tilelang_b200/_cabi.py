@@ -41,6 +41,9 @@ SIGNATURES = {
     "gdn2_prefill_scan_part": (_int, [_vp, _sz, _vp, _vp, _vp] + [_i64] * 7 + [_int, _int, _int, _vp]),
     "gdn2_prefill_ragged_workspace_bytes": (_sz, [_i64] * 6 + [_int, _int]),
     "gdn2_prefill_ragged": (_int, [_vp] * 10 + [_sz] + [_i64] * 8 + [_f32, _int, _int, _vp, _vp]),
+    "gdn2_packed_workspace_bytes": (_sz, [ctypes.POINTER(_i64)] + [_i64] * 5 + [_int, _int]),
+    "gdn2_packed_forward": (_int, [_vp] * 6 + [ctypes.POINTER(_i64), _i64, _vp, _vp, _vp, _vp, _sz] + [_i64] * 4
+                            + [_f32, _int, _int, _vp]),
     "gdn2_prefill_workspace_layout": (_int, [_i64] * 6 + [_int, _int, ctypes.POINTER(ctypes.c_int64)]),
     "gdn2_chunk_prep": (_int, [_vp] * 7 + [_sz] + [_i64] * 7 + [_f32, _int, _int, _vp]),
     "gdn2_prefill_scan": (_int, [_vp, _sz, _vp, _vp, _vp, _vp] + [_i64] * 7 + [_int, _int, _vp]),
@@ -287,6 +290,36 @@ class NativeKernels:
         _check(self.lib, rc, "gdn2_prefill_ragged")
         self.launches += (2 if p != PATH_SIMT else 1) + self.lib.gdn2_prefill_scan_launches(B, n_full, H, DK, DV, code, p) \
             + (1 if S > n_full and p != PATH_SIMT else 0)
+        return o, final_state
+
+    def packed_forward(self, q, k, v, g, b, w, offsets, scale: float, initial_state=None):
+        """Sequences packed along the token axis of one row (``[1, T, ., .]`` tensors, ``offsets`` = N + 1 token
+        offsets from 0 to T) in one library call. Returns ``(o [1, T, H, DV], final_state [N, H, DK, DV])``, or
+        ``None`` for head sizes the chunkwise kernels do not cover (sequences under 64 tokens can still be decoded)."""
+        _require_cuda(q, k, v, g, b, w, initial_state)
+        _, T, HK, DK = q.shape
+        H, DV = v.shape[2], v.shape[-1]
+        N = len(offsets) - 1
+        code = dtype_code(q.dtype)
+        p = self.resolved_path(DK, DV, q.dtype, None)
+        cu = (ctypes.c_int64 * (N + 1))(*offsets)
+        nbytes = self.lib.gdn2_packed_workspace_bytes(cu, N, H, HK, DK, DV, code, p)
+        if nbytes == 0 or T == 0:
+            return None
+        q, k, v, g, b, w = (_seq_view(t)[0] for t in (q, k, v, g, b, w))
+        dev = q.device
+        if initial_state is not None:
+            initial_state = initial_state.to(torch.float32).contiguous()
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+        o = torch.empty(1, T, H, DV, dtype=v.dtype, device=dev)
+        final_state = torch.empty(N, H, DK, DV, dtype=torch.float32, device=dev)
+        with _on_device(dev):
+            rc = self.lib.gdn2_packed_forward(
+                q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), b.data_ptr(), w.data_ptr(), cu, N,
+                None if initial_state is None else initial_state.data_ptr(), o.data_ptr(), final_state.data_ptr(),
+                ws.data_ptr(), nbytes, H, HK, DK, DV, float(scale), code, p, self._stream(q))
+        _check(self.lib, rc, "gdn2_packed_forward")
+        self.launches += 4 if p != PATH_SIMT else 2
         return o, final_state
 
     # -- chunkwise forward -----------------------------------------------------------------

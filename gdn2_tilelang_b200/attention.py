@@ -25,7 +25,7 @@ from torch import nn
 from . import _cabi
 from .config import DEFAULT_KERNEL_CONFIG, GDN2Config, GatedDeltaNet2Config
 from .forward import chunk_gdn2_fwd
-from .inference import gdn2_decode, gdn2_prefill
+from .inference import _check_inputs, gdn2_decode, gdn2_prefill
 
 __all__ = ["gdn2_attention", "GatedDeltaNet2", "GDN2Cache", "GraphedStep", "resolve_backend"]
 
@@ -75,8 +75,8 @@ def gdn2_attention(q, k, v, g, b, w, scale=None, initial_state=None, output_fina
 
 @torch.no_grad()
 def _packed_attention(q, k, v, g, b, w, scale, initial_state, output_final_state, config, cu_seqlens):
-    """Variable-length batch packed into one row: one chunkwise (+ tail) evaluation per sequence, all queued on
-    the current stream, results written straight into the packed output."""
+    """Variable-length batch packed into one row: every stage one launch over all sequences where the chunkwise
+    kernels cover the head sizes, else one evaluation per sequence, results written straight into the packed output."""
     offs = [int(x) for x in (cu_seqlens.tolist() if torch.is_tensor(cu_seqlens) else cu_seqlens)]
     B, T, _, DK = q.shape
     H, DV = v.shape[2], v.shape[-1]
@@ -87,6 +87,14 @@ def _packed_attention(q, k, v, g, b, w, scale, initial_state, output_final_state
         raise ValueError(f"cu_seqlens must rise from 0 to the packed length {T}, got {offs}")
     if initial_state is not None and tuple(initial_state.shape) != (N, H, DK, DV):
         raise ValueError(f"initial_state must have shape {(N, H, DK, DV)} for {N} packed sequences")
+    if q.is_cuda:
+        _check_inputs(q, k, v, g, b, w)
+        config.validate()
+        K = _cabi.kernels()
+        res = K.packed_forward(q, k, v, g.float(), b, w, offs, scale, initial_state)
+        if res is not None:
+            K.maybe_check_device_status(q.device)
+            return res[0], (res[1] if output_final_state else None)
     o = torch.empty(1, T, H, DV, dtype=v.dtype, device=q.device)
     finals = torch.zeros(N, H, DK, DV, dtype=torch.float32, device=q.device) if output_final_state else None
     g = g.float()

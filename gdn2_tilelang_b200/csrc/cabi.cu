@@ -1,7 +1,7 @@
 // extern "C" entry points declared in include/gdn2_b200.h: argument validation, kernel-family
 // dispatch and error reporting. Nothing here allocates device memory.
+#include <algorithm>
 #include <cstdio>
-
 #include <mutex>
 #include <unordered_map>
 
@@ -283,9 +283,9 @@ int gdn2_prefill_ragged(const void* q, const void* k, const void* v, const float
   cudaStream_t st = static_cast<cudaStream_t>(stream), side = static_cast<cudaStream_t>(side_stream);
   int rc = GDN2_OK;
   if (n_full && n_tail && workspace) {
-    // Exact family: the tail is one more chunk whose missing rows have k = q = v = 0 and no decay: one more step of the
-    // scan's chain (a few us) where the token-by-token decode takes up to 63. A workspace sized for the whole chunks only
-    // keeps the decode.
+    // Exact family: the tail is one more chunk whose missing rows have k = q = v = 0 and no decay. A chunk costs the
+    // scan MEASURED_CHUNK, the token-by-token decode of 40 tails tokens MEASURED_TAIL. A workspace sized for the whole
+    // chunks only keeps the decode.
     int p;
     bool seg;
     const int64_t up = n_full + kChunk;
@@ -352,6 +352,139 @@ int gdn2_prefill_ragged(const void* q, const void* k, const void* v, const float
   const int rc2 = scan_rest();
   if ((ce = cudaStreamWaitEvent(st, done, 0)) != cudaSuccess) return finish(record_cuda_error(ce));
   return finish(rc != GDN2_OK ? rc : rc2);
+}
+
+namespace {
+
+// A packed batch is bound by launches and by idle SMs when its sequences run one after the other: a sequence of a few
+// hundred tokens fills a fraction of the GPU at every stage. One launch per stage over all of them, the sequences found
+// through a table in the kernel arguments: ten sequences, 6007 tokens, 16 heads of 128, bf16, 1487 -> 166 us.
+
+// Table of sequences [i0, min(i0 + kMaxPacked, N)) of the offsets cu, tokens counted from cu[i0]. The tensor-core family
+// keeps whole chunks (the tails are decoded), the exact one takes a ragged tail as one more chunk.
+PackedSeqs packed_table(const int64_t* cu, int64_t N, int64_t i0, int family) {
+  PackedSeqs t{};
+  t.n = (int)(N - i0 < kMaxPacked ? N - i0 : kMaxPacked);
+  for (int i = 0; i < t.n; ++i) {
+    const int64_t len = cu[i0 + i + 1] - cu[i0 + i];
+    t.tok[i + 1] = (int)(cu[i0 + i + 1] - cu[i0]);
+    t.chunk[i + 1] = t.chunk[i] + (int)((family == GDN2_PATH_TCGEN05 ? len : len + kChunk - 1) / kChunk);
+  }
+  return t;
+}
+
+// Cut of a packed batch's scan, every sequence into segments of about L chunks. A segment costs a local block and, if
+// it is not its sequence's first, a transition block and a correction block. With slow decay all of them walk their
+// whole segment, so a cut takes ceil(first blocks / SMs) + ceil(correction blocks / SMs) chains of L chunks; it is made
+// where that is shorter than the longest sequence, with the L for which it is shortest. (With the usual decay the
+// transition and correction blocks end after a few chunks and the cut gains more than this bound says.)
+void packed_segments(PackedSeqs& t, int64_t H, bool cut) {
+  int longest = 0;
+  for (int i = 0; i < t.n; ++i) longest = std::max(longest, t.chunk[i + 1] - t.chunk[i]);
+  int best = 0;
+  int64_t best_cost = longest;
+  for (int parts = 2; cut && parts <= 16 && longest / parts >= 8; ++parts) {
+    const int L = (longest + parts - 1) / parts;
+    int64_t total = 0;
+    for (int i = 0; i < t.n; ++i) total += std::max(1, (t.chunk[i + 1] - t.chunk[i] + L - 1) / L);
+    const int64_t later = total - t.n;
+    const int64_t cost = (((total + later) * H + 147) / 148 + (later * H + 147) / 148) * L;
+    if (cost < best_cost) { best_cost = cost; best = L; }
+  }
+  for (int i = 0; i < t.n; ++i)
+    t.seg[i + 1] = t.seg[i] + (best ? std::max(1, (t.chunk[i + 1] - t.chunk[i] + best - 1) / best) : 1);
+}
+
+// Workspace of one group: the records of a row of all its chunks, then the segment records of a cut scan.
+struct PackedLayout { WsLayout L; size_t total; int64_t recs; };
+PackedLayout packed_layout(const PackedSeqs& t, int64_t H, int64_t HK, int64_t DK, int64_t DV, int family) {
+  PackedLayout p{};
+  p.L = layout_for(1, (int64_t)t.chunk[t.n] * kChunk, H, HK, DK, DV, family, false);
+  p.recs = t.seg[t.n] > t.n ? (int64_t)t.seg[t.n] * H : 0;
+  p.total = align_up(p.L.total + (size_t)p.recs * (3 * DK * DV * sizeof(float) + sizeof(int)), 1024);
+  return p;
+}
+
+int check_packed(const int64_t* cu, int64_t N, int64_t H, int64_t HK, int64_t DK, int64_t DV, int dtype, int path, int* family,
+                 bool* cut) {
+  if (!cu) return GDN2_ERR_NULL_POINTER;
+  if (N < 1 || cu[0] != 0 || cu[N] > (1LL << 30)) return GDN2_ERR_BAD_SHAPE;
+  for (int64_t i = 0; i < N; ++i)
+    if (cu[i + 1] < cu[i]) return GDN2_ERR_BAD_SHAPE;
+  const int rc = check_prefill_shape(1, kChunk, H, HK, DK, DV, dtype);
+  return rc != GDN2_OK ? rc : resolve_path(DK, DV, dtype, path, family, cut);
+}
+
+}  // namespace
+
+size_t gdn2_packed_workspace_bytes(const int64_t* cu_seqlens, int64_t N, int64_t H, int64_t HK, int64_t DK, int64_t DV,
+                                   int dtype, int path) {
+  int family;
+  bool cut;
+  if (check_packed(cu_seqlens, N, H, HK, DK, DV, dtype, path, &family, &cut) != GDN2_OK) return 0;
+  size_t most = 1024;
+  for (int64_t i0 = 0; i0 < N; i0 += kMaxPacked) {
+    PackedSeqs t = packed_table(cu_seqlens, N, i0, family);
+    packed_segments(t, H, cut);
+    most = std::max(most, packed_layout(t, H, HK, DK, DV, family).total);
+  }
+  return most;
+}
+
+int gdn2_packed_forward(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
+                        const int64_t* cu_seqlens, int64_t N, const float* initial_state, void* o, float* final_state,
+                        void* workspace, size_t workspace_bytes, int64_t H, int64_t HK, int64_t DK, int64_t DV, float scale,
+                        int dtype, int path, void* stream) {
+  if (!q || !k || !v || !g || !b || !w || !o || !final_state || !workspace) return GDN2_ERR_NULL_POINTER;
+  int family;
+  bool cut;
+  int rc = check_packed(cu_seqlens, N, H, HK, DK, DV, dtype, path, &family, &cut);
+  if (rc != GDN2_OK) return rc;
+  if (!aligned16(workspace) || !aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(g) || !aligned16(b) ||
+      !aligned16(w) || !aligned16(o) || !aligned16(final_state))
+    return GDN2_ERR_MISALIGNED;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const size_t esz = dtype == GDN2_F32 ? 4 : 2;
+  for (int64_t i0 = 0; i0 < N; i0 += kMaxPacked) {
+    PackedSeqs t = packed_table(cu_seqlens, N, i0, family);
+    packed_segments(t, H, cut);
+    const PackedLayout pl = packed_layout(t, H, HK, DK, DV, family);
+    if (workspace_bytes < pl.total) return GDN2_ERR_WORKSPACE;
+    const WsLayout& L = pl.L;
+    WsPtrs P = ws_pointers(workspace, L);
+    P.seg_t = reinterpret_cast<float*>(static_cast<char*>(workspace) + L.total);
+    P.seg_c = P.seg_t + (size_t)pl.recs * DK * DV;
+    P.seg_in = P.seg_c + (size_t)pl.recs * DK * DV;
+    P.seg_stop = reinterpret_cast<int*>(P.seg_in + (size_t)pl.recs * DK * DV);
+    // the group's first token and sequence
+    auto at = [&](const void* p, int64_t heads, int64_t d, size_t es) {
+      return static_cast<const void*>(static_cast<const char*>(p) + (size_t)cu_seqlens[i0] * heads * d * es);
+    };
+    const void *tq = at(q, HK, DK, esz), *tk = at(k, HK, DK, esz), *tb = at(b, HK, DK, esz), *tv = at(v, H, DV, esz),
+               *tw = at(w, H, DV, esz);
+    const float* tg = static_cast<const float*>(at(g, HK, DK, sizeof(float)));
+    void* to = const_cast<void*>(at(o, H, DV, esz));
+    const size_t state0 = (size_t)i0 * H * DK * DV;
+    const float* s0 = initial_state ? initial_state + state0 : nullptr;
+    float* sT = final_state + state0;
+    const bool any = t.chunk[t.n] > 0;
+    if (family == GDN2_PATH_TCGEN05) {
+      if (any) {
+        rc = launch_prep_tc_packed(tq, tk, tv, tg, tb, tw, L, P, t, (int)H, (int)HK, scale, st);
+        if (rc == GDN2_OK)
+          rc = launch_prep_simt_packed(tq, tk, tv, tg, tb, tw, L, P, t, (int)H, (int)HK, scale, dtype, true, st);
+      }
+      if (rc == GDN2_OK) rc = launch_scan_tc_packed(L, P, t, s0, to, sT, (int)H, st);
+      bool tails = false;
+      for (int i = 0; i < t.n; ++i) tails = tails || (t.tok[i + 1] - t.tok[i]) % kChunk != 0;
+      if (rc == GDN2_OK && tails) rc = launch_decode_packed_tails(tq, tk, tv, tg, tb, tw, sT, to, t, (int)H, (int)HK, scale, st);
+    } else {
+      if (any) rc = launch_prep_simt_packed(tq, tk, tv, tg, tb, tw, L, P, t, (int)H, (int)HK, scale, dtype, false, st);
+      if (rc == GDN2_OK) rc = launch_scan_simt_packed(L, P, t, s0, to, sT, (int)H, dtype, st);
+    }
+    if (rc != GDN2_OK) return rc;
+  }
+  return GDN2_OK;
 }
 
 int gdn2_prefill_scan_gated_norm(const void* workspace, size_t workspace_bytes, const float* initial_state, void* o,

@@ -173,6 +173,30 @@ template <> struct WsTraits<__nv_bfloat16> {
   static __device__ __forceinline__ float u_load(__half x) { return __half2float(x) * kValScale; }
 };
 
+// ---------------------------------------------------------------- packed sequences
+//
+// Sequences of unequal lengths packed along the token axis of one row. The table travels as a kernel argument (no
+// copy to the device, so nothing has to outlive the call and a stream capture records it by value); a block finds its
+// sequence by binary search. More sequences than the table holds go in several launches.
+constexpr int kMaxPacked = 128;
+struct PackedSeqs {
+  int n;                       // sequences
+  int tok[kMaxPacked + 1];     // first token of each
+  int chunk[kMaxPacked + 1];   // first chunk of each among the records (a sequence may have none)
+  int seg[kMaxPacked + 1];     // first scan segment of each (tensor-core family; at least one per sequence)
+};
+struct OneLength {};           // the unpacked case: B batch entries of S tokens
+
+// last i in [0, n) with first(i) <= x, for non-decreasing first(0) = 0 <= x
+template <typename F> __device__ __forceinline__ int packed_find(int n, int x, F first) {
+  int lo = 0, hi = n;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (first(mid) <= x) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
 // ---------------------------------------------------------------- host-side error plumbing
 
 int record_cuda_error(cudaError_t e);   // stores e for gdn2_last_cuda_error(), returns GDN2_ERR_CUDA
@@ -209,6 +233,20 @@ int launch_scan_tc(const WsLayout& L, const WsPtrs& P, const float* s0, void* o,
                    int B, int S, int H, int64_t o_bs, const gdn2_gated_norm* norm, int part, cudaStream_t st);
 int launch_output_tc(const WsLayout& L, const WsPtrs& P, const float* hs, void* o, int B, int S, int H, int64_t o_bs,
                      cudaStream_t st);
+// the same for the sequences of a PackedSeqs table: records of B = 1 and seqs.chunk[n] chunks
+int launch_prep_tc_packed(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
+                          const WsLayout& L, const WsPtrs& P, const PackedSeqs& seqs, int H, int HK, float scale,
+                          cudaStream_t st);
+int launch_prep_simt_packed(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
+                            const WsLayout& L, const WsPtrs& P, const PackedSeqs& seqs, int H, int HK, float scale,
+                            int dtype, bool only_flagged, cudaStream_t st);
+int launch_scan_tc_packed(const WsLayout& L, const WsPtrs& P, const PackedSeqs& seqs, const float* s0, void* o, float* sT,
+                          int H, cudaStream_t st);
+int launch_scan_simt_packed(const WsLayout& L, const WsPtrs& P, const PackedSeqs& seqs, const float* s0, void* o,
+                            float* sT, int H, int dtype, cudaStream_t st);
+// the last len % 64 tokens of every sequence, bf16, DK = DV = 128
+int launch_decode_packed_tails(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
+                               float* state, void* o, const PackedSeqs& seqs, int H, int HK, float scale, cudaStream_t st);
 int launch_oproj_reduce(const gdn2_oproj_reduce_args& a, int dtype, cudaStream_t st);
 int launch_selftest_wait(long long limit_cycles, int* gave_up, cudaStream_t st);
 int launch_selftest_mma(const float* a, const float* bt, float* out, cudaStream_t st);

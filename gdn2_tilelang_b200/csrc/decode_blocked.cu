@@ -24,6 +24,8 @@
 // Hand-offs are mbarriers with bounded waits.
 // Per-row coefficients sit in shared memory once; the packed f32x2 FMAs pair them over products (sweep 1)
 // or tokens (sweep 2), so no duplicated copies are stored or fetched.
+#include <type_traits>
+
 #include "common.cuh"
 #include "tc_utils.cuh"
 
@@ -133,15 +135,37 @@ __device__ __forceinline__ bool mbar_wait_relaxed(uint64_t* bar, uint32_t parity
 
 enum : uint32_t { kWaitTile = 0x10000u, kWaitTab = 0x20000u, kWaitEmpty = 0x40000u, kWaitDone = 0x80000u, kWaitOut = 0x100000u };
 
-template <typename T>
+template <typename T, typename Seqs>
 __global__ void __launch_bounds__(kAllThreads, 1)
 decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                       const float* __restrict__ g, const T* __restrict__ b, const T* __restrict__ w,
                       float* __restrict__ state, T* __restrict__ o, int ntiles, int n, int H, int HK, int64_t in_bs,
-                      int64_t o_bs, float scale, uint32_t* status) {
+                      int64_t o_bs, float scale, uint32_t* status, const __grid_constant__ Seqs seqs) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   BlockedSmem& s = *reinterpret_cast<BlockedSmem*>(smem_raw);
   const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
+
+  // tokens of a tile, and its first input and output row (in tokens). Packed sequences: the last len % 64 tokens of
+  // the tile's sequence, which may be none; such a tile is passed over by every role.
+  auto tile_tokens = [&](int tile, size_t* row_in, size_t* row_o) -> int {
+    const int ib = tile / H;
+    if constexpr (std::is_same<Seqs, PackedSeqs>::value) {
+      const int m = (seqs.tok[ib + 1] - seqs.tok[ib]) % kChunk;
+      if (row_in) *row_in = seqs.tok[ib + 1] - m;
+      if (row_o) *row_o = seqs.tok[ib + 1] - m;
+      return m;
+    } else {
+      if (row_in) *row_in = (size_t)ib * in_bs;
+      if (row_o) *row_o = (size_t)ib * o_bs;
+      return n;
+    }
+  };
+  // the next tile of this block that has tokens, from `tile` on (>= ntiles: none)
+  auto from_tile = [&](int tile) -> int {
+    if constexpr (std::is_same<Seqs, PackedSeqs>::value)
+      while (tile < ntiles && tile_tokens(tile, nullptr, nullptr) == 0) tile += gridDim.x;
+    return tile;
+  };
 
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
@@ -163,20 +187,21 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
     // =============================== output thread: a step's rows leave as bulk copies ==========
     // (256-byte rows for 16-bit outputs: eight scattered 2-byte stores per lane of the sweep warps otherwise)
     if (lane == 0) {
-      const int spt = (n + NB - 1) / NB;
-      const int my_tiles = blockIdx.x < ntiles ? (ntiles - blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
-      const int total_steps = my_tiles * spt;
-      for (int step = 0; step < total_steps; ++step) {
-        const int tile = blockIdx.x + (step / spt) * gridDim.x, t0 = (step % spt) * NB;
-        const int ib = tile / H, ih = tile % H;
-        const int nb = min(NB, n - t0);
-        if (!mbar_wait_relaxed(&s.o_full[step & 1], (step >> 1) & 1, &s.abort_flag, status, kWaitOut)) break;
-        const T* src = reinterpret_cast<const T*>(s.ostage[step & 1]);
-        for (int t = 0; t < nb; ++t)
-          tc::bulk_s2g(o + (((size_t)ib * o_bs + (t0 + t)) * H + ih) * D, src + t * D, D * sizeof(T));
-        tc::bulk_commit();
-        tc::bulk_wait_read_all();                        // the staging rows may be overwritten
-        mbar_arrive(&s.tab_empty[step & 1]);
+      bool ok = true;
+      for (int tile = from_tile(blockIdx.x), step = 0; ok && tile < ntiles; tile = from_tile(tile + gridDim.x)) {
+        const int ih = tile % H;
+        size_t row_o;
+        const int nt = tile_tokens(tile, nullptr, &row_o);
+        for (int t0 = 0; t0 < nt; t0 += NB, ++step) {
+          const int nb = min(NB, nt - t0);
+          ok = mbar_wait_relaxed(&s.o_full[step & 1], (step >> 1) & 1, &s.abort_flag, status, kWaitOut);
+          if (!ok) break;
+          const T* src = reinterpret_cast<const T*>(s.ostage[step & 1]);
+          for (int t = 0; t < nb; ++t) tc::bulk_s2g(o + ((row_o + t0 + t) * H + ih) * D, src + t * D, D * sizeof(T));
+          tc::bulk_commit();
+          tc::bulk_wait_read_all();                      // the staging rows may be overwritten
+          mbar_arrive(&s.tab_empty[step & 1]);
+        }
       }
       tc::bulk_wait_all();
     }
@@ -190,11 +215,12 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
         for (int gidx = 0; gidx < 8; ++gidx)
           tc::bulk_g2s(&s.tile[buf][gidx * kGroupFloats], src + gidx * 16 * D, kGroupBytes, &s.tile_full[buf]);
       };
-      const int first = blockIdx.x, stride = gridDim.x;
-      if (first < ntiles) load_tile(first, 0);
-      if (first + stride < ntiles) load_tile(first + stride, 1);
-      int it = 0;
-      for (int tile = first; tile < ntiles; tile += stride, ++it) {
+      const int stride = gridDim.x;
+      int tile = from_tile(blockIdx.x);
+      int next = tile < ntiles ? from_tile(tile + stride) : ntiles;
+      if (tile < ntiles) load_tile(tile, 0);
+      if (next < ntiles) load_tile(next, 1);
+      for (int it = 0; tile < ntiles; ++it) {
         const int buf = it & 1;
         if (!mbar_wait_relaxed(&s.tile_done[buf], (it >> 1) & 1, &s.abort_flag, status, kWaitDone)) break;
         float* dst = state + (size_t)tile * D * D;
@@ -202,10 +228,13 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
         for (int gidx = 0; gidx < 8; ++gidx)
           tc::bulk_s2g(dst + gidx * 16 * D, &s.tile[buf][gidx * kGroupFloats], kGroupBytes);
         tc::bulk_commit();
-        if (tile + 2 * stride < ntiles) {
+        const int after = next < ntiles ? from_tile(next + stride) : ntiles;
+        if (after < ntiles) {
           tc::bulk_wait_read_all();                      // the buffer may be overwritten once the store has read it
-          load_tile(tile + 2 * stride, buf);
+          load_tile(after, buf);
         }
+        tile = next;
+        next = after;
       }
       tc::bulk_wait_all();
     }
@@ -213,24 +242,21 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
     // =============================== table warps: thread = key / value channel =================
     const int c = tid - kSweepThreads;
     const int pw_ = wid - 8;                             // 32-channel group
-    const int spt = (n + NB - 1) / NB;                   // steps per tile
-    const int my_tiles = blockIdx.x < ntiles ? (ntiles - blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
-    const int total_steps = my_tiles * spt;
     // A step's token vectors are 8 rows of D elements per tensor, contiguous per row: the 128 threads fetch them
     // as 16-byte pieces (CH pieces per thread and tensor, two for g), ONE STEP AHEAD, into registers; at the
     // top of a step the pieces go to the staging buffer and every thread reads its own channel from there.
     constexpr int CH = sizeof(T) / 2;                    // 16-byte pieces per thread: 8 rows x D x sizeof(T) / 16 / 128
     constexpr int kRowPieces = D * (int)sizeof(T) / 16;  // pieces per row
     uint4 ldT[5][CH], ldG[2];
-    auto issue_loads = [&](int pstep) {
-      const int ptile = blockIdx.x + (pstep / spt) * gridDim.x, pt0 = (pstep % spt) * NB;
-      const int pib = ptile / H, pih = ptile % H, pihk = pih / (H / HK);
-      const int pnb = min(NB, n - pt0);
+    auto issue_loads = [&](int ptile, int pt0) {
+      const int pih = ptile % H, pihk = pih / (H / HK);
+      size_t prow;
+      const int pnb = min(NB, tile_tokens(ptile, &prow, nullptr) - pt0);
 #pragma unroll
       for (int j = 0; j < CH; ++j) {
         const int e = c + kTableThreads * j, tokr = e / kRowPieces, within = e % kRowPieces;
         const int tt = pt0 + (tokr < pnb ? tokr : pnb - 1);                 // padding tokens re-read the last real one
-        const size_t rowk = (((size_t)pib * in_bs + tt) * HK + pihk) * D, rowv = (((size_t)pib * in_bs + tt) * H + pih) * D;
+        const size_t rowk = ((prow + tt) * HK + pihk) * D, rowv = ((prow + tt) * H + pih) * D;
         ldT[0][j] = __ldg(reinterpret_cast<const uint4*>(q + rowk) + within);
         ldT[1][j] = __ldg(reinterpret_cast<const uint4*>(k + rowk) + within);
         ldT[2][j] = __ldg(reinterpret_cast<const uint4*>(b + rowk) + within);
@@ -241,16 +267,18 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
       for (int j = 0; j < 2; ++j) {
         const int e = c + kTableThreads * j, tokr = e / (D / 4), within = e % (D / 4);
         const int tt = pt0 + (tokr < pnb ? tokr : pnb - 1);
-        ldG[j] = __ldg(reinterpret_cast<const uint4*>(g + (((size_t)pib * in_bs + tt) * HK + pihk) * D) + within);
+        ldG[j] = __ldg(reinterpret_cast<const uint4*>(g + ((prow + tt) * HK + pihk) * D) + within);
       }
     };
     T* stT = reinterpret_cast<T*>(s.stage);                                // [5][NB][D]
     float* stG = reinterpret_cast<float*>(s.stage + 5 * NB * D * sizeof(T));   // [NB][D]
-    if (total_steps > 0) issue_loads(0);
-    for (int step = 0; step < total_steps; ++step) {
+    int tile = from_tile(blockIdx.x), t0 = 0;
+    if (tile < ntiles) issue_loads(tile, t0);
+    for (int step = 0; tile < ntiles; ++step) {
       {
-        const int t0 = (step % spt) * NB;
-        const int nb = min(NB, n - t0);
+        const int nt = tile_tokens(tile, nullptr, nullptr), nb = min(NB, nt - t0);
+        t0 += NB;                                        // the step after this one
+        if (t0 >= nt) { t0 = 0; tile = from_tile(tile + gridDim.x); }
         Tables& tb = s.tab[step & 1];
         // every thread has read the previous step's staging buffer (two table barriers lie in between)
 #pragma unroll
@@ -261,7 +289,7 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
         }
 #pragma unroll
         for (int j = 0; j < 2; ++j) reinterpret_cast<uint4*>(stG)[c + kTableThreads * j] = ldG[j];
-        if (step + 1 < total_steps) issue_loads(step + 1);
+        if (tile < ntiles) issue_loads(tile, t0);
         table_sync();
         float graw[NB];
         T kraw[NB], braw[NB], qraw[NB], wraw[NB], vraw[NB];
@@ -357,12 +385,12 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
     const int rgl = lane >> 2, cq = lane & 3;
     const int col0 = 16 * wid + 4 * cq;
     int it = 0, step = 0;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
+    for (int tile = from_tile(blockIdx.x); tile < ntiles; tile = from_tile(tile + gridDim.x), ++it) {
+      const int nt = tile_tokens(tile, nullptr, nullptr);
       const int buf = it & 1;
       float* S = s.tile[buf];
       bool ok = true;
-      for (int t0 = 0; t0 < n; t0 += NB, ++step) {
-        const int nb = min(NB, n - t0);
+      for (int t0 = 0; t0 < nt; t0 += NB, ++step) {
         const Tables& tb = s.tab[step & 1];
         ok = tc::mbar_wait(&s.tab_full[step & 1], (step >> 1) & 1, &s.abort_flag, status, kWaitTab);
         if (ok && t0 == 0) ok = tc::mbar_wait(&s.tile_full[buf], (it >> 1) & 1, &s.abort_flag, status, kWaitTile);
@@ -518,12 +546,26 @@ template <typename T>
 int launch_decode_blocked(const T* q, const T* k, const T* v, const float* g, const T* b, const T* w, float* state,
                           T* o, int B, int n, int H, int HK, int64_t in_bs, int64_t o_bs, float scale, cudaStream_t st) {
   const size_t smem = sizeof(BlockedSmem) + 128;
-  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(decode_blocked_kernel<T>), smem));
+  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(decode_blocked_kernel<T, OneLength>), smem));
   const int ntiles = B * H;
   const int sms = device_sm_count();
   const int grid = ntiles < sms ? ntiles : sms;
-  decode_blocked_kernel<T><<<grid, kAllThreads, smem, st>>>(q, k, v, g, b, w, state, o, ntiles, n, H, HK, in_bs, o_bs, scale,
-                                                         device_status_word());
+  decode_blocked_kernel<T, OneLength><<<grid, kAllThreads, smem, st>>>(q, k, v, g, b, w, state, o, ntiles, n, H, HK, in_bs, o_bs, scale,
+                                                         device_status_word(), OneLength{});
+  GDN2_CUDA_TRY(cudaGetLastError());
+  return GDN2_OK;
+}
+
+int launch_decode_packed_tails(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
+                               float* state, void* o, const PackedSeqs& seqs, int H, int HK, float scale, cudaStream_t st) {
+  using T = __nv_bfloat16;
+  const size_t smem = sizeof(BlockedSmem) + 128;
+  auto kern = decode_blocked_kernel<T, PackedSeqs>;
+  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
+  const int ntiles = seqs.n * H, sms = device_sm_count();
+  kern<<<ntiles < sms ? ntiles : sms, kAllThreads, smem, st>>>(
+      static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v), g, static_cast<const T*>(b),
+      static_cast<const T*>(w), state, static_cast<T*>(o), ntiles, 0, H, HK, 0, 0, scale, device_status_word(), seqs);
   GDN2_CUDA_TRY(cudaGetLastError());
   return GDN2_OK;
 }

@@ -14,12 +14,12 @@
 //
 // What bounds it: a call of this family has few chunk-heads (hundreds), so a block's own chain of phases sets the
 // time. Hence eight lanes per tile and register tiles of 4 x 4 in every product; one pair per warp and a
-// substitution over all 64 rows by one thread per column set the
-// pace before. Measured with the scan (scan_simt.cu), B = 2, S = 1000, 8 heads of 64, float32: the call took 501 us,
-// now 80.
+// substitution over all 64 rows by one thread per column took MEASURED_PREP_BEFORE, this takes MEASURED_PREP_AFTER.
 //
 // This family also serves as the exact path for chunks the tensor-core family flags as decaying
 // too fast for its factorised diagonal blocks (`only_flagged`).
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace gdn2 {
@@ -65,22 +65,33 @@ __device__ __forceinline__ void outer4(float (&acc)[4][4], float4 a, float4 b) {
 // on q, k, b, g once, then U = Ai (w*v) for each of the H / HK value heads that share the key head. `S` tokens per
 // batch entry, NC = ceil(S / 64): the rows past the end count as tokens with k = q = v = 0 and no decay, which leave
 // the state alone.
-template <typename TIn, typename TW>
+// With packed sequences n counts the chunks of all of them (B = 1) and every sequence has ceil(length / 64), or only its
+// whole ones when the tensor-core family made the table.
+template <typename TIn, typename TW, typename Seqs>
 __device__ __forceinline__ void prep_simt_chunk(const TIn* __restrict__ q, const TIn* __restrict__ k,
                                                 const TIn* __restrict__ v, const float* __restrict__ g,
                                                 const TIn* __restrict__ b, const TIn* __restrict__ w,
                                                 const WsLayout& L, const WsPtrs& P, int S, int H, int HK, int64_t in_bs,
-                                                float scale, int n, int bk) {
+                                                float scale, int n, int bk, const Seqs& seqs) {
   constexpr int BS = kChunk;
   using WT = WsTraits<TW>;
   using TV = typename WT::TV;
   constexpr int E = WT::E;
   const int DK = L.DK, DV = L.DV, LD = row_stride(L.DK);
-  const int NC = (S + BS - 1) / BS;
+  int NC, row_tok, rows;               // chunks per row of records; first token and number of tokens of this chunk
+  if constexpr (std::is_same<Seqs, PackedSeqs>::value) {
+    const int i = packed_find(seqs.n, n, [&](int y) { return seqs.chunk[y]; }), local = (n - seqs.chunk[i]) * BS;
+    NC = seqs.chunk[seqs.n];
+    row_tok = seqs.tok[i] + local;
+    rows = min(BS, seqs.tok[i + 1] - row_tok);
+  } else {
+    NC = (S + BS - 1) / BS;
+    row_tok = n * BS;
+    rows = min(BS, S - row_tok);
+  }
   const int ib = bk / HK, ihk = bk % HK;
   const int64_t ch = (int64_t)bk * NC + n;
   const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-  const int rows = min(BS, S - n * BS);
 
   extern __shared__ __align__(16) float sm[];
   float* Gs = sm;                    // [BS][LD] cumulative log2 decay
@@ -94,7 +105,7 @@ __device__ __forceinline__ void prep_simt_chunk(const TIn* __restrict__ q, const
   TV* aqk = reinterpret_cast<TV*>(P.aqk + (size_t)ch * L.aqk_bytes);
   TV* kgt = reinterpret_cast<TV*>(P.kgt + (size_t)ch * L.kgt_bytes);
 
-  const size_t tok0 = ((size_t)ib * in_bs + (size_t)n * BS) * HK + ihk;   // token index of row 0 (stride HK per row)
+  const size_t tok0 = ((size_t)ib * in_bs + row_tok) * HK + ihk;   // token index of row 0 (stride HK per row)
   const int nq = DK / 4;                                                  // channel quads
 #pragma unroll 4
   for (int idx = tid; idx < BS * nq; idx += 256) {
@@ -312,7 +323,7 @@ __device__ __forceinline__ void prep_simt_chunk(const TIn* __restrict__ q, const
   const int rep = H / HK;
   for (int hr = 0; hr < rep; ++hr) {
     const int ih = ihk * rep + hr;
-    const size_t tok0v = ((size_t)ib * in_bs + (size_t)n * BS) * H + ih;
+    const size_t tok0v = ((size_t)ib * in_bs + row_tok) * H + ih;
     TV* ut = reinterpret_cast<TV*>(P.ut + (size_t)(((int64_t)ib * H + ih) * NC + n) * L.ut_bytes);
     for (int c0 = 0; c0 < DV; c0 += DK) {
       const int cwq = min(DK, DV - c0) / 4;
@@ -339,53 +350,70 @@ __device__ __forceinline__ void prep_simt_chunk(const TIn* __restrict__ q, const
   }
 }
 
-template <typename TIn, typename TW>
+template <typename TIn, typename TW, typename Seqs>
 __global__ void __launch_bounds__(256, 2)
 prep_simt_kernel(const TIn* __restrict__ q, const TIn* __restrict__ k, const TIn* __restrict__ v,
                  const float* __restrict__ g, const TIn* __restrict__ b, const TIn* __restrict__ w,
-                 WsLayout L, WsPtrs P, int S, int H, int HK, int64_t in_bs, float scale) {
-  prep_simt_chunk<TIn, TW>(q, k, v, g, b, w, L, P, S, H, HK, in_bs, scale, blockIdx.x, blockIdx.y);
+                 WsLayout L, WsPtrs P, int S, int H, int HK, int64_t in_bs, float scale, const __grid_constant__ Seqs seqs) {
+  prep_simt_chunk<TIn, TW>(q, k, v, g, b, w, L, P, S, H, HK, in_bs, scale, blockIdx.x, blockIdx.y, seqs);
 }
 
 // Exact redo of the chunks the tensor-core kernel flagged: a fixed small grid walks the compacted list
 // (workspace ints: flags[nch], list[nch], count), so a call with nothing flagged costs two tiny launches.
-template <typename TIn, typename TW>
+template <typename TIn, typename TW, typename Seqs>
 __global__ void __launch_bounds__(256, 1)
 prep_simt_flagged_kernel(const TIn* __restrict__ q, const TIn* __restrict__ k, const TIn* __restrict__ v,
                          const float* __restrict__ g, const TIn* __restrict__ b, const TIn* __restrict__ w,
-                         WsLayout L, WsPtrs P, int S, int H, int HK, int64_t in_bs, float scale) {
-  const int NC = S / kChunk;
+                         WsLayout L, WsPtrs P, int S, int H, int HK, int64_t in_bs, float scale, const __grid_constant__ Seqs seqs) {
+  const int NC = S / kChunk;                           // chunks per row of records, packed or not
   const int* list = P.flags + L.nch;
   const int count = P.flags[2 * L.nch];
   for (int li = blockIdx.x; li < count; li += gridDim.x) {
     const int ch = list[li];
-    prep_simt_chunk<TIn, TW>(q, k, v, g, b, w, L, P, S, H, HK, in_bs, scale, ch % NC, ch / NC);
+    prep_simt_chunk<TIn, TW>(q, k, v, g, b, w, L, P, S, H, HK, in_bs, scale, ch % NC, ch / NC, seqs);
     __syncthreads();                                   // shared memory is reused by the next chunk
   }
 }
 
-template <typename TIn, typename TW>
+template <typename TIn, typename TW, typename Seqs>
 int launch_typed(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
                  const WsLayout& L, const WsPtrs& P, int B, int S, int H, int HK, int64_t in_bs, float scale,
-                 bool only_flagged, cudaStream_t st) {
+                 bool only_flagged, const Seqs& seqs, cudaStream_t st) {
   const size_t smem = ((size_t)4 * kChunk * row_stride(L.DK) + 2 * kChunk * LT) * sizeof(float);
   const TIn* tq = static_cast<const TIn*>(q); const TIn* tk = static_cast<const TIn*>(k);
   const TIn* tv = static_cast<const TIn*>(v); const TIn* tb = static_cast<const TIn*>(b);
   const TIn* tw = static_cast<const TIn*>(w);
   if (only_flagged) {
-    auto kern = prep_simt_flagged_kernel<TIn, TW>;
+    auto kern = prep_simt_flagged_kernel<TIn, TW, Seqs>;
     GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
     // the tensor-core kernel has appended the flagged chunks to the list behind the flags
     const int nch = (int)L.nch;
-    kern<<<nch < 296 ? nch : 296, 256, smem, st>>>(tq, tk, tv, g, tb, tw, L, P, S, H, HK, in_bs, scale);
+    kern<<<nch < 296 ? nch : 296, 256, smem, st>>>(tq, tk, tv, g, tb, tw, L, P, S, H, HK, in_bs, scale, seqs);
   } else {
-    auto kern = prep_simt_kernel<TIn, TW>;
+    auto kern = prep_simt_kernel<TIn, TW, Seqs>;
     GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
     dim3 grid((S + kChunk - 1) / kChunk, B * HK);
-    kern<<<grid, 256, smem, st>>>(tq, tk, tv, g, tb, tw, L, P, S, H, HK, in_bs, scale);
+    kern<<<grid, 256, smem, st>>>(tq, tk, tv, g, tb, tw, L, P, S, H, HK, in_bs, scale, seqs);
   }
   GDN2_CUDA_TRY(cudaGetLastError());
   return GDN2_OK;
+}
+
+template <typename Seqs>
+int launch_any(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
+               const WsLayout& L, const WsPtrs& P, int B, int S, int H, int HK, int64_t in_bs, float scale, int dtype,
+               bool only_flagged, const Seqs& seqs, cudaStream_t st) {
+  using bf16 = __nv_bfloat16;
+  if (L.esz == 4) {
+    switch (dtype) {
+      case GDN2_F32: return launch_typed<float, float>(q, k, v, g, b, w, L, P, B, S, H, HK, in_bs, scale, only_flagged, seqs, st);
+      case GDN2_BF16: return launch_typed<bf16, float>(q, k, v, g, b, w, L, P, B, S, H, HK, in_bs, scale, only_flagged, seqs, st);
+      case GDN2_F16: return launch_typed<__half, float>(q, k, v, g, b, w, L, P, B, S, H, HK, in_bs, scale, only_flagged, seqs, st);
+      default: return GDN2_ERR_BAD_DTYPE;
+    }
+  }
+  if (dtype != GDN2_BF16) return GDN2_ERR_UNSUPPORTED;
+  return launch_typed<bf16, bf16>(q, k, v, g, b, w, L, P, B, S, H, HK, in_bs, scale, only_flagged, seqs, st);
 }
 
 }  // namespace
@@ -393,16 +421,13 @@ int launch_typed(const void* q, const void* k, const void* v, const float* g, co
 int launch_prep_simt(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
                      const WsLayout& L, const WsPtrs& P, int B, int S, int H, int HK, int64_t in_bs, float scale,
                      int dtype, bool only_flagged, cudaStream_t st) {
-  if (L.esz == 4) {
-    switch (dtype) {
-      case GDN2_F32: return launch_typed<float, float>(q, k, v, g, b, w, L, P, B, S, H, HK, in_bs, scale, only_flagged, st);
-      case GDN2_BF16: return launch_typed<__nv_bfloat16, float>(q, k, v, g, b, w, L, P, B, S, H, HK, in_bs, scale, only_flagged, st);
-      case GDN2_F16: return launch_typed<__half, float>(q, k, v, g, b, w, L, P, B, S, H, HK, in_bs, scale, only_flagged, st);
-      default: return GDN2_ERR_BAD_DTYPE;
-    }
-  }
-  if (dtype != GDN2_BF16) return GDN2_ERR_UNSUPPORTED;
-  return launch_typed<__nv_bfloat16, __nv_bfloat16>(q, k, v, g, b, w, L, P, B, S, H, HK, in_bs, scale, only_flagged, st);
+  return launch_any(q, k, v, g, b, w, L, P, B, S, H, HK, in_bs, scale, dtype, only_flagged, OneLength{}, st);
+}
+
+int launch_prep_simt_packed(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
+                            const WsLayout& L, const WsPtrs& P, const PackedSeqs& seqs, int H, int HK, float scale,
+                            int dtype, bool only_flagged, cudaStream_t st) {
+  return launch_any(q, k, v, g, b, w, L, P, 1, seqs.chunk[seqs.n] * kChunk, H, HK, 0, scale, dtype, only_flagged, seqs, st);
 }
 
 }  // namespace gdn2

@@ -36,6 +36,8 @@
 //   X (72.5 KiB): MMA1 operands, then Tm + Ai + (w*v)^T;   Y (32.25 KiB): E^T, then the WQ staging.
 // Qg = scale*q*gamma is produced in step 1 but only needed in step 5; it waits in 32 spare TMEM
 // columns (packed bf16 pairs: the two channels of one token per word).
+#include <type_traits>
+
 #include "common.cuh"
 #include "tc_utils.cuh"
 
@@ -123,15 +125,26 @@ __device__ __forceinline__ float2 pick4(int j, float2 a0, float2 a1, float2 a2, 
 // HT > 0: the number of key heads is a compile-time constant (and RT > 0 the value heads per key head), so every
 // token offset of the strided channel loads folds into the load instruction's immediate; 0 takes them from the
 // arguments.
-template <int HT, int RT>
+template <int HT, int RT, typename Seqs>
 __global__ void __launch_bounds__(kThreads, 2)
 prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
                const __nv_bfloat16* __restrict__ v, const float* __restrict__ g,
                const __nv_bfloat16* __restrict__ b, const __nv_bfloat16* __restrict__ w, WsPtrs P, int S, int H,
-               int HK_arg, int64_t in_bs, float scale, int a_sm_count, uint32_t* status) {
+               int HK_arg, int64_t in_bs, float scale, int a_sm_count, uint32_t* status,
+               const __grid_constant__ Seqs seqs) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   PrepTcSmem& s = *reinterpret_cast<PrepTcSmem*>(smem_raw);
+  constexpr bool kPacked = std::is_same<Seqs, PackedSeqs>::value;
   const int NC = S / BS;
+  // first token of chunk x of the row (packed sequences: the chunks of all of them in one row of records)
+  auto chunk_token = [&](int x) {
+    if constexpr (kPacked) {
+      const int i = packed_find(seqs.n, x, [&](int y) { return seqs.chunk[y]; });
+      return (size_t)(seqs.tok[i] + (x - seqs.chunk[i]) * BS);
+    } else {
+      return (size_t)x * BS;
+    }
+  };
   const int HK = HT > 0 ? HT : HK_arg;                                  // key heads
   const int rep = RT > 0 ? RT : H / HK;                                 // value heads per key head
   const int n = blockIdx.x, bh = blockIdx.y;                            // bh: (batch, key head)
@@ -145,12 +158,13 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
   const int cp = tid & 63;                                              // channels 2 cp, 2 cp + 1
   const int sbk = tid >> 6;
   const int c0 = 2 * cp;
-  const size_t row0 = ((size_t)ib * in_bs + (size_t)n * BS) * HK + ih;  // q, k, b, g: token row of t = 0
+  const size_t tok_n = (size_t)ib * in_bs + chunk_token(n);
+  const size_t row0 = tok_n * HK + ih;  // q, k, b, g: token row of t = 0
   const size_t rstride = (size_t)HK * D;                                // ... and elements between tokens
   const size_t pstride = rstride / 2;                                   // channel pairs between tokens
   const size_t soff = (size_t)(16 * sbk) * rstride;                     // first token of this thread's sub-block
   // v, w: the same for the first value head of this key head (the others follow at +D elements each)
-  const size_t vrow0 = ((size_t)ib * in_bs + (size_t)n * BS) * HK * rep + (size_t)ih * rep;
+  const size_t vrow0 = tok_n * HK * rep + (size_t)ih * rep;
   const size_t vstride = rstride * rep, vpstride = vstride / 2;
   const size_t vsoff = (size_t)(16 * sbk) * vstride;
   const float2* gp = reinterpret_cast<const float2*>(g + row0 * D + soff) + cp;
@@ -336,7 +350,7 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
     const int64_t nxt = (int64_t)blockIdx.y * gridDim.x + blockIdx.x + 2 * (int64_t)a_sm_count;
     if (nxt < (int64_t)gridDim.x * gridDim.y) {
       const int nb_ = (int)(nxt / gridDim.x), nn_ = (int)(nxt % gridDim.x);
-      const size_t r0n = ((size_t)(nb_ / HK) * in_bs + (size_t)nn_ * BS) * HK + (nb_ % HK);
+      const size_t r0n = ((size_t)(nb_ / HK) * in_bs + chunk_token(nn_)) * HK + (nb_ % HK);
       const char* ptr = reinterpret_cast<const char*>(g + r0n * D + (size_t)(tid >> 2) * rstride) + (tid & 3) * 128;
       asm volatile("prefetch.global.L2 [%0];" ::"l"(ptr));
     }
@@ -654,9 +668,11 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
 
 }  // namespace
 
-int launch_prep_tc(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
-                   const WsLayout& L, const WsPtrs& P, int B, int S, int H, int HK, int64_t in_bs, float scale,
-                   cudaStream_t st) {
+namespace {
+template <typename Seqs>
+int launch_any(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
+               const WsLayout& L, const WsPtrs& P, int B, int S, int H, int HK, int64_t in_bs, float scale, const Seqs& seqs,
+               cudaStream_t st) {
   if (L.DK != D || L.DV != D || L.esz != 2) return GDN2_ERR_UNSUPPORTED;
   const size_t smem = sizeof(PrepTcSmem) + 128;
   dim3 grid(S / BS, B * HK);
@@ -667,30 +683,43 @@ int launch_prep_tc(const void* q, const void* k, const void* v, const float* g, 
     kern<<<grid, kThreads, smem, st>>>(static_cast<const bf16*>(q), static_cast<const bf16*>(k),
                                        static_cast<const bf16*>(v), g, static_cast<const bf16*>(b),
                                        static_cast<const bf16*>(w), P, S, H, HK, in_bs, scale, device_sm_count(),
-                                       device_status_word());
+                                       device_status_word(), seqs);
     GDN2_CUDA_TRY(cudaGetLastError());
     return GDN2_OK;
   };
   const int rep = H / HK;
   if (rep == 1) {
     switch (HK) {                               // common head counts, whole and sharded
-      case 16: return launch(prep_tc_kernel<16, 1>);
-      case 8: return launch(prep_tc_kernel<8, 1>);
-      case 4: return launch(prep_tc_kernel<4, 1>);
-      case 2: return launch(prep_tc_kernel<2, 1>);
-      default: return launch(prep_tc_kernel<0, 1>);
+      case 16: return launch(prep_tc_kernel<16, 1, Seqs>);
+      case 8: return launch(prep_tc_kernel<8, 1, Seqs>);
+      case 4: return launch(prep_tc_kernel<4, 1, Seqs>);
+      case 2: return launch(prep_tc_kernel<2, 1, Seqs>);
+      default: return launch(prep_tc_kernel<0, 1, Seqs>);
     }
   }
   if (rep == 2) {                               // two value heads per key head, whole and sharded
     switch (HK) {
-      case 8: return launch(prep_tc_kernel<8, 2>);
-      case 4: return launch(prep_tc_kernel<4, 2>);
-      case 2: return launch(prep_tc_kernel<2, 2>);
-      case 1: return launch(prep_tc_kernel<1, 2>);
+      case 8: return launch(prep_tc_kernel<8, 2, Seqs>);
+      case 4: return launch(prep_tc_kernel<4, 2, Seqs>);
+      case 2: return launch(prep_tc_kernel<2, 2, Seqs>);
+      case 1: return launch(prep_tc_kernel<1, 2, Seqs>);
       default: break;
     }
   }
-  return launch(prep_tc_kernel<0, 0>);
+  return launch(prep_tc_kernel<0, 0, Seqs>);
+}
+}  // namespace
+
+int launch_prep_tc(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
+                   const WsLayout& L, const WsPtrs& P, int B, int S, int H, int HK, int64_t in_bs, float scale,
+                   cudaStream_t st) {
+  return launch_any(q, k, v, g, b, w, L, P, B, S, H, HK, in_bs, scale, OneLength{}, st);
+}
+
+int launch_prep_tc_packed(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
+                          const WsLayout& L, const WsPtrs& P, const PackedSeqs& seqs, int H, int HK, float scale,
+                          cudaStream_t st) {
+  return launch_any(q, k, v, g, b, w, L, P, 1, seqs.chunk[seqs.n] * BS, H, HK, 0, scale, seqs, st);
 }
 
 }  // namespace gdn2

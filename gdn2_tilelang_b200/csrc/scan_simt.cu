@@ -9,11 +9,12 @@
 // columns never meet, so a head is spread over tiles of 8 of them while SMs are free (16 and 32 beyond that: the
 // records are read once per tile). The records arrive by bulk copies in the layout they are stored in, each one
 // refilled for the next chunk as soon as its last reader is through, and the two halves of the block form the output
-// rows and the new state at the same time: two barriers per chunk. Measured
-// with the chunk-local stage (prep_simt.cu), B = 2, S = 1000, 8 heads of 64, float32: the call took 501 us, now 80.
+// rows and the new state at the same time: two barriers per chunk. MEASURED_SCAN
 //
 // Output: one block per (value tile, chunk, batch*head) doing the first two lines from a stored
 // chunk state (output_kernel, gdn2/forward.py:710-725).
+#include <type_traits>
+
 #include "common.cuh"
 #include "tc_utils.cuh"
 
@@ -130,15 +131,16 @@ template <int NVT> struct ScanTile {
   }
 };
 
-// S tokens per batch entry, NC = ceil(S / 64): the rows past the end are not written (the chunk-local stage has made
+// S tokens per batch entry, ceil(S / 64) chunks: the rows past the end are not written (the chunk-local stage has made
 // them neutral). Threads: tid & 127 = row of the W | Qg image, tid >> 7 = half of the tile's columns. The W rows' threads
 // go on to the state update (row & 63 = key channel, two of them when DK > 64), the Qg rows' threads to the output.
-template <typename TOut, int NVT>
+template <typename TOut, int NVT, typename Seqs>
 __global__ void __launch_bounds__(256, 1)
 scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __restrict__ o,
-                 float* __restrict__ sT, float* __restrict__ hs, int S, int H, int64_t o_bs, uint32_t* status) {
+                 float* __restrict__ sT, float* __restrict__ hs, int S, int H, int64_t o_bs, uint32_t* status,
+                 const __grid_constant__ Seqs seqs) {
   constexpr int CT = NVT / 2;                             // columns per thread
-  const int DK = L.DK, DV = L.DV, NC = (S + kChunk - 1) / kChunk;
+  const int DK = L.DK, DV = L.DV;
   const int bh = blockIdx.x, ib = bh / H, ih = bh % H;
   const int lo = blockIdx.y * NVT, nv = min(NVT, DV - lo);
   const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
@@ -149,12 +151,28 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
   __shared__ uint64_t bar_wq, bar_ut, bar_aqk, bar_kgt;
   __shared__ int abort_flag;
 
-  const int64_t bk = (int64_t)ib * (H / L.rep) + ih / L.rep;       // (batch, key head) whose records this value head reads
-  const char* g_wq = P.wq + (size_t)(bk * NC) * L.wq_bytes;
-  const char* g_aqk = P.aqk + (size_t)(bk * NC) * L.aqk_bytes;
-  const char* g_kgt = P.kgt + (size_t)(bk * NC) * L.kgt_bytes;
-  const char* g_ut = P.ut + (size_t)((int64_t)bh * NC) * L.ut_bytes + (size_t)lo * 16;
-  const float* g_gl = P.gl + (size_t)(bk * NC) * DK;
+  // this block's run of chunks: how many, its records (those of its key head, and U of its value head), its first
+  // output row and its number of tokens. With packed sequences `ib` is the sequence and there is one row of records.
+  int NC, len;
+  int64_t ch0, chv0, o_row0;
+  if constexpr (std::is_same<Seqs, PackedSeqs>::value) {
+    NC = seqs.chunk[ib + 1] - seqs.chunk[ib];
+    len = seqs.tok[ib + 1] - seqs.tok[ib];
+    ch0 = (int64_t)(ih / L.rep) * seqs.chunk[seqs.n] + seqs.chunk[ib];
+    chv0 = (int64_t)ih * seqs.chunk[seqs.n] + seqs.chunk[ib];
+    o_row0 = seqs.tok[ib];
+  } else {
+    NC = (S + kChunk - 1) / kChunk;
+    len = S;
+    ch0 = ((int64_t)ib * (H / L.rep) + ih / L.rep) * NC;
+    chv0 = (int64_t)bh * NC;
+    o_row0 = (int64_t)ib * o_bs;
+  }
+  const char* g_wq = P.wq + (size_t)ch0 * L.wq_bytes;
+  const char* g_aqk = P.aqk + (size_t)ch0 * L.aqk_bytes;
+  const char* g_kgt = P.kgt + (size_t)ch0 * L.kgt_bytes;
+  const char* g_ut = P.ut + (size_t)chv0 * L.ut_bytes + (size_t)lo * 16;
+  const float* g_gl = P.gl + (size_t)ch0 * DK;
 
   // copies of chunk n, issued by the first warp (the 16 column pieces of U by its first 16 lanes)
   auto load_wq_ut = [&](int n) {
@@ -190,7 +208,7 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
     for (int idx = tid; idx < kChunk * NVT; idx += 256) s.ut[idx] = 0.f;
   tc::fence_async_smem();
   __syncthreads();
-  if (wid == 0) { load_wq_ut(0); load_aqk_kgt(0); }
+  if (wid == 0 && NC > 0) { load_wq_ut(0); load_aqk_kgt(0); }
 
   float2 acc[CT / 2];
   for (int n = 0; n < NC; ++n) {
@@ -246,8 +264,8 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
         }
       }
       const int t = n * kChunk + r;
-      if (t < S) {
-        TOut* op = o + (((size_t)ib * o_bs + t) * H + ih) * DV + lo + col0;
+      if (t < len) {
+        TOut* op = o + ((size_t)(o_row0 + t) * H + ih) * DV + lo + col0;
 #pragma unroll
         for (int x = 0; x < CT / 2; ++x) {
           if (col0 + 2 * x < nv) {                         // nv is a multiple of 4
@@ -311,22 +329,22 @@ output_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ hs, TOut* __r
   un_and_output<TOut>(s, DK, DV, lo, o_rows, (size_t)H * DV);
 }
 
-template <typename TOut>
+template <typename TOut, typename Seqs>
 int launch_scan_typed(const WsLayout& L, const WsPtrs& P, const float* s0, void* o, float* sT, float* hs,
-                      int B, int S, int H, int64_t o_bs, cudaStream_t st) {
+                      int B, int S, int H, int64_t o_bs, const Seqs& seqs, cudaStream_t st) {
   const int BH = B * H, sms = device_sm_count();
   auto launch = [&](auto kern, int nvt, size_t smem) -> int {
     GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
     kern<<<dim3(BH, (L.DV + nvt - 1) / nvt), 256, smem, st>>>(L, P, s0, static_cast<TOut*>(o), sT, hs, S, H, o_bs,
-                                                              device_status_word());
+                                                              device_status_word(), seqs);
     GDN2_CUDA_TRY(cudaGetLastError());
     return GDN2_OK;
   };
   // the narrowest tile whose blocks all run at once (two per SM while the records of DK <= 64 leave room)
   const int64_t room = L.DK <= 64 ? 2 * sms : sms;
-  if ((int64_t)BH * ((L.DV + 7) / 8) <= room) return launch(scan_simt_kernel<TOut, 8>, 8, ScanTile<8>::bytes(L.DK));
-  if ((int64_t)BH * ((L.DV + 15) / 16) <= room) return launch(scan_simt_kernel<TOut, 16>, 16, ScanTile<16>::bytes(L.DK));
-  return launch(scan_simt_kernel<TOut, 32>, 32, ScanTile<32>::bytes(L.DK));
+  if ((int64_t)BH * ((L.DV + 7) / 8) <= room) return launch(scan_simt_kernel<TOut, 8, Seqs>, 8, ScanTile<8>::bytes(L.DK));
+  if ((int64_t)BH * ((L.DV + 15) / 16) <= room) return launch(scan_simt_kernel<TOut, 16, Seqs>, 16, ScanTile<16>::bytes(L.DK));
+  return launch(scan_simt_kernel<TOut, 32, Seqs>, 32, ScanTile<32>::bytes(L.DK));
 }
 
 template <typename TOut, typename TW>
@@ -341,17 +359,28 @@ int launch_output_typed(const WsLayout& L, const WsPtrs& P, const float* hs, voi
   return GDN2_OK;
 }
 
+template <typename Seqs>
+int launch_scan_any(const WsLayout& L, const WsPtrs& P, const float* s0, void* o, float* sT, float* hs,
+                    int B, int S, int H, int64_t o_bs, int dtype, const Seqs& seqs, cudaStream_t st) {
+  if (L.esz != 4) return GDN2_ERR_UNSUPPORTED;   // 16-bit records belong to the tensor-core family's kernels
+  switch (dtype) {
+    case GDN2_F32: return launch_scan_typed<float>(L, P, s0, o, sT, hs, B, S, H, o_bs, seqs, st);
+    case GDN2_BF16: return launch_scan_typed<__nv_bfloat16>(L, P, s0, o, sT, hs, B, S, H, o_bs, seqs, st);
+    case GDN2_F16: return launch_scan_typed<__half>(L, P, s0, o, sT, hs, B, S, H, o_bs, seqs, st);
+    default: return GDN2_ERR_BAD_DTYPE;
+  }
+}
+
 }  // namespace
 
 int launch_scan_simt(const WsLayout& L, const WsPtrs& P, const float* s0, void* o, float* sT, float* hs,
                      int B, int S, int H, int64_t o_bs, int dtype, cudaStream_t st) {
-  if (L.esz != 4) return GDN2_ERR_UNSUPPORTED;   // 16-bit records belong to the tensor-core family's kernels
-  switch (dtype) {
-    case GDN2_F32: return launch_scan_typed<float>(L, P, s0, o, sT, hs, B, S, H, o_bs, st);
-    case GDN2_BF16: return launch_scan_typed<__nv_bfloat16>(L, P, s0, o, sT, hs, B, S, H, o_bs, st);
-    case GDN2_F16: return launch_scan_typed<__half>(L, P, s0, o, sT, hs, B, S, H, o_bs, st);
-    default: return GDN2_ERR_BAD_DTYPE;
-  }
+  return launch_scan_any(L, P, s0, o, sT, hs, B, S, H, o_bs, dtype, OneLength{}, st);
+}
+
+int launch_scan_simt_packed(const WsLayout& L, const WsPtrs& P, const PackedSeqs& seqs, const float* s0, void* o,
+                            float* sT, int H, int dtype, cudaStream_t st) {
+  return launch_scan_any(L, P, s0, o, sT, nullptr, seqs.n, 0, H, 0, dtype, seqs, st);
 }
 
 int launch_output_simt(const WsLayout& L, const WsPtrs& P, const float* hs, void* o, int B, int S, int H,

@@ -49,6 +49,8 @@
 // a few chunks.
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "tc_utils.cuh"
 
@@ -208,64 +210,101 @@ __device__ __noinline__ void store_rows_normed(const __nv_bfloat16* ostage, __nv
   }
 }
 
+template <typename Seqs>
 __global__ void __launch_bounds__(kThreads, 1)
 scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* __restrict__ s0,
                __nv_bfloat16* __restrict__ o, float* __restrict__ sT, float* __restrict__ hs, int S, int H, int64_t o_bs,
-               uint32_t* status) {
+               uint32_t* status, const __grid_constant__ Seqs seqs) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   ScanTcSmem& s = *reinterpret_cast<ScanTcSmem*>(smem_raw);
-  const int NC_all = S / BS;
+  constexpr bool kPacked = std::is_same<Seqs, PackedSeqs>::value;
   const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
 
   // ---- this block's job: which (batch, head), which run of chunks, where the state comes from and goes to
-  const int BH = (int)L.BH;
-  int bh = blockIdx.x, seg = 0;
   bool transition = false;                  // identity start, no U, no outputs: yields the segment's transition matrix
-  if (plan.pass != kWhole) {
-    const int slot = blockIdx.x / BH;
-    bh = blockIdx.x % BH;
-    if (plan.pass == kFirst) {
-      transition = slot < plan.nseg - 1;
-      seg = transition ? slot + 1 : slot - (plan.nseg - 1);
-    } else if (plan.pass == kRedo) {
-      seg = slot + 1;
-    } else {
-      seg = slot;
-    }
-  }
   const bool output_only = plan.pass == kOutput;
-  if (plan.guarded && *P.seg_mode != 0) {                  // slow decay: no cut after all (uniform over the launch)
-    if (plan.pass != kFirst || transition || seg != 0) return;
-    plan.pass = kWhole;
+  int bh, ib, ih, seg = 0;                  // (batch entry or packed sequence, head) and segment
+  int NC_all, c_first, NC;                  // chunks per row of records; first chunk and number of chunks of this block
+  int64_t ch0, chv0, o_row0;                // first record of the key head and of the value head; first output row
+  if constexpr (kPacked) {
+    // slot -> segment, over all segments or (transition blocks, correction pass) over those with a predecessor
+    const int slot = blockIdx.x / H;
+    ih = blockIdx.x % H;
+    const int later_total = seqs.seg[seqs.n] - seqs.n;
+    transition = plan.pass == kFirst && slot < later_total;
+    const int later = transition || plan.pass == kRedo ? 1 : 0;
+    const int x = plan.pass == kFirst && !transition ? slot - later_total : slot;
+    ib = packed_find(seqs.n, x, [&](int y) { return seqs.seg[y] - later * y; });
+    seg = x - (seqs.seg[ib] - later * ib) + later;
+    bh = ib * H + ih;
+    const int nseg = seqs.seg[ib + 1] - seqs.seg[ib], len = seqs.chunk[ib + 1] - seqs.chunk[ib];
+    NC_all = seqs.chunk[seqs.n];
+    c_first = len * seg / nseg;
+    NC = len * (seg + 1) / nseg - c_first;
+    ch0 = (int64_t)(ih / L.rep) * NC_all + seqs.chunk[ib] + c_first;
+    chv0 = (int64_t)ih * NC_all + seqs.chunk[ib] + c_first;
+    o_row0 = seqs.tok[ib] + c_first * BS;
+  } else {
+    const int BH = (int)L.BH;
+    bh = blockIdx.x;
+    NC_all = S / BS;
+    if (plan.pass != kWhole) {
+      const int slot = blockIdx.x / BH;
+      bh = blockIdx.x % BH;
+      if (plan.pass == kFirst) {
+        transition = slot < plan.nseg - 1;
+        seg = transition ? slot + 1 : slot - (plan.nseg - 1);
+      } else if (plan.pass == kRedo) {
+        seg = slot + 1;
+      } else {
+        seg = slot;
+      }
+    }
+    if (plan.guarded && *P.seg_mode != 0) {                // slow decay: no cut after all (uniform over the launch)
+      if (plan.pass != kFirst || transition || seg != 0) return;
+      plan.pass = kWhole;
+    }
+    ib = bh / H; ih = bh % H;
+    c_first = plan.pass == kWhole ? 0 : (int)((int64_t)NC_all * seg / plan.nseg);
+    NC = (plan.pass == kWhole ? NC_all : (int)((int64_t)NC_all * (seg + 1) / plan.nseg)) - c_first;
+    // records that depend on q, k, b, g only exist once per KEY head; U^T per value head
+    ch0 = ((int64_t)ib * (H / L.rep) + ih / L.rep) * NC_all + c_first;
+    chv0 = (int64_t)bh * NC_all + c_first;
+    o_row0 = (int64_t)ib * o_bs + (int64_t)c_first * BS;
   }
-  const int ib = bh / H, ih = bh % H;
-  const int c_first = plan.pass == kWhole ? 0 : (int)((int64_t)NC_all * seg / plan.nseg);
-  const int c_end = plan.pass == kWhole ? NC_all : (int)((int64_t)NC_all * (seg + 1) / plan.nseg);
-  int NC = c_end - c_first;                 // chunks this block walks
+  auto segment_record = [&]() -> size_t {
+    if constexpr (kPacked) return (size_t)(seqs.seg[ib] + seg) * H + ih;
+    else return (size_t)bh * plan.nseg + seg;
+  };
   if (plan.pass == kRedo) {
-    const int redo = P.seg_stop[bh * plan.nseg + seg];
+    const int redo = P.seg_stop[segment_record()];
     NC = redo < NC ? redo : NC;
   }
   if (plan.pass == kFirst || plan.pass == kRedo) hs = nullptr;
   // where the state comes from (nullptr = zero, or the identity for a transition block) and where it goes;
   // evaluated where they are used so that they do not occupy registers across the chunk loop
   auto state_source = [&]() -> const float* {
-    const size_t seg_rec = ((size_t)bh * plan.nseg + seg) * D * D;
+    const size_t seg_rec = segment_record() * D * D;
     if (plan.pass == kRedo) return P.seg_in + seg_rec;
     if (plan.pass == kFirst && seg != 0) return nullptr;
     if (output_only) return hs + (((size_t)ib * NC_all + c_first) * H + ih) * D * D;
     return s0 ? s0 + (size_t)bh * D * D : nullptr;
   };
   auto state_sink = [&]() -> float* {
-    const size_t seg_rec = ((size_t)bh * plan.nseg + seg) * D * D;
+    const size_t seg_rec = segment_record() * D * D;
     if (plan.pass == kRedo || output_only) return nullptr;
     if (plan.pass == kFirst) return (transition ? P.seg_t : P.seg_c) + seg_rec;
     return sT ? sT + (size_t)bh * D * D : nullptr;
   };
   const bool write_o = !transition;
-  // records that depend on q, k, b, g only exist once per KEY head; U^T per value head
-  const int64_t ch0 = ((int64_t)ib * (H / L.rep) + ih / L.rep) * NC_all + c_first;
-  const int64_t chv0 = (int64_t)bh * NC_all + c_first;
+  if constexpr (kPacked) {
+    if (NC == 0) {                          // a sequence without a whole chunk: its state passes through
+      const float* src = state_source();
+      float* dst = state_sink();
+      for (int i = tid; dst && i < D * D; i += kThreads) dst[i] = src ? src[i] : 0.f;
+      return;
+    }
+  }
 
   const char* g_wq = P.wq + (size_t)ch0 * kWqBytes;
   const char* g_aqk = P.aqk + (size_t)ch0 * kAqkBytes;
@@ -412,7 +451,7 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
       output_sync();
       if (write_o && !s.abort_flag) {
         // 64 rows x 256 bytes = 1024 16-byte pieces, 8 per thread, 128-bit coalesced stores
-        __nv_bfloat16* obase = o + (((size_t)ib * o_bs + (size_t)(c_first + n) * BS) * H + ih) * D;
+        __nv_bfloat16* obase = o + ((size_t)(o_row0 + (int64_t)n * BS) * H + ih) * D;
         if (norm.gate == nullptr) {
 #pragma unroll
           for (int x = 0; x < 8; ++x) {
@@ -589,7 +628,7 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
     int last = -1;
     for (int i = 0; i < kComputeThreads / 32; ++i) last = s.last_big[i] > last ? s.last_big[i] : last;
     const int redo = last + 2;                               // < NC whenever the block stopped early: then no matrix was stored
-    P.seg_stop[bh * plan.nseg + seg] = redo < NC ? redo : NC;
+    P.seg_stop[segment_record()] = redo < NC ? redo : NC;
   }
 }
 
@@ -622,15 +661,26 @@ scan_mode_kernel(WsPtrs P, int BK, int nseg, int NC_all) {
 // columns evolve independently, so the slices need no exchange.
 constexpr int kCombineCols = 16;
 constexpr int kTPad = D + 1;
+template <typename Seqs>
 __global__ void __launch_bounds__(256)
-scan_combine_kernel(WsPtrs P, int nseg, int NC_all, int guarded, float* __restrict__ sT) {
+scan_combine_kernel(WsPtrs P, int nseg, int NC_all, int guarded, float* __restrict__ sT, int H,
+                    const __grid_constant__ Seqs seqs) {
   extern __shared__ __align__(16) float csm[];
   if (guarded && *P.seg_mode != 0) return;                 // the first pass walked the whole sequences itself
   float* Ts = csm;                         // [128][129] transition matrix of the current segment
   float* Ss = csm + D * kTPad;             // [128][16] current state slice
   const int bh = blockIdx.x, col0 = blockIdx.y * kCombineCols;
   const int tid = threadIdx.x, r = tid & (D - 1), cg = tid >> 7;      // row, 8-column group
-  const size_t rec0 = (size_t)bh * nseg * D * D;
+  // record of segment j: unpacked, the segments of a (batch, head) lie together; packed, the heads of a segment do
+  size_t first = (size_t)bh * nseg, step = 1;
+  if constexpr (std::is_same<Seqs, PackedSeqs>::value) {
+    const int ib = bh / H;
+    nseg = seqs.seg[ib + 1] - seqs.seg[ib];
+    NC_all = seqs.chunk[ib + 1] - seqs.chunk[ib];
+    first = (size_t)seqs.seg[ib] * H + bh % H;
+    step = H;
+  }
+  const size_t rec0 = first * D * D;
   float acc[8];
   {
     const float* c0p = P.seg_c + rec0 + (size_t)r * D + col0 + 8 * cg;
@@ -638,12 +688,12 @@ scan_combine_kernel(WsPtrs P, int nseg, int NC_all, int guarded, float* __restri
     acc[0] = a.x; acc[1] = a.y; acc[2] = a.z; acc[3] = a.w; acc[4] = b.x; acc[5] = b.y; acc[6] = b.z; acc[7] = b.w;
   }
   for (int j = 1; j < nseg; ++j) {
-    const size_t rec = rec0 + (size_t)j * D * D;
+    const size_t rec = rec0 + (size_t)j * step * D * D;
     float* inp = P.seg_in + rec + (size_t)r * D + col0 + 8 * cg;
     *reinterpret_cast<float4*>(inp) = make_float4(acc[0], acc[1], acc[2], acc[3]);
     *reinterpret_cast<float4*>(inp + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
     const int len = (int)((int64_t)NC_all * (j + 1) / nseg) - (int)((int64_t)NC_all * j / nseg);
-    const bool vanished = P.seg_stop[bh * nseg + j] < len;             // uniform over the block
+    const bool vanished = P.seg_stop[first + j * step] < len;             // uniform over the block
     const float* cp = P.seg_c + rec + (size_t)r * D + col0 + 8 * cg;
     const float4 ca = *reinterpret_cast<const float4*>(cp), cb = *reinterpret_cast<const float4*>(cp + 4);
     if (vanished) {
@@ -685,7 +735,7 @@ int launch_scan_tc(const WsLayout& L, const WsPtrs& P, const float* s0, void* o,
                    int B, int S, int H, int64_t o_bs, const gdn2_gated_norm* gn, int part, cudaStream_t st) {
   if (L.DK != D || L.DV != D || L.esz != 2) return GDN2_ERR_UNSUPPORTED;
   const size_t smem = sizeof(ScanTcSmem) + 128;
-  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(scan_tc_kernel), smem));
+  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(scan_tc_kernel<OneLength>), smem));
   __nv_bfloat16* ob = static_cast<__nv_bfloat16*>(o);
   uint32_t* status = device_status_word();
   const int BH = B * H, NC = S / BS;
@@ -696,14 +746,14 @@ int launch_scan_tc(const WsLayout& L, const WsPtrs& P, const float* s0, void* o,
   const int nseg = hs ? 1 : L.nseg;
   if (nseg <= 1) {
     if (part == 2) return GDN2_OK;
-    scan_tc_kernel<<<BH, kThreads, smem, st>>>(L, P, ScanPlan{kWhole, 1, 0}, norm, s0, ob, sT, hs, S, H, o_bs, status);
+    scan_tc_kernel<OneLength><<<BH, kThreads, smem, st>>>(L, P, ScanPlan{kWhole, 1, 0}, norm, s0, ob, sT, hs, S, H, o_bs, status, OneLength{});
     GDN2_CUDA_TRY(cudaGetLastError());
     return GDN2_OK;
   }
   const int guarded = L.nseg_guarded ? 1 : 0;
   if (part == 2) {
-    scan_tc_kernel<<<BH * (nseg - 1), kThreads, smem, st>>>(L, P, ScanPlan{kRedo, nseg, guarded}, norm, nullptr, ob, nullptr, nullptr,
-                                                           S, H, o_bs, status);
+    scan_tc_kernel<OneLength><<<BH * (nseg - 1), kThreads, smem, st>>>(L, P, ScanPlan{kRedo, nseg, guarded}, norm, nullptr, ob, nullptr, nullptr,
+                                                           S, H, o_bs, status, OneLength{});
     GDN2_CUDA_TRY(cudaGetLastError());
     return GDN2_OK;
   }
@@ -713,18 +763,43 @@ int launch_scan_tc(const WsLayout& L, const WsPtrs& P, const float* s0, void* o,
     scan_mode_kernel<<<(BK * (nseg - 1) + 7) / 8, 256, 0, st>>>(P, BK, nseg, NC);
     GDN2_CUDA_TRY(cudaGetLastError());
   }
-  scan_tc_kernel<<<BH * (2 * nseg - 1), kThreads, smem, st>>>(L, P, ScanPlan{kFirst, nseg, guarded}, norm, s0, ob, sT, nullptr,
-                                                             S, H, o_bs, status);
+  scan_tc_kernel<OneLength><<<BH * (2 * nseg - 1), kThreads, smem, st>>>(L, P, ScanPlan{kFirst, nseg, guarded}, norm, s0, ob, sT, nullptr,
+                                                             S, H, o_bs, status, OneLength{});
   GDN2_CUDA_TRY(cudaGetLastError());
   const size_t csmem = (size_t)(D * kTPad + D * kCombineCols) * sizeof(float);
-  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(scan_combine_kernel), csmem));
-  scan_combine_kernel<<<dim3(BH, D / kCombineCols), 256, csmem, st>>>(P, nseg, NC, guarded, sT);
+  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(scan_combine_kernel<OneLength>), csmem));
+  scan_combine_kernel<OneLength><<<dim3(BH, D / kCombineCols), 256, csmem, st>>>(P, nseg, NC, guarded, sT, H, OneLength{});
   GDN2_CUDA_TRY(cudaGetLastError());
   if (part == 1) return GDN2_OK;
-  scan_tc_kernel<<<BH * (nseg - 1), kThreads, smem, st>>>(L, P, ScanPlan{kRedo, nseg, guarded}, norm, nullptr, ob, nullptr, nullptr,
-                                                         S, H, o_bs, status);
+  scan_tc_kernel<OneLength><<<BH * (nseg - 1), kThreads, smem, st>>>(L, P, ScanPlan{kRedo, nseg, guarded}, norm, nullptr, ob, nullptr, nullptr,
+                                                         S, H, o_bs, status, OneLength{});
   GDN2_CUDA_TRY(cudaGetLastError());
   return GDN2_OK;
+}
+
+// Packed sequences: one block per (segment, head); seqs.seg holds the cut (one segment each = none).
+int launch_scan_tc_packed(const WsLayout& L, const WsPtrs& P, const PackedSeqs& seqs, const float* s0, void* o, float* sT,
+                          int H, cudaStream_t st) {
+  if (L.DK != D || L.DV != D || L.esz != 2) return GDN2_ERR_UNSUPPORTED;
+  const size_t smem = sizeof(ScanTcSmem) + 128;
+  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(scan_tc_kernel<PackedSeqs>), smem));
+  __nv_bfloat16* ob = static_cast<__nv_bfloat16*>(o);
+  const ScanNorm norm{nullptr, nullptr, 0, 0, 0.f};
+  const int total = seqs.seg[seqs.n], later = total - seqs.n;
+  auto pass = [&](int which, int blocks) -> int {
+    scan_tc_kernel<PackedSeqs><<<blocks, kThreads, smem, st>>>(L, P, ScanPlan{which, 0, 0}, norm, s0, ob, sT, nullptr, 0, H, 0,
+                                                               device_status_word(), seqs);
+    GDN2_CUDA_TRY(cudaGetLastError());
+    return GDN2_OK;
+  };
+  if (later == 0) return pass(kWhole, seqs.n * H);
+  int rc = pass(kFirst, (total + later) * H);
+  if (rc != GDN2_OK) return rc;
+  const size_t csmem = (size_t)(D * kTPad + D * kCombineCols) * sizeof(float);
+  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(scan_combine_kernel<PackedSeqs>), csmem));
+  scan_combine_kernel<PackedSeqs><<<dim3(seqs.n * H, D / kCombineCols), 256, csmem, st>>>(P, 1, 0, 0, sT, H, seqs);
+  GDN2_CUDA_TRY(cudaGetLastError());
+  return pass(kRedo, later * H);
 }
 
 // Chunk-parallel output from stored chunk states on the tensor-core family: the scan kernel's chunk body without
@@ -733,15 +808,15 @@ int launch_output_tc(const WsLayout& L, const WsPtrs& P, const float* hs, void* 
                      cudaStream_t st) {
   if (L.DK != D || L.DV != D || L.esz != 2) return GDN2_ERR_UNSUPPORTED;
   const size_t smem = sizeof(ScanTcSmem) + 128;
-  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(scan_tc_kernel), smem));
+  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(scan_tc_kernel<OneLength>), smem));
   const int BH = B * H, NC = S / BS;
   // enough runs to give every SM a few blocks, none shorter than 4 chunks
   int runs = (4 * device_sm_count() + BH - 1) / BH;
   if (runs > NC / 4) runs = NC / 4;
   if (runs < 1) runs = 1;
-  scan_tc_kernel<<<BH * runs, kThreads, smem, st>>>(L, P, ScanPlan{kOutput, runs, 0}, ScanNorm{nullptr, nullptr, 0, 0, 0.f}, nullptr,
+  scan_tc_kernel<OneLength><<<BH * runs, kThreads, smem, st>>>(L, P, ScanPlan{kOutput, runs, 0}, ScanNorm{nullptr, nullptr, 0, 0, 0.f}, nullptr,
                                                    static_cast<__nv_bfloat16*>(o),
-                                                   nullptr, const_cast<float*>(hs), S, H, o_bs, device_status_word());
+                                                   nullptr, const_cast<float*>(hs), S, H, o_bs, device_status_word(), OneLength{});
   GDN2_CUDA_TRY(cudaGetLastError());
   return GDN2_OK;
 }

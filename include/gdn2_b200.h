@@ -186,6 +186,23 @@ int gdn2_prefill_ragged(const void* q, const void* k, const void* v, const float
                         int64_t o_batch_stride, float scale, int dtype, int path, void* side_stream, void* stream);
 
 /*
+ * The functional op on N sequences packed along the token axis of one row (the cu_seqlens convention of the reference's
+ * signature, gdn2/attention.py:142-145, where it raises): one launch per stage for all of them.
+ *   q,k,b [T,HK,DK]  v,w,o [T,H,DV]  g [T,HK,DK] fp32, T = cu_seqlens[N]; dense, 16-byte aligned
+ *   cu_seqlens     N + 1 token offsets IN HOST MEMORY, rising from 0; sequences may be empty
+ *   initial_state  [N,H,DK,DV] fp32 or NULL (zero); final_state the same, always written, 16-byte aligned, not the
+ *                  same memory
+ *   workspace      gdn2_packed_workspace_bytes(...) bytes, 16-byte aligned (0 = unsupported combination)
+ * Every sequence gets what gdn2_prefill_ragged gives it alone, up to the rounding of where its scan is cut.
+ */
+size_t gdn2_packed_workspace_bytes(const int64_t* cu_seqlens, int64_t N, int64_t H, int64_t HK, int64_t DK, int64_t DV,
+                                   int dtype, int path);
+int gdn2_packed_forward(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
+                        const int64_t* cu_seqlens, int64_t N, const float* initial_state, void* o, float* final_state,
+                        void* workspace, size_t workspace_bytes, int64_t H, int64_t HK, int64_t DK, int64_t DV, float scale,
+                        int dtype, int path, void* stream);
+
+/*
  * gdn2_prefill_scan with the layer's gated RMSNorm as the epilogue of the output rows:
  *   o[b,t,h,:] <- o * rsqrt(mean(o^2) + eps) * weight * silu(gate[b,t,h,:]),
  * evaluated on the rows as they leave the chip (rounded to `dtype` first, as the separate kernel would read
