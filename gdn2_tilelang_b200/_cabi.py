@@ -437,7 +437,7 @@ class NativeKernels:
                 _check(self.lib, rc, "gdn2_prefill_scan")
                 state_ptr = states[i].data_ptr()
                 launched += (2 if p != PATH_SIMT else 1) + (
-                    1 if want_chunk_states else self.lib.gdn2_prefill_scan_launches(B, S_i, H, DK, DV, code, p))
+                    self.lib.gdn2_prefill_scan_launches(B, S_i, H, DK, DV, code, p))
             if side is not None:
                 main.wait_stream(side)             # from here on the caller's stream is ordered after every scan
             del scratch                            # ... so only now may the allocator hand these blocks out again
