@@ -114,6 +114,17 @@ def load_library(build_if_missing: bool = True) -> ctypes.CDLL:
         return lib
 
 
+def load_host():
+    """The host extension (``csrc/host/binding.cpp``), built in-tree first if it is missing."""
+    from . import build as _build
+
+    if not _build.HOST_LIB.exists():
+        _build.build_host()
+    from . import _gdn2_host
+
+    return _gdn2_host
+
+
 def dtype_code(dtype: torch.dtype) -> int:
     try:
         return _DTYPES[dtype]
@@ -178,6 +189,7 @@ class NativeKernels:
 
     def __init__(self):
         self.lib = load_library()
+        self.host = load_host()     # decode, prefill and the layer's decode in one native call, where the case is plain
         self.prefill_path = _PATHS[os.environ.get("GDN2_B200_PREFILL_PATH", "auto")]
         self.launches = 0   # kernels launched through this object (for the benchmark's accounting)
         self._side_streams = {}
@@ -246,6 +258,15 @@ class NativeKernels:
         _check(self.lib, rc, "gdn2_decode")
         self.launches += 1
         return o
+
+    def prefill_plain(self, q, k, v, g, b, w, scale, state):
+        """``gdn2_prefill_ragged`` through the host extension: ``(o, final_state)``, or ``None`` when the call is not plain."""
+        side = self._side_stream(q.device).cuda_stream if q.is_cuda and q.shape[1] % CHUNK else 0
+        res = self.host.prefill(q, k, v, g, b, w, scale, state, self.prefill_path, side)
+        if res is None:
+            return None
+        self.launches += res[2]
+        return res[0], res[1]
 
     # -- prefill in one call ---------------------------------------------------------------
     def prefill_ragged(self, q, k, v, g, b, w, scale: float, initial_state=None):

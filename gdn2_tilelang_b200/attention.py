@@ -143,6 +143,9 @@ class _GatedRMSNorm(nn.Module):
         self.weight = nn.Parameter(torch.ones(dim))
 
 
+_PROJECTIONS = ("q_proj", "k_proj", "v_proj", "b_proj", "w_proj", "f_proj", "o_gate_proj")
+
+
 class GatedDeltaNet2(nn.Module):
     """Gated DeltaNet-2 token mixer: projections, short convolution, L2-normalised q/k, the decay /
     erase / write gates, the recurrent attention kernels, gated RMSNorm and the output projection."""
@@ -185,14 +188,24 @@ class GatedDeltaNet2(nn.Module):
         self.erase_scale = config.erase_gate_scale
 
     # ------------------------------------------------------------------ pieces
+    def _table_parameters(self):
+        """The projection modules, the convolution modules and the parameters ``_fused_tables`` is made of."""
+        m = self._modules                                  # (plain dictionary look-ups: this runs on every one-token step)
+        lin = [m[n] for n in _PROJECTIONS]
+        convs = [] if m.get("q_conv") is None else [m[n]._modules["conv"] for n in ("q_conv", "k_conv", "v_conv")]
+        weights = [x._parameters.get("weight") for x in lin + convs]
+        if any(p is None for p in weights):                # parametrised modules compute their weight
+            weights = [x.weight for x in lin + convs]
+        return lin, convs, weights + [c.bias for c in convs if c.bias is not None]
+
     def _fused_tables(self):
         """Concatenated projection weight ``[NP, hidden]`` (q | k | v | b | w | f | o_gate), its column
         offsets, and the convolution weight ``[CC, K]`` / bias ``[CC]`` (q | k | v); rebuilt when a
         parameter changes."""
-        lin = (self.q_proj, self.k_proj, self.v_proj, self.b_proj, self.w_proj, self.f_proj, self.o_gate_proj)
-        convs = () if self.q_conv is None else (self.q_conv.conv, self.k_conv.conv, self.v_conv.conv)
-        params = [m.weight for m in lin] + [c.weight for c in convs] + [c.bias for c in convs if c.bias is not None]
-        key = tuple((p.data_ptr(), p._version, p.dtype) for p in params)
+        lin, convs, params = self._table_parameters()
+        host = getattr(_cabi.kernels(), "host", None)
+        key = (host.parameter_key(params) if host is not None
+               else tuple((p.data_ptr(), p._version, p.dtype) for p in params))
         if getattr(self, "_fused_key", None) != key:
             w_cat = torch.cat([m.weight for m in lin], 0).contiguous()
             sizes = [m.weight.shape[0] for m in lin]
@@ -273,6 +286,30 @@ class GatedDeltaNet2(nn.Module):
         """``o_proj``; the head-parallel variant overrides it to add the sum over ranks."""
         return self.o_proj(normed)
 
+    def _decode_plain(self, x, cache):
+        """The whole of ``decode`` as one native call, or ``None`` where something about the layer, the cache or the input
+        needs the general path (a subclass, hooks, a missing or converted convolution cache, strided tensors)."""
+        K = _cabi.kernels()
+        host = getattr(K, "host", None)
+        if host is None or type(self) is not GatedDeltaNet2 or cache.conv_state is None:
+            return None
+        m = self._modules
+        o_proj = m["o_proj"]
+        if (type(o_proj) is not nn.Linear or o_proj.bias is not None or o_proj._forward_hooks or o_proj._forward_pre_hooks
+                or any(m[n]._parameters.get("bias") is not None for n in _PROJECTIONS)):
+            return None
+        w_cat, offs, cw, cb = self._fused_tables()
+        own = self._parameters
+        res = host.layer_decode(x, cache.recurrent_state, cache.conv_state, w_cat, cw, cb, own["A_log"], own["dt_bias"],
+                                m["o_norm"].weight, o_proj.weight, offs, self.num_heads, self.num_kv_heads, self.head_dim_k,
+                                self.head_dim_v, self.cfg.conv_size, self.erase_scale, m["o_norm"].eps, self.scale)
+        if res is None:
+            return None
+        K.launches += 3
+        K.maybe_check_device_status(x.device)
+        out, cache.conv_state = res
+        return out
+
     # ------------------------------------------------------------------ public API
     @torch.no_grad()
     def forward(self, hidden_states, cache: GDN2Cache | None = None, use_cache: bool = False, cu_seqlens=None):
@@ -311,6 +348,9 @@ class GatedDeltaNet2(nn.Module):
     @torch.no_grad()
     def decode(self, hidden_states, cache: GDN2Cache):
         """Decode ``n`` tokens ``[B, n, hidden]``; ``cache.recurrent_state`` is updated in place."""
+        res = self._decode_plain(hidden_states, cache)
+        if res is not None:
+            return res, cache
         q, k, v, g, b, w, conv, proj = self._front(hidden_states, cache.conv_state, cached=self.q_conv is not None)
         if conv is not None:
             cache.conv_state = conv

@@ -1,0 +1,181 @@
+// The short calls' host path: argument checks, allocations and launches of one call without going back to Python in
+// between. A one-token decode is a few microseconds of device work, and the same sequence in Python (views, shape
+// comparisons, a 20-argument foreign call) took 34 us, a layer step of it 165 us.
+//
+// Every function takes the plain case only -- dense, aligned CUDA tensors of the expected shapes and types on the
+// current device -- and returns None for anything else, so that the general path in Python handles it or raises the
+// error that belongs to it. Nothing is kept between calls.
+#include <ATen/ATen.h>
+#include <ATen/core/grad_mode.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include "../../../include/gdn2_b200.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using Pair = std::tuple<Tensor, Tensor>;
+
+namespace {
+
+// a dense, 16-byte aligned tensor of this dtype on the current device, not wrapped by a transform or a subclass
+bool plain(const Tensor& t, at::ScalarType dt, c10::DeviceIndex dev) {
+  return t.defined() && t.is_cuda() && t.get_device() == dev && t.scalar_type() == dt && t.is_contiguous() &&
+         !t.is_conj() && !t.is_neg() && t.key_set().has(c10::DispatchKey::CUDA) && !t.key_set().has(c10::DispatchKey::Python) &&
+         !t.key_set().has(c10::DispatchKey::FuncTorchBatched) && !t.key_set().has(c10::DispatchKey::FuncTorchGradWrapper) &&
+         !t.key_set().has(c10::DispatchKey::Functionalize) && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0;
+}
+
+int dtype_code(at::ScalarType dt) {
+  return dt == at::kBFloat16 ? GDN2_BF16 : dt == at::kHalf ? GDN2_F16 : dt == at::kFloat ? GDN2_F32 : -1;
+}
+
+struct Problem {
+  int64_t B, S, H, HK, DK, DV;
+  int dtype;
+  at::ScalarType type;
+  c10::DeviceIndex dev;
+};
+
+// q, k, b, g [.., HK, DK] and v, w [.., H, DV] with `lead` leading dimensions (batch, and tokens when lead == 2)
+bool plain_tokens(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& b, const Tensor& w, Problem& p,
+                  int64_t lead) {
+  if (q.dim() != lead + 2 || v.dim() != lead + 2 || !q.is_cuda()) return false;
+  p.type = q.scalar_type();
+  p.dtype = dtype_code(p.type);
+  p.dev = c10::cuda::current_device();
+  if (p.dtype < 0 || !plain(q, p.type, p.dev) || !plain(k, p.type, p.dev) || !plain(v, p.type, p.dev) || !plain(b, p.type, p.dev) ||
+      !plain(w, p.type, p.dev) || !plain(g, at::kFloat, p.dev))
+    return false;
+  const auto qs = q.sizes(), vs = v.sizes();
+  if (k.sizes() != qs || b.sizes() != qs || g.sizes() != qs || w.sizes() != vs) return false;
+  p.B = qs[0];
+  p.S = lead == 2 ? qs[1] : 1;
+  if (vs[0] != p.B || (lead == 2 && vs[1] != p.S)) return false;
+  p.HK = qs[lead]; p.DK = qs[lead + 1];
+  p.H = vs[lead]; p.DV = vs[lead + 1];
+  return p.B > 0 && p.S > 0 && p.HK > 0 && p.DK > 0 && p.DV > 0 && p.H > 0 && p.H % p.HK == 0;
+}
+
+bool plain_state(const Tensor& s, const Problem& p) {
+  return plain(s, at::kFloat, p.dev) && s.dim() == 4 && s.size(0) == p.B && s.size(1) == p.H && s.size(2) == p.DK && s.size(3) == p.DV;
+}
+
+void* stream_of(const Problem& p) { return c10::cuda::getCurrentCUDAStream(p.dev).stream(); }
+
+// gdn2_decode ([B, n, H, D] tokens) and gdn2_decode_step ([B, H, D]); the state is updated in place. Returns o or None.
+std::optional<Tensor> decode(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& b, const Tensor& w,
+                  const Tensor& state, std::optional<double> scale) {
+  Problem p;
+  if (!plain_tokens(q, k, v, g, b, w, p, q.dim() == 3 ? 1 : 2) || !plain_state(state, p)) return std::nullopt;
+  Tensor o = at::empty(v.sizes(), v.options().requires_grad(false));
+  const float sc = scale ? (float)*scale : (float)(1.0 / std::sqrt((double)p.DK));
+  const int rc = gdn2_decode(q.data_ptr(), k.data_ptr(), v.data_ptr(), static_cast<const float*>(g.data_ptr()), b.data_ptr(),
+                             w.data_ptr(), static_cast<float*>(state.data_ptr()), o.data_ptr(), p.B, p.S, p.H, p.HK, p.DK, p.DV,
+                             p.S, p.S, sc, p.dtype, stream_of(p));
+  if (rc != GDN2_OK) return std::nullopt;
+  return o;
+}
+
+// gdn2_prefill_ragged. `side`: the second stream (0: none). Returns (o, final state, kernels launched) or None.
+std::optional<std::tuple<Tensor, Tensor, int64_t>> prefill(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& b, const Tensor& w,
+                   std::optional<double> scale, const std::optional<Tensor>& state, int path, uint64_t side) {
+  Problem p;
+  if (q.dim() != 4 || !plain_tokens(q, k, v, g, b, w, p, 2)) return std::nullopt;
+  if (state && !plain_state(*state, p)) return std::nullopt;
+  const int64_t n_full = p.S / 64 * 64;
+  if (n_full == 0) return std::nullopt;
+  if (path == GDN2_PATH_AUTO) path = p.DK == 128 && p.DV == 128 && p.dtype == GDN2_BF16 ? GDN2_PATH_TCGEN05 : GDN2_PATH_SIMT;
+  // the caller overlaps the stages of long, uncut problems segment by segment
+  if (path != GDN2_PATH_SIMT && n_full / 64 >= 32 && gdn2_prefill_scan_segments(p.B, n_full, p.H, p.DK, p.DV, p.dtype, path) <= 1)
+    return std::nullopt;
+  const size_t bytes = gdn2_prefill_ragged_workspace_bytes(p.B, p.S, p.H, p.HK, p.DK, p.DV, p.dtype, path);
+  if (bytes == 0) return std::nullopt;
+  const auto opt = v.options().requires_grad(false);
+  Tensor ws = at::empty({(int64_t)bytes}, opt.dtype(at::kByte));
+  Tensor o = at::empty(v.sizes(), opt);
+  Tensor fin = at::empty({p.B, p.H, p.DK, p.DV}, opt.dtype(at::kFloat));
+  const float sc = scale ? (float)*scale : (float)(1.0 / std::sqrt((double)p.DK));
+  const int rc = gdn2_prefill_ragged(
+      q.data_ptr(), k.data_ptr(), v.data_ptr(), static_cast<const float*>(g.data_ptr()), b.data_ptr(), w.data_ptr(),
+      state ? static_cast<const float*>(state->data_ptr()) : nullptr, o.data_ptr(), static_cast<float*>(fin.data_ptr()), ws.data_ptr(),
+      bytes, p.B, p.S, p.H, p.HK, p.DK, p.DV, p.S, p.S, sc, p.dtype, path, p.S > n_full ? reinterpret_cast<void*>(side) : nullptr,
+      stream_of(p));
+  if (rc != GDN2_OK) return std::nullopt;
+  const bool tc = path != GDN2_PATH_SIMT;
+  const int64_t launched = (tc ? 2 : 1) + gdn2_prefill_scan_launches(p.B, n_full, p.H, p.DK, p.DV, p.dtype, path) + (tc && p.S > n_full);
+  return std::make_tuple(o, fin, launched);
+}
+
+
+// GatedDeltaNet2.decode on x [B, n, hidden]: projections, layer_front, decode, layer_back, output projection. The recurrent
+// state is updated in place. Returns (out [B, n, hidden], new convolution cache) or None.
+std::optional<Pair> layer_decode(const Tensor& x, const Tensor& state, const std::optional<Tensor>& conv_state, const Tensor& w_cat,
+                        const std::optional<Tensor>& conv_w, const std::optional<Tensor>& conv_b, const Tensor& A_log,
+                        const Tensor& dt_bias, const Tensor& norm_w, const Tensor& o_w, const std::vector<int64_t>& offs, int64_t H,
+                        int64_t HK, int64_t DK, int64_t DV, int64_t K, double erase_scale, double eps, double scale) {
+  Problem p;
+  p.type = x.scalar_type();
+  p.dtype = dtype_code(p.type);
+  if (p.dtype < 0 || x.dim() != 3 || !x.is_cuda() || x.numel() == 0 || DK > 256 || DV > 256 || offs.size() != 7) return std::nullopt;
+  p.dev = c10::cuda::current_device();
+  p.B = x.size(0); p.S = x.size(1); p.H = H; p.HK = HK; p.DK = DK; p.DV = DV;
+  for (const Tensor* t : {&w_cat, &A_log, &dt_bias, &norm_w, &o_w})
+    if (!plain(*t, p.type, p.dev)) return std::nullopt;
+  if (!plain(x, p.type, p.dev) || !plain_state(state, p) || x.size(2) != w_cat.size(1)) return std::nullopt;
+  const int64_t CC = 2 * HK * DK + H * DV;
+  if (K < 2 || !conv_w || !plain(*conv_w, p.type, p.dev) || (conv_b && !plain(*conv_b, p.type, p.dev)) || !conv_state ||
+      !plain(*conv_state, p.type, p.dev) || conv_state->dim() != 3 || conv_state->size(0) != p.B || conv_state->size(1) != CC ||
+      conv_state->size(2) != K - 1)
+    return std::nullopt;
+  at::NoGradGuard no_grad;
+  Tensor proj = at::linear(x, w_cat);
+  if (proj.scalar_type() != p.type || !proj.is_contiguous()) return std::nullopt;       // an autocast region
+  const auto opt = x.options().requires_grad(false);
+  Tensor q = at::empty({p.B, p.S, HK, DK}, opt), k = at::empty({p.B, p.S, HK, DK}, opt), b = at::empty({p.B, p.S, HK, DK}, opt);
+  Tensor g = at::empty({p.B, p.S, HK, DK}, opt.dtype(at::kFloat));
+  Tensor v = at::empty({p.B, p.S, H, DV}, opt), w = at::empty({p.B, p.S, H, DV}, opt), o = at::empty({p.B, p.S, H, DV}, opt);
+  Tensor conv = at::empty({p.B, CC, K - 1}, opt), normed = at::empty({p.B, p.S, H * DV}, opt);
+  void* st = stream_of(p);
+  gdn2_layer_front_args a{};
+  a.proj = proj.data_ptr(); a.conv_state = conv_state->data_ptr(); a.conv_weight = conv_w->data_ptr();
+  a.conv_bias = conv_b ? conv_b->data_ptr() : nullptr;
+  a.A_log = A_log.data_ptr(); a.dt_bias = dt_bias.data_ptr();
+  a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.g = static_cast<float*>(g.data_ptr()); a.b = b.data_ptr();
+  a.w = w.data_ptr(); a.new_conv_state = conv.data_ptr();
+  a.B = p.B; a.S = p.S; a.H = H; a.HK = HK; a.DK = DK; a.DV = DV; a.K = K; a.NP = proj.size(2);
+  a.off_q = offs[0]; a.off_k = offs[1]; a.off_v = offs[2]; a.off_b = offs[3]; a.off_w = offs[4]; a.off_f = offs[5];
+  a.erase_scale = (float)erase_scale;
+  // up to the decode nothing of the cache has changed, so the general path can still take the call over
+  if (gdn2_layer_front(&a, p.dtype, st) != GDN2_OK) return std::nullopt;
+  if (gdn2_decode(q.data_ptr(), k.data_ptr(), v.data_ptr(), a.g, b.data_ptr(), w.data_ptr(), static_cast<float*>(state.data_ptr()),
+                  o.data_ptr(), p.B, p.S, H, HK, DK, DV, p.S, p.S, (float)scale, p.dtype, st) != GDN2_OK)
+    return std::nullopt;
+  const int rc = gdn2_layer_back(o.data_ptr(), proj.data_ptr(), norm_w.data_ptr(), normed.data_ptr(), p.B * p.S, H, DV,
+                                 proj.size(2), offs[6], (float)eps, p.dtype, st);
+  if (rc != GDN2_OK) throw std::runtime_error(std::string("gdn2_layer_back: ") + gdn2_status_string(rc));
+  return Pair{at::linear(normed, o_w), conv};
+}
+
+// The state of a list of parameters: where each lies, its version and its type. Equal bytes = nothing was replaced,
+// moved, converted or written to since.
+py::bytes parameter_key(const std::vector<Tensor>& params) {
+  std::string key;
+  for (const Tensor& t : params) {
+    const uint64_t rec[3] = {reinterpret_cast<uint64_t>(t.data_ptr()), (uint64_t)t._version(), (uint64_t)t.scalar_type()};
+    key.append(reinterpret_cast<const char*>(rec), sizeof(rec));
+  }
+  return py::bytes(key);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_gdn2_host, m) {
+  // none of them touches Python objects: the lock is released meanwhile, as a foreign call does
+  const auto unlocked = py::call_guard<py::gil_scoped_release>();
+  m.def("decode", &decode, unlocked);
+  m.def("prefill", &prefill, unlocked);
+  m.def("layer_decode", &layer_decode, unlocked);
+  m.def("parameter_key", &parameter_key);
+}

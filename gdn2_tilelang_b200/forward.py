@@ -14,7 +14,7 @@ import torch
 
 from . import _cabi
 from .config import DEFAULT_KERNEL_CONFIG, GDN2Config
-from .inference import _check_inputs
+from .inference import _check_inputs, _prefill_plain
 
 __all__ = ["chunk_gdn2_fwd", "chunk_gdn2_output"]
 
@@ -29,6 +29,10 @@ def chunk_gdn2_fwd(q, k, v, g, b, w, scale, initial_state=None, output_final_sta
     tensor or view with dense ``[S, H, DV]`` blocks that receives ``o`` (a slice of a packed batch, for instance).
     """
     config.validate()
+    if out is None and not return_chunk_states:
+        res = _prefill_plain(q, k, v, g, b, w, initial_state, scale)
+        if res is not None:
+            return res[0], (res[1] if output_final_state else None)
     B, S, H, DK, DV = _check_inputs(q, k, v, g, b, w)
     BS = config.chunk_size
     n_full = (S // BS) * BS

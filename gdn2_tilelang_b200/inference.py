@@ -42,11 +42,26 @@ def _check_inputs(q, k, v, g, b, w):
     return B, S, H, DK, DV
 
 
+def _decode_plain(q, k, v, g, b, w, state, scale):
+    """The decode in one native call (dense, aligned CUDA tensors of matching shapes and types), or ``None``."""
+    K = _cabi.kernels()
+    host = getattr(K, "host", None)
+    o = None if host is None else host.decode(q, k, v, g, b, w, state, scale)
+    if o is not None:
+        K.launches += 1
+        K.maybe_check_device_status(q.device)
+    return o
+
+
 def gdn2_decode(q, k, v, g, b, w, state, scale=None):
     """Decode ``n`` tokens (``[B, n, H, D]``), updating ``state [B, H, DK, DV]`` in place.
 
     Returns ``o [B, n, H, DV]`` in ``v.dtype``. ``g`` is coerced to float32.
     """
+    if q.dim() == 4:
+        o = _decode_plain(q, k, v, g, b, w, state, scale)
+        if o is not None:
+            return o
     B, n, H, DK, DV = _check_inputs(q, k, v, g, b, w)
     scale = DK**-0.5 if scale is None else scale
     if state.shape != (B, H, DK, DV):
@@ -61,8 +76,22 @@ def gdn2_decode_step(q, k, v, g, b, w, state, scale=None):
     """One token with ``[B, H, D]``-shaped inputs; ``state`` is updated in place. Returns ``[B, H, DV]``."""
     if q.dim() != 3:
         raise ValueError(f"expected [B, H, D] tensors, got shape {tuple(q.shape)}")
+    o = _decode_plain(q, k, v, g, b, w, state, scale)
+    if o is not None:
+        return o
     o = gdn2_decode(*(t.unsqueeze(1) for t in (q, k, v, g, b, w)), state, scale)
     return o[:, 0]
+
+
+def _prefill_plain(q, k, v, g, b, w, state, scale):
+    """A prefill of at least 64 tokens in one native call, or ``None`` where the call is not plain."""
+    K = _cabi.kernels()
+    if getattr(K, "host", None) is None:
+        return None
+    res = K.prefill_plain(q, k, v, g, b, w, scale, state)
+    if res is not None:
+        K.maybe_check_device_status(q.device)
+    return res
 
 
 @torch.no_grad()
@@ -77,6 +106,10 @@ def gdn2_prefill(q, k, v, g, b, w, state=None, scale=None, config: GDN2Config = 
     ``NativeKernels.chunk_forward``); the rows of a ragged tail are left plain for the caller to finish.
     """
     config.validate()
+    if gated_norm is None:
+        res = _prefill_plain(q, k, v, g, b, w, state, scale)
+        if res is not None:
+            return res
     B, S, H, DK, DV = _check_inputs(q, k, v, g, b, w)
     BS = config.chunk_size
     scale = DK**-0.5 if scale is None else scale
