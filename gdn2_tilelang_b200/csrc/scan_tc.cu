@@ -6,16 +6,21 @@
 // project) is evaluated TRANSPOSED so that every product has the 128 value channels as the MMA M
 // dimension (= TMEM lane = thread), tokens or key channels as N:
 //
-//   MMA1   [WS | O][dv, tok] = S^T[dv,dk] * [W ; Qg][tok,dk]^T  (W S)^T and (Qg S)^T, one N = 128 product, bf16
+//   MMA1w  WS[dv, tok]       = S^T[dv,dk] * W[tok,dk]^T         (W S)^T            bf16
+//   MMA1q  O [dv, tok]       = S^T[dv,dk] * Qg[tok,dk]^T        (Qg S)^T           bf16
 //   regs   Un^T[dv,tok] = U^T - WS
 //   MMA3   P [dv,dk]    = Un^T[dv,tok] * KG^T[dk,tok]^T       (KG^T Un)^T      fp16 (scaled, see common.cuh)
 //   MMA2   O [dv, r]   += Un^T[dv,s] * Aqk[r,s]^T             (tril(Aqk) Un)^T fp16 (same scaled Un^T image)
 //   regs   S^T         <- gamma_C[dk] * S^T + P   (the fp32 state lives in registers, 64 values per thread)
 //
-// Only MMA1, the Un pass, MMA3 and the state pass are on the recurrence's critical path; the
+// Only MMA1w, the Un pass, MMA3 and the state pass are on the recurrence's critical path; the
 // kernel is organised around that:
 //   * warp 8 issues every MMA (converged, one elected lane), MMA3 before MMA2 so the state update never
 //     queues behind the output product; one thread of warp 9 issues every bulk copy.
+//   * the products on the critical path are as short as they can be made: MMA1q runs under the Un pass, and the state
+//     goes around in two halves of 64 key channels, so that the first half's state pass runs under the second half's
+//     MMA3 and MMA1w starts on the first half while the second is still being written (with one product of N = 128 for
+//     both row kinds and undivided hand-offs the forward with chunk states above took 245 us, this way 235)
 //   * warps 10-13 read each finished O accumulator into registers, release it, and write the rows
 //     out through a shared staging tile with 128-bit coalesced stores, off the critical path.
 //   * warps 0-7 (256 threads; two warps share each 32-lane quarter of TMEM and split its columns)
@@ -82,8 +87,9 @@ struct ScanTcSmem {
   __nv_bfloat16 ostage[BS * D];      // output rows [tok][dv] on their way to global memory
   float gl[4][D];                    // gamma at the last token of chunk n (slot n & 3), copied with KG^T
   uint64_t bar_wq[2], bar_kgt[2], bar_ut[2], bar_aqk;   // bulk-copy arrival
-  uint64_t bar_m1, bar_m3, bar_m2;                      // MMA completion
-  uint64_t bar_sb, bar_un;                              // compute threads -> issuer (256 arrivals)
+  uint64_t bar_m1, bar_m3[2], bar_m2;                   // MMA completion: (W S)^T; the two key-channel halves of P; O
+  uint64_t bar_sb[2], bar_un;                           // compute threads -> issuer: S^T by key-channel half, Un^T
+  uint64_t bar_of;                                      // output warps -> issuer: the O accumulator has been read out
   uint32_t tmem_base;
   int abort_flag;
   int last_big[kComputeThreads / 32];                   // transition blocks: last chunk after which an entry was still >= kVanish
@@ -319,9 +325,10 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
     for (int i = 0; i < 2; ++i) {
       tc::mbar_init(&s.bar_wq[i], 1); tc::mbar_init(&s.bar_kgt[i], 1); tc::mbar_init(&s.bar_ut[i], 1);
     }
-    tc::mbar_init(&s.bar_aqk, 1); tc::mbar_init(&s.bar_m1, 1); tc::mbar_init(&s.bar_m3, 1); tc::mbar_init(&s.bar_m2, 1);
+    tc::mbar_init(&s.bar_aqk, 1); tc::mbar_init(&s.bar_m1, 1); tc::mbar_init(&s.bar_m2, 1);
     // one arrival per warp; a transition block has no outputs, its output warps take no part
-    tc::mbar_init(&s.bar_sb, (kComputeThreads + (transition ? 0 : kOutputThreads)) / 32);
+    for (int i = 0; i < 2; ++i) { tc::mbar_init(&s.bar_m3[i], 1); tc::mbar_init(&s.bar_sb[i], kComputeThreads / 64); }
+    tc::mbar_init(&s.bar_of, kOutputThreads / 32);
     tc::mbar_init(&s.bar_un, kComputeThreads / 32);
     s.abort_flag = 0;
     s.nc_limit = NC;
@@ -390,11 +397,11 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
     // The whole warp runs this loop converged (identical waits and operands on every lane); one
     // elected lane issues each instruction.
     {
-      constexpr uint32_t idesc_n128 = tc::instr_desc(1, 128, 128);   // bf16 operands, N = 128
-      constexpr uint32_t idesc_f16 = tc::instr_desc(0, 128, 128);    // fp16 operands, N = 128
+      constexpr uint32_t idesc_bf16 = tc::instr_desc(1, 128, 64);    // bf16 operands, N = 64
       constexpr uint32_t idesc_f16_n64 = tc::instr_desc(0, 128, 64); // fp16 operands, N = 64
       const uint32_t a_sb = tc::tmem_addr(tm, 0, kColSb), a_un16 = tc::tmem_addr(tm, 0, kColUn16);
       const uint32_t a_aqk = tc::smem_u32(s.aqk);
+      const uint32_t t_ws = tc::tmem_addr(tm, 0, kColWs), t_o = tc::tmem_addr(tm, 0, kColO);
       auto wait_all = [&](uint64_t* bar, uint32_t parity, uint32_t code) {
         return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity, &s.abort_flag, status, code)) != 0;
       };
@@ -402,26 +409,40 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
         if (n >= *(volatile int*)&s.nc_limit) break;         // uniform: every lane reads the same word
         const int b = n & 1;
         const uint32_t ph = n & 1, ph2 = (n >> 1) & 1;
-        // S^T (bf16) of chunk n is in place and the O accumulator has been read out
+        // (W S)^T first, one key-channel half of S^T as soon as it is in place: the Un pass waits for nothing else.
+        // The query rows' half of the product runs under that pass.
         bool ok = wait_all(&s.bar_wq[b], ph2, kWaitWq);
-        ok = ok && wait_all(&s.bar_sb, ph, kWaitSb);
+        const uint32_t b_wq = tc::smem_u32(s.wq[b]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          ok = ok && wait_all(&s.bar_sb[h], ph, kWaitSb);
+          if (ok) {
+            tc::tc_fence_after_sync();
+            tc::mma_f16_ts_ktile_warp(t_ws, a_sb + h * (D / 4), b_wq + h * (D / 16) * (2 * BS * 16), 2 * BS, D / 2, idesc_bf16, h != 0);
+          }
+        }
+        if (ok && !output_only) tc::mma_commit_warp(&s.bar_m1);
+        if (!transition) ok = ok && wait_all(&s.bar_of, ph, kWaitSb);   // the O accumulator has been read out
         if (ok) {
           tc::tc_fence_after_sync();
-          // one N = 128 product: columns [128,192) = (W S)^T, [192,256) = (Qg S)^T
-          tc::mma_f16_ts_ktile_warp(tc::tmem_addr(tm, 0, kColWs), a_sb, tc::smem_u32(s.wq[b]), 2 * BS, D, idesc_n128, false);
-          tc::mma_commit_warp(&s.bar_m1);
+          tc::mma_f16_ts_ktile_warp(t_o, a_sb, b_wq + BS * 16, 2 * BS, D, idesc_bf16, false);
+          if (output_only) tc::mma_commit_warp(&s.bar_m1);   // the next chunk's S^T replaces this one right after the Un pass
         }
-        ok = output_only || wait_all(&s.bar_kgt[b], ph2, kWaitKgt);
+        ok = ok && (output_only || wait_all(&s.bar_kgt[b], ph2, kWaitKgt));
         ok = ok && wait_all(&s.bar_un, ph, kWaitUn);
         if (ok && !output_only) {
           tc::tc_fence_after_sync();
-          tc::mma_f16_ts_ktile_warp(tc::tmem_addr(tm, 0, 0), a_un16, tc::smem_u32(s.kgt[b]), D, BS, idesc_f16, false);
-          tc::mma_commit_warp(&s.bar_m3);
+          const uint32_t b_kgt = tc::smem_u32(s.kgt[b]);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {                      // key-channel halves: the state pass of the first starts early
+            tc::mma_f16_ts_ktile_warp(tc::tmem_addr(tm, 0, h * (D / 2)), a_un16, b_kgt + h * (D / 2) * 16, D, BS, idesc_f16_n64, false);
+            tc::mma_commit_warp(&s.bar_m3[h]);
+          }
         }
         ok = ok && wait_all(&s.bar_aqk, ph, kWaitAqk);
         if (ok) {
           tc::tc_fence_after_sync();
-          tc::mma_f16_ts_ktile_warp(tc::tmem_addr(tm, 0, kColO), a_un16, a_aqk, BS, BS, idesc_f16_n64, true);
+          tc::mma_f16_ts_ktile_warp(t_o, a_un16, a_aqk, BS, BS, idesc_f16_n64, true);
           tc::mma_commit_warp(&s.bar_m2);
         }
       }
@@ -432,7 +453,7 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
     const int dv = lq * 32 + lane;
     const int otid = tid - (kComputeThreads + 64);
     const uint32_t t_o = tc::tmem_addr(tm, lq * 32, kColO);
-    if (!transition) warp_arrive(&s.bar_sb, lane);         // nothing to read out before chunk 0
+    if (!transition) warp_arrive(&s.bar_of, lane);         // nothing to read out before chunk 0
     for (int n = 0; n < (transition ? 0 : NC); ++n) {
       float ov[64];
       if (norm.gate) {                                     // this chunk's gate rows towards L2 while its products run
@@ -447,7 +468,7 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
       tc::tmem_ld32(t_o + 32, *reinterpret_cast<float(*)[32]>(&ov[32]));
       tc::tmem_ld_wait();
       tc::tc_fence_before_sync();
-      if (n + 1 < NC) warp_arrive(&s.bar_sb, lane);        // the accumulator may be overwritten by the next MMA1
+      if (n + 1 < NC) warp_arrive(&s.bar_of, lane);        // the accumulator may be overwritten by the next MMA1
       output_sync();                                       // the previous chunk's rows have left the staging buffer
 #pragma unroll
       for (int i = 0; i < 64; ++i) s.ostage[i * D + dv] = __float2bfloat16_rn(ov[i]);
@@ -498,7 +519,7 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
       tc::tmem_st_wait();
     }
     tc::tc_fence_before_sync();
-    warp_arrive(&s.bar_sb, lane);
+    warp_arrive(&s.bar_sb[part], lane);
     for (int n = 0; n < NC; ++n) {
       if (n >= *(volatile int*)&s.nc_limit) break;
       const int b = n & 1;
@@ -555,7 +576,7 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
           tc::tmem_st32(t_lane + kColSb + dkp / 2, pk);
           tc::tmem_st_wait();
           tc::tc_fence_before_sync();
-          warp_arrive(&s.bar_sb, lane);
+          warp_arrive(&s.bar_sb[part], lane);
         }
         if (s.abort_flag) break;
         continue;
@@ -563,7 +584,7 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
 
       // ---- new state S <- gamma_C * S + P, its bf16 operand copy for the next chunk, optional snapshot
       tc::mbar_wait(&s.bar_kgt[b], ph2, &s.abort_flag, status, kWaitKgt);   // gamma arrived with KG^T
-      tc::mbar_wait(&s.bar_m3, ph, &s.abort_flag, status, kWaitM3);
+      tc::mbar_wait(&s.bar_m3[part], ph, &s.abort_flag, status, kWaitM3);
       tc::tc_fence_after_sync();
       {
         const float* gln = s.gl[n & 3];
@@ -590,7 +611,7 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
         if (more) {
           tc::tmem_st_wait();
           tc::tc_fence_before_sync();
-          warp_arrive(&s.bar_sb, lane);
+          warp_arrive(&s.bar_sb[part], lane);
         }
         float* hn = (hs && more) ? hs + (((size_t)ib * NC_all + (c_first + n + 1)) * H + ih) * D * D : nullptr;
         if (hn) {
