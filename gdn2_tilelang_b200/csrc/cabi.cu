@@ -283,9 +283,9 @@ int gdn2_prefill_ragged(const void* q, const void* k, const void* v, const float
   cudaStream_t st = static_cast<cudaStream_t>(stream), side = static_cast<cudaStream_t>(side_stream);
   int rc = GDN2_OK;
   if (n_full && n_tail && workspace) {
-    // Exact family: the tail is one more chunk whose missing rows have k = q = v = 0 and no decay. A chunk costs the
-    // scan MEASURED_CHUNK, the token-by-token decode of 40 tails tokens MEASURED_TAIL. A workspace sized for the whole
-    // chunks only keeps the decode.
+    // Exact family: the tail is one more chunk whose missing rows have k = q = v = 0 and no decay: one more step of the
+    // scan's chain (a few us) where the token-by-token decode takes up to 63. A workspace sized for the whole chunks only
+    // keeps the decode.
     int p;
     bool seg;
     const int64_t up = n_full + kChunk;

