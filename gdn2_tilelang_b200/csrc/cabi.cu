@@ -126,9 +126,10 @@ const char* gdn2_status_string(int status) {
 
 int gdn2_last_cuda_error(void) { return g_last_cuda_error; }
 
-int gdn2_decode(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
+namespace {
+int decode_impl(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
                 float* state, void* o, int64_t B, int64_t n, int64_t H, int64_t HK, int64_t DK, int64_t DV,
-                int64_t in_batch_stride, int64_t o_batch_stride, float scale, int dtype, void* stream) {
+                int64_t in_batch_stride, int64_t o_batch_stride, float scale, int dtype, bool chained, void* stream) {
   if (!q || !k || !v || !g || !b || !w || !state || !o) return GDN2_ERR_NULL_POINTER;
   if (!valid_dtype(dtype)) return GDN2_ERR_BAD_DTYPE;
   if (B <= 0 || n <= 0 || H <= 0 || DK <= 0 || DV <= 0 || DK > 256) return GDN2_ERR_BAD_SHAPE;
@@ -139,7 +140,14 @@ int gdn2_decode(const void* q, const void* k, const void* v, const float* g, con
                                  !aligned16(b) || !aligned16(w) || !aligned16(o)))
     return GDN2_ERR_MISALIGNED;                            // bulk copies and 16-byte loads on this path
   return launch_decode(q, k, v, g, b, w, state, o, (int)B, (int)n, (int)H, (int)HK, (int)DK, (int)DV, in_batch_stride,
-                       o_batch_stride, scale, dtype, static_cast<cudaStream_t>(stream));
+                       o_batch_stride, scale, dtype, chained, static_cast<cudaStream_t>(stream));
+}
+}  // namespace
+
+int gdn2_decode(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
+                float* state, void* o, int64_t B, int64_t n, int64_t H, int64_t HK, int64_t DK, int64_t DV,
+                int64_t in_batch_stride, int64_t o_batch_stride, float scale, int dtype, void* stream) {
+  return decode_impl(q, k, v, g, b, w, state, o, B, n, H, HK, DK, DV, in_batch_stride, o_batch_stride, scale, dtype, true, stream);
 }
 
 size_t gdn2_prefill_workspace_bytes(int64_t B, int64_t S, int64_t H, int64_t HK, int64_t DK, int64_t DV, int dtype,
@@ -327,10 +335,10 @@ int gdn2_prefill_ragged(const void* q, const void* k, const void* v, const float
     return static_cast<const void*>(static_cast<const char*>(p) + (size_t)n_full * heads * d * es);
   };
   auto decode_tail = [&](void* on) -> int {
-    return gdn2_decode(at(q, HK, DK, esz), at(k, HK, DK, esz), at(v, H, DV, esz),
+    return decode_impl(at(q, HK, DK, esz), at(k, HK, DK, esz), at(v, H, DV, esz),
                        static_cast<const float*>(at(g, HK, DK, sizeof(float))), at(b, HK, DK, esz), at(w, H, DV, esz),
                        final_state, const_cast<void*>(at(o, H, DV, esz)), B, n_tail, H, HK, DK, DV, in_batch_stride,
-                       o_batch_stride, scale, dtype, on);
+                       o_batch_stride, scale, dtype, false, on);
   };
   const bool beside = n_full && side && side != st &&
                       gdn2_prefill_scan_launches(B, n_full, H, DK, DV, dtype, path) > 1;

@@ -24,7 +24,8 @@ namespace gdn2 {
 // decode_blocked.cu: blocks of up to 8 tokens without a per-token dependent sweep (DK = DV = 128)
 template <typename T>
 int launch_decode_blocked(const T* q, const T* k, const T* v, const float* g, const T* b, const T* w, float* state,
-                          T* o, int B, int n, int H, int HK, int64_t in_bs, int64_t o_bs, float scale, cudaStream_t st);
+                          T* o, int B, int n, int H, int HK, int64_t in_bs, int64_t o_bs, float scale, bool chained,
+                          cudaStream_t st);
 
 namespace {
 
@@ -71,6 +72,8 @@ decode_square_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* 
   __shared__ float s_wv[kTokBatch][D];                   // w * v
   __shared__ float s_qk[kTokBatch][D / 32];              // per-warp partial sums of scale * q . k
 
+  grid_wait();
+  grid_launch_dependents();
   float4 S[R];
   float4* gS = reinterpret_cast<float4*>(state + ((size_t)bh * D + R * rg) * D + col0);
 #pragma unroll
@@ -165,6 +168,8 @@ decode_generic_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
   float* s_q = s_k + DK;
   __shared__ float s_red[2][4][32];
 
+  grid_wait();
+  grid_launch_dependents();
   float S[MAXR];
 #pragma unroll
   for (int i = 0; i < MAXR; ++i) {
@@ -218,30 +223,29 @@ decode_generic_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
 template <typename T>
 int launch_typed(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
                  float* state, void* o, int B, int n, int H, int HK, int DK, int DV, int64_t in_bs, int64_t o_bs, float scale,
-                 cudaStream_t st) {
+                 bool chained, cudaStream_t st) {
   const T* tq = static_cast<const T*>(q); const T* tk = static_cast<const T*>(k);
   const T* tv = static_cast<const T*>(v); const T* tb = static_cast<const T*>(b);
   const T* tw = static_cast<const T*>(w); T* to = static_cast<T*>(o);
   if (DK == 128 && DV == 128 && n >= kBlockedMinTokens) {
-    return launch_decode_blocked<T>(tq, tk, tv, g, tb, tw, state, to, B, n, H, HK, in_bs, o_bs, scale, st);
+    return launch_decode_blocked<T>(tq, tk, tv, g, tb, tw, state, to, B, n, H, HK, in_bs, o_bs, scale, chained, st);
   } else if (DK == 128 && DV == 128) {
-    decode_square_kernel<T, 128><<<B * H, 128, 0, st>>>(tq, tk, tv, g, tb, tw, state, to, n, H, HK, in_bs, o_bs, scale);
+    GDN2_CUDA_TRY(launch_chained(chained, decode_square_kernel<T, 128>, dim3(B * H), 128, 0, st, tq, tk, tv, g, tb, tw, state, to, n, H, HK, in_bs, o_bs, scale));
   } else if (DK == 64 && DV == 64 && (reinterpret_cast<uintptr_t>(state) & 15u) == 0) {
     // The generic kernel reads the state 4 bytes per lane, holds a quarter of a column per warp and meets at a barrier three
     // times per token; it stays for the other sizes and for a state without 16-byte alignment. B = 256, 16 heads, bf16: one
     // token 39.1 us there, 28.6 here; eight tokens 144 and 60.7.
-    decode_square_kernel<T, 64><<<B * H, 64, 0, st>>>(tq, tk, tv, g, tb, tw, state, to, n, H, HK, in_bs, o_bs, scale);
+    GDN2_CUDA_TRY(launch_chained(chained, decode_square_kernel<T, 64>, dim3(B * H), 64, 0, st, tq, tk, tv, g, tb, tw, state, to, n, H, HK, in_bs, o_bs, scale));
   } else {
     dim3 grid(B * H, (DV + 31) / 32);
     const size_t sm = (size_t)4 * DK * sizeof(float);
     if (DK <= 64)
-      decode_generic_kernel<T, 16><<<grid, 128, sm, st>>>(tq, tk, tv, g, tb, tw, state, to, n, H, HK, DK, DV, in_bs, o_bs, scale);
+      GDN2_CUDA_TRY(launch_chained(chained, decode_generic_kernel<T, 16>, grid, 128, sm, st, tq, tk, tv, g, tb, tw, state, to, n, H, HK, DK, DV, in_bs, o_bs, scale));
     else if (DK <= 128)
-      decode_generic_kernel<T, 32><<<grid, 128, sm, st>>>(tq, tk, tv, g, tb, tw, state, to, n, H, HK, DK, DV, in_bs, o_bs, scale);
+      GDN2_CUDA_TRY(launch_chained(chained, decode_generic_kernel<T, 32>, grid, 128, sm, st, tq, tk, tv, g, tb, tw, state, to, n, H, HK, DK, DV, in_bs, o_bs, scale));
     else
-      decode_generic_kernel<T, 64><<<grid, 128, sm, st>>>(tq, tk, tv, g, tb, tw, state, to, n, H, HK, DK, DV, in_bs, o_bs, scale);
+      GDN2_CUDA_TRY(launch_chained(chained, decode_generic_kernel<T, 64>, grid, 128, sm, st, tq, tk, tv, g, tb, tw, state, to, n, H, HK, DK, DV, in_bs, o_bs, scale));
   }
-  GDN2_CUDA_TRY(cudaGetLastError());
   return GDN2_OK;
 }
 
@@ -249,11 +253,11 @@ int launch_typed(const void* q, const void* k, const void* v, const float* g, co
 
 int launch_decode(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
                   float* state, void* o, int B, int n, int H, int HK, int DK, int DV, int64_t in_bs, int64_t o_bs,
-                  float scale, int dtype, cudaStream_t st) {
+                  float scale, int dtype, bool chained, cudaStream_t st) {
   switch (dtype) {
-    case GDN2_F32: return launch_typed<float>(q, k, v, g, b, w, state, o, B, n, H, HK, DK, DV, in_bs, o_bs, scale, st);
-    case GDN2_BF16: return launch_typed<__nv_bfloat16>(q, k, v, g, b, w, state, o, B, n, H, HK, DK, DV, in_bs, o_bs, scale, st);
-    case GDN2_F16: return launch_typed<__half>(q, k, v, g, b, w, state, o, B, n, H, HK, DK, DV, in_bs, o_bs, scale, st);
+    case GDN2_F32: return launch_typed<float>(q, k, v, g, b, w, state, o, B, n, H, HK, DK, DV, in_bs, o_bs, scale, chained, st);
+    case GDN2_BF16: return launch_typed<__nv_bfloat16>(q, k, v, g, b, w, state, o, B, n, H, HK, DK, DV, in_bs, o_bs, scale, chained, st);
+    case GDN2_F16: return launch_typed<__half>(q, k, v, g, b, w, state, o, B, n, H, HK, DK, DV, in_bs, o_bs, scale, chained, st);
     default: return GDN2_ERR_BAD_DTYPE;
   }
 }

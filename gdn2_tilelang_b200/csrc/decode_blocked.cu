@@ -183,6 +183,9 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
   }
   __syncthreads();
 
+  grid_wait();
+  grid_launch_dependents();
+
   if (wid == 13) {
     // =============================== output thread: a step's rows leave as bulk copies ==========
     // (256-byte rows for 16-bit outputs: eight scattered 2-byte stores per lane of the sweep warps otherwise)
@@ -544,15 +547,15 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
 
 template <typename T>
 int launch_decode_blocked(const T* q, const T* k, const T* v, const float* g, const T* b, const T* w, float* state,
-                          T* o, int B, int n, int H, int HK, int64_t in_bs, int64_t o_bs, float scale, cudaStream_t st) {
+                          T* o, int B, int n, int H, int HK, int64_t in_bs, int64_t o_bs, float scale, bool chained,
+                          cudaStream_t st) {
   const size_t smem = sizeof(BlockedSmem) + 128;
   GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(decode_blocked_kernel<T, OneLength>), smem));
   const int ntiles = B * H;
   const int sms = device_sm_count();
   const int grid = ntiles < sms ? ntiles : sms;
-  decode_blocked_kernel<T, OneLength><<<grid, kAllThreads, smem, st>>>(q, k, v, g, b, w, state, o, ntiles, n, H, HK, in_bs, o_bs, scale,
-                                                         device_status_word(), OneLength{});
-  GDN2_CUDA_TRY(cudaGetLastError());
+  GDN2_CUDA_TRY(launch_chained(chained, decode_blocked_kernel<T, OneLength>, dim3(grid), kAllThreads, smem, st, q, k, v, g, b, w, state, o, ntiles,
+                               n, H, HK, in_bs, o_bs, scale, device_status_word(), OneLength{}));
   return GDN2_OK;
 }
 
@@ -563,21 +566,18 @@ int launch_decode_packed_tails(const void* q, const void* k, const void* v, cons
   auto kern = decode_blocked_kernel<T, PackedSeqs>;
   GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
   const int ntiles = seqs.n * H, sms = device_sm_count();
-  kern<<<ntiles < sms ? ntiles : sms, kAllThreads, smem, st>>>(
-      static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v), g, static_cast<const T*>(b),
-      static_cast<const T*>(w), state, static_cast<T*>(o), ntiles, 0, H, HK, 0, 0, scale, device_status_word(), seqs);
-  GDN2_CUDA_TRY(cudaGetLastError());
+  GDN2_CUDA_TRY(launch_chained(false, kern, dim3(ntiles < sms ? ntiles : sms), kAllThreads, smem, st, static_cast<const T*>(q),
+                               static_cast<const T*>(k), static_cast<const T*>(v), g, static_cast<const T*>(b), static_cast<const T*>(w),
+                               state, static_cast<T*>(o), ntiles, 0, H, HK, 0, 0, scale, device_status_word(), seqs));
   return GDN2_OK;
 }
 
 template int launch_decode_blocked<float>(const float*, const float*, const float*, const float*, const float*,
-                                          const float*, float*, float*, int, int, int, int, int64_t, int64_t, float,
-                                          cudaStream_t);
+                                          const float*, float*, float*, int, int, int, int, int64_t, int64_t, float, bool, cudaStream_t);
 template int launch_decode_blocked<__nv_bfloat16>(const __nv_bfloat16*, const __nv_bfloat16*, const __nv_bfloat16*,
                                                   const float*, const __nv_bfloat16*, const __nv_bfloat16*, float*,
-                                                  __nv_bfloat16*, int, int, int, int, int64_t, int64_t, float, cudaStream_t);
+                                                  __nv_bfloat16*, int, int, int, int, int64_t, int64_t, float, bool, cudaStream_t);
 template int launch_decode_blocked<__half>(const __half*, const __half*, const __half*, const float*, const __half*,
-                                           const __half*, float*, __half*, int, int, int, int, int64_t, int64_t, float,
-                                           cudaStream_t);
+                                           const __half*, float*, __half*, int, int, int, int, int64_t, int64_t, float, bool, cudaStream_t);
 
 }  // namespace gdn2

@@ -56,6 +56,8 @@ __device__ __forceinline__ float tap(const T* P, const T* conv_state, int64_t b,
 template <typename T>
 __global__ void __launch_bounds__(32 * kWarps)
 layer_front_kernel(gdn2_layer_front_args a) {
+  grid_wait();
+  grid_launch_dependents();
   const int lane = threadIdx.x & 31;
   const int64_t item = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
   if (item >= a.B * a.S * a.HK) return;
@@ -204,6 +206,8 @@ __device__ __forceinline__ void conv4(const T* P, const T* cs, const T* cw, cons
 template <typename T>
 __global__ void __launch_bounds__(32 * kWarps)
 layer_front_d128_kernel(gdn2_layer_front_args a) {
+  grid_wait();
+  grid_launch_dependents();
   constexpr int DK = 128, DV = 128;
   const int lane = threadIdx.x & 31;
   const int64_t item = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
@@ -274,6 +278,8 @@ layer_front_d128_kernel(gdn2_layer_front_args a) {
 template <typename T>
 __global__ void __launch_bounds__(32 * kWarps, 6)
 layer_front_d128x4_kernel(gdn2_layer_front_args a) {
+  grid_wait();
+  grid_launch_dependents();
   constexpr int D = 128, K = 4, TT = 4;
   const int lane = threadIdx.x & 31;
   const int S = (int)a.S, NP = (int)a.NP, H = (int)a.H, HK = (int)a.HK;
@@ -392,6 +398,8 @@ layer_front_d128x4_kernel(gdn2_layer_front_args a) {
 // new_conv[b, cch, s] = pre-convolution value at time S - (K-1) + s (from P, the old cache, or zero)
 template <typename T>
 __global__ void layer_conv_tail_kernel(gdn2_layer_front_args a) {
+  grid_wait();
+  grid_launch_dependents();
   const int K = (int)a.K, S = (int)a.S, NP = (int)a.NP;
   const int Cqk = (int)(a.HK * a.DK), Cv = (int)(a.H * a.DV), CC = 2 * Cqk + Cv;
   const int64_t total = a.B * CC * (K - 1);
@@ -410,6 +418,8 @@ template <typename T>
 __global__ void __launch_bounds__(32 * kWarps)
 layer_back_kernel(const T* __restrict__ o, const T* __restrict__ proj, const T* __restrict__ weight, T* __restrict__ out,
                   int64_t BS, int H, int DV, int NP, int off_gate, float eps) {
+  grid_wait();
+  grid_launch_dependents();
   const int lane = threadIdx.x & 31;
   const int64_t item = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
   if (item >= BS * H) return;
@@ -446,18 +456,15 @@ int launch_front_typed(const gdn2_layer_front_args& a, cudaStream_t st) {
   if (sizeof(T) == 2 && a.DK == 128 && a.DV == 128 && a.K == 4 && aligned && a.S >= 8 &&
       a.B * ((a.S + 3) / 4) * (4 * a.HK + 2 * a.H) < (int64_t)1 << 31) {
     const int64_t items4 = a.B * ((a.S + 3) / 4) * (4 * a.HK + 2 * a.H);   // prompts: a slot of four tokens per warp
-    layer_front_d128x4_kernel<T><<<(unsigned)((items4 + kWarps - 1) / kWarps), 32 * kWarps, 0, st>>>(a);
+    GDN2_CUDA_TRY(launch_chained(true, layer_front_d128x4_kernel<T>, dim3((unsigned)((items4 + kWarps - 1) / kWarps)), 32 * kWarps, 0, st, a));
   } else if (sizeof(T) == 2 && a.DK == 128 && a.DV == 128 && a.K == 4 && aligned) {
-    layer_front_d128_kernel<T><<<(unsigned)((items + kWarps - 1) / kWarps), 32 * kWarps, 0, st>>>(a);
-    GDN2_CUDA_TRY(cudaGetLastError());
+    GDN2_CUDA_TRY(launch_chained(true, layer_front_d128_kernel<T>, dim3((unsigned)((items + kWarps - 1) / kWarps)), 32 * kWarps, 0, st, a));
     return GDN2_OK;                                          // this form writes the new convolution cache itself
   } else
-    layer_front_kernel<T><<<(unsigned)((items + kWarps - 1) / kWarps), 32 * kWarps, 0, st>>>(a);
-  GDN2_CUDA_TRY(cudaGetLastError());
+    GDN2_CUDA_TRY(launch_chained(true, layer_front_kernel<T>, dim3((unsigned)((items + kWarps - 1) / kWarps)), 32 * kWarps, 0, st, a));
   if (a.K > 1 && a.new_conv_state) {
     const int64_t total = a.B * (2 * a.HK * a.DK + a.H * a.DV) * (a.K - 1);
-    layer_conv_tail_kernel<T><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(a);
-    GDN2_CUDA_TRY(cudaGetLastError());
+    GDN2_CUDA_TRY(launch_chained(true, layer_conv_tail_kernel<T>, dim3((unsigned)((total + 255) / 256)), 256, 0, st, a));
   }
   return GDN2_OK;
 }
@@ -468,6 +475,8 @@ template <typename T>
 __global__ void __launch_bounds__(32 * kWarps)
 layer_back_d128_kernel(const T* __restrict__ o, const T* __restrict__ proj, const T* __restrict__ weight, T* __restrict__ out,
                        int64_t items, int H, int NP, int off_gate, float eps) {
+  grid_wait();
+  grid_launch_dependents();
   constexpr int DV = 128, R = 4;
   const int lane = threadIdx.x & 31;
   const int c = 4 * lane;
@@ -507,16 +516,10 @@ int launch_back_typed(const void* o, const void* proj, const void* weight, void*
                          reinterpret_cast<uintptr_t>(out)) & 7) == 0;
   if (sizeof(T) == 2 && DV == 128 && aligned && items < (int64_t)1 << 32) {
     const int64_t warps = (items + 3) / 4;
-    layer_back_d128_kernel<T><<<(unsigned)((warps + kWarps - 1) / kWarps), 32 * kWarps, 0, st>>>(
-        static_cast<const T*>(o), static_cast<const T*>(proj), static_cast<const T*>(weight), static_cast<T*>(out), items, H,
-        NP, off_gate, eps);
-    GDN2_CUDA_TRY(cudaGetLastError());
+    GDN2_CUDA_TRY(launch_chained(true, layer_back_d128_kernel<T>, dim3((unsigned)((warps + kWarps - 1) / kWarps)), 32 * kWarps, 0, st, static_cast<const T*>(o), static_cast<const T*>(proj), static_cast<const T*>(weight), static_cast<T*>(out), items, H, NP, off_gate, eps));
     return GDN2_OK;
   }
-  layer_back_kernel<T><<<(unsigned)((items + kWarps - 1) / kWarps), 32 * kWarps, 0, st>>>(
-      static_cast<const T*>(o), static_cast<const T*>(proj), static_cast<const T*>(weight), static_cast<T*>(out), BS, H,
-      DV, NP, off_gate, eps);
-  GDN2_CUDA_TRY(cudaGetLastError());
+  GDN2_CUDA_TRY(launch_chained(true, layer_back_kernel<T>, dim3((unsigned)((items + kWarps - 1) / kWarps)), 32 * kWarps, 0, st, static_cast<const T*>(o), static_cast<const T*>(proj), static_cast<const T*>(weight), static_cast<T*>(out), BS, H, DV, NP, off_gate, eps));
   return GDN2_OK;
 }
 

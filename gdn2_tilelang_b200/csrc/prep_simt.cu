@@ -357,6 +357,7 @@ __global__ void __launch_bounds__(256, 2)
 prep_simt_kernel(const TIn* __restrict__ q, const TIn* __restrict__ k, const TIn* __restrict__ v,
                  const float* __restrict__ g, const TIn* __restrict__ b, const TIn* __restrict__ w,
                  WsLayout L, WsPtrs P, int S, int H, int HK, int64_t in_bs, float scale, const __grid_constant__ Seqs seqs) {
+  grid_wait();
   prep_simt_chunk<TIn, TW>(q, k, v, g, b, w, L, P, S, H, HK, in_bs, scale, blockIdx.x, blockIdx.y, seqs);
 }
 
@@ -395,7 +396,7 @@ int launch_typed(const void* q, const void* k, const void* v, const float* g, co
     auto kern = prep_simt_kernel<TIn, TW, Seqs>;
     GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
     dim3 grid((S + kChunk - 1) / kChunk, B * HK);
-    kern<<<grid, 256, smem, st>>>(tq, tk, tv, g, tb, tw, L, P, S, H, HK, in_bs, scale, seqs);
+    GDN2_CUDA_TRY(launch_chained(true, kern, grid, 256, smem, st, tq, tk, tv, g, tb, tw, L, P, S, H, HK, in_bs, scale, seqs));
   }
   GDN2_CUDA_TRY(cudaGetLastError());
   return GDN2_OK;

@@ -201,6 +201,7 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
     abort_flag = 0;
     tc::mbar_init_fence();
   }
+  grid_wait();
   for (int idx = tid; idx < DK * NVT; idx += 256) {
     const int c = idx / NVT, d = idx % NVT;
     s.St[idx] = (s0 != nullptr && d < nv) ? s0[((size_t)bh * DK + c) * DV + lo + d] : 0.f;
@@ -336,9 +337,8 @@ int launch_scan_typed(const WsLayout& L, const WsPtrs& P, const float* s0, void*
   const int BH = B * H, sms = device_sm_count();
   auto launch = [&](auto kern, int nvt, size_t smem) -> int {
     GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
-    kern<<<dim3(BH, (L.DV + nvt - 1) / nvt), 256, smem, st>>>(L, P, s0, static_cast<TOut*>(o), sT, hs, S, H, o_bs,
-                                                              device_status_word(), seqs);
-    GDN2_CUDA_TRY(cudaGetLastError());
+    GDN2_CUDA_TRY(launch_chained(true, kern, dim3(BH, (L.DV + nvt - 1) / nvt), 256, smem, st, L, P, s0, static_cast<TOut*>(o), sT, hs, S, H,
+                                 o_bs, device_status_word(), seqs));
     return GDN2_OK;
   };
   // the narrowest tile whose blocks all run at once (two per SM while the records of DK <= 64 leave room)
