@@ -2,15 +2,21 @@
 // of 8), any DV (multiple of 4), fp32 arithmetic throughout. One 256-thread block per
 // (chunk, batch*head).
 //
-// The two intra-chunk matrices are sums over channels of x_r * k_s * exp2(G_r - G_s), r >= s (exponent <= 0 by
-// construction), evaluated in 4 x 4 tiles of (r, s). On a tile of the diagonal every pair has its own exponential
-// (the form the reference uses for its diagonal sub-blocks, intra_diag_kernel, gdn2/forward.py:220-235 of the
-// reference project). Below it the decay is split at the tile's first row, exp2(G_r - G_ref) * exp2(G_ref - G_s):
-// both exponents are <= 0 whatever the inputs, so nothing can overflow and a factor flushes to zero only where the
-// product is below 2^-126; 7 exponentials per channel stand for the tile's 16. The inverse (I + Tm)^-1 is built by
-// 16 x 16 blocks (solve_kernel, gdn2/forward.py:424-434, substitutes column by column), then W = Ai E, U = Ai (w*v),
-// KG and Qg follow wy_kernel (gdn2/forward.py:512-533) and the query scaling of prefill_scan_kernel
-// (gdn2/inference.py:461).
+// The two intra-chunk matrices are sums over channels of x_r * k_s * exp2(l_{s+1} + .. + l_r), r >= s, l = g * log2(e)
+// (exponents <= 0 for decays), evaluated in 4 x 4 tiles of (r, s). On a tile of the diagonal every pair has its own
+// exponential (the form the reference uses for its diagonal sub-blocks, intra_diag_kernel, gdn2/forward.py:220-235 of the
+// reference project). Below it the exponent is split at the tile's first row, 7 exponentials per channel for the tile's 16.
+//
+// An exponent is never the difference of two rounded prefix sums: a strong gate (-100, or -inf) would swallow the ones
+// after it, and a token-by-token evaluation knows no such loss. The decays stay one by one in shared memory; a span is the
+// sum of the up to three at each end and of the four-token groups in between, whose prefix sums are kept as unevaluated
+// pairs (high, low), so their difference is right to its own size. Gates are read as max(g, kMinGate), whose exponential is
+// zero already: sums stay finite. With one gate of -1e6 in 40 tokens, D = 64, the outputs are off by 1.3e-7 of their norm;
+// differences of prefix sums over the chunk gave 4e-2, and NaN for -inf.
+//
+// The inverse (I + Tm)^-1 is built by 16 x 16 blocks (solve_kernel, gdn2/forward.py:424-434, substitutes column by column),
+// then W = Ai E, U = Ai (w*v), KG and Qg follow wy_kernel (gdn2/forward.py:512-533) and the query scaling of
+// prefill_scan_kernel (gdn2/inference.py:461).
 //
 // What bounds it: a call of this family has few chunk-heads (hundreds), so a block's own chain of phases sets the
 // time. Hence eight lanes per tile and register tiles of 4 x 4 in every product; one pair per warp and a
@@ -31,11 +37,18 @@ namespace {
 constexpr int LT = kChunk + 4;        // floats per row of the transposed 64 x 64 matrices
 __host__ __device__ inline int row_stride(int DK) { return DK + 4; }   // floats per token row: 16-byte aligned, rows 4 banks apart
 
+constexpr float kMinGate = -110.f;    // exp(-104) is already below half of float32's smallest number
+constexpr int kGroups = kChunk / 4;   // groups of four tokens
+
+// 2^x to the instruction's documented error, a relative 2^-22; zero far below float32's range
 __device__ __forceinline__ float ex2(float x) {
   float y;
-  asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));   // what exp2f is made of; here it need not be inlined with range checks
+  asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+__device__ __forceinline__ float gate_log2(float g) { return (g < kMinGate ? kMinGate : g) * kLog2e; }   // (a NaN stays one)
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 __device__ __forceinline__ float4 load4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
 __device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
   const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
@@ -96,12 +109,14 @@ __device__ __forceinline__ void prep_simt_chunk(const TIn* __restrict__ q, const
   const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
 
   extern __shared__ __align__(16) float sm[];
-  float* Gs = sm;                    // [BS][LD] cumulative log2 decay
-  float* ks = Gs + BS * LD;          // [BS][LD] k
+  float* Ls = sm;                    // [BS][LD] log2 decay of every token
+  float* ks = Ls + BS * LD;          // [BS][LD] k
   float* es = ks + BS * LD;          // [BS][LD] b*k, later E = b*k*gamma
   float* qs = es + BS * LD;          // [BS][LD] q, later the w*v tiles
   float* TT = qs + BS * LD;          // [BS][LT] Tm transposed (row s, column r; strictly s < r), later N
-  float* AT = TT + BS * LT;          // [BS][LT] (I + Tm)^-1 transposed; before that, partial sums of the decay
+  float* AT = TT + BS * LT;          // [BS][LT] (I + Tm)^-1 transposed
+  float* Ch = AT + BS * LT;          // [17][LD] decay of the four-token groups before group x: high part ...
+  float* Cl = Ch + (kGroups + 1) * LD;   // ... and what its rounding lost
 
   TW* wq = reinterpret_cast<TW*>(P.wq + (size_t)ch * L.wq_bytes);
   TV* aqk = reinterpret_cast<TV*>(P.aqk + (size_t)ch * L.aqk_bytes);
@@ -118,24 +133,27 @@ __device__ __forceinline__ void prep_simt_chunk(const TIn* __restrict__ q, const
     *reinterpret_cast<float4*>(&ks[t * LD + c]) = kk;
     *reinterpret_cast<float4*>(&qs[t * LD + c]) = qq;
     *reinterpret_cast<float4*>(&es[t * LD + c]) = mul4(bb, kk);
-    *reinterpret_cast<float4*>(&Gs[t * LD + c]) = gg;
+    *reinterpret_cast<float4*>(&Ls[t * LD + c]) = make_float4(gate_log2(gg.x), gate_log2(gg.y), gate_log2(gg.z), gate_log2(gg.w));
   }
   __syncthreads();
-  // cumulative decay: four runs of 16 tokens per channel, then the totals of the runs before
-  for (int it = tid; it < 4 * DK; it += 256) {
-    const int c = it % DK, sg = it / DK;
-    float run = 0.f;
-#pragma unroll
-    for (int t = 0; t < 16; ++t) { run += Gs[(16 * sg + t) * LD + c]; Gs[(16 * sg + t) * LD + c] = run; }
-    AT[sg * DK + c] = run;
+  // totals of the groups, then their prefix sums as (high, low) pairs: the rounding error of every addition is collected
+  // (Knuth's two-sum)
+  for (int it = tid; it < kGroups * DK; it += 256) {
+    const int c = it % DK, x = it / DK;
+    const float* l = &Ls[4 * x * LD + c];
+    Ch[(x + 1) * LD + c] = (l[0] + l[LD]) + (l[2 * LD] + l[3 * LD]);
   }
   __syncthreads();
-  for (int it = tid; it < 4 * DK; it += 256) {
-    const int c = it % DK, sg = it / DK;
-    float base = 0.f;
-    for (int x = 0; x < sg; ++x) base += AT[x * DK + c];
+  for (int c = tid; c < DK; c += 256) {
+    float hi = 0.f, lo = 0.f;
+    Ch[c] = 0.f; Cl[c] = 0.f;
 #pragma unroll
-    for (int t = 0; t < 16; ++t) Gs[(16 * sg + t) * LD + c] = (Gs[(16 * sg + t) * LD + c] + base) * kLog2e;
+    for (int x = 1; x <= kGroups; ++x) {
+      const float t = Ch[x * LD + c], sum = hi + t, part = sum - hi;
+      lo += (hi - (sum - part)) + (t - part);
+      hi = sum;
+      Ch[x * LD + c] = hi; Cl[x * LD + c] = lo;
+    }
   }
   // the part of the Aqk image above the diagonal tiles
   for (int idx = tid; idx < BS * (BS / 4); idx += 256) {
@@ -143,6 +161,15 @@ __device__ __forceinline__ void prep_simt_chunk(const TIn* __restrict__ q, const
     if (sq > r / 4) store4(aqk + kc_index<E>(r, 4 * sq, BS), WT::kg_store(0.f), WT::kg_store(0.f), WT::kg_store(0.f), WT::kg_store(0.f));
   }
   __syncthreads();
+
+  // exponent of gamma_t: the groups before t's, then its own group up to t
+  auto gamma_log2 = [&](int t, int c) {
+    float4 a = *reinterpret_cast<const float4*>(&Ls[(t & ~3) * LD + c]);
+#pragma unroll
+    for (int x = 1; x < 4; ++x)
+      if (x <= (t & 3)) a = add4(a, *reinterpret_cast<const float4*>(&Ls[((t & ~3) + x) * LD + c]));
+    return add4(*reinterpret_cast<const float4*>(&Ch[(t >> 2) * LD + c]), add4(*reinterpret_cast<const float4*>(&Cl[(t >> 2) * LD + c]), a));
+  };
 
   // The two matrices: 120 tiles below the diagonal, then the 16 on it; eight lanes per tile share its channels.
   const int l8 = lane & 7;
@@ -159,19 +186,25 @@ __device__ __forceinline__ void prep_simt_chunk(const TIn* __restrict__ q, const
       st = p - rt * (rt - 1) / 2;
       for (int u = l8; u < DK / 2; u += 8) {
         const int o_r = 4 * rt * LD + 2 * u, o_s = 4 * st * LD + 2 * u;
-        const float2 gref = *reinterpret_cast<const float2*>(&Gs[o_r]);
-        float2 kf[4];
+        auto at2 = [&](const float* m, int off) { return *reinterpret_cast<const float2*>(m + off); };
+        // from the last source token to the tile's first row: the groups in between and that row's own decay
+        const float2 h1 = at2(Ch, rt * LD + 2 * u), h0 = at2(Ch, (st + 1) * LD + 2 * u);
+        const float2 w1 = at2(Cl, rt * LD + 2 * u), w0 = at2(Cl, (st + 1) * LD + 2 * u), lr = at2(Ls, o_r);
+        float2 e = make_float2(((h1.x - h0.x) + (w1.x - w0.x)) + lr.x, ((h1.y - h0.y) + (w1.y - w0.y)) + lr.y);
+        float2 kf[4], tail = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 gj = *reinterpret_cast<const float2*>(&Gs[o_s + j * LD]), kj = *reinterpret_cast<const float2*>(&ks[o_s + j * LD]);
-          kf[j] = make_float2(kj.x * ex2(gref.x - gj.x), kj.y * ex2(gref.y - gj.y));
+        for (int j = 3; j >= 0; --j) {
+          const float2 kj = at2(ks, o_s + j * LD);
+          kf[j] = make_float2(kj.x * ex2(e.x + tail.x), kj.y * ex2(e.y + tail.y));
+          if (j > 0) tail = add2(tail, at2(Ls, o_s + j * LD));
         }
+        float2 head = make_float2(0.f, 0.f);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          float2 qi = *reinterpret_cast<const float2*>(&qs[o_r + i * LD]), ei = *reinterpret_cast<const float2*>(&es[o_r + i * LD]);
+          float2 qi = at2(qs, o_r + i * LD), ei = at2(es, o_r + i * LD);
           if (i > 0) {
-            const float2 gi = *reinterpret_cast<const float2*>(&Gs[o_r + i * LD]);
-            const float ax = ex2(gi.x - gref.x), ay = ex2(gi.y - gref.y);
+            head = add2(head, at2(Ls, o_r + i * LD));
+            const float ax = ex2(head.x), ay = ex2(head.y);
             qi.x *= ax; qi.y *= ay; ei.x *= ax; ei.y *= ay;
           }
 #pragma unroll
@@ -185,18 +218,20 @@ __device__ __forceinline__ void prep_simt_chunk(const TIn* __restrict__ q, const
       rt = st = p - 120;
       for (int u = l8; u < DK / 2; u += 8) {
         const int o_r = 4 * rt * LD + 2 * u;
-        float2 gg[4], kk[4];
+        float2 kk[4];                                      // k_j with the decay up to row i
+#pragma unroll
+        for (int i = 0; i < 4; ++i) kk[i] = *reinterpret_cast<const float2*>(&ks[o_r + i * LD]);
+        float2 span[3];                                    // exponents from rows 0, 1, 2 to row i
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          gg[i] = *reinterpret_cast<const float2*>(&Gs[o_r + i * LD]); kk[i] = *reinterpret_cast<const float2*>(&ks[o_r + i * LD]);
-        }
+          const float2 li = *reinterpret_cast<const float2*>(&Ls[o_r + i * LD]);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+          for (int j = 0; j < i; ++j) span[j] = j == i - 1 ? li : add2(span[j], li);
           const float2 qi = *reinterpret_cast<const float2*>(&qs[o_r + i * LD]), ei = *reinterpret_cast<const float2*>(&es[o_r + i * LD]);
 #pragma unroll
           for (int j = 0; j <= i; ++j) {
             float2 kd = kk[j];
-            if (j < i) { kd.x *= ex2(gg[i].x - gg[j].x); kd.y *= ex2(gg[i].y - gg[j].y); }
+            if (j < i) { kd.x *= ex2(span[j].x); kd.y *= ex2(span[j].y); }
             val[4 * i + j] = fmaf(qi.x, kd.x, fmaf(qi.y, kd.y, val[4 * i + j]));
             if (j < i) val[16 + 4 * i + j] = fmaf(ei.x, kd.x, fmaf(ei.y, kd.y, val[16 + 4 * i + j]));
           }
@@ -248,24 +283,29 @@ __device__ __forceinline__ void prep_simt_chunk(const TIn* __restrict__ q, const
     for (int r4 = 0; r4 < 4; ++r4)
       *reinterpret_cast<float4*>(&AT[tid * LT + 16 * i + 4 * r4]) = make_float4(x[4 * r4], x[4 * r4 + 1], x[4 * r4 + 2], x[4 * r4 + 3]);
   } else {
-    // meanwhile the other six warps: gamma_last, the query rows Qg and KG^T, which need G, q, k only
+    // meanwhile the other six warps: gamma_last, the query rows Qg and KG^T, which need the decays, q and k only
     const int z = tid - BS, nz = 256 - BS;
-    const float* glast = Gs + (BS - 1) * LD;
     for (int idx = z; idx < BS * nq; idx += nz) {          // tokens fastest: 16-byte pieces in a row
       const int t = idx % BS, c = 4 * (idx / BS);
-      const float4 G = *reinterpret_cast<const float4*>(&Gs[t * LD + c]), qq = *reinterpret_cast<const float4*>(&qs[t * LD + c]);
+      const float4 G = gamma_log2(t, c), qq = *reinterpret_cast<const float4*>(&qs[t * LD + c]);
       store4(wq + kc_index<E>(BS + t, c, 2 * BS), from_f32<TW>(scale * qq.x * ex2(G.x)), from_f32<TW>(scale * qq.y * ex2(G.y)),
              from_f32<TW>(scale * qq.z * ex2(G.z)), from_f32<TW>(scale * qq.w * ex2(G.w)));
     }
     for (int idx = z; idx < (BS / 4) * DK; idx += nz) {
       const int c = idx % DK, t = 4 * (idx / DK);
+      // from t + 3 to the chunk's last token: the groups after this one
+      const int x = t / 4 + 1;
+      float e = (Ch[kGroups * LD + c] - Ch[x * LD + c]) + (Cl[kGroups * LD + c] - Cl[x * LD + c]), tail = 0.f;
       float kg[4];
 #pragma unroll
-      for (int x = 0; x < 4; ++x) kg[x] = ks[(t + x) * LD + c] * ex2(glast[c] - Gs[(t + x) * LD + c]);
+      for (int y = 3; y >= 0; --y) {
+        kg[y] = ks[(t + y) * LD + c] * ex2(e + tail);
+        if (y > 0) tail += Ls[(t + y) * LD + c];
+      }
       store4(kgt + kc_index<E>(c, t, DK), WT::kg_store(kg[0]), WT::kg_store(kg[1]), WT::kg_store(kg[2]), WT::kg_store(kg[3]));
     }
     float* gl = P.gl + (size_t)ch * DK;
-    for (int c = z; c < DK; c += nz) gl[c] = ex2(glast[c]);
+    for (int c = z; c < DK; c += nz) gl[c] = ex2(Ch[kGroups * LD + c] + Cl[kGroups * LD + c]);
   }
   __syncthreads();
   for (int pass = 0; pass < 2; ++pass) {                   // N^T in place over T^T: 6 blocks x 16 rows t x 4 row quads
@@ -288,7 +328,7 @@ __device__ __forceinline__ void prep_simt_chunk(const TIn* __restrict__ q, const
   // E = b k gamma in place (needed from here on)
   for (int idx = tid; idx < BS * nq; idx += 256) {
     const int t = idx / nq, c = 4 * (idx % nq);
-    const float4 G = *reinterpret_cast<const float4*>(&Gs[t * LD + c]);
+    const float4 G = gamma_log2(t, c);
     float4* ep = reinterpret_cast<float4*>(&es[t * LD + c]);
     *ep = mul4(*ep, make_float4(ex2(G.x), ex2(G.y), ex2(G.z), ex2(G.w)));
   }
@@ -391,7 +431,7 @@ template <typename TIn, typename TW, typename Seqs>
 int launch_typed(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
                  const WsLayout& L, const WsPtrs& P, int B, int S, int H, int HK, int64_t in_bs, float scale,
                  bool only_flagged, const Seqs& seqs, cudaStream_t st) {
-  const size_t smem = ((size_t)4 * kChunk * row_stride(L.DK) + 2 * kChunk * LT) * sizeof(float);
+  const size_t smem = ((size_t)(4 * kChunk + 2 * (kGroups + 1)) * row_stride(L.DK) + 2 * kChunk * LT) * sizeof(float);
   const TIn* tq = static_cast<const TIn*>(q); const TIn* tk = static_cast<const TIn*>(k);
   const TIn* tv = static_cast<const TIn*>(v); const TIn* tb = static_cast<const TIn*>(b);
   const TIn* tw = static_cast<const TIn*>(w);

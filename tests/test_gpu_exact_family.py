@@ -57,3 +57,32 @@ def test_workspace_for_whole_chunks_keeps_the_decoded_tail():
         assert rc == 0
         res.append((o.cpu(), s.cpu()))
     assert orc.rel_max_err(res[0][0], res[1][0]) < 2e-5 and orc.rel_max_err(res[0][1], res[1][1]) < 2e-5
+
+
+@pytest.mark.parametrize("gate", [None, -20.0, -100.0, -1e4, -1e6, -1e30, float("-inf")])
+@pytest.mark.parametrize("form", ["tail", "packed", "whole"])
+def test_strong_gates_keep_the_ones_after_them(gate, form):
+    """A gate that wipes a channel must not cost the later, ordinary ones any digits: the recurrence forms every decay by
+    itself. Against it in 64 bits the float32 outputs are sums of a few hundred rounded terms, 1.6e-7 of their norm when
+    evaluated token by token; 1e-6 leaves room for another order and is below what prefix sums lose from -100 on (5e-6)."""
+    D, H = 64, 2
+    lengths = {"tail": [64 + 40], "packed": [40, 3, 64, 41], "whole": [128]}[form]
+    T = sum(lengths)
+    q, k, v, g, b, w = orc.make_inputs(1, T, H, D, D, seed=5)
+    if gate is not None:                                    # whole tokens, single channels, neighbours inside a group of four
+        g[:, 9::31] = gate
+        g[:, 10::37, :, ::3] = gate
+        g[:, 17::29, :, 1::2] = gate
+    s0 = golden_state(len(lengths), H, D, D, 1, 0.3)
+    dev = [t.to(DEV) for t in (q, k, v, g, b, w)]
+    cu = [0]
+    for n in lengths:
+        cu.append(cu[-1] + n)
+    o, s = gdn2.gdn2_attention(*dev, initial_state=s0.to(DEV), output_final_state=True,
+                               **({"cu_seqlens": cu} if form == "packed" else {}))
+    _cabi.kernels().check_device_status()
+    for i, n in enumerate(lengths):
+        part = [t[:, cu[i]:cu[i + 1]] for t in (q, k, v, g, b, w)]
+        o_ref, s_ref = orc.recurrence(*part, initial_state=s0[i:i + 1], dtype=torch.float64)
+        assert orc.rel_fro_err(o[:, cu[i]:cu[i + 1]].cpu(), o_ref) < 1e-6
+        assert orc.rel_fro_err(s[i:i + 1].cpu(), s_ref) < 1e-6
