@@ -370,14 +370,12 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
       for (; n < NC; ++n) {
         if (n >= *limit) break;                              // a transition block whose matrix has vanished stops early
         const uint32_t ph = n & 1;
-        // the Un pass of chunk n has consumed its U^T buffer
-        bool ok = tc::mbar_wait(&s.bar_un, ph, &s.abort_flag, status, kWaitUn);
-        if (ok && n + 2 < *limit) { load_ut(n + 2); ut_ahead = n + 2; }
-        // every product of chunk n has completed: refill the operand buffers it read
-        ok = ok && tc::mbar_wait(&s.bar_m2, ph, &s.abort_flag, status, kWaitM2);
-        if (ok) {
+        // Every product of chunk n has completed, the last of them after the Un pass: refill the buffers they and that
+        // pass read. The Un hand-off itself is not waited for: it can complete twice before this thread looks, because
+        // chunk n + 1 needs nothing from here until its last product, and a wait sees a phase's parity only.
+        if (tc::mbar_wait(&s.bar_m2, ph, &s.abort_flag, status, kWaitM2)) {
           if (n + 1 < *limit) { load_aqk(n + 1); aqk_ahead = n + 1; }
-          if (n + 2 < *limit) { load_wq(n + 2); load_kgt(n + 2); ahead = n + 2; }
+          if (n + 2 < *limit) { load_wq(n + 2); load_ut(n + 2); load_kgt(n + 2); ahead = ut_ahead = n + 2; }
         }
       }
       // Copies issued for chunks that no one will consume any more (the limit dropped after they were issued)
@@ -564,6 +562,9 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
         tc::tmem_st16(t_lane + kColUn16 + tokp / 2, p16);
         tc::tmem_st_wait();
         tc::tc_fence_before_sync();
+        // gamma arrived with KG^T. Waited for here and not in the state pass: once this hand-off is given the buffer may be
+        // refilled, and its barrier complete a second time, before this warp would look.
+        if (!output_only) tc::mbar_wait(&s.bar_kgt[b], ph2, &s.abort_flag, status, kWaitKgt);
         warp_arrive(&s.bar_un, lane);
       }
 
@@ -583,7 +584,6 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
       }
 
       // ---- new state S <- gamma_C * S + P, its bf16 operand copy for the next chunk, optional snapshot
-      tc::mbar_wait(&s.bar_kgt[b], ph2, &s.abort_flag, status, kWaitKgt);   // gamma arrived with KG^T
       tc::mbar_wait(&s.bar_m3[part], ph, &s.abort_flag, status, kWaitM3);
       tc::tc_fence_after_sync();
       {
@@ -629,7 +629,8 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
           // Has the running transition matrix vanished? All 256 compute threads agree through one barrier with
           // an AND reduction. If it has, chunks n + 1 and n + 2 are still walked (other warps of the block are
           // already working on them) and every role stops before chunk n + 3: they all pass a hand-off of chunk
-          // n + 2 that is ordered after this store before they look at the limit again.
+          // n + 2 that is ordered after this store (the copy thread's through the issuer) before they look at the
+          // limit again.
           float m = 0.f;
 #pragma unroll
           for (int i = 0; i < 64; ++i) m = fmaxf(m, fabsf(S[i]));
