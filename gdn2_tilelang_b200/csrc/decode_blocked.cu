@@ -117,7 +117,7 @@ __device__ __forceinline__ bool table_sync_or(bool pred) {
 
 // Bounded wait for hand-offs that have thousands of cycles of slack: the polling thread sleeps between probes
 // instead of competing with the sweep warps for issue slots.
-__device__ __forceinline__ bool mbar_wait_relaxed(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+[[nodiscard]] __device__ __forceinline__ bool mbar_wait_relaxed(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                                   uint32_t* status_word, uint32_t code) {
   if (tc::mbar_try_wait(bar, parity)) return true;
   const long long t_begin = clock64();
@@ -221,8 +221,9 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
       const int stride = gridDim.x;
       int tile = from_tile(blockIdx.x);
       int next = tile < ntiles ? from_tile(tile + stride) : ntiles;
-      if (tile < ntiles) load_tile(tile, 0);
-      if (next < ntiles) load_tile(next, 1);
+      int loaded = 0;                                    // tiles whose copies were issued
+      if (tile < ntiles) { load_tile(tile, 0); ++loaded; }
+      if (next < ntiles) { load_tile(next, 1); ++loaded; }
       for (int it = 0; tile < ntiles; ++it) {
         const int buf = it & 1;
         if (!mbar_wait_relaxed(&s.tile_done[buf], (it >> 1) & 1, &s.abort_flag, status, kWaitDone)) break;
@@ -235,11 +236,14 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
         if (after < ntiles) {
           tc::bulk_wait_read_all();                      // the buffer may be overwritten once the store has read it
           load_tile(after, buf);
+          ++loaded;
         }
         tile = next;
         next = after;
       }
       tc::bulk_wait_all();
+      // a block that gave up leaves copies behind: they must land before it gives its shared memory back
+      for (int x = loaded > 1 ? loaded - 2 : 0; x < loaded; ++x) tc::mbar_drain(&s.tile_full[x & 1], (x >> 1) & 1);
     }
   } else if (wid >= 8) {
     // =============================== table warps: thread = key / value channel =================
@@ -381,7 +385,7 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
         }
         warp_arrive(&s.tab_full[step & 1], lane);
       }
-      if (s.abort_flag) break;
+      // (a block that gave up is left at the next step's table_sync_or, by all four warps together)
     }
   } else {
     // =============================== sweep warps ================================================

@@ -358,10 +358,24 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
 #pragma unroll
     for (int u = 0; u < 16; ++u) { vr[u] = __ldg(vp + u * vpstride); wr[u] = __ldg(wp + u * vpstride); }
   }
-  // one warp polls the MMA barrier; the rest sleep at the block barrier instead of spending issue slots
-  if (wid == 0) tc::mbar_wait(&s.bar_m1, 0, &s.abort_flag, status, 0x1000u);
-  __syncthreads();
-  tc::tc_fence_after_sync();
+  // One warp polls the MMA barrier; the rest sleep at the block barrier instead of spending issue slots. If the wait runs
+  // out the whole block leaves: the products may still be under way, so tensor memory is not read, and given back only
+  // when they are through (or a second limit has passed).
+  auto products_done = [&](uint64_t* bar, uint32_t parity, uint32_t code) {
+    bool ok = true;
+    if (wid == 0) ok = tc::mbar_wait_warp(bar, parity, &s.abort_flag, status, code);
+    if (!__syncthreads_or(ok ? 0 : 1)) {
+      tc::tc_fence_after_sync();
+      return true;
+    }
+    if (wid == 0) {
+      tc::mbar_drain(bar, parity);
+      __syncwarp();
+      tc::tmem_dealloc(tm, kTmemCols);
+    }
+    return false;
+  };
+  if (!products_done(&s.bar_m1, 0, 0x1000u)) return;
 
   // ---- 2b. read back: lane = row (0..63 Tm, 64..127 Aqk); a warp spans sub-blocks i0 and i0+1, and
   //          the two threads of a row split the four 16-column groups.
@@ -529,16 +543,14 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
   __syncthreads();
 
   // ---- 4. MMA2 (tf32): W^T at TMEM columns 0..63, U^T at 64..127
-  if (wid < 2 && !s.abort_flag) {  // warp 0: W^T, warp 1: U^T
+  if (wid < 2) {  // warp 0: W^T, warp 1: U^T
     tc::tc_fence_after_sync();
     constexpr uint32_t idesc = tc::instr_desc(2, 128, BS);
     tc::mma_tf32_ktile_warp(tc::tmem_addr(tm, 0, 64 * wid), tc::smem_u32(wid == 0 ? s.y.et : s.x.sol.zt), D,
                             tc::smem_u32(s.x.sol.ai), BS, BS, idesc);
     tc::mma_commit_warp(&s.bar_m2);
   }
-  if (wid == 0) tc::mbar_wait(&s.bar_m2, 0, &s.abort_flag, status, 0x2000u);
-  __syncthreads();
-  tc::tc_fence_after_sync();
+  if (!products_done(&s.bar_m2, 0, 0x2000u)) return;
 
   // ---- 5. W and Qg rows into the WQ staging image (E^T is dead now), U^T straight to global; each
   //         thread handles the 32 tokens of its half
@@ -577,7 +589,7 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
   __syncthreads();
   // WQ record: 16 K chunks x 128 rows x 16 bytes; every thread copies 8 pieces with 128-bit accesses
   // (16 consecutive threads cover 256 contiguous bytes) and nothing waits on them
-  if (!s.abort_flag) {
+  {
     char* g_wq = P.wq + (size_t)ch * (2 * BS * D * 2);
     const char* stage = reinterpret_cast<const char*>(s.y.wq);
 #pragma unroll
@@ -616,15 +628,13 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
     tc::fence_async_smem();
     tc::tc_fence_before_sync();
     __syncthreads();
-    if (wid == 1 && !s.abort_flag) {
+    if (wid == 1) {
       tc::tc_fence_after_sync();
       constexpr uint32_t idesc = tc::instr_desc(2, 128, BS);
       tc::mma_tf32_ktile_warp(tc::tmem_addr(tm, 0, 64), tc::smem_u32(s.x.sol.zt), D, tc::smem_u32(s.x.sol.ai), BS, BS, idesc);
       tc::mma_commit_warp(&s.bar_m2v);
     }
-    if (wid == 0) tc::mbar_wait(&s.bar_m2v, (hr - 1) & 1, &s.abort_flag, status, 0x2000u);
-    __syncthreads();
-    tc::tc_fence_after_sync();
+    if (!products_done(&s.bar_m2v, (hr - 1) & 1, 0x2000u)) return;
     {
       char* ut_g = P.ut + (size_t)(((int64_t)ib * HK * rep + (int64_t)ih * rep + hr) * NC + n) * (D * BS * 2) + c * 16;
       float val[32];

@@ -212,9 +212,16 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
   __syncthreads();
   if (wid == 0 && NC > 0) { load_wq_ut(0); load_aqk_kgt(0); }
 
+  // A wait that ran out leaves `ok` false in its warp: it computes on what is there (the status word says that the results
+  // are void) and the block leaves together at the end of the chunk.
+  auto wait_all = [&](uint64_t* bar, uint32_t parity, uint32_t code) {
+    return tc::mbar_wait_warp(bar, parity, &abort_flag, status, code);
+  };
   float2 acc[CT / 2];
+  int wq_ahead = 0, kgt_ahead = 0;                         // last chunk whose copies were issued
   for (int n = 0; n < NC; ++n) {
     const uint32_t ph = n & 1;
+    bool ok = true;
     if (hs != nullptr) {
       float* hp = hs + (((size_t)ib * NC + n) * H + ih) * DK * DV + lo;
       for (int idx = tid; idx < DK * NVT; idx += 256) {
@@ -225,7 +232,7 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
     // ---- row of W S or Qg S
 #pragma unroll
     for (int x = 0; x < CT / 2; ++x) acc[x] = make_float2(0.f, 0.f);
-    tc::mbar_wait(&bar_wq, ph, &abort_flag, status, kWaitSimtWq);
+    ok = wait_all(&bar_wq, ph, kWaitSimtWq);
     const float4* wrow = reinterpret_cast<const float4*>(s.wq) + row;
 #pragma unroll 4
     for (int c4 = 0; c4 < DK / 4; ++c4) {
@@ -238,20 +245,24 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
         for (int x = 0; x < CT / 2; ++x) acc[x] = ffma2(make_float2(wv[y], wv[y]), st[x], acc[x]);
       }
     }
-    tc::mbar_wait(&bar_ut, ph, &abort_flag, status, kWaitSimtUt);
+    ok = ok && wait_all(&bar_ut, ph, kWaitSimtUt);
     if (!is_q) {
       const float* u = s.ut + ((row >> 2) * NVT + col0) * 4 + (row & 3);
       float2* un = reinterpret_cast<float2*>(&s.Un[row * NVT + col0]);
 #pragma unroll
       for (int x = 0; x < CT / 2; ++x) un[x] = make_float2(u[8 * x] - acc[x].x, u[8 * x + 4] - acc[x].y);
     }
-    __syncthreads();                                       // Un complete; the state and W | Qg have been read
-    if (wid == 0 && n + 1 < NC && !abort_flag) load_wq_ut(n + 1);
+    // Un complete; the state and W | Qg have been read
+    if (__syncthreads_or(ok ? 0 : 1)) break;
+    if (n + 1 < NC) {
+      wq_ahead = n + 1;
+      if (wid == 0) load_wq_ut(n + 1);
+    }
 
     if (is_q) {
       // ---- o = Qg S + tril(Aqk) Un: source tokens up to the warp's last row (Aqk is zero above the diagonal)
       const int r = row - kChunk;
-      tc::mbar_wait(&bar_aqk, ph, &abort_flag, status, kWaitSimtAqk);
+      ok = wait_all(&bar_aqk, ph, kWaitSimtAqk);
       const float4* arow = reinterpret_cast<const float4*>(s.aqk) + r;
       const int tq = ((r & ~31) + 32) / 4;
 #pragma unroll 4
@@ -277,7 +288,7 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
       }
     } else {
       // ---- S <- gamma_C S + KG^T Un, this thread's channel(s)
-      tc::mbar_wait(&bar_kgt, ph, &abort_flag, status, kWaitSimtKgt);
+      ok = wait_all(&bar_kgt, ph, kWaitSimtKgt);
       for (int c = row; c < DK; c += kChunk) {
         float2* st = reinterpret_cast<float2*>(&s.St[c * NVT + col0]);
         const float gm = s.gl[c];
@@ -299,8 +310,16 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
         for (int x = 0; x < CT / 2; ++x) st[x] = acc[x];
       }
     }
-    __syncthreads();                                       // the new state is complete; Un, Aqk and KG have been read
-    if (wid == 0 && n + 1 < NC && !abort_flag) load_aqk_kgt(n + 1);
+    // the new state is complete; Un, Aqk and KG have been read
+    if (__syncthreads_or(ok ? 0 : 1)) break;
+    if (n + 1 < NC) {
+      kgt_ahead = n + 1;
+      if (wid == 0) load_aqk_kgt(n + 1);
+    }
+  }
+  if (wid == 0 && NC > 0) {                                // copies that no one waited for must land before the block ends
+    tc::mbar_drain(&bar_wq, wq_ahead & 1); tc::mbar_drain(&bar_ut, wq_ahead & 1);
+    tc::mbar_drain(&bar_kgt, kgt_ahead & 1); tc::mbar_drain(&bar_aqk, kgt_ahead & 1);
   }
   if (sT != nullptr) {
     for (int idx = tid; idx < DK * NVT; idx += 256) {

@@ -90,6 +90,7 @@ struct ScanTcSmem {
   uint64_t bar_m1, bar_m3[2], bar_m2;                   // MMA completion: (W S)^T; the two key-channel halves of P; O
   uint64_t bar_sb[2], bar_un;                           // compute threads -> issuer: S^T by key-channel half, Un^T
   uint64_t bar_of;                                      // output warps -> issuer: the O accumulator has been read out
+  uint64_t bar_drain;                                   // every product of the block
   uint32_t tmem_base;
   int abort_flag;
   int last_big[kComputeThreads / 32];                   // transition blocks: last chunk after which an entry was still >= kVanish
@@ -140,6 +141,21 @@ __device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
 }
 // barrier among the 128 output threads only (hardware barrier 2)
 __device__ __forceinline__ void output_sync() { asm volatile("bar.sync 2, 128;" ::: "memory"); }
+// the same barrier fused with an AND over one predicate per thread
+__device__ __forceinline__ bool output_all(bool pred) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.and.pred q, 2, 128, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t"
+      "}"
+      : "=r"(r)
+      : "r"((uint32_t)pred)
+      : "memory");
+  return r != 0;
+}
 // barrier among the 256 compute threads (hardware barrier 3) fused with an AND over one predicate per thread
 __device__ __forceinline__ bool compute_all(bool pred) {
   uint32_t r;
@@ -330,6 +346,7 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
     for (int i = 0; i < 2; ++i) { tc::mbar_init(&s.bar_m3[i], 1); tc::mbar_init(&s.bar_sb[i], kComputeThreads / 64); }
     tc::mbar_init(&s.bar_of, kOutputThreads / 32);
     tc::mbar_init(&s.bar_un, kComputeThreads / 32);
+    tc::mbar_init(&s.bar_drain, 1);
     s.abort_flag = 0;
     s.nc_limit = NC;
     tc::mbar_init_fence();
@@ -363,32 +380,27 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
         tc::bulk_g2s(s.aqk, g_aqk + (size_t)n * kAqkBytes, kAqkBytes, &s.bar_aqk);
       };
       const volatile int* limit = &s.nc_limit;
-      int ahead = 0, ut_ahead = 0, aqk_ahead = 0;            // highest chunk whose WQ + KG^T, U^T and Aqk copies were issued
+      int ahead = 0, aqk_ahead = 0;                          // highest chunk whose WQ + KG^T + U^T and Aqk copies were issued
       load_wq(0); load_ut(0); load_kgt(0); load_aqk(0);
-      if (NC > 1) { load_wq(1); load_ut(1); load_kgt(1); ahead = ut_ahead = 1; }
-      int n = 0;
-      for (; n < NC; ++n) {
+      if (NC > 1) { load_wq(1); load_ut(1); load_kgt(1); ahead = 1; }
+      for (int n = 0; n < NC; ++n) {
         if (n >= *limit) break;                              // a transition block whose matrix has vanished stops early
         const uint32_t ph = n & 1;
         // Every product of chunk n has completed, the last of them after the Un pass: refill the buffers they and that
         // pass read. The Un hand-off itself is not waited for: it can complete twice before this thread looks, because
         // chunk n + 1 needs nothing from here until its last product, and a wait sees a phase's parity only.
-        if (tc::mbar_wait(&s.bar_m2, ph, &s.abort_flag, status, kWaitM2)) {
-          if (n + 1 < *limit) { load_aqk(n + 1); aqk_ahead = n + 1; }
-          if (n + 2 < *limit) { load_wq(n + 2); load_ut(n + 2); load_kgt(n + 2); ahead = ut_ahead = n + 2; }
-        }
+        if (!tc::mbar_wait(&s.bar_m2, ph, &s.abort_flag, status, kWaitM2)) break;
+        if (n + 1 < *limit) { load_aqk(n + 1); aqk_ahead = n + 1; }
+        if (n + 2 < *limit) { load_wq(n + 2); load_ut(n + 2); load_kgt(n + 2); ahead = n + 2; }
       }
-      // Copies issued for chunks that no one will consume any more (the limit dropped after they were issued)
-      // must land before the block gives its shared memory back.
-      if (!s.abort_flag) {
-        for (int c = n; c <= ahead; ++c) {
-          tc::mbar_wait(&s.bar_wq[c & 1], (c >> 1) & 1, &s.abort_flag, status, kWaitWq);
-          if (!output_only) tc::mbar_wait(&s.bar_kgt[c & 1], (c >> 1) & 1, &s.abort_flag, status, kWaitKgt);
-        }
-        if (!transition)
-          for (int c = n; c <= ut_ahead; ++c) tc::mbar_wait(&s.bar_ut[c & 1], (c >> 1) & 1, &s.abort_flag, status, kWaitUt);
-        if (aqk_ahead >= n && n < NC) tc::mbar_wait(&s.bar_aqk, aqk_ahead & 1, &s.abort_flag, status, kWaitAqk);
+      // The last copy into every buffer must have landed before the block gives its shared memory back: copies issued for
+      // chunks that no one consumes any more (the limit dropped, or a wait ran out) are still on their way.
+      for (int c = ahead > 0 ? ahead - 1 : 0; c <= ahead; ++c) {
+        tc::mbar_drain(&s.bar_wq[c & 1], (c >> 1) & 1);
+        if (!output_only) tc::mbar_drain(&s.bar_kgt[c & 1], (c >> 1) & 1);
+        if (!transition) tc::mbar_drain(&s.bar_ut[c & 1], (c >> 1) & 1);
       }
+      tc::mbar_drain(&s.bar_aqk, aqk_ahead & 1);
     }
   } else if (wid == 8) {
     // =============================== issuer: every MMA, in critical-path order ==================
@@ -401,15 +413,16 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
       const uint32_t a_aqk = tc::smem_u32(s.aqk);
       const uint32_t t_ws = tc::tmem_addr(tm, 0, kColWs), t_o = tc::tmem_addr(tm, 0, kColO);
       auto wait_all = [&](uint64_t* bar, uint32_t parity, uint32_t code) {
-        return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity, &s.abort_flag, status, code)) != 0;
+        return tc::mbar_wait_warp(bar, parity, &s.abort_flag, status, code);
       };
-      for (int n = 0; n < NC; ++n) {
+      bool ok = true;
+      for (int n = 0; ok && n < NC; ++n) {
         if (n >= *(volatile int*)&s.nc_limit) break;         // uniform: every lane reads the same word
         const int b = n & 1;
         const uint32_t ph = n & 1, ph2 = (n >> 1) & 1;
         // (W S)^T first, one key-channel half of S^T as soon as it is in place: the Un pass waits for nothing else.
         // The query rows' half of the product runs under that pass.
-        bool ok = wait_all(&s.bar_wq[b], ph2, kWaitWq);
+        ok = wait_all(&s.bar_wq[b], ph2, kWaitWq);
         const uint32_t b_wq = tc::smem_u32(s.wq[b]);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -444,6 +457,10 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
           tc::mma_commit_warp(&s.bar_m2);
         }
       }
+      // no product is under way when the block gives its shared and tensor memory back, whichever wait ended the loops
+      tc::mma_commit_warp(&s.bar_drain);
+      tc::mbar_drain(&s.bar_drain, 0);
+      __syncwarp();
     }
   } else if (wid >= 10) {
     // =============================== output warps: O^T -> bf16 rows in global memory =============
@@ -460,18 +477,18 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
 #pragma unroll
         for (int x = 0; x < 8; ++x) asm volatile("prefetch.global.L2 [%0];" ::"l"(gp_ + (size_t)(8 * x) * norm.row_stride));
       }
-      tc::mbar_wait(&s.bar_m2, n & 1, &s.abort_flag, status, kWaitM2);
+      // the four warps leave the loop together; past this barrier the previous chunk's rows have left the staging buffer
+      if (!output_all(tc::mbar_wait_warp(&s.bar_m2, n & 1, &s.abort_flag, status, kWaitM2))) break;
       tc::tc_fence_after_sync();
       tc::tmem_ld32(t_o, *reinterpret_cast<float(*)[32]>(&ov[0]));
       tc::tmem_ld32(t_o + 32, *reinterpret_cast<float(*)[32]>(&ov[32]));
       tc::tmem_ld_wait();
       tc::tc_fence_before_sync();
       if (n + 1 < NC) warp_arrive(&s.bar_of, lane);        // the accumulator may be overwritten by the next MMA1
-      output_sync();                                       // the previous chunk's rows have left the staging buffer
 #pragma unroll
       for (int i = 0; i < 64; ++i) s.ostage[i * D + dv] = __float2bfloat16_rn(ov[i]);
       output_sync();
-      if (write_o && !s.abort_flag) {
+      if (write_o) {
         // 64 rows x 256 bytes = 1024 16-byte pieces, 8 per thread, 128-bit coalesced stores
         __nv_bfloat16* obase = o + ((size_t)(o_row0 + (int64_t)n * BS) * H + ih) * D;
         if (norm.gate == nullptr) {
@@ -518,7 +535,12 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
     }
     tc::tc_fence_before_sync();
     warp_arrive(&s.bar_sb[part], lane);
-    for (int n = 0; n < NC; ++n) {
+    auto wait_all = [&](uint64_t* bar, uint32_t parity, uint32_t code) {
+      return tc::mbar_wait_warp(bar, parity, &s.abort_flag, status, code);
+    };
+    // After a wait that ran out a warp leaves the loop: it touches tensor memory no more and gives no hand-off.
+    int n = 0;
+    for (; n < NC; ++n) {
       if (n >= *(volatile int*)&s.nc_limit) break;
       const int b = n & 1;
       const uint32_t ph = n & 1, ph2 = (n >> 1) & 1;
@@ -536,14 +558,14 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
       // both the state update and the output product
       uint4 uraw[4];
       if (!transition) {
-        tc::mbar_wait(&s.bar_ut[b], ph2, &s.abort_flag, status, kWaitUt);
+        if (!wait_all(&s.bar_ut[b], ph2, kWaitUt)) break;
 #pragma unroll
         for (int j = 0; j < 4; ++j) uraw[j] = *reinterpret_cast<const uint4*>(&s.ut[b][((tokp / 8 + j) * D + dv) * 8]);
       } else {
 #pragma unroll
         for (int j = 0; j < 4; ++j) uraw[j] = make_uint4(0u, 0u, 0u, 0u);
       }
-      tc::mbar_wait(&s.bar_m1, ph, &s.abort_flag, status, kWaitM1);
+      if (!wait_all(&s.bar_m1, ph, kWaitM1)) break;
       tc::tc_fence_after_sync();
       {
         float ws[32];
@@ -564,7 +586,7 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
         tc::tc_fence_before_sync();
         // gamma arrived with KG^T. Waited for here and not in the state pass: once this hand-off is given the buffer may be
         // refilled, and its barrier complete a second time, before this warp would look.
-        if (!output_only) tc::mbar_wait(&s.bar_kgt[b], ph2, &s.abort_flag, status, kWaitKgt);
+        if (!output_only && !wait_all(&s.bar_kgt[b], ph2, kWaitKgt)) break;
         warp_arrive(&s.bar_un, lane);
       }
 
@@ -579,12 +601,11 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
           tc::tc_fence_before_sync();
           warp_arrive(&s.bar_sb[part], lane);
         }
-        if (s.abort_flag) break;
         continue;
       }
 
       // ---- new state S <- gamma_C * S + P, its bf16 operand copy for the next chunk, optional snapshot
-      tc::mbar_wait(&s.bar_m3[part], ph, &s.abort_flag, status, kWaitM3);
+      if (!wait_all(&s.bar_m3[part], ph, kWaitM3)) break;
       tc::tc_fence_after_sync();
       {
         const float* gln = s.gl[n & 3];
@@ -638,8 +659,13 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
           else if (tid == 0 && n + 3 < s.nc_limit) s.nc_limit = n + 3;
         }
       }
-      if (s.abort_flag) break;                             // per thread: no block-level barrier in this loop
     }
+    // a warp that left early still owes the others their barrier of every chunk that is left
+    if (transition)
+      for (; n < NC && n < *(volatile int*)&s.nc_limit; ++n) {
+        compute_all(false);
+        last_big = n;
+      }
     if (lane == 0) s.last_big[wid] = last_big;
   }
 

@@ -48,7 +48,12 @@ selftest_kernel(const float* __restrict__ a, const float* __restrict__ bt, float
     tc::mbar_expect_tx(&s.bar_copy, M * K * 4);
     tc::bulk_g2s(s.raw_a, a, M * K * 4, &s.bar_copy);
   }
-  tc::mbar_wait(&s.bar_copy, 0, &s.abort_flag, status, 0x1u);
+  if (__syncthreads_or(tc::mbar_wait_warp(&s.bar_copy, 0, &s.abort_flag, status, 0x1u) ? 0 : 1)) {
+    tc::mbar_drain(&s.bar_copy, 0);
+    __syncwarp();
+    if (wid == 0) tc::tmem_dealloc(tm, 512);
+    return;
+  }
 
   // build the operand images: thread = row
   {
@@ -79,7 +84,7 @@ selftest_kernel(const float* __restrict__ a, const float* __restrict__ bt, float
   tc::tc_fence_before_sync();
   __syncthreads();
 
-  if (tid == 0 && !s.abort_flag) {
+  if (tid == 0) {
     tc::tc_fence_after_sync();
     tc::mma_f16_ts_ktile(tc::tmem_addr(tm, 0, 384), tc::tmem_addr(tm, 0, 320), tc::smem_u32(s.b16), N, K,
                          tc::instr_desc(1, M, N), false);
@@ -92,7 +97,12 @@ selftest_kernel(const float* __restrict__ a, const float* __restrict__ bt, float
                        tc::instr_desc(2, M, 64), false);
     tc::mma_commit(&s.bar_mma);
   }
-  tc::mbar_wait(&s.bar_mma, 0, &s.abort_flag, status, 0x2u);
+  if (__syncthreads_or(tc::mbar_wait_warp(&s.bar_mma, 0, &s.abort_flag, status, 0x2u) ? 0 : 1)) {
+    tc::mbar_drain(&s.bar_mma, 0);
+    __syncwarp();
+    if (wid == 0) tc::tmem_dealloc(tm, 512);
+    return;
+  }
   tc::tc_fence_after_sync();
 
   const uint32_t lane_base = (wid & 3) * 32;

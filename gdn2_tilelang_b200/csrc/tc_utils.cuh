@@ -49,7 +49,7 @@ constexpr long long kWaitCycles = 400LL * 1000 * 1000;
 // Bounded wait. `abort_flag` is a shared-memory word shared by the whole block: once any wait has
 // run out every later wait returns false at once, so a broken pipeline drains in bounded time.
 // On the first failure `code` is OR-ed into the device status word.
-__device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+[[nodiscard]] __device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                                 uint32_t* status_word, uint32_t code, long long limit_cycles) {
   if (mbar_try_wait(bar, parity)) return true;   // the common case costs one probe and no shared-memory load
   if (*abort_flag) return false;
@@ -64,9 +64,23 @@ __device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, 
     }
   }
 }
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                          uint32_t* status_word, uint32_t code) {
+[[nodiscard]] __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                                        uint32_t* status_word, uint32_t code) {
   return mbar_wait_limit(bar, parity, abort_flag, status_word, code, kWaitCycles);
+}
+// The same for a whole warp, with one result: the lanes leave a wait by different exits and at different times, and what
+// follows is usually warp-collective (.sync.aligned tensor-memory instructions, shuffles). Only a warp whose wait has
+// succeeded may touch what the wait stands for.
+[[nodiscard]] __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                                             uint32_t* status_word, uint32_t code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status_word, code)) != 0;
+}
+// Waits for asynchronous work of the block's own (copies, products) before the block gives up its shared or tensor memory:
+// bounded, and whatever the abort flag says, because a block that gave up leaves such work behind. A barrier whose phase
+// has completed costs one probe.
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, parity) && clock64() - t0 <= kWaitCycles) {}
 }
 
 // ------------------------------------------------------------------ proxy / tcgen05 fences
