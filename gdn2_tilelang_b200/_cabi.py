@@ -35,6 +35,7 @@ SIGNATURES = {
     "gdn2_status_string": (ctypes.c_char_p, [_int]),
     "gdn2_last_cuda_error": (_int, []),
     "gdn2_decode": (_int, [_vp] * 8 + [_i64] * 8 + [_f32, _int, _vp]),
+    "gdn2_decode_tail": (_int, [_vp] * 8 + [_i64] * 8 + [_f32, _int, _vp]),
     "gdn2_prefill_workspace_bytes": (_sz, [_i64] * 6 + [_int, _int]),
     "gdn2_prefill_scan_segments": (_int, [_i64] * 5 + [_int, _int]),
     "gdn2_prefill_scan_launches": (_int, [_i64] * 5 + [_int, _int]),
@@ -231,7 +232,9 @@ class NativeKernels:
     def decode(self, q, k, v, g, b, w, state, scale: float, out=None) -> torch.Tensor:
         """``[B,n,H,D]`` tokens, ``state [B,H,DK,DV]`` fp32 contiguous, updated in place. Returns ``o``.
 
-        ``out`` may be a ``[B,n,H,DV]`` view into a longer preallocated sequence tensor.
+        ``out`` may be a ``[B,n,H,DV]`` view into a longer preallocated sequence tensor. The tokens are then a
+        prompt's ragged tail, queued on or beside the streams of its prefill, and launched plainly like the rest of it
+        (``gdn2_decode_tail``).
         """
         _require_cuda(q, k, v, g, b, w, state)
         B, n, HK, DK = q.shape
@@ -252,9 +255,9 @@ class NativeKernels:
             if o is not out or out.dtype != v.dtype or tuple(out.shape) != (B, n, H, DV):
                 raise ValueError("`out` must be a [B,n,H,DV] view with dense [n,H,DV] blocks in v's dtype")
         with _on_device(q.device):
-            rc = self.lib.gdn2_decode(q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), b.data_ptr(),
-                                      w.data_ptr(), state.data_ptr(), o.data_ptr(), B, n, H, HK, DK, DV, in_bs, o_bs,
-                                      float(scale), code, self._stream(q))
+            fn = self.lib.gdn2_decode if out is None else self.lib.gdn2_decode_tail
+            rc = fn(q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), b.data_ptr(), w.data_ptr(), state.data_ptr(),
+                    o.data_ptr(), B, n, H, HK, DK, DV, in_bs, o_bs, float(scale), code, self._stream(q))
         _check(self.lib, rc, "gdn2_decode")
         self.launches += 1
         return o

@@ -150,6 +150,12 @@ int gdn2_decode(const void* q, const void* k, const void* v, const float* g, con
   return decode_impl(q, k, v, g, b, w, state, o, B, n, H, HK, DK, DV, in_batch_stride, o_batch_stride, scale, dtype, true, stream);
 }
 
+int gdn2_decode_tail(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
+                     float* state, void* o, int64_t B, int64_t n, int64_t H, int64_t HK, int64_t DK, int64_t DV,
+                     int64_t in_batch_stride, int64_t o_batch_stride, float scale, int dtype, void* stream) {
+  return decode_impl(q, k, v, g, b, w, state, o, B, n, H, HK, DK, DV, in_batch_stride, o_batch_stride, scale, dtype, false, stream);
+}
+
 size_t gdn2_prefill_workspace_bytes(int64_t B, int64_t S, int64_t H, int64_t HK, int64_t DK, int64_t DV, int dtype,
                                     int path) {
   if (check_prefill_shape(B, S, H, HK, DK, DV, dtype) != GDN2_OK) return 0;

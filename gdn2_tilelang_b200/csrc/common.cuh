@@ -218,7 +218,8 @@ int record_cuda_error(cudaError_t e);   // stores e for gdn2_last_cuda_error(), 
 // with it, 75 without). What chaining saves is launch latency between short kernels: five
 // draft tokens for 24 conversations, f16, 18.4 -> 16.3 us; one token for 256 conversations 86.7 -> 85.3, eight 132.6 -> 129.5;
 // the float32 call above 80 -> 75.
-// The tensor-core prefill, whose calls fork to a second stream, is launched plainly (chained = false).
+// The tensor-core prefill, whose calls fork to a second stream, is launched plainly (chained = false), the decode of its
+// ragged tail included, whether this library queues it or a caller that composes the stages (gdn2_decode_tail).
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... P, typename... A>

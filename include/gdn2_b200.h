@@ -82,6 +82,15 @@ int gdn2_decode(const void* q, const void* k, const void* v, const float* g, con
                 int64_t in_batch_stride, int64_t o_batch_stride, float scale, int dtype, void* stream);
 
 /*
+ * The same for the ragged tail of a prompt whose whole chunks a caller has queued itself with gdn2_chunk_prep and
+ * gdn2_prefill_scan(_part), on one or two streams: gdn2_decode may be set up while the kernel before it in the stream still
+ * runs (programmatic stream serialization), this one starts after it, as the kernels of the tensor-core prefill do.
+ */
+int gdn2_decode_tail(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
+                     float* state, void* o, int64_t B, int64_t n, int64_t H, int64_t HK, int64_t DK, int64_t DV,
+                     int64_t in_batch_stride, int64_t o_batch_stride, float scale, int dtype, void* stream);
+
+/*
  * Bytes of scratch the chunkwise prefill needs for a [B,S,H,DK,DV] problem (S a multiple of 64).
  * Returns 0 for an unsupported combination. `path` is a gdn2_prefill_path.
  */

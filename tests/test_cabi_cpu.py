@@ -59,6 +59,27 @@ def test_workspace_query(lib):
     assert f(1, 64, 1, 1, 32, 24, 7, 0) == 0                           # bad dtype
 
 
+def test_a_tail_is_launched_plainly(monkeypatch):
+    """Tokens decoded into a view of a longer output are a prefill's tail: they take the plain-launch entry point."""
+    import torch
+
+    called = []
+
+    class Lib:
+        def __getattr__(self, name):
+            return lambda *a: called.append(name) or 0
+
+    K = _cabi.NativeKernels.__new__(_cabi.NativeKernels)
+    K.lib, K.launches = Lib(), 0
+    monkeypatch.setattr(_cabi, "_require_cuda", lambda *t: None)
+    monkeypatch.setattr(_cabi, "_on_device", lambda dev: __import__("contextlib").nullcontext())
+    monkeypatch.setattr(K, "_stream", lambda t: 0, raising=False)
+    x, s, o = torch.zeros(1, 3, 2, 8), torch.zeros(1, 2, 8, 8), torch.zeros(1, 67, 2, 8)
+    K.decode(x, x, x, x, x, x, s, 1.0)
+    K.decode(x, x, x, x, x, x, s, 1.0, out=o[:, 64:])
+    assert called == ["gdn2_decode", "gdn2_decode_tail"]
+
+
 def test_argument_validation_returns_status_without_device_work(lib):
     null = None
     one = ctypes.c_void_p(16)   # never dereferenced: validation fails first
