@@ -201,7 +201,9 @@ int gdn2_prefill_ragged(const void* q, const void* k, const void* v, const float
  *   cu_seqlens     N + 1 token offsets IN HOST MEMORY, rising from 0; sequences may be empty
  *   initial_state  [N,H,DK,DV] fp32 or NULL (zero); final_state the same, always written, 16-byte aligned, not the
  *                  same memory
- *   workspace      gdn2_packed_workspace_bytes(...) bytes, 16-byte aligned (0 = unsupported combination)
+ *   workspace      gdn2_packed_workspace_bytes(...) bytes, 16-byte aligned (0 = unsupported combination). Bounded however
+ *                  long the batch: the sequences go through it in groups of at most 128 and of at most 8192 (chunk, head)
+ *                  pairs, or one sequence where that has more
  * Every sequence gets what gdn2_prefill_ragged gives it alone, up to the rounding of where its scan is cut.
  */
 size_t gdn2_packed_workspace_bytes(const int64_t* cu_seqlens, int64_t N, int64_t H, int64_t HK, int64_t DK, int64_t DV,

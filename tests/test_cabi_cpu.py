@@ -59,6 +59,24 @@ def test_workspace_query(lib):
     assert f(1, 64, 1, 1, 32, 24, 7, 0) == 0                           # bad dtype
 
 
+@pytest.mark.parametrize("dtype", [_cabi.GDN2_BF16, _cabi.GDN2_F32])
+def test_packed_workspace_does_not_grow_with_the_batch(lib, dtype):
+    def packed(lens, H=16):
+        cu = [0]
+        for n in lens:
+            cu.append(cu[-1] + n)
+        return lib.gdn2_packed_workspace_bytes((ctypes.c_int64 * len(cu))(*cu), len(lens), H, H, 128, 128, dtype, 0)
+
+    alone = packed([8192])
+    bound = 8192 * 64 * (2400 if dtype == _cabi.GDN2_F32 else 1200) + (1 << 28)      # records of the group, and a cut's
+    assert 0 < alone <= bound
+    assert packed([8192] * 128) <= bound and packed([8192] * 1000) <= bound
+    assert packed([8192] * 128) == packed([8192] * 300)
+    # a sequence beyond the bound takes what it takes alone
+    assert packed([100, 1 << 18, 77]) == packed([1 << 18])
+    assert lib.gdn2_packed_workspace_bytes((ctypes.c_int64 * 3)(0, 5, 5), 2, 1, 1, 128, 128, dtype, 0) > 0
+
+
 def test_a_tail_is_launched_plainly(monkeypatch):
     """Tokens decoded into a view of a longer output are a prefill's tail: they take the plain-launch entry point."""
     import torch

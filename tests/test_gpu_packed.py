@@ -63,3 +63,31 @@ def test_packed_equals_one_call_per_sequence(name, H, HK, DK, DV, dtype, with_st
             assert orc.max_abs_err(o[:, lo:hi].float().cpu(), o1.float().cpu()) < 2e-2, i
             assert orc.rel_fro_err(s[i:i + 1].cpu(), s1.cpu()) < 1e-3, i
     _cabi.kernels().check_device_status()
+
+
+@pytest.mark.parametrize("H,D,DV,dtype,lens", [
+    (64, 128, 128, torch.bfloat16, [64 * 70 + 9, 64 * 61, 0, 130, 64 * 2]),     # the second sequence opens a new group
+    (128, 8, 4, torch.float32, [64 * 30 + 1, 64 * 34, 70, 5]),                  # the third does
+    (70, 8, 4, torch.float32, [10, 64 * 118, 3]),                               # a sequence beyond the bound by itself
+])
+def test_groups_that_share_a_workspace(H, D, DV, dtype, lens):
+    offs = [0]
+    for n in lens:
+        offs.append(offs[-1] + n)
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    q, k = (torch.nn.functional.normalize(torch.randn(1, offs[-1], H, D, generator=gen, device=DEV), dim=-1).to(dtype) for _ in "qk")
+    v, w = (torch.randn(1, offs[-1], H, DV, generator=gen, device=DEV).to(dtype) for _ in "vw")
+    g = torch.nn.functional.logsigmoid(torch.randn(1, offs[-1], H, D, generator=gen, device=DEV)) / 16
+    b = torch.sigmoid(torch.randn(1, offs[-1], H, D, generator=gen, device=DEV)).to(dtype)
+    w = torch.sigmoid(w)
+    s0 = torch.randn(len(lens), H, D, DV, generator=gen, device=DEV) * 0.1
+    o, s = gdn2.gdn2_attention(q, k, v, g, b, w, initial_state=s0, output_final_state=True, cu_seqlens=offs)
+    _cabi.kernels().check_device_status()
+    for i, (lo, hi) in enumerate(zip(offs, offs[1:])):
+        if hi == lo:
+            assert torch.equal(s[i], s0[i])
+            continue
+        o1, s1 = gdn2.gdn2_attention(*(t[:, lo:hi] for t in (q, k, v, g, b, w)), initial_state=s0[i:i + 1], output_final_state=True)
+        tol = 2e-5 if dtype == torch.float32 else 1e-2
+        assert orc.rel_fro_err(o[:, lo:hi].cpu(), o1.cpu()) < tol and orc.rel_fro_err(s[i:i + 1].cpu(), s1.cpu()) < min(tol, 1e-3)
+    _cabi.kernels().check_device_status()
