@@ -21,6 +21,7 @@ from dataclasses import dataclass
 import torch
 import torch.nn.functional as F
 from torch import nn
+from torch.nn.modules.module import _has_any_global_hook
 
 from . import _cabi
 from .config import DEFAULT_KERNEL_CONFIG, GDN2Config, GatedDeltaNet2Config
@@ -143,6 +144,7 @@ class _GatedRMSNorm(nn.Module):
         self.weight = nn.Parameter(torch.ones(dim))
 
 
+_STAGES = frozenset(("_front", "_back", "_project_out", "_fused_tables", "_check_supported"))   # what the native call stands for
 _PROJECTIONS = ("q_proj", "k_proj", "v_proj", "b_proj", "w_proj", "f_proj", "o_gate_proj")
 
 
@@ -288,7 +290,8 @@ class GatedDeltaNet2(nn.Module):
 
     def _decode_plain(self, x, cache):
         """The whole of ``decode`` as one native call, or ``None`` where something about the layer, the cache or the input
-        needs the general path (a subclass, hooks, a missing or converted convolution cache, strided tensors)."""
+        needs the general path (a subclass, hooks, replaced methods, a missing or converted convolution cache, strided
+        tensors): whatever would have run when ``o_proj`` is called as a module still runs."""
         K = _cabi.kernels()
         host = getattr(K, "host", None)
         if host is None or type(self) is not GatedDeltaNet2 or cache.conv_state is None:
@@ -296,6 +299,7 @@ class GatedDeltaNet2(nn.Module):
         m = self._modules
         o_proj = m["o_proj"]
         if (type(o_proj) is not nn.Linear or o_proj.bias is not None or o_proj._forward_hooks or o_proj._forward_pre_hooks
+                or "forward" in o_proj.__dict__ or _has_any_global_hook() or not _STAGES.isdisjoint(self.__dict__)
                 or any(m[n]._parameters.get("bias") is not None for n in _PROJECTIONS)):
             return None
         w_cat, offs, cw, cb = self._fused_tables()
