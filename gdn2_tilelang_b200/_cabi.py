@@ -11,9 +11,12 @@ tensors into raw pointers, sizes and the current CUDA stream.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 import pathlib
+import sys
 import threading
+import warnings
 
 import torch
 
@@ -116,14 +119,22 @@ def load_library(build_if_missing: bool = True) -> ctypes.CDLL:
 
 
 def load_host():
-    """The host extension (``csrc/host/binding.cpp``), built in-tree first if it is missing."""
+    """The host extension (``csrc/host/binding.cpp``), built in-tree first if there is none for this Python and PyTorch, or
+    ``None`` with a warning where it cannot be built or loaded: every caller has the general path to fall back on."""
     from . import build as _build
 
-    if not _build.HOST_LIB.exists():
-        _build.build_host()
-    from . import _gdn2_host
-
-    return _gdn2_host
+    name = f"{__package__}._gdn2_host"
+    if name in sys.modules:
+        return sys.modules[name]
+    try:
+        spec = importlib.util.spec_from_file_location(name, _build.build_host_if_missing())
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        sys.modules[name] = module
+        return module
+    except (RuntimeError, OSError, ImportError) as e:
+        warnings.warn(f"the host extension cannot be used, short calls go through Python: {e}")
+        return None
 
 
 def dtype_code(dtype: torch.dtype) -> int:
@@ -190,7 +201,7 @@ class NativeKernels:
 
     def __init__(self):
         self.lib = load_library()
-        self.host = load_host()     # decode, prefill and the layer's decode in one native call, where the case is plain
+        self.host = load_host()     # decode, prefill and the layer's decode in one native call, where the case is plain; or None
         self.prefill_path = _PATHS[os.environ.get("GDN2_B200_PREFILL_PATH", "auto")]
         self.launches = 0   # kernels launched through this object (for the benchmark's accounting)
         self._side_streams = {}

@@ -1,5 +1,6 @@
 """Build ``libgdn2_b200.so`` in-tree with nvcc for sm_100a (cross-compiles without a GPU), and beside it the host
-extension ``_gdn2_host.so`` (g++, PyTorch's headers) that makes the short calls without going through Python.
+extension ``_gdn2_host.*.so`` (g++, PyTorch's headers) that makes the short calls without going through Python. The package
+works without the extension: a failure to build it is a warning.
 
     python -m gdn2_tilelang_b200.build [--force] [--verbose]
 """
@@ -13,13 +14,26 @@ import pathlib
 import shutil
 import subprocess
 import sys
+import warnings
 
 PKG = pathlib.Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = PKG / "build"
 LIB = PKG / "libgdn2_b200.so"
 HOST_SRC = CSRC / "host" / "binding.cpp"
-HOST_LIB = PKG / "_gdn2_host.so"
+
+
+def host_lib() -> pathlib.Path:
+    """The host extension for THIS Python and PyTorch: it is linked against PyTorch's C++ interface, so one that was built
+    under another version must not be loaded."""
+    import re
+    import sysconfig
+
+    import torch
+
+    tag = re.sub(r"[^A-Za-z0-9_]+", "_", f"torch_{torch.__version__}_{sysconfig.get_config_var('SOABI')}")
+    return PKG / f"_gdn2_host.{tag}.so"
+
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -66,13 +80,22 @@ def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
-    build_host(force)
+    try:
+        build_host(force)
+    except (RuntimeError, OSError) as e:
+        warnings.warn(f"the host extension was not built, short calls go through Python: {e}")
     return LIB
+
+
+def build_host_if_missing() -> pathlib.Path:
+    target = host_lib()
+    return target if target.exists() else build_host()
 
 
 def build_host(force: bool = False) -> pathlib.Path:
     header = PKG.parent / "include" / "gdn2_b200.h"
-    if force or _stale(HOST_LIB, [HOST_SRC, header]):
+    target = host_lib()
+    if force or _stale(target, [HOST_SRC, header]):
         import sysconfig
 
         import torch
@@ -81,15 +104,15 @@ def build_host(force: bool = False) -> pathlib.Path:
         cuda = pathlib.Path(find_nvcc()).resolve().parent.parent
         includes = [*include_paths(), sysconfig.get_paths()["include"], str(cuda / "include")]
         torch_lib = pathlib.Path(torch.__file__).parent / "lib"
-        tmp = HOST_LIB.with_suffix(f".{os.getpid()}.tmp")
+        tmp = target.with_suffix(f".{os.getpid()}.tmp")
         cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
                *(f"-I{i}" for i in includes), str(HOST_SRC), "-o", str(tmp), f"-L{torch_lib}", "-lc10", "-lc10_cuda",
                "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-ltorch", f"-L{PKG}", f"-l:{LIB.name}", "-Wl,-rpath,$ORIGIN"]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"g++ failed on {HOST_SRC.name}:\n{r.stdout}\n{r.stderr}")
-        os.replace(tmp, HOST_LIB)
-    return HOST_LIB
+        os.replace(tmp, target)
+    return target
 
 
 if __name__ == "__main__":
