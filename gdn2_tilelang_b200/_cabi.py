@@ -45,6 +45,7 @@ SIGNATURES = {
     "gdn2_prefill_scan_part": (_int, [_vp, _sz, _vp, _vp, _vp] + [_i64] * 7 + [_int, _int, _int, _vp]),
     "gdn2_prefill_ragged_workspace_bytes": (_sz, [_i64] * 6 + [_int, _int]),
     "gdn2_prefill_ragged": (_int, [_vp] * 10 + [_sz] + [_i64] * 8 + [_f32, _int, _int, _vp, _vp]),
+    "gdn2_packed_launches": (_int, [ctypes.POINTER(_i64)] + [_i64] * 5 + [_int, _int]),
     "gdn2_packed_workspace_bytes": (_sz, [ctypes.POINTER(_i64)] + [_i64] * 5 + [_int, _int]),
     "gdn2_packed_forward": (_int, [_vp] * 6 + [ctypes.POINTER(_i64), _i64, _vp, _vp, _vp, _vp, _sz] + [_i64] * 4
                             + [_f32, _int, _int, _vp]),
@@ -354,7 +355,7 @@ class NativeKernels:
                 None if initial_state is None else initial_state.data_ptr(), o.data_ptr(), final_state.data_ptr(),
                 ws.data_ptr(), nbytes, H, HK, DK, DV, float(scale), code, p, self._stream(q))
         _check(self.lib, rc, "gdn2_packed_forward")
-        self.launches += 4 if p != PATH_SIMT else 2
+        self.launches += self.lib.gdn2_packed_launches(cu, N, H, HK, DK, DV, code, p)
         return o, final_state
 
     # -- chunkwise forward -----------------------------------------------------------------

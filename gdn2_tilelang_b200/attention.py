@@ -309,9 +309,9 @@ class GatedDeltaNet2(nn.Module):
                                 self.head_dim_v, self.cfg.conv_size, self.erase_scale, m["o_norm"].eps, self.scale)
         if res is None:
             return None
-        K.launches += 3
+        out, cache.conv_state, launched = res
+        K.launches += launched
         K.maybe_check_device_status(x.device)
-        out, cache.conv_state = res
         return out
 
     # ------------------------------------------------------------------ public API

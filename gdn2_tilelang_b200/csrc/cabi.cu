@@ -419,6 +419,12 @@ void packed_segments(PackedSeqs& t, int64_t H, bool cut) {
     t.seg[i + 1] = t.seg[i] + (best ? std::max(1, (t.chunk[i + 1] - t.chunk[i] + best - 1) / best) : 1);
 }
 
+bool has_tails(const PackedSeqs& t) {
+  for (int i = 0; i < t.n; ++i)
+    if ((t.tok[i + 1] - t.tok[i]) % kChunk != 0) return true;
+  return false;
+}
+
 // Workspace of one group: the records of a row of all its chunks, then the segment records of a cut scan.
 struct PackedLayout { WsLayout L; size_t total; int64_t recs; };
 PackedLayout packed_layout(const PackedSeqs& t, int64_t H, int64_t HK, int64_t DK, int64_t DV, int family) {
@@ -454,6 +460,22 @@ size_t gdn2_packed_workspace_bytes(const int64_t* cu_seqlens, int64_t N, int64_t
     most = std::max(most, packed_layout(t, H, HK, DK, DV, family).total);
   }
   return most;
+}
+
+int gdn2_packed_launches(const int64_t* cu_seqlens, int64_t N, int64_t H, int64_t HK, int64_t DK, int64_t DV, int dtype,
+                         int path) {
+  int family;
+  bool cut;
+  if (check_packed(cu_seqlens, N, H, HK, DK, DV, dtype, path, &family, &cut) != GDN2_OK) return -1;
+  int launches = 0;
+  for (int64_t i0 = 0, n; i0 < N; i0 += n) {
+    PackedSeqs t = packed_table(cu_seqlens, N, i0, H, family);
+    n = t.n;
+    packed_segments(t, H, cut);
+    const bool any = t.chunk[t.n] > 0;
+    launches += family == GDN2_PATH_TCGEN05 ? (any ? 2 : 0) + (t.seg[t.n] > t.n ? 3 : 1) + (has_tails(t) ? 1 : 0) : (any ? 1 : 0) + 1;
+  }
+  return launches;
 }
 
 int gdn2_packed_forward(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
@@ -501,9 +523,7 @@ int gdn2_packed_forward(const void* q, const void* k, const void* v, const float
           rc = launch_prep_simt_packed(tq, tk, tv, tg, tb, tw, L, P, t, (int)H, (int)HK, scale, dtype, true, st);
       }
       if (rc == GDN2_OK) rc = launch_scan_tc_packed(L, P, t, s0, to, sT, (int)H, st);
-      bool tails = false;
-      for (int i = 0; i < t.n; ++i) tails = tails || (t.tok[i + 1] - t.tok[i]) % kChunk != 0;
-      if (rc == GDN2_OK && tails) rc = launch_decode_packed_tails(tq, tk, tv, tg, tb, tw, sT, to, t, (int)H, (int)HK, scale, st);
+      if (rc == GDN2_OK && has_tails(t)) rc = launch_decode_packed_tails(tq, tk, tv, tg, tb, tw, sT, to, t, (int)H, (int)HK, scale, st);
     } else {
       if (any) rc = launch_prep_simt_packed(tq, tk, tv, tg, tb, tw, L, P, t, (int)H, (int)HK, scale, dtype, false, st);
       if (rc == GDN2_OK) rc = launch_scan_simt_packed(L, P, t, s0, to, sT, (int)H, dtype, st);

@@ -16,7 +16,6 @@
 
 namespace py = pybind11;
 using at::Tensor;
-using Pair = std::tuple<Tensor, Tensor>;
 
 namespace {
 
@@ -111,8 +110,8 @@ std::optional<std::tuple<Tensor, Tensor, int64_t>> prefill(const Tensor& q, cons
 
 
 // GatedDeltaNet2.decode on x [B, n, hidden]: projections, layer_front, decode, layer_back, output projection. The recurrent
-// state is updated in place. Returns (out [B, n, hidden], new convolution cache) or None.
-std::optional<Pair> layer_decode(const Tensor& x, const Tensor& state, const std::optional<Tensor>& conv_state, const Tensor& w_cat,
+// state is updated in place. Returns (out [B, n, hidden], new convolution cache, kernels launched) or None.
+std::optional<std::tuple<Tensor, Tensor, int64_t>> layer_decode(const Tensor& x, const Tensor& state, const std::optional<Tensor>& conv_state, const Tensor& w_cat,
                         const std::optional<Tensor>& conv_w, const std::optional<Tensor>& conv_b, const Tensor& A_log,
                         const Tensor& dt_bias, const Tensor& norm_w, const Tensor& o_w, const std::vector<int64_t>& offs, int64_t H,
                         int64_t HK, int64_t DK, int64_t DV, int64_t K, double erase_scale, double eps, double scale) {
@@ -156,7 +155,10 @@ std::optional<Pair> layer_decode(const Tensor& x, const Tensor& state, const std
   const int rc = gdn2_layer_back(o.data_ptr(), proj.data_ptr(), norm_w.data_ptr(), normed.data_ptr(), p.B * p.S, H, DV,
                                  proj.size(2), offs[6], (float)eps, p.dtype, st);
   if (rc != GDN2_OK) throw std::runtime_error(std::string("gdn2_layer_back: ") + gdn2_status_string(rc));
-  return Pair{at::linear(normed, o_w), conv};
+  // the front kernel writes the new convolution cache itself in its one-token form, else a second one does
+  bool fused = p.dtype != GDN2_F32 && DK == 128 && DV == 128 && K == 4 && p.S < 8 && a.NP % 4 == 0;
+  for (int i = 0; i < 6; ++i) fused = fused && offs[i] % 4 == 0;
+  return std::make_tuple(at::linear(normed, o_w), conv, int64_t(fused ? 3 : 4));
 }
 
 // The state of a list of parameters: where each lies, its version and its type. Equal bytes = nothing was replaced,

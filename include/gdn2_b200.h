@@ -212,6 +212,10 @@ int gdn2_packed_forward(const void* q, const void* k, const void* v, const float
                         const int64_t* cu_seqlens, int64_t N, const float* initial_state, void* o, float* final_state,
                         void* workspace, size_t workspace_bytes, int64_t H, int64_t HK, int64_t DK, int64_t DV, float scale,
                         int dtype, int path, void* stream);
+/* Kernels gdn2_packed_forward launches for these sequences (-1: unsupported combination), for callers that account for
+ * their launches. */
+int gdn2_packed_launches(const int64_t* cu_seqlens, int64_t N, int64_t H, int64_t HK, int64_t DK, int64_t DV, int dtype,
+                         int path);
 
 /*
  * gdn2_prefill_scan with the layer's gated RMSNorm as the epilogue of the output rows:

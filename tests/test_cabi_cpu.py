@@ -77,6 +77,24 @@ def test_packed_workspace_does_not_grow_with_the_batch(lib, dtype):
     assert lib.gdn2_packed_workspace_bytes((ctypes.c_int64 * 3)(0, 5, 5), 2, 1, 1, 128, 128, dtype, 0) > 0
 
 
+def test_packed_launches(lib):
+    def count(lens, H=2, D=128, dtype=_cabi.GDN2_BF16, path=0):
+        cu = [0]
+        for n in lens:
+            cu.append(cu[-1] + n)
+        return lib.gdn2_packed_launches((ctypes.c_int64 * len(cu))(*cu), len(lens), H, H, D, D, dtype, path)
+
+    assert count([64]) == 3                                  # chunk stage, redo of flagged chunks, scan
+    assert count([64, 5]) == 4                               # ... and the tails
+    assert count([5, 0]) == 2                                # nothing but tails: the states pass through the scan
+    assert count([64 * 70, 9]) == 6                          # the scan cut: first pass, chaining, correction pass
+    assert count([64 * 70, 9], path=_cabi.PATH_TCGEN05_SERIAL) == 4
+    assert count([5] * 128) == 2 and count([5] * 129) == 4   # a second table
+    assert count([100, 3], D=64, dtype=_cabi.GDN2_F32) == 2
+    assert count([0, 0], D=64, dtype=_cabi.GDN2_F32) == 1
+    assert count([64], D=36, dtype=_cabi.GDN2_F32) == -1
+
+
 def test_a_tail_is_launched_plainly(monkeypatch):
     """Tokens decoded into a view of a longer output are a prefill's tail: they take the plain-launch entry point."""
     import torch

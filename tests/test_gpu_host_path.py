@@ -104,6 +104,22 @@ def test_layer_step(monkeypatch, dtype):
     assert len(seen) == 4                                # hooks on the output projection still run, in every call
 
 
+@pytest.mark.parametrize("D,launched", [(128, 3), (64, 4)])
+def test_launches_are_counted(monkeypatch, D, launched):
+    """The benchmark's accounting, by either path: the general front of the layer is two kernels."""
+    cfg = gdn2.GatedDeltaNet2Config(hidden_size=256, num_heads=2, head_dim_k=D)
+    layer = gdn2.GatedDeltaNet2(cfg).to(DEV, torch.bfloat16)
+    x = torch.randn(2, 256, device=DEV, dtype=torch.bfloat16)
+    K = _cabi.kernels()
+
+    def call():
+        cache, before = layer.init_cache(2), K.launches
+        layer.step(x, cache)
+        return K.launches - before
+
+    assert _both(monkeypatch, call) == (launched, launched)
+
+
 def test_a_failed_allocation_is_torch_s_own_error():
     """Programs catch torch.OutOfMemoryError to retry with a smaller batch, whichever path the call takes."""
     ins = _inputs(4, 64 * 16, 16, 16, 128, torch.bfloat16)            # 76 MB of workspace
