@@ -52,7 +52,7 @@ constexpr int A_PAD = 129;        // rows per K chunk of a 128-row bf16 image, +
 constexpr int B_PAD = 161;        // 160 key rows (16 + 32 + 48 + 64) + 1 pad row
 constexpr int TM_STRIDE = 68;     // floats per Tm row (row-major, padded against bank conflicts)
 constexpr float kMaxSpanLog2 = 96.f;     // 2^96 keeps every scaled operand inside bf16 and fp32 range (|k|, |q| << 2^30)
-constexpr uint32_t kTmemCols = 256;
+constexpr uint32_t kTmemCols = 256;              // 192 are used; an allocation is a power of two
 constexpr uint32_t kQgCol = 160;  // TMEM columns [160,192): packed Qg of the thread's channel
 
 struct PrepTcSmem {

@@ -25,39 +25,36 @@ namespace {
 
 constexpr int NV = 32;   // value columns per block of the output kernel
 
-struct ScanSmem {
-  float *Ws, *Qs, *As, *Ks, *Us, *Un, *St, *gl;
-  __device__ ScanSmem(float* base, int DK) {
+// Shared memory of the output kernel.
+struct OutputSmem {
+  float *Ws, *Qs, *As, *Us, *Un, *St;
+  __device__ OutputSmem(float* base, int DK) {
     Ws = base;                    // [64][DK]
     Qs = Ws + kChunk * DK;        // [64][DK]
-    Ks = Qs + kChunk * DK;        // [64][DK]   KG[t][k]
-    As = Ks + kChunk * DK;        // [64][64]
+    As = Qs + kChunk * DK;        // [64][64]
     Us = As + kChunk * kChunk;    // [64][NV]
     Un = Us + kChunk * NV;        // [64][NV]
     St = Un + kChunk * NV;        // [DK][NV]
-    gl = St + DK * NV;            // [DK]
   }
   static size_t bytes(int DK) {
-    return ((size_t)3 * kChunk * DK + kChunk * kChunk + 2 * kChunk * NV + (size_t)DK * NV + DK) * sizeof(float);
+    return ((size_t)2 * kChunk * DK + kChunk * kChunk + 2 * kChunk * NV + (size_t)DK * NV) * sizeof(float);
   }
 };
 
 template <typename TW>
 __device__ __forceinline__ void load_chunk_operands(const WsLayout& L, const WsPtrs& P, int64_t ch, int64_t chv, int lo,
-                                                    ScanSmem& s, bool want_kg) {
+                                                    OutputSmem& s) {
   using WT = WsTraits<TW>;
   using TV = typename WT::TV;
   constexpr int E = WT::E;
   const int DK = L.DK, DV = L.DV, tid = threadIdx.x;
   const TW* wq = reinterpret_cast<const TW*>(P.wq + (size_t)ch * L.wq_bytes);
   const TV* aqk = reinterpret_cast<const TV*>(P.aqk + (size_t)ch * L.aqk_bytes);
-  const TV* kgt = reinterpret_cast<const TV*>(P.kgt + (size_t)ch * L.kgt_bytes);
   const TV* ut = reinterpret_cast<const TV*>(P.ut + (size_t)chv * L.ut_bytes);   // per value head; the rest per key head
   for (int idx = tid; idx < kChunk * DK; idx += 256) {
     const int t = idx / DK, c = idx % DK;
     s.Ws[idx] = to_f32(wq[kc_index<E>(t, c, 2 * kChunk)]);
     s.Qs[idx] = to_f32(wq[kc_index<E>(kChunk + t, c, 2 * kChunk)]);
-    if (want_kg) s.Ks[idx] = WT::kg_load(kgt[kc_index<E>(c, t, DK)]);
   }
   for (int idx = tid; idx < kChunk * kChunk; idx += 256)
     s.As[idx] = WT::kg_load(aqk[kc_index<E>(idx / kChunk, idx % kChunk, kChunk)]);
@@ -65,12 +62,11 @@ __device__ __forceinline__ void load_chunk_operands(const WsLayout& L, const WsP
     const int t = idx / NV, c = lo + idx % NV;
     s.Us[idx] = c < DV ? WT::u_load(ut[kc_index<E>(c, t, DV)]) : 0.f;
   }
-  if (want_kg && tid < DK) s.gl[tid] = P.gl[(size_t)ch * DK + tid];
 }
 
 // Un = U - W S and o = Qg S + tril(Aqk) Un for the 8 tokens [wid*8, wid*8+8) and column `lane`.
 template <typename TOut>
-__device__ __forceinline__ void un_and_output(ScanSmem& s, int DK, int DV, int lo, TOut* __restrict__ o_rows,
+__device__ __forceinline__ void un_and_output(OutputSmem& s, int DK, int DV, int lo, TOut* __restrict__ o_rows,
                                               size_t o_row_stride) {
   const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
   float acc[8];
@@ -337,14 +333,14 @@ output_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ hs, TOut* __r
   const int lo = blockIdx.x * NV;
   const int tid = threadIdx.x;
   extern __shared__ float sm[];
-  ScanSmem s(sm, DK);
+  OutputSmem s(sm, DK);
   const int64_t ch = ((int64_t)ib * (H / L.rep) + ih / L.rep) * NC + n;
   const float* hp = hs + (((size_t)ib * NC + n) * H + ih) * DK * DV;
   for (int idx = tid; idx < DK * NV; idx += 256) {
     const int c = idx / NV, d = lo + idx % NV;
     s.St[idx] = d < DV ? hp[(size_t)c * DV + d] : 0.f;
   }
-  load_chunk_operands<TW>(L, P, ch, (int64_t)bh * NC + n, lo, s, false);
+  load_chunk_operands<TW>(L, P, ch, (int64_t)bh * NC + n, lo, s);
   __syncthreads();
   TOut* o_rows = o + (((size_t)ib * o_bs + (size_t)n * kChunk) * H + ih) * DV;
   un_and_output<TOut>(s, DK, DV, lo, o_rows, (size_t)H * DV);
@@ -370,7 +366,7 @@ int launch_scan_typed(const WsLayout& L, const WsPtrs& P, const float* s0, void*
 template <typename TOut, typename TW>
 int launch_output_typed(const WsLayout& L, const WsPtrs& P, const float* hs, void* o, int B, int S, int H,
                         int64_t o_bs, cudaStream_t st) {
-  const size_t smem = ScanSmem::bytes(L.DK);
+  const size_t smem = OutputSmem::bytes(L.DK);
   auto kern = output_simt_kernel<TOut, TW>;
   GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
   dim3 grid((L.DV + NV - 1) / NV, S / kChunk, B * H);
