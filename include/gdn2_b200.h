@@ -122,7 +122,7 @@ int gdn2_prefill_workspace_layout(int64_t B, int64_t S, int64_t H, int64_t HK, i
 int gdn2_prefill_scan_segments(int64_t B, int64_t S, int64_t H, int64_t DK, int64_t DV, int dtype, int path);
 
 /*
- * Kernels gdn2_prefill_scan launches for this problem without chunk_states: 1 (one walk), 3 (first pass, chaining
+ * Kernels gdn2_prefill_scan launches for this problem: 1 (one walk), 3 (first pass, chaining
  * of the segment records, redo pass) or 4 (the same behind the decay check of a guarded cut); 0 for an
  * unsupported combination. For callers that account for their launches. No counterpart in the reference.
  */
@@ -148,13 +148,16 @@ int gdn2_chunk_prep(const void* q, const void* k, const void* v, const float* g,
  * Replaces prefill_scan_kernel (gdn2/inference.py:356-479) and, with chunk_states, the
  * state_kernel + output_kernel pair of the training-style forward (gdn2/forward.py:538-727).
  *
- * Few (batch, head) pairs (tcgen05 family, no chunk_states; B*H <= 28 and 24 chunks or more: always; B*H <= 72 and
+ * Few (batch, head) pairs (tcgen05 family; B*H <= 28 and 24 chunks or more: always; B*H <= 72 and
  * 48 chunks or more: "guarded", only when a check of the decay on the device finds that a segment forgets the
  * state entering it): the sequence is cut into segments. Every segment is scanned from a zero state while a second block
  * accumulates the segment's state-transition matrix; a small kernel chains the segments' affine maps
  * and a last launch redoes, from the true entering state, the leading chunks of each segment that the
- * entering state still reaches. The result equals the one-block walk up to the rounding of the state
- * hand-over (below 1e-6 of the state); the form used is reported by gdn2_prefill_scan_segments.
+ * entering state still reaches; chunk_states come from the same launches. What is left out of a segment's states is the
+ * entering state's share once every entry of the transition matrix is under 2^-27 (below 1e-6 of that state). Where the
+ * matrix stays, its products round as the walk's do: either form is off 64-bit arithmetic by 6e-4 of the state's norm with
+ * ordinary decay and by 1.7e-3 without any, and the two forms differ from each other by as much. The form used is reported
+ * by gdn2_prefill_scan_segments; GDN2_PATH_TCGEN05_SERIAL is always the one-block walk.
  */
 int gdn2_prefill_scan(const void* workspace, size_t workspace_bytes, const float* initial_state, void* o,
                       float* final_state, float* chunk_states, int64_t B, int64_t S, int64_t H, int64_t HK, int64_t DK,
