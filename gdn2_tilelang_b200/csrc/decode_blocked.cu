@@ -6,6 +6,8 @@
 //     u_t = w_t*v_t - (b_t*k_t*A_t)^T S_0 - sum_{s<t} Akk[t,s] u_s      Akk[t,s] = sum_c b_t k_t k_s A_t/A_s
 //     o_t = (scale*q_t*A_t)^T S_0 + sum_{s<=t} Aqk[t,s] u_s              Aqk[t,s] = scale * sum_c q_t k_s A_t/A_s
 //     S_8 = diag(A_8) S_0 + sum_s (k_s * A_8/A_s) u_s^T
+// (the exponent of every A_t / A_s is the sum of the gates s+1 .. t, not a difference of prefix sums, in which one strong gate
+// would swallow the ordinary ones after it; gates are read as max(g, kMinGate), whose exponential is zero already)
 // which is the token-by-token recurrence S <- diag(exp g) S; u = w*v - S^T(b*k); S <- S + k u^T;
 // o = scale S^T q with the sums regrouped: two sweeps over the state tile with 64 and 36 independent
 // accumulation chains per thread instead of 2 n sweeps that each wait for a cross-thread reduction.
@@ -35,6 +37,7 @@ namespace {
 
 constexpr int D = 128;
 constexpr int NB = 8;                       // tokens per block step
+constexpr float kMinGate = -110.f;          // exp(-104) is already below half of float32's smallest number
 constexpr int kGroupFloats = 16 * D + 16;   // 16 state rows + 64 bytes: adjacent row groups land 64 B apart mod 128
 constexpr int kTileFloats = 8 * kGroupFloats;
 constexpr uint32_t kGroupBytes = 16 * D * 4;
@@ -306,17 +309,15 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
           qraw[t] = stT[(0 * NB + t) * D + c]; kraw[t] = stT[(1 * NB + t) * D + c]; braw[t] = stT[(2 * NB + t) * D + c];
           vraw[t] = stT[(3 * NB + t) * D + c]; wraw[t] = stT[(4 * NB + t) * D + c];
         }
-        float G[NB], kk[NB], bk[NB], qs[NB], wvv[NB];
-        float run = 0.f;
+        float l[NB], kk[NB], bk[NB], qs[NB], wvv[NB];
 #pragma unroll
         for (int t = 0; t < NB; ++t) {
           const bool real = t < nb;                      // padding token: no decay, no write, no read
-          run += real ? graw[t] * kLog2e : 0.f;
+          l[t] = real ? (graw[t] < kMinGate ? kMinGate : graw[t]) * kLog2e : 0.f;   // (a NaN stays one)
           kk[t] = real ? to_f32(kraw[t]) : 0.f;
           bk[t] = real ? to_f32(braw[t]) * kk[t] : 0.f;
           qs[t] = real ? to_f32(qraw[t]) * scale : 0.f;
           wvv[t] = real ? to_f32(wraw[t]) * to_f32(vraw[t]) : 0.f;
-          G[t] = run;                                    // log2 of A_t
         }
         // the sweep warps have finished with this table buffer (two steps ago)
         // (one warp polls, with pauses; the other three sleep at the barrier below)
@@ -326,36 +327,49 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
         if (table_sync_or(!okw)) break;
         {
           const int pr = crow(c);
-          float c1v[16], c2v[8];
+          float c1v[16], c2v[8], An = 1.f;
+          float run = 0.f, rest = 0.f;                   // log2 of A_t and of A_8 / A_t
 #pragma unroll
           for (int t = 0; t < NB; ++t) {
-            const float At = ex2(G[t]);
-            c1v[t] = bk[t] * At;
-            c1v[8 + t] = qs[t] * At;
-            c2v[t] = kk[t] * ex2(G[NB - 1] - G[t]);
+            run += l[t];
+            An = ex2(run);
+            c1v[t] = bk[t] * An;
+            c1v[8 + t] = qs[t] * An;
             tb.wv[t][c] = wvv[t];
+          }
+#pragma unroll
+          for (int t = NB - 1; t >= 0; --t) {
+            c2v[t] = kk[t] * ex2(rest);
+            rest += l[t];
           }
 #pragma unroll
           for (int j = 0; j < 4; ++j) tb.c1[j][pr] = make_float4(c1v[4 * j], c1v[4 * j + 1], c1v[4 * j + 2], c1v[4 * j + 3]);
 #pragma unroll
           for (int j = 0; j < 2; ++j) tb.c2[j][pr] = make_float4(c2v[4 * j], c2v[4 * j + 1], c2v[4 * j + 2], c2v[4 * j + 3]);
-          const float An = ex2(G[NB - 1]);
           tb.gam[pr] = An;
         }
         // Slot (t, sx) holds the Akk[t, sx] term for sx < t and the Aqk[sx, t] term for sx >= t (the upper
         // triangle is free). Summing over the warp's 32 channels: each step halves what a lane keeps.
+        float span[NB];                                  // span[sx] = l[sx + 1] + .. + l[t], log2 of A_t / A_sx
 #pragma unroll
         for (int hb = 0; hb < 2; ++hb) {
           float term[32];
 #pragma unroll
           for (int tt = 0; tt < 4; ++tt) {
             const int t = 4 * hb + tt;
+            float ahead = 0.f;
 #pragma unroll
             for (int sx = 0; sx < NB; ++sx) {
               float val;
-              if (sx < t) val = bk[t] * kk[sx] * ex2(G[t] - G[sx]);          // Akk[t, sx], A_t / A_s <= 1
-              else if (sx == t) val = qs[t] * kk[t];                          // Aqk[t, t]
-              else val = qs[sx] * kk[t] * ex2(G[sx] - G[t]);                  // Aqk[sx, t]
+              if (sx < t) {                                                   // Akk[t, sx], A_t / A_s <= 1
+                span[sx] = sx == t - 1 ? l[t] : span[sx] + l[t];
+                val = bk[t] * kk[sx] * ex2(span[sx]);
+              } else if (sx == t) {                                           // Aqk[t, t]
+                val = qs[t] * kk[t];
+              } else {                                                        // Aqk[sx, t]
+                ahead = sx == t + 1 ? l[sx] : ahead + l[sx];
+                val = qs[sx] * kk[t] * ex2(ahead);
+              }
               term[tt * 8 + sx] = val;
             }
           }
