@@ -9,7 +9,6 @@
 #include <ATen/core/grad_mode.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
-#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/utils/pybind.h>
 
 #include "../../../include/gdn2_b200.h"
@@ -175,10 +174,10 @@ py::bytes parameter_key(const std::vector<Tensor>& params) {
 }  // namespace
 
 PYBIND11_MODULE(_gdn2_host, m) {
-  // None of them touches Python objects: the lock is released meanwhile, as a foreign call does. Exceptions become the ones
-  // PyTorch's own functions raise: an allocation that fails is torch.OutOfMemoryError.
-  m.def("decode", torch::wrap_pybind_function_no_gil(&decode));
-  m.def("prefill", torch::wrap_pybind_function_no_gil(&prefill));
-  m.def("layer_decode", torch::wrap_pybind_function_no_gil(&layer_decode));
-  m.def("parameter_key", torch::wrap_pybind_function(&parameter_key));
+  // none of them touches Python objects: the lock is released meanwhile, as a foreign call does
+  const auto unlocked = py::call_guard<py::gil_scoped_release>();
+  m.def("decode", &decode, unlocked);
+  m.def("prefill", &prefill, unlocked);
+  m.def("layer_decode", &layer_decode, unlocked);
+  m.def("parameter_key", &parameter_key);
 }

@@ -118,20 +118,3 @@ def test_launches_are_counted(monkeypatch, D, launched):
         return K.launches - before
 
     assert _both(monkeypatch, call) == (launched, launched)
-
-
-def test_a_failed_allocation_is_torch_s_own_error():
-    """Programs catch torch.OutOfMemoryError to retry with a smaller batch, whichever path the call takes."""
-    ins = _inputs(4, 64 * 16, 16, 16, 128, torch.bfloat16)            # 76 MB of workspace
-    torch.cuda.synchronize()
-    torch.cuda.empty_cache()
-    total = torch.cuda.get_device_properties(0).total_memory
-    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (1 << 20)) / total)
-    try:
-        with pytest.raises(torch.OutOfMemoryError):
-            gdn2.gdn2_prefill(*ins)
-    finally:
-        torch.cuda.set_per_process_memory_fraction(1.0)
-    o, _ = gdn2.gdn2_prefill(*ins)
-    torch.cuda.synchronize()
-    assert torch.isfinite(o).all()
