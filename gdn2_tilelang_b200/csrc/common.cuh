@@ -217,7 +217,7 @@ int record_cuda_error(cudaError_t e);   // stores e for gdn2_last_cuda_error(), 
 // places while a kernel drains crowd onto the SMs that happen to be free first (B = 2, S = 1000, 8 heads of 64: call 103 us
 // with it, 75 without). What chaining saves is launch latency between short kernels: five
 // draft tokens for 24 conversations, f16, 18.4 -> 16.3 us; one token for 256 conversations 86.7 -> 85.3, eight 132.6 -> 129.5;
-// the float32 call above 80 -> 75.
+// the float32 call above 80 -> 75 (as it was then; 79 now).
 // The tensor-core prefill, whose calls fork to a second stream, is launched plainly (chained = false), the decode of its
 // ragged tail included, whether this library queues it or a caller that composes the stages (gdn2_decode_tail).
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
