@@ -21,7 +21,7 @@
 
 namespace gdn2 {
 
-// decode_blocked.cu: blocks of up to 8 tokens without a per-token dependent sweep (DK = DV = 128)
+// decode_blocked.cu: blocks of 2 to 8 tokens without a per-token dependent sweep (DK = DV = 128)
 template <typename T>
 int launch_decode_blocked(const T* q, const T* k, const T* v, const float* g, const T* b, const T* w, float* state,
                           T* o, int B, int n, int H, int HK, int64_t in_bs, int64_t o_bs, float scale, bool chained,
@@ -29,7 +29,10 @@ int launch_decode_blocked(const T* q, const T* k, const T* v, const float* g, co
 
 namespace {
 
-constexpr int kBlockedMinTokens = 4;   // from here on the blocked form wins over the token-by-token sweeps
+// From here on the blocked form wins over the token-by-token sweeps whatever the number of tiles; for two and three tokens it
+// wins where a block has more than one tile to walk (bf16, 16 heads, us: n = 3, 8 conversations 7.4 here and 8.3 there, 16 of
+// them 13.0 and 11.2, 256 of them 121 and 90; n = 2, 256 of them 101 and 88).
+constexpr int kBlockedMinTokens = 4;
 constexpr int kTokBatch = 8;   // token vectors staged in shared memory per barrier round
 
 // packed fp32 pairs (Blackwell): two FMAs / multiplies per instruction on 64-bit register pairs
@@ -227,7 +230,7 @@ int launch_typed(const void* q, const void* k, const void* v, const float* g, co
   const T* tq = static_cast<const T*>(q); const T* tk = static_cast<const T*>(k);
   const T* tv = static_cast<const T*>(v); const T* tb = static_cast<const T*>(b);
   const T* tw = static_cast<const T*>(w); T* to = static_cast<T*>(o);
-  if (DK == 128 && DV == 128 && n >= kBlockedMinTokens) {
+  if (DK == 128 && DV == 128 && (n >= kBlockedMinTokens || (n > 1 && B * H > device_sm_count()))) {
     return launch_decode_blocked<T>(tq, tk, tv, g, tb, tw, state, to, B, n, H, HK, in_bs, o_bs, scale, chained, st);
   } else if (DK == 128 && DV == 128) {
     GDN2_CUDA_TRY(launch_chained(chained, decode_square_kernel<T, 128>, dim3(B * H), 128, 0, st, tq, tk, tv, g, tb, tw, state, to, n, H, HK, in_bs, o_bs, scale));

@@ -1,15 +1,15 @@
 // Recurrent decode of several tokens at once, DK = DV = 128: the n-token recurrence of
-// decode_multi_kernel (gdn2/inference.py:199-303 of the reference project) evaluated in blocks of up
-// to 8 tokens without a per-token dependent sweep over the state.
+// decode_multi_kernel (gdn2/inference.py:199-303 of the reference project) evaluated in blocks of NB = 2, 4, 6
+// or 8 tokens without a per-token dependent sweep over the state.
 //
 // With A_t = exp(g_1 + .. + g_t) per key channel (A_t / A_s <= 1 for s <= t, so nothing can overflow):
 //     u_t = w_t*v_t - (b_t*k_t*A_t)^T S_0 - sum_{s<t} Akk[t,s] u_s      Akk[t,s] = sum_c b_t k_t k_s A_t/A_s
 //     o_t = (scale*q_t*A_t)^T S_0 + sum_{s<=t} Aqk[t,s] u_s              Aqk[t,s] = scale * sum_c q_t k_s A_t/A_s
-//     S_8 = diag(A_8) S_0 + sum_s (k_s * A_8/A_s) u_s^T
+//     S_NB = diag(A_NB) S_0 + sum_s (k_s * A_NB/A_s) u_s^T
 // (the exponent of every A_t / A_s is the sum of the gates s+1 .. t, not a difference of prefix sums, in which one strong gate
 // would swallow the ordinary ones after it; gates are read as max(g, kMinGate), whose exponential is zero already)
 // which is the token-by-token recurrence S <- diag(exp g) S; u = w*v - S^T(b*k); S <- S + k u^T;
-// o = scale S^T q with the sums regrouped: two sweeps over the state tile with 64 and 36 independent
+// o = scale S^T q with the sums regrouped: two sweeps over the state tile with 64 and 36 (NB = 8) independent
 // accumulation chains per thread instead of 2 n sweeps that each wait for a cross-thread reduction.
 //
 // Persistent blocks, one per SM, walk over the (batch, head) tiles with four kinds of warps:
@@ -20,7 +20,7 @@
 //     bulk copy per token row;
 //   * four table warps (thread = channel) fetch the token vectors a step ahead as 16-byte pieces, pass them
 //     through a staging buffer to read their own channel, and build the step's coefficient tables and the
-//     8 x 8 pair matrices while the current step is swept;
+//     NB x NB pair matrices while the current step is swept;
 //   * eight sweep warps do the two sweeps in place: warp w owns value columns 16w .. 16w+15, lane
 //     (rgl = lane >> 2, cq = lane & 3) columns 16w + 4cq .. +3 of key rows 16 rgl .. 16 rgl + 15.
 // Hand-offs are mbarriers with bounded waits.
@@ -36,7 +36,6 @@ namespace gdn2 {
 namespace {
 
 constexpr int D = 128;
-constexpr int NB = 8;                       // tokens per block step
 constexpr float kMinGate = -110.f;          // exp(-104) is already below half of float32's smallest number
 constexpr int kGroupFloats = 16 * D + 16;   // 16 state rows + 64 bytes: adjacent row groups land 64 B apart mod 128
 constexpr int kTileFloats = 8 * kGroupFloats;
@@ -65,20 +64,22 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+template <int NB>
 struct Tables {
-  // per key row: chunks 0, 1 = b*k*A_t for t < 8, chunks 2, 3 = scale*q*A_t (four consecutive products per chunk)
-  float4 c1[4][kCoefRows];
-  // per key row: k * A_8/A_s for s = 0..3 (chunk 0) and s = 4..7 (chunk 1); A_8 itself
-  float4 c2[2][kCoefRows];
+  // per key row the 2 NB products, four per chunk: b*k*A_t for t < NB, then scale*q*A_t
+  float4 c1[NB / 2][kCoefRows];
+  // per key row: k * A_NB/A_s, four per chunk; A_NB itself
+  float4 c2[(NB + 3) / 4][kCoefRows];
   float gam[kCoefRows];
   float wv[NB][D];                    // w * v
-  float akk[NB][NB];                  // strictly lower
-  float aqk[NB][NB];                  // lower incl. diagonal, scale folded in
+  float akk[NB][8];                   // strictly lower
+  float aqk[NB][8];                   // lower incl. diagonal, scale folded in
 };
 
+template <int NB>
 struct alignas(128) BlockedSmem {
   float tile[2][kTileFloats];         // the state of two (batch, head) tiles
-  Tables tab[2];                      // coefficient tables of two consecutive steps
+  Tables<NB> tab[2];                      // coefficient tables of two consecutive steps
   float part[4][64];                  // per 32-channel group: partial sums of the 64 pair entries
   // one step's token vectors as they lie in memory: q, k, b, v, w rows of D elements (up to 4 bytes each), then g
   alignas(16) unsigned char stage[6 * NB * D * 4];
@@ -138,14 +139,16 @@ __device__ __forceinline__ bool table_sync_or(bool pred) {
 
 enum : uint32_t { kWaitTile = 0x10000u, kWaitTab = 0x20000u, kWaitEmpty = 0x40000u, kWaitDone = 0x80000u, kWaitOut = 0x100000u };
 
-template <typename T, typename Seqs>
+template <typename T, typename Seqs, int NB>
 __global__ void __launch_bounds__(kAllThreads, 1)
 decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                       const float* __restrict__ g, const T* __restrict__ b, const T* __restrict__ w,
                       float* __restrict__ state, T* __restrict__ o, int ntiles, int n, int H, int HK, int64_t in_bs,
                       int64_t o_bs, float scale, uint32_t* status, const __grid_constant__ Seqs seqs) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  BlockedSmem& s = *reinterpret_cast<BlockedSmem*>(smem_raw);
+  static_assert(NB % 2 == 0 && NB >= 2 && NB <= 8, "products are paired, pair matrices have eight columns");
+  using Smem = BlockedSmem<NB>;
+  Smem& s = *reinterpret_cast<Smem*>(smem_raw);
   const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
 
   // tokens of a tile, and its first input and output row (in tokens). Packed sequences: the last len % 64 tokens of
@@ -252,12 +255,13 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
     // =============================== table warps: thread = key / value channel =================
     const int c = tid - kSweepThreads;
     const int pw_ = wid - 8;                             // 32-channel group
-    // A step's token vectors are 8 rows of D elements per tensor, contiguous per row: the 128 threads fetch them
-    // as 16-byte pieces (CH pieces per thread and tensor, two for g), ONE STEP AHEAD, into registers; at the
+    // A step's token vectors are NB rows of D elements per tensor, contiguous per row: the 128 threads fetch them
+    // as 16-byte pieces (CH pieces per thread and tensor, CG for g), ONE STEP AHEAD, into registers; at the
     // top of a step the pieces go to the staging buffer and every thread reads its own channel from there.
-    constexpr int CH = sizeof(T) / 2;                    // 16-byte pieces per thread: 8 rows x D x sizeof(T) / 16 / 128
-    constexpr int kRowPieces = D * (int)sizeof(T) / 16;  // pieces per row
-    uint4 ldT[5][CH], ldG[2];
+    constexpr int kRowPieces = D * (int)sizeof(T) / 16;  // 16-byte pieces per row
+    constexpr int CH = (NB * kRowPieces + kTableThreads - 1) / kTableThreads;   // ... per thread and tensor, the last ones perhaps past NB rows
+    constexpr int CG = (NB * (D / 4) + kTableThreads - 1) / kTableThreads;
+    uint4 ldT[5][CH], ldG[CG];
     auto issue_loads = [&](int ptile, int pt0) {
       const int pih = ptile % H, pihk = pih / (H / HK);
       size_t prow;
@@ -274,7 +278,7 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
         ldT[4][j] = __ldg(reinterpret_cast<const uint4*>(w + rowv) + within);
       }
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
+      for (int j = 0; j < CG; ++j) {
         const int e = c + kTableThreads * j, tokr = e / (D / 4), within = e % (D / 4);
         const int tt = pt0 + (tokr < pnb ? tokr : pnb - 1);
         ldG[j] = __ldg(reinterpret_cast<const uint4*>(g + ((prow + tt) * HK + pihk) * D) + within);
@@ -289,16 +293,17 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
         const int nt = tile_tokens(tile, nullptr, nullptr), nb = min(NB, nt - t0);
         t0 += NB;                                        // the step after this one
         if (t0 >= nt) { t0 = 0; tile = from_tile(tile + gridDim.x); }
-        Tables& tb = s.tab[step & 1];
+        Tables<NB>& tb = s.tab[step & 1];
         // every thread has read the previous step's staging buffer (two table barriers lie in between)
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
 #pragma unroll
           for (int x = 0; x < 5; ++x)
-            reinterpret_cast<uint4*>(stT + (size_t)x * NB * D)[c + kTableThreads * j] = ldT[x][j];
+            if (c + kTableThreads * j < NB * kRowPieces) reinterpret_cast<uint4*>(stT + (size_t)x * NB * D)[c + kTableThreads * j] = ldT[x][j];
         }
 #pragma unroll
-        for (int j = 0; j < 2; ++j) reinterpret_cast<uint4*>(stG)[c + kTableThreads * j] = ldG[j];
+        for (int j = 0; j < CG; ++j)
+          if (c + kTableThreads * j < NB * (D / 4)) reinterpret_cast<uint4*>(stG)[c + kTableThreads * j] = ldG[j];
         if (tile < ntiles) issue_loads(tile, t0);
         table_sync();
         float graw[NB];
@@ -327,14 +332,14 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
         if (table_sync_or(!okw)) break;
         {
           const int pr = crow(c);
-          float c1v[16], c2v[8], An = 1.f;
-          float run = 0.f, rest = 0.f;                   // log2 of A_t and of A_8 / A_t
+          float c1v[2 * NB], c2v[4 * ((NB + 3) / 4)], An = 1.f;
+          float run = 0.f, rest = 0.f;                   // log2 of A_t and of A_NB / A_t
 #pragma unroll
           for (int t = 0; t < NB; ++t) {
             run += l[t];
             An = ex2(run);
             c1v[t] = bk[t] * An;
-            c1v[8 + t] = qs[t] * An;
+            c1v[NB + t] = qs[t] * An;
             tb.wv[t][c] = wvv[t];
           }
 #pragma unroll
@@ -343,25 +348,28 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
             rest += l[t];
           }
 #pragma unroll
-          for (int j = 0; j < 4; ++j) tb.c1[j][pr] = make_float4(c1v[4 * j], c1v[4 * j + 1], c1v[4 * j + 2], c1v[4 * j + 3]);
+          for (int t = NB; t < 4 * ((NB + 3) / 4); ++t) c2v[t] = 0.f;
 #pragma unroll
-          for (int j = 0; j < 2; ++j) tb.c2[j][pr] = make_float4(c2v[4 * j], c2v[4 * j + 1], c2v[4 * j + 2], c2v[4 * j + 3]);
+          for (int j = 0; j < NB / 2; ++j) tb.c1[j][pr] = make_float4(c1v[4 * j], c1v[4 * j + 1], c1v[4 * j + 2], c1v[4 * j + 3]);
+#pragma unroll
+          for (int j = 0; j < (NB + 3) / 4; ++j) tb.c2[j][pr] = make_float4(c2v[4 * j], c2v[4 * j + 1], c2v[4 * j + 2], c2v[4 * j + 3]);
           tb.gam[pr] = An;
         }
         // Slot (t, sx) holds the Akk[t, sx] term for sx < t and the Aqk[sx, t] term for sx >= t (the upper
         // triangle is free). Summing over the warp's 32 channels: each step halves what a lane keeps.
         float span[NB];                                  // span[sx] = l[sx + 1] + .. + l[t], log2 of A_t / A_sx
 #pragma unroll
-        for (int hb = 0; hb < 2; ++hb) {
+        for (int hb = 0; hb < (NB + 3) / 4; ++hb) {
           float term[32];
 #pragma unroll
           for (int tt = 0; tt < 4; ++tt) {
             const int t = 4 * hb + tt;
             float ahead = 0.f;
 #pragma unroll
-            for (int sx = 0; sx < NB; ++sx) {
-              float val;
-              if (sx < t) {                                                   // Akk[t, sx], A_t / A_s <= 1
+            for (int sx = 0; sx < 8; ++sx) {
+              float val = 0.f;
+              if (t >= NB || sx >= NB) {                                      // (slots of no token)
+              } else if (sx < t) {                                                   // Akk[t, sx], A_t / A_s <= 1
                 span[sx] = sx == t - 1 ? l[t] : span[sx] + l[t];
                 val = bk[t] * kk[sx] * ex2(span[sx]);
               } else if (sx == t) {                                           // Aqk[t, t]
@@ -394,7 +402,8 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
         if (c < 64) {
           const float sum = s.part[0][c] + s.part[1][c] + s.part[2][c] + s.part[3][c];
           const int t = c >> 3, sx = c & 7;
-          if (sx < t) tb.akk[t][sx] = sum;               // Akk[t, sx]
+          if (t >= NB || sx >= NB) {}
+          else if (sx < t) tb.akk[t][sx] = sum;          // Akk[t, sx]
           else tb.aqk[sx][t] = sum;                      // slot (t, sx) with sx >= t holds Aqk[sx, t]
         }
         warp_arrive(&s.tab_full[step & 1], lane);
@@ -412,19 +421,19 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
       float* S = s.tile[buf];
       bool ok = true;
       for (int t0 = 0; t0 < nt; t0 += NB, ++step) {
-        const Tables& tb = s.tab[step & 1];
+        const Tables<NB>& tb = s.tab[step & 1];
         ok = tc::mbar_wait(&s.tab_full[step & 1], (step >> 1) & 1, &s.abort_flag, status, kWaitTab);
         if (ok && t0 == 0) ok = tc::mbar_wait(&s.tile_full[buf], (it >> 1) & 1, &s.abort_flag, status, kWaitTile);
         ok = __all_sync(0xffffffffu, ok);                // the warp leaves together: what follows uses full-warp shuffles
         if (!ok) break;
 
-        // ---- sweep 1: the 16 products (8 erase rows, 8 query rows) of S_0 for this thread's rows and columns
+        // ---- sweep 1: the 2 NB products (NB erase rows, NB query rows) of S_0 for this thread's rows and columns
         //      packed over PAIRS OF PRODUCTS: acc[pp][col] = (product 2pp, product 2pp+1) of column col, so the
         //      coefficients are used as stored (no duplicated copies in shared memory) and the state value is
         //      the operand that is duplicated, in registers
-        float2 acc[8][4];
+        float2 acc[NB][4];
 #pragma unroll
-        for (int p = 0; p < 8; ++p) {
+        for (int p = 0; p < NB; ++p) {
 #pragma unroll
           for (int cc = 0; cc < 4; ++cc) acc[p][cc] = make_float2(0.f, 0.f);
         }
@@ -436,7 +445,7 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
           const float2 sd[4] = {make_float2(sv.x, sv.x), make_float2(sv.y, sv.y), make_float2(sv.z, sv.z),
                                 make_float2(sv.w, sv.w)};
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
+          for (int j = 0; j < NB / 2; ++j) {
             const float4 cf = tb.c1[j][cr0 + i];
 #pragma unroll
             for (int cc = 0; cc < 4; ++cc) {
@@ -445,20 +454,20 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
             }
           }
         }
-        // reduce over the 8 row groups. Index = half*32 + column*8 + t (half 0: erase products, 1: query
-        // products); lane (rgl) ends with the 8 values of half rgl >> 2, column rgl & 3.
-        float pv[8];
+        // reduce over the 8 row groups. Index = (half * 4 + column) * NB + t (half 0: erase products, 1: query
+        // products); lane (rgl) ends with the NB values of half rgl >> 2, column rgl & 3.
+        float pv[NB];
         {
-          float val[64];
+          float val[8 * NB];
 #pragma unroll
-          for (int pp = 0; pp < 8; ++pp) {
-            const int base = (pp >> 2) * 32 + 2 * (pp & 3);       // products 2pp, 2pp + 1
+          for (int pp = 0; pp < NB; ++pp) {
+            const int half = pp / (NB / 2), base = half * 4 * NB + 2 * pp - half * NB;       // products 2pp, 2pp + 1
 #pragma unroll
-            for (int cc = 0; cc < 4; ++cc) { val[base + cc * 8] = acc[pp][cc].x; val[base + cc * 8 + 1] = acc[pp][cc].y; }
+            for (int cc = 0; cc < 4; ++cc) { val[base + cc * NB] = acc[pp][cc].x; val[base + cc * NB + 1] = acc[pp][cc].y; }
           }
 #pragma unroll
           for (int m = 0; m < 3; ++m) {
-            const int half = 32 >> m;
+            const int half = (4 * NB) >> m;
             const int bit = 16 >> m;                     // lane bits 4, 3, 2 = rgl bits 2, 1, 0
             const bool up = (lane & bit) != 0;
 #pragma unroll
@@ -469,13 +478,13 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
             }
           }
 #pragma unroll
-          for (int t = 0; t < 8; ++t) pv[t] = val[t];
+          for (int t = 0; t < NB; ++t) pv[t] = val[t];
         }
         // ---- forward substitution for u on the lanes that hold the erase products; the lanes that hold
         //      the query products of the same column take u from them and form the outputs
         const bool has_q = (rgl & 4) != 0;
         const int mycol = col0 + (rgl & 3);
-        float u[8];
+        float u[NB];
         {
           float4 ak[NB][2];                              // rows of Akk, fetched ahead of the dependent chain
 #pragma unroll
@@ -516,7 +525,7 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
         warp_arrive(&s.o_full[step & 1], lane);
         // gather u of the thread's four columns from the lanes that share cq (rgl bits 0 and 1 = lane bits 2, 3)
         //      and pair them over tokens: up[tp][c] = (u_{2tp}, u_{2tp+1}) of column col0 + c
-        float2 up[4][4];
+        float2 up[NB / 2][4];
 #pragma unroll
         for (int t = 0; t < NB; ++t) {
           const float o4 = __shfl_xor_sync(0xffffffffu, u[t], 4);      // column (rgl & 3) ^ 1
@@ -531,22 +540,28 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
             else up[t >> 1][cc].x = uc[cc];
           }
         }
-        // ---- sweep 2: S <- A_8 * S + sum_s (k_s A_8/A_s) u_s^T, in place
+        // ---- sweep 2: S <- A_NB * S + sum_s (k_s A_NB/A_s) u_s^T, in place
         {
           float* Sw = S + rgl * kGroupFloats + col0;
 #pragma unroll 4
           for (int i = 0; i < 16; ++i) {
-            // per column a dot product over the 8 tokens, packed over token pairs (coefficients as stored)
+            // per column a dot product over the NB tokens, packed over token pairs (coefficients as stored)
             const float4 sv = *reinterpret_cast<const float4*>(Sw + i * D);
-            const float4 ka = tb.c2[0][cr0 + i], kb = tb.c2[1][cr0 + i];
+            float2 kp[NB / 2];
+#pragma unroll
+            for (int j = 0; j < (NB + 3) / 4; ++j) {
+              const float4 kq = tb.c2[j][cr0 + i];
+              kp[2 * j] = make_float2(kq.x, kq.y);
+              if (2 * j + 1 < NB / 2) kp[2 * j + 1] = make_float2(kq.z, kq.w);
+            }
             const float ga = tb.gam[cr0 + i];
-            const float2 k01 = make_float2(ka.x, ka.y), k23 = make_float2(ka.z, ka.w);
-            const float2 k45 = make_float2(kb.x, kb.y), k67 = make_float2(kb.z, kb.w);
             const float svv[4] = {sv.x, sv.y, sv.z, sv.w};
             float nn[4];
 #pragma unroll
             for (int cc = 0; cc < 4; ++cc) {
-              const float2 d = ffma2(k01, up[0][cc], ffma2(k23, up[1][cc], ffma2(k45, up[2][cc], fmul2(k67, up[3][cc]))));
+              float2 d = fmul2(kp[NB / 2 - 1], up[NB / 2 - 1][cc]);
+#pragma unroll
+              for (int j = NB / 2 - 2; j >= 0; --j) d = ffma2(kp[j], up[j][cc], d);
               nn[cc] = fmaf(ga, svv[cc], d.x + d.y);
             }
             *reinterpret_cast<float4*>(Sw + i * D) = make_float4(nn[0], nn[1], nn[2], nn[3]);
@@ -567,21 +582,33 @@ template <typename T>
 int launch_decode_blocked(const T* q, const T* k, const T* v, const float* g, const T* b, const T* w, float* state,
                           T* o, int B, int n, int H, int HK, int64_t in_bs, int64_t o_bs, float scale, bool chained,
                           cudaStream_t st) {
-  const size_t smem = sizeof(BlockedSmem) + 128;
-  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(decode_blocked_kernel<T, OneLength>), smem));
   const int ntiles = B * H;
   const int sms = device_sm_count();
   const int grid = ntiles < sms ? ntiles : sms;
-  GDN2_CUDA_TRY(launch_chained(chained, decode_blocked_kernel<T, OneLength>, dim3(grid), kAllThreads, smem, st, q, k, v, g, b, w, state, o, ntiles,
-                               n, H, HK, in_bs, o_bs, scale, device_status_word(), OneLength{}));
-  return GDN2_OK;
+  auto launch = [&](auto kern, size_t smem) -> int {
+    GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
+    GDN2_CUDA_TRY(launch_chained(chained, kern, dim3(grid), kAllThreads, smem, st, q, k, v, g, b, w, state, o, ntiles, n, H, HK, in_bs, o_bs,
+                                 scale, device_status_word(), OneLength{}));
+    return GDN2_OK;
+  };
+  // Tokens per step: padding tokens cost what real ones do, so the fewest that n needs; in several steps 6 or 8, whichever takes
+  // less, a step of 6 being about four fifths of one of 8. bf16, 16 heads, 256 / 24 conversations, us (steps of 8 before, and
+  // token by token for n = 2 and 3): n = 2 101 -> 88 / 12.9 -> 12.8, n = 3 121 -> 90 / 14.8 -> 14.1, n = 4 113 -> 91 / 18.6 -> 14.3,
+  // n = 5 114 -> 97 / 18.9 -> 16.6, n = 12 213 -> 171 / 30.1 -> 25.4; steps of 6 for n = 16 would take 251 / 34.3 in place of 214 / 30.3.
+  // A prompt's ragged tail (not chained) takes steps of 8 however short it is: in a packed batch the tails of all lengths share a
+  // launch, and a sequence has the same bits there and alone.
+  if (!chained) return launch(decode_blocked_kernel<T, OneLength, 8>, sizeof(BlockedSmem<8>) + 128);
+  if (n <= 2) return launch(decode_blocked_kernel<T, OneLength, 2>, sizeof(BlockedSmem<2>) + 128);
+  if (n <= 4) return launch(decode_blocked_kernel<T, OneLength, 4>, sizeof(BlockedSmem<4>) + 128);
+  if ((n + 5) / 6 * 4 < (n + 7) / 8 * 5) return launch(decode_blocked_kernel<T, OneLength, 6>, sizeof(BlockedSmem<6>) + 128);
+  return launch(decode_blocked_kernel<T, OneLength, 8>, sizeof(BlockedSmem<8>) + 128);
 }
 
 int launch_decode_packed_tails(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
                                float* state, void* o, const PackedSeqs& seqs, int H, int HK, float scale, cudaStream_t st) {
   using T = __nv_bfloat16;
-  const size_t smem = sizeof(BlockedSmem) + 128;
-  auto kern = decode_blocked_kernel<T, PackedSeqs>;
+  const size_t smem = sizeof(BlockedSmem<8>) + 128;
+  auto kern = decode_blocked_kernel<T, PackedSeqs, 8>;
   GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
   const int ntiles = seqs.n * H, sms = device_sm_count();
   GDN2_CUDA_TRY(launch_chained(false, kern, dim3(ntiles < sms ? ntiles : sms), kAllThreads, smem, st, static_cast<const T*>(q),
