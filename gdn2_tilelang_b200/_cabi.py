@@ -61,6 +61,8 @@ SIGNATURES = {
     "gdn2_layer_front": (_int, [_vp, _int, _vp]),
     "gdn2_oproj_reduce_buffer_bytes": (_sz, [_i64, _i64, ctypes.POINTER(_sz)]),
     "gdn2_oproj_reduce": (_int, [_vp, _int, _vp]),
+    "gdn2_layer_step_workspace_bytes": (_sz, [_i64] * 7 + [_int]),
+    "gdn2_layer_step": (_int, [_vp, _int, _vp]),
     "gdn2_layer_back": (_int, [_vp] * 4 + [_i64] * 5 + [_f32, _int, _vp]),
 }
 
@@ -73,6 +75,18 @@ class LayerFrontArgs(ctypes.Structure):
                 + [(n, _i64) for n in ("B", "S", "H", "HK", "DK", "DV", "K", "NP",
                                        "off_q", "off_k", "off_v", "off_b", "off_w", "off_f")]
                 + [("erase_scale", _f32)])
+
+
+class LayerStepArgs(ctypes.Structure):
+    """``gdn2_layer_step_args`` of include/gdn2_b200.h."""
+
+    _fields_ = ([(n, _vp) for n in ("x", "w_cat", "conv_state", "conv_weight", "conv_bias", "A_log", "dt_bias", "norm_weight",
+                                    "o_weight", "state", "new_conv_state", "out", "workspace")]
+                + [("workspace_bytes", _sz)]
+                + [(n, _i64) for n in ("B", "hidden", "H", "HK", "DK", "DV", "K",
+                                       "off_q", "off_k", "off_v", "off_b", "off_w", "off_f", "off_gate")]
+                + [("erase_scale", _f32), ("eps", _f32), ("scale", _f32)])
+
 
 class GatedNormArgs(ctypes.Structure):
     """``gdn2_gated_norm`` of include/gdn2_b200.h."""
@@ -559,6 +573,41 @@ class NativeKernels:
         _check(self.lib, rc, "gdn2_layer_front")
         self.launches += 2 if (new_conv is not None and not fused_tail) else 1
         return q, k, v, g, b, w, new_conv
+
+    def layer_step(self, x, state, conv_state, w_cat, conv_weight, conv_bias, A_log, dt_bias, norm_weight, o_weight, offsets, H, HK,
+                   DK, DV, K, erase_scale, eps, scale, conv_in_place):
+        """``gdn2_layer_step``: one token per sequence, ``x [B, 1, hidden]``, through the whole layer, ``state`` updated in place
+        (what the host extension's ``layer_decode`` does for such a call). Returns ``(out, new_conv_state, kernels launched)``,
+        or ``None`` where these kernels do not apply and the stages are called one by one."""
+        if x.dim() != 3 or x.shape[1] != 1 or not x.is_cuda or torch.is_autocast_enabled("cuda"):
+            return None
+        B, _, hidden = x.shape
+        dt, dev = x.dtype, x.device
+        if dt not in (torch.bfloat16, torch.float16) or K != 4 or w_cat.shape[1] != hidden or o_weight.shape != (hidden, H * DV):
+            return None
+        CC = 2 * HK * DK + H * DV
+        x = x.contiguous()
+        if x.data_ptr() % 16:
+            x = x.clone()
+        tensors = [w_cat, conv_state, conv_weight, A_log, dt_bias, norm_weight, o_weight] + ([] if conv_bias is None else [conv_bias])
+        if (any(t.dtype != dt or t.device != dev or not t.is_contiguous() or t.data_ptr() % 16 for t in tensors)
+                or conv_state.shape != (B, CC, K - 1) or state.shape != (B, H, DK, DV) or state.dtype != torch.float32
+                or state.device != dev or not state.is_contiguous() or state.data_ptr() % 16):
+            return None
+        nbytes = self.lib.gdn2_layer_step_workspace_bytes(B, hidden, H, HK, DK, DV, K, dtype_code(dt))
+        if nbytes == 0:
+            return None
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+        out = torch.empty(B, 1, hidden, dtype=dt, device=dev)
+        conv = conv_state if conv_in_place else torch.empty_like(conv_state)
+        a = LayerStepArgs(x.data_ptr(), w_cat.data_ptr(), conv_state.data_ptr(), conv_weight.data_ptr(),
+                          None if conv_bias is None else conv_bias.data_ptr(), A_log.data_ptr(), dt_bias.data_ptr(),
+                          norm_weight.data_ptr(), o_weight.data_ptr(), state.data_ptr(), conv.data_ptr(), out.data_ptr(),
+                          ws.data_ptr(), nbytes, B, hidden, H, HK, DK, DV, K, *offsets, erase_scale, eps, scale)
+        with _on_device(dev):
+            rc = self.lib.gdn2_layer_step(ctypes.byref(a), dtype_code(dt), self._stream(x))
+        _check(self.lib, rc, "gdn2_layer_step")
+        return out, conv, 3
 
     def layer_back(self, o, proj, norm_weight, off_gate, eps):
         """Fused gated RMSNorm: ``o [B, S, H, DV]`` and the o_gate columns of ``proj`` -> ``[B, S, H*DV]``."""

@@ -288,13 +288,14 @@ class GatedDeltaNet2(nn.Module):
         """``o_proj``; the head-parallel variant overrides it to add the sum over ranks."""
         return self.o_proj(normed)
 
-    def _decode_plain(self, x, cache):
-        """The whole of ``decode`` as one native call, or ``None`` where something about the layer, the cache or the input
+    def _decode_plain(self, x, cache, conv_in_place=False):
+        """The whole of ``decode`` as one native call (with ``conv_in_place`` the convolution cache is written into, too), or ``None`` where something about the layer, the cache or the input
         needs the general path (a subclass, hooks, replaced methods, a missing or converted convolution cache, strided
         tensors): whatever would have run when ``o_proj`` is called as a module still runs."""
         K = _cabi.kernels()
         host = getattr(K, "host", None)
-        if host is None or type(self) is not GatedDeltaNet2 or cache.conv_state is None:
+        call = getattr(K, "layer_step", None) if host is None else host.layer_decode
+        if call is None or type(self) is not GatedDeltaNet2 or cache.conv_state is None:
             return None
         m = self._modules
         o_proj = m["o_proj"]
@@ -304,12 +305,14 @@ class GatedDeltaNet2(nn.Module):
             return None
         w_cat, offs, cw, cb = self._fused_tables()
         own = self._parameters
-        res = host.layer_decode(x, cache.recurrent_state, cache.conv_state, w_cat, cw, cb, own["A_log"], own["dt_bias"],
-                                m["o_norm"].weight, o_proj.weight, offs, self.num_heads, self.num_kv_heads, self.head_dim_k,
-                                self.head_dim_v, self.cfg.conv_size, self.erase_scale, m["o_norm"].eps, self.scale)
+        res = call(x, cache.recurrent_state, cache.conv_state, w_cat, cw, cb, own["A_log"], own["dt_bias"],
+                   m["o_norm"].weight, o_proj.weight, offs, self.num_heads, self.num_kv_heads, self.head_dim_k,
+                   self.head_dim_v, self.cfg.conv_size, self.erase_scale, m["o_norm"].eps, self.scale, conv_in_place)
         if res is None:
             return None
-        out, cache.conv_state, launched = res
+        out, conv, launched = res
+        if not conv_in_place:
+            cache.conv_state = conv
         K.launches += launched
         K.maybe_check_device_status(x.device)
         return out
@@ -361,10 +364,14 @@ class GatedDeltaNet2(nn.Module):
         o = gdn2_decode(q, k, v, g, b, w, cache.recurrent_state, scale=self.scale)
         return self._back(hidden_states, o, proj), cache
 
-    @torch.no_grad()
     def step(self, hidden_states, cache: GDN2Cache):
         """Decode one token ``[B, hidden]``."""
-        out, cache = self.decode(hidden_states.unsqueeze(1), cache)
+        x = hidden_states.unsqueeze(1)
+        if "decode" not in self.__dict__ and type(self).decode is _DECODE:   # (what it does first, without its no-grad region)
+            out = self._decode_plain(x, cache)
+            if out is not None:
+                return out[:, 0], cache
+        out, cache = self.decode(x, cache)
         return out[:, 0], cache
 
     def init_cache(self, batch_size: int, device=None, dtype=torch.float32) -> GDN2Cache:
@@ -379,6 +386,9 @@ class GatedDeltaNet2(nn.Module):
             conv_state = torch.zeros(batch_size, channels, self.cfg.conv_size - 1, device=device,
                                      dtype=self.o_proj.weight.dtype)
         return GDN2Cache(state, conv_state)
+
+
+_DECODE = GatedDeltaNet2.decode
 
 
 class GraphedStep:
@@ -422,6 +432,9 @@ class GraphedStep:
     def _step_in_place(self):
         layer, cache = self.layer, self.cache
         x = self.x.unsqueeze(1)
+        out = layer._decode_plain(x, cache, conv_in_place=True)
+        if out is not None:
+            return out[:, 0]
         q, k, v, g, b, w, conv, proj = layer._front(x, cache.conv_state, cached=layer.q_conv is not None,
                                                      update_cache_in_place=True)
         if conv is not None and conv is not cache.conv_state:

@@ -6,7 +6,9 @@
 // current device -- and returns None for anything else, so that the general path in Python handles it or raises the
 // error that belongs to it. Nothing is kept between calls.
 #include <ATen/ATen.h>
+#include <ATen/autocast_mode.h>
 #include <ATen/core/grad_mode.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/utils/pybind.h>
@@ -18,13 +20,16 @@ using at::Tensor;
 
 namespace {
 
-// a dense, 16-byte aligned tensor of this dtype on the current device, not wrapped by a transform or a subclass
-bool plain(const Tensor& t, at::ScalarType dt, c10::DeviceIndex dev) {
-  return t.defined() && t.is_cuda() && t.get_device() == dev && t.scalar_type() == dt && t.is_contiguous() &&
+// a tensor of this dtype on the current device, not wrapped by a transform or a subclass
+bool unwrapped(const Tensor& t, at::ScalarType dt, c10::DeviceIndex dev) {
+  return t.defined() && t.is_cuda() && t.get_device() == dev && t.scalar_type() == dt &&
          !t.is_conj() && !t.is_neg() && t.key_set().has(c10::DispatchKey::CUDA) && !t.key_set().has(c10::DispatchKey::Python) &&
          !t.key_set().has(c10::DispatchKey::FuncTorchBatched) && !t.key_set().has(c10::DispatchKey::FuncTorchGradWrapper) &&
-         !t.key_set().has(c10::DispatchKey::Functionalize) && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0;
+         !t.key_set().has(c10::DispatchKey::Functionalize);
 }
+// dense and 16-byte aligned
+bool dense(const Tensor& t) { return t.is_contiguous() && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0; }
+bool plain(const Tensor& t, at::ScalarType dt, c10::DeviceIndex dev) { return unwrapped(t, dt, dev) && dense(t); }
 
 int dtype_code(at::ScalarType dt) {
   return dt == at::kBFloat16 ? GDN2_BF16 : dt == at::kHalf ? GDN2_F16 : dt == at::kFloat ? GDN2_F32 : -1;
@@ -108,12 +113,13 @@ std::optional<std::tuple<Tensor, Tensor, int64_t>> prefill(const Tensor& q, cons
 }
 
 
-// GatedDeltaNet2.decode on x [B, n, hidden]: projections, layer_front, decode, layer_back, output projection. The recurrent
-// state is updated in place. Returns (out [B, n, hidden], new convolution cache, kernels launched) or None.
-std::optional<std::tuple<Tensor, Tensor, int64_t>> layer_decode(const Tensor& x, const Tensor& state, const std::optional<Tensor>& conv_state, const Tensor& w_cat,
+// GatedDeltaNet2.decode on x [B, n, hidden]: gdn2_layer_step where it applies, else projections, layer_front, decode,
+// layer_back, output projection. The recurrent state is updated in place. Returns (out [B, n, hidden], new convolution cache,
+// kernels launched) or None. `conv_in_place`: the convolution cache is updated in place too, or the call is not made.
+std::optional<std::tuple<Tensor, Tensor, int64_t>> layer_decode(Tensor x, const Tensor& state, const std::optional<Tensor>& conv_state, const Tensor& w_cat,
                         const std::optional<Tensor>& conv_w, const std::optional<Tensor>& conv_b, const Tensor& A_log,
                         const Tensor& dt_bias, const Tensor& norm_w, const Tensor& o_w, const std::vector<int64_t>& offs, int64_t H,
-                        int64_t HK, int64_t DK, int64_t DV, int64_t K, double erase_scale, double eps, double scale) {
+                        int64_t HK, int64_t DK, int64_t DV, int64_t K, double erase_scale, double eps, double scale, bool conv_in_place) {
   Problem p;
   p.type = x.scalar_type();
   p.dtype = dtype_code(p.type);
@@ -122,36 +128,65 @@ std::optional<std::tuple<Tensor, Tensor, int64_t>> layer_decode(const Tensor& x,
   p.B = x.size(0); p.S = x.size(1); p.H = H; p.HK = HK; p.DK = DK; p.DV = DV;
   for (const Tensor* t : {&w_cat, &A_log, &dt_bias, &norm_w, &o_w})
     if (!plain(*t, p.type, p.dev)) return std::nullopt;
+  at::NoGradGuard no_grad;
+  // one token out of a prompt that lies in memory whole (x[:, t]): its rows are brought together
+  if (p.S == 1 && unwrapped(x, p.type, p.dev) && !dense(x)) x = x.clone(at::MemoryFormat::Contiguous);
   if (!plain(x, p.type, p.dev) || !plain_state(state, p) || x.size(2) != w_cat.size(1)) return std::nullopt;
   const int64_t CC = 2 * HK * DK + H * DV;
   if (K < 2 || !conv_w || !plain(*conv_w, p.type, p.dev) || (conv_b && !plain(*conv_b, p.type, p.dev)) || !conv_state ||
       !plain(*conv_state, p.type, p.dev) || conv_state->dim() != 3 || conv_state->size(0) != p.B || conv_state->size(1) != CC ||
       conv_state->size(2) != K - 1)
     return std::nullopt;
-  at::NoGradGuard no_grad;
+  const auto opt = x.options().requires_grad(false);
+  const int64_t hidden = x.size(2);
+  // (an autocast region or a dispatch mode would have seen the two linear layers)
+  const size_t step_bytes = p.S == 1 && o_w.dim() == 2 && o_w.size(0) == hidden && o_w.size(1) == H * DV &&
+                                    !at::autocast::is_autocast_enabled(at::kCUDA) && !c10::impl::TorchDispatchModeTLS::any_modes_set()
+                                ? gdn2_layer_step_workspace_bytes(p.B, hidden, H, HK, DK, DV, K, p.dtype)
+                                : 0;
+  if (step_bytes > 0) {
+    Tensor ws = at::empty({(int64_t)step_bytes}, opt.dtype(at::kByte)), out = at::empty({p.B, 1, hidden}, opt);
+    Tensor conv = conv_in_place ? *conv_state : at::empty({p.B, CC, K - 1}, opt);
+    gdn2_layer_step_args s{};
+    s.x = x.data_ptr(); s.w_cat = w_cat.data_ptr(); s.conv_state = conv_state->data_ptr(); s.conv_weight = conv_w->data_ptr();
+    s.conv_bias = conv_b ? conv_b->data_ptr() : nullptr;
+    s.A_log = A_log.data_ptr(); s.dt_bias = dt_bias.data_ptr(); s.norm_weight = norm_w.data_ptr(); s.o_weight = o_w.data_ptr();
+    s.state = static_cast<float*>(state.data_ptr()); s.new_conv_state = conv.data_ptr(); s.out = out.data_ptr();
+    s.workspace = ws.data_ptr(); s.workspace_bytes = step_bytes;
+    s.B = p.B; s.hidden = hidden; s.H = H; s.HK = HK; s.DK = DK; s.DV = DV; s.K = K;
+    s.off_q = offs[0]; s.off_k = offs[1]; s.off_v = offs[2]; s.off_b = offs[3]; s.off_w = offs[4]; s.off_f = offs[5]; s.off_gate = offs[6];
+    s.erase_scale = (float)erase_scale; s.eps = (float)eps; s.scale = (float)scale;
+    const int rc = gdn2_layer_step(&s, p.dtype, stream_of(p));
+    if (rc == GDN2_OK) return std::make_tuple(out, conv, int64_t(3));
+    // refused before anything ran; after a launch that failed part of the cache may have been written
+    if (rc == GDN2_ERR_CUDA) throw std::runtime_error(std::string("gdn2_layer_step: ") + gdn2_status_string(rc));
+  }
+  if (conv_in_place) return std::nullopt;
   Tensor proj = at::linear(x, w_cat);
   if (proj.scalar_type() != p.type || !proj.is_contiguous()) return std::nullopt;       // an autocast region
-  const auto opt = x.options().requires_grad(false);
-  Tensor q = at::empty({p.B, p.S, HK, DK}, opt), k = at::empty({p.B, p.S, HK, DK}, opt), b = at::empty({p.B, p.S, HK, DK}, opt);
-  Tensor g = at::empty({p.B, p.S, HK, DK}, opt.dtype(at::kFloat));
-  Tensor v = at::empty({p.B, p.S, H, DV}, opt), w = at::empty({p.B, p.S, H, DV}, opt), o = at::empty({p.B, p.S, H, DV}, opt);
-  Tensor conv = at::empty({p.B, CC, K - 1}, opt), normed = at::empty({p.B, p.S, H * DV}, opt);
+  // one allocation for what lives between the stages, every part 256-byte aligned
+  const int64_t esz = p.dtype == GDN2_F32 ? 4 : 2, tokens = p.B * p.S;
+  auto part = [](int64_t bytes) { return (bytes + 255) / 256 * 256; };
+  const int64_t key = part(tokens * HK * DK * esz), decay = part(tokens * HK * DK * 4), value = part(tokens * H * DV * esz);
+  Tensor mid = at::empty({3 * key + decay + 3 * value}, opt.dtype(at::kByte)), normed = at::empty({p.B, p.S, H * DV}, opt);
+  Tensor conv = at::empty({p.B, CC, K - 1}, opt);
+  char* at_ = static_cast<char*>(mid.data_ptr());
+  auto take = [&](int64_t bytes) { char* r = at_; at_ += bytes; return r; };
+  char *q = take(key), *k = take(key), *b = take(key), *g = take(decay), *v = take(value), *w = take(value), *o = take(value);
   void* st = stream_of(p);
   gdn2_layer_front_args a{};
   a.proj = proj.data_ptr(); a.conv_state = conv_state->data_ptr(); a.conv_weight = conv_w->data_ptr();
   a.conv_bias = conv_b ? conv_b->data_ptr() : nullptr;
   a.A_log = A_log.data_ptr(); a.dt_bias = dt_bias.data_ptr();
-  a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.g = static_cast<float*>(g.data_ptr()); a.b = b.data_ptr();
-  a.w = w.data_ptr(); a.new_conv_state = conv.data_ptr();
+  a.q = q; a.k = k; a.v = v; a.g = reinterpret_cast<float*>(g); a.b = b; a.w = w; a.new_conv_state = conv.data_ptr();
   a.B = p.B; a.S = p.S; a.H = H; a.HK = HK; a.DK = DK; a.DV = DV; a.K = K; a.NP = proj.size(2);
   a.off_q = offs[0]; a.off_k = offs[1]; a.off_v = offs[2]; a.off_b = offs[3]; a.off_w = offs[4]; a.off_f = offs[5];
   a.erase_scale = (float)erase_scale;
   // up to the decode nothing of the cache has changed, so the general path can still take the call over
   if (gdn2_layer_front(&a, p.dtype, st) != GDN2_OK) return std::nullopt;
-  if (gdn2_decode(q.data_ptr(), k.data_ptr(), v.data_ptr(), a.g, b.data_ptr(), w.data_ptr(), static_cast<float*>(state.data_ptr()),
-                  o.data_ptr(), p.B, p.S, H, HK, DK, DV, p.S, p.S, (float)scale, p.dtype, st) != GDN2_OK)
+  if (gdn2_decode(q, k, v, a.g, b, w, static_cast<float*>(state.data_ptr()), o, p.B, p.S, H, HK, DK, DV, p.S, p.S, (float)scale, p.dtype, st) != GDN2_OK)
     return std::nullopt;
-  const int rc = gdn2_layer_back(o.data_ptr(), proj.data_ptr(), norm_w.data_ptr(), normed.data_ptr(), p.B * p.S, H, DV,
+  const int rc = gdn2_layer_back(o, proj.data_ptr(), norm_w.data_ptr(), normed.data_ptr(), p.B * p.S, H, DV,
                                  proj.size(2), offs[6], (float)eps, p.dtype, st);
   if (rc != GDN2_OK) throw std::runtime_error(std::string("gdn2_layer_back: ") + gdn2_status_string(rc));
   // the front kernel writes the new convolution cache itself in its one-token form, else a second one does

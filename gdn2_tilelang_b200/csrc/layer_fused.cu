@@ -13,35 +13,13 @@
 // and as many round trips through HBM per call become three. All arithmetic is fp32 with one rounding to
 // the storage type at the end. One warp per (token, kv head) in front, per (token, value head) in back.
 #include "common.cuh"
+#include "layer_math.cuh"
 
 namespace gdn2 {
 
 namespace {
 
 constexpr int kWarps = 4;
-
-// Hardware exponential, reciprocal, logarithm and reciprocal square root, one instruction each (flush-to-zero
-// forms: no denormal fix-up code). A few ulp each, far inside the 16-bit storage rounding and the 2e-5 the
-// float32 form is tested to; the precise division and log1pf were most of these kernels' instructions.
-__device__ __forceinline__ float ex2_(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-__device__ __forceinline__ float rcp_(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-__device__ __forceinline__ float lg2_(float x) { float y; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-__device__ __forceinline__ float rsq_(float x) { float y; asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
-__device__ __forceinline__ float silu(float x) { return x * rcp_(1.f + ex2_(-kLog2e * x)); }
-__device__ __forceinline__ float sigmoidf_(float x) { return rcp_(1.f + ex2_(-kLog2e * x)); }
-__device__ __forceinline__ float softplusf_(float x) {
-  const float e = ex2_(-kLog2e * fabsf(x));                // softplus(x) = max(x, 0) + log1p(exp(-|x|))
-  const float l = e < 0x1p-12f ? e * (1.f - 0.5f * e) : kLn2 * lg2_(1.f + e);
-  return fmaxf(x, 0.f) + l;
-}
-// 1 / max(sqrt(ss), 1e-12): the scale of F.normalize
-__device__ __forceinline__ float inv_norm(float ss) { return rsq_(fmaxf(ss, 1e-24f)); }
-__device__ __forceinline__ float warp_sum(float x) {
-#pragma unroll
-  for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  return x;
-}
 
 // value at time tt (may be negative: the cached columns, or zero) of projection column `col`, whose
 // position among the convolved channels q | k | v is `cch`
@@ -151,23 +129,6 @@ layer_front_kernel(gdn2_layer_front_args a) {
 // The common shape (DK = DV = 128, four taps, 16-bit storage): lane owns channels 4 lane .. 4 lane + 3 of a
 // head, so every access to the projection buffer, the weights and the outputs is one 8- or 16-byte access
 // and a warp covers a head's 256 bytes in one instruction.
-template <typename T>
-struct alignas(4 * sizeof(T)) Vec4 { T x[4]; };
-
-template <typename T>
-__device__ __forceinline__ void load4(const T* p, float (&o)[4]) {
-  const Vec4<T> v = *reinterpret_cast<const Vec4<T>*>(p);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) o[i] = to_f32(v.x[i]);
-}
-template <typename T>
-__device__ __forceinline__ void store4(T* p, const float (&o)[4]) {
-  Vec4<T> v;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) v.x[i] = from_f32<T>(o[i]);
-  *reinterpret_cast<Vec4<T>*>(p) = v;
-}
-
 // convolution + SiLU of 4 adjacent channels: projection columns col.., convolved-channel index cch..
 // `tail` (or null): where the new convolution cache of these channels goes, [4 channels][K - 1]; the last three taps
 // of the LAST token are exactly its contents.

@@ -353,6 +353,38 @@ int gdn2_layer_back(const void* o, const void* proj, const void* norm_weight, vo
                     int64_t DV, int64_t NP, int64_t off_gate, float eps, int dtype, void* stream);
 
 /*
+ * One token per sequence through the whole layer: projections, gdn2_layer_front, gdn2_decode with n = 1, gdn2_layer_back and
+ * the output projection (gdn2/attention.py:290-356 with a cache) as three kernels. `state` is updated in place;
+ * new_conv_state receives the new convolution cache and may be conv_state itself. The projections are rounded to `dtype`
+ * before the element-wise stages, as separate products leave them. The column offsets are rows of w_cat.
+ * gdn2_layer_step_workspace_bytes returns 0 for what these kernels do not cover (they take 16-bit types, DK = DV = 128, K = 4,
+ * at most 16 sequences, hidden a multiple of 64, and a sequence block of rows that fits in shared memory); gdn2_layer_step
+ * then returns GDN2_ERR_UNSUPPORTED and has launched nothing.
+ */
+typedef struct gdn2_layer_step_args {
+  const void* x;               /* [B, hidden] */
+  const void* w_cat;           /* [NP, hidden] */
+  const void* conv_state;      /* [B, CC, K-1] */
+  const void* conv_weight;     /* [CC, K] */
+  const void* conv_bias;       /* [CC] or NULL */
+  const void* A_log;           /* [HK] */
+  const void* dt_bias;         /* [HK, DK] */
+  const void* norm_weight;     /* [DV] */
+  const void* o_weight;        /* [hidden, H*DV] */
+  float* state;                /* [B, H, DK, DV] */
+  void* new_conv_state;        /* [B, CC, K-1] */
+  void* out;                   /* [B, hidden] */
+  void* workspace;
+  size_t workspace_bytes;
+  int64_t B, hidden, H, HK, DK, DV, K;
+  int64_t off_q, off_k, off_v, off_b, off_w, off_f, off_gate;
+  float erase_scale, eps, scale;
+} gdn2_layer_step_args;
+
+size_t gdn2_layer_step_workspace_bytes(int64_t B, int64_t hidden, int64_t H, int64_t HK, int64_t DK, int64_t DV, int64_t K, int dtype);
+int gdn2_layer_step(const gdn2_layer_step_args* args, int dtype, void* stream);
+
+/*
  * Output projection of a head-parallel layer fused with its all-reduce, for decode-sized inputs (1..8 token
  * rows): out [rows, hidden] = sum over the `world` ranks of x_r [rows, K] * weight_r [hidden, K]^T, the same
  * bits on every rank. One launch per rank and call; all ranks must make the same sequence of calls.
