@@ -33,7 +33,7 @@
 //     passes store them as packed 16-bit pairs into tensor memory and the MMAs read them from there.
 //
 // TMEM columns: [0,128) the update product P; [128,192) WS; [192,256) the O accumulator;
-// [320,384) S^T bf16 pairs; [384,416) Un^T/256 fp16 pairs.
+// [320,384) S^T bf16 pairs; [384,416) Un^T/256 fp16 pairs; [256,320) and [416,480) S^T in fp32 where chunk states are wanted.
 //
 // Sequence-parallel form. One block per (batch, head) leaves most of the GPU idle when a GPU holds few
 // (batch, head) pairs (a head-sharded layer), and its chunk-to-chunk chain then sets the time. The
@@ -78,6 +78,7 @@ constexpr uint32_t kKgtBytes = D * BS * 2;       // 16 KiB (fp16)
 constexpr uint32_t kUtBytes = D * BS * 2;        // 16 KiB (fp16)
 constexpr uint32_t kColWs = 128, kColO = 192;
 constexpr uint32_t kColSb = 320, kColUn16 = 384;   // packed 16-bit A operands in TMEM
+constexpr uint32_t kColH0 = 256, kColH1 = 416;     // fp32 state on its way to memory, one half of the key channels each
 
 struct ScanTcSmem {
   __nv_bfloat16 wq[2][2 * BS * D];   // B of MMA1w/q: [dk/8][128 rows: W tok 0..63, Qg tok 0..63][8]
@@ -90,6 +91,7 @@ struct ScanTcSmem {
   uint64_t bar_m1, bar_m3[2], bar_m2;                   // MMA completion: (W S)^T; the two key-channel halves of P; O
   uint64_t bar_sb[2], bar_un;                           // compute threads -> issuer: S^T by key-channel half, Un^T
   uint64_t bar_of;                                      // output warps -> issuer: the O accumulator has been read out
+  uint64_t bar_hf, bar_he;                              // chunk states: compute threads -> output warps (in place), and back (read out)
   uint64_t bar_drain;                                   // every product of the block
   uint32_t tmem_base;
   int abort_flag;
@@ -127,7 +129,8 @@ struct ScanNorm {
 
 enum : uint32_t {
   kWaitWq = 0x10, kWaitUt = 0x20, kWaitAqk = 0x40, kWaitKgt = 0x80, kWaitM1 = 0x100, kWaitM2 = 0x200,
-  kWaitM3 = 0x400, kWaitSb = 0x800, kWaitUn = 0x4000
+  kWaitM3 = 0x400, kWaitSb = 0x800, kWaitUn = 0x4000,
+  kWaitHs = 0x8000
 };
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -235,7 +238,10 @@ __device__ __noinline__ void store_rows_normed(const __nv_bfloat16* ostage, __nv
   }
 }
 
-template <typename Seqs>
+// kForm: the plain scan, with chunk states stored, the chunk-parallel output from stored states (ScanPlan::pass is kOutput), or
+// with the gated norm behind it; kernels of their own, because the plain form has no register to spare.
+enum ScanForm : int { kPlain = 0, kStoreStates = 1, kFromStates = 2, kNormed = 3 };
+template <typename Seqs, int kForm>
 __global__ void __launch_bounds__(kThreads, 1)
 scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* __restrict__ s0,
                __nv_bfloat16* __restrict__ o, float* __restrict__ sT, float* __restrict__ hs, int S, int H, int64_t o_bs,
@@ -247,7 +253,9 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
 
   // ---- this block's job: which (batch, head), which run of chunks, where the state comes from and goes to
   bool transition = false;                  // identity start, no U, no outputs: yields the segment's transition matrix
-  const bool output_only = plan.pass == kOutput;
+  constexpr bool output_only = kForm == kFromStates;
+  if constexpr (kForm == kPlain || kForm == kNormed) hs = nullptr;
+  if constexpr (kForm != kNormed) norm.gate = nullptr;
   int bh, ib, ih, seg = 0;                  // (batch entry or packed sequence, head) and segment
   int NC_all, c_first, NC;                  // chunks per row of records; first chunk and number of chunks of this block
   int64_t ch0, chv0, o_row0;                // first record of the key head and of the value head; first output row
@@ -345,6 +353,7 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
     // one arrival per warp; a transition block has no outputs, its output warps take no part
     for (int i = 0; i < 2; ++i) { tc::mbar_init(&s.bar_m3[i], 1); tc::mbar_init(&s.bar_sb[i], kComputeThreads / 64); }
     tc::mbar_init(&s.bar_of, kOutputThreads / 32);
+    tc::mbar_init(&s.bar_hf, kComputeThreads / 32); tc::mbar_init(&s.bar_he, kOutputThreads / 32);
     tc::mbar_init(&s.bar_un, kComputeThreads / 32);
     tc::mbar_init(&s.bar_drain, 1);
     s.abort_flag = 0;
@@ -505,6 +514,26 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
           store_rows_normed(s.ostage, obase, gbase, norm.row_stride, norm.weight, norm.eps, otid, H);
         }
       }
+      if (hs && !output_only && n + 1 < NC) {
+        // The state entering the next chunk, out of tensor memory: 64 KiB per chunk, a thousand cycles of the SM's store path,
+        // which the compute threads, whose chain sets the pace, spent waiting when they stored it themselves
+        // (B = 2, S = 4096, 16 heads: 238 -> 220 us a call).
+        if (!output_all(tc::mbar_wait_warp(&s.bar_hf, n & 1, &s.abort_flag, status, kWaitHs))) break;
+        tc::tc_fence_after_sync();
+        float* hn = hs + (((size_t)ib * NC_all + (c_first + n + 1)) * H + ih) * D * D + dv;
+#pragma unroll 1
+        for (int x = 0; x < 4; ++x) {
+          float v[32];
+          tc::tmem_ld32(tc::tmem_addr(tm, lq * 32, (x < 2 ? kColH0 : kColH1) + 32 * (x & 1)), v);
+          tc::tmem_ld_wait();
+          if (x == 3) {
+            tc::tc_fence_before_sync();
+            warp_arrive(&s.bar_he, lane);
+          }
+#pragma unroll
+          for (int i = 0; i < 32; ++i) hn[(size_t)(32 * x + i) * D] = v[i];
+        }
+      }
     }
   } else {
     // =============================== compute threads ============================================
@@ -634,10 +663,15 @@ scan_tc_kernel(WsLayout L, WsPtrs P, ScanPlan plan, ScanNorm norm, const float* 
           tc::tc_fence_before_sync();
           warp_arrive(&s.bar_sb[part], lane);
         }
-        float* hn = (hs && more) ? hs + (((size_t)ib * NC_all + (c_first + n + 1)) * H + ih) * D * D : nullptr;
-        if (hn) {
-#pragma unroll
-          for (int i = 0; i < 64; ++i) hn[(size_t)(dkp + i) * D + dv] = S[i];
+        if (hs && more) {                                  // the output warps store it from tensor memory
+          if (n > 0 && !wait_all(&s.bar_he, (n - 1) & 1, kWaitHs)) break;
+          tc::tc_fence_after_sync();
+          const uint32_t t_h = t_lane + (part ? kColH1 : kColH0);
+          tc::tmem_st32(t_h, *reinterpret_cast<const float(*)[32]>(&S[0]));
+          tc::tmem_st32(t_h + 32, *reinterpret_cast<const float(*)[32]>(&S[32]));
+          tc::tmem_st_wait();
+          tc::tc_fence_before_sync();
+          warp_arrive(&s.bar_hf, lane);
         }
         if (!more) {
           float* fin = state_sink();
@@ -786,7 +820,9 @@ int launch_scan_tc(const WsLayout& L, const WsPtrs& P, const float* s0, void* o,
                    int B, int S, int H, int64_t o_bs, const gdn2_gated_norm* gn, int part, cudaStream_t st) {
   if (L.DK != D || L.DV != D || L.esz != 2) return GDN2_ERR_UNSUPPORTED;
   const size_t smem = sizeof(ScanTcSmem) + 128;
-  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(scan_tc_kernel<OneLength>), smem));
+  if (gn && hs) return GDN2_ERR_UNSUPPORTED;               // (no caller wants both)
+  const auto kern = hs ? scan_tc_kernel<OneLength, kStoreStates> : gn ? scan_tc_kernel<OneLength, kNormed> : scan_tc_kernel<OneLength, kPlain>;
+  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
   __nv_bfloat16* ob = static_cast<__nv_bfloat16*>(o);
   uint32_t* status = device_status_word();
   const int BH = B * H, NC = S / BS;
@@ -796,13 +832,13 @@ int launch_scan_tc(const WsLayout& L, const WsPtrs& P, const float* s0, void* o,
   const int nseg = L.nseg;
   if (nseg <= 1) {
     if (part == 2) return GDN2_OK;
-    scan_tc_kernel<OneLength><<<BH, kThreads, smem, st>>>(L, P, ScanPlan{kWhole, 1, 0}, norm, s0, ob, sT, hs, S, H, o_bs, status, OneLength{});
+    kern<<<BH, kThreads, smem, st>>>(L, P, ScanPlan{kWhole, 1, 0}, norm, s0, ob, sT, hs, S, H, o_bs, status, OneLength{});
     GDN2_CUDA_TRY(cudaGetLastError());
     return GDN2_OK;
   }
   const int guarded = L.nseg_guarded ? 1 : 0;
   if (part == 2) {
-    scan_tc_kernel<OneLength><<<BH * (nseg - 1), kThreads, smem, st>>>(L, P, ScanPlan{kRedo, nseg, guarded}, norm, nullptr, ob, nullptr, nullptr,
+    kern<<<BH * (nseg - 1), kThreads, smem, st>>>(L, P, ScanPlan{kRedo, nseg, guarded}, norm, nullptr, ob, nullptr, nullptr,
                                                            S, H, o_bs, status, OneLength{});
     GDN2_CUDA_TRY(cudaGetLastError());
     return GDN2_OK;
@@ -813,7 +849,7 @@ int launch_scan_tc(const WsLayout& L, const WsPtrs& P, const float* s0, void* o,
     scan_mode_kernel<<<(BK * (nseg - 1) + 7) / 8, 256, 0, st>>>(P, BK, nseg, NC);
     GDN2_CUDA_TRY(cudaGetLastError());
   }
-  scan_tc_kernel<OneLength><<<BH * (2 * nseg - 1), kThreads, smem, st>>>(L, P, ScanPlan{kFirst, nseg, guarded}, norm, s0, ob, sT, hs,
+  kern<<<BH * (2 * nseg - 1), kThreads, smem, st>>>(L, P, ScanPlan{kFirst, nseg, guarded}, norm, s0, ob, sT, hs,
                                                              S, H, o_bs, status, OneLength{});
   GDN2_CUDA_TRY(cudaGetLastError());
   const size_t csmem = (size_t)(D * kTPad + D * kCombineCols) * sizeof(float);
@@ -821,7 +857,7 @@ int launch_scan_tc(const WsLayout& L, const WsPtrs& P, const float* s0, void* o,
   scan_combine_kernel<OneLength><<<dim3(BH, D / kCombineCols), 256, csmem, st>>>(P, nseg, NC, guarded, sT, H, OneLength{});
   GDN2_CUDA_TRY(cudaGetLastError());
   if (part == 1) return GDN2_OK;
-  scan_tc_kernel<OneLength><<<BH * (nseg - 1), kThreads, smem, st>>>(L, P, ScanPlan{kRedo, nseg, guarded}, norm, nullptr, ob, nullptr, hs,
+  kern<<<BH * (nseg - 1), kThreads, smem, st>>>(L, P, ScanPlan{kRedo, nseg, guarded}, norm, nullptr, ob, nullptr, hs,
                                                          S, H, o_bs, status, OneLength{});
   GDN2_CUDA_TRY(cudaGetLastError());
   return GDN2_OK;
@@ -832,12 +868,12 @@ int launch_scan_tc_packed(const WsLayout& L, const WsPtrs& P, const PackedSeqs& 
                           int H, cudaStream_t st) {
   if (L.DK != D || L.DV != D || L.esz != 2) return GDN2_ERR_UNSUPPORTED;
   const size_t smem = sizeof(ScanTcSmem) + 128;
-  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(scan_tc_kernel<PackedSeqs>), smem));
+  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(scan_tc_kernel<PackedSeqs, kPlain>), smem));
   __nv_bfloat16* ob = static_cast<__nv_bfloat16*>(o);
   const ScanNorm norm{nullptr, nullptr, 0, 0, 0.f};
   const int total = seqs.seg[seqs.n], later = total - seqs.n;
   auto pass = [&](int which, int blocks) -> int {
-    scan_tc_kernel<PackedSeqs><<<blocks, kThreads, smem, st>>>(L, P, ScanPlan{which, 0, 0}, norm, s0, ob, sT, nullptr, 0, H, 0,
+    scan_tc_kernel<PackedSeqs, kPlain><<<blocks, kThreads, smem, st>>>(L, P, ScanPlan{which, 0, 0}, norm, s0, ob, sT, nullptr, 0, H, 0,
                                                                device_status_word(), seqs);
     GDN2_CUDA_TRY(cudaGetLastError());
     return GDN2_OK;
@@ -858,13 +894,13 @@ int launch_output_tc(const WsLayout& L, const WsPtrs& P, const float* hs, void* 
                      cudaStream_t st) {
   if (L.DK != D || L.DV != D || L.esz != 2) return GDN2_ERR_UNSUPPORTED;
   const size_t smem = sizeof(ScanTcSmem) + 128;
-  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(scan_tc_kernel<OneLength>), smem));
+  GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(scan_tc_kernel<OneLength, kFromStates>), smem));
   const int BH = B * H, NC = S / BS;
   // enough runs to give every SM a few blocks, none shorter than 4 chunks
   int runs = (4 * device_sm_count() + BH - 1) / BH;
   if (runs > NC / 4) runs = NC / 4;
   if (runs < 1) runs = 1;
-  scan_tc_kernel<OneLength><<<BH * runs, kThreads, smem, st>>>(L, P, ScanPlan{kOutput, runs, 0}, ScanNorm{nullptr, nullptr, 0, 0, 0.f}, nullptr,
+  scan_tc_kernel<OneLength, kFromStates><<<BH * runs, kThreads, smem, st>>>(L, P, ScanPlan{kOutput, runs, 0}, ScanNorm{nullptr, nullptr, 0, 0, 0.f}, nullptr,
                                                    static_cast<__nv_bfloat16*>(o),
                                                    nullptr, const_cast<float*>(hs), S, H, o_bs, device_status_word(), OneLength{});
   GDN2_CUDA_TRY(cudaGetLastError());
