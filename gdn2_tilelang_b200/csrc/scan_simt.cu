@@ -9,8 +9,12 @@
 // columns never meet, so a head is spread over tiles of 8 of them while SMs are free (16 and 32 beyond that: the
 // records are read once per tile). The records arrive by bulk copies in the layout they are stored in, each one
 // refilled for the next chunk as soon as its last reader is through, and the two halves of the block form the output
-// rows and the new state at the same time: two barriers per chunk. Measured
-// with the chunk-local stage (prep_simt.cu), B = 2, S = 1000, 8 heads of 64, float32: the call took 501 us, now 79.
+// rows and the new state at the same time: two barriers per chunk.
+// Inside a chunk the pace is set by what shared memory can return, 128 bytes a cycle whether lanes share an address or not. A
+// thread therefore forms 4 rows x 4 columns over a quarter of the reduction (8 loads of 16 bytes per 64 FMAs, where one row by
+// four columns took 5 for 16), and the four quarters, neighbours in a warp, meet in 12 shuffles. Two buffers per record, so that a
+// copy has a whole chunk to land, gained nothing (79 -> 84 us). Measured
+// with the chunk-local stage (prep_simt.cu), B = 2, S = 1000, 8 heads of 64, float32: 75.7 us a call, 78.9 before.
 //
 // Output: one block per (value tile, chunk, batch*head) doing the first two lines from a stored
 // chunk state (output_kernel, gdn2/forward.py:710-725).
@@ -111,7 +115,7 @@ __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
 
 enum : uint32_t { kWaitSimtWq = 0x200000u, kWaitSimtUt = 0x400000u, kWaitSimtAqk = 0x800000u, kWaitSimtKgt = 0x1000000u };
 
-// Shared memory of the scan: the chunk's records as stored (fp32 images), the state tile and Un, value columns inside.
+// Shared memory of the scan: the chunk's records as stored (fp32 images), the state tile and Un, value columns outside.
 template <int NVT> struct ScanTile {
   float *wq, *aqk, *kgt, *ut, *gl, *St, *Un;
   __device__ ScanTile(float* base, int DK) {
@@ -120,29 +124,68 @@ template <int NVT> struct ScanTile {
     aqk = kgt + kChunk * DK;            // [64/4][64 r][4]
     ut = aqk + kChunk * kChunk;         // [64/4][NVT][4]
     gl = ut + kChunk * NVT;             // [DK]
-    St = gl + DK;                       // [DK][NVT]
-    Un = St + DK * NVT;                 // [64][NVT]
+    St = gl + DK;                       // [NVT][DK]: the state transposed
+    Un = St + DK * NVT;                 // [NVT][64]
   }
   static size_t bytes(int DK) {
     return ((size_t)3 * kChunk * DK + kChunk * kChunk + 2 * kChunk * NVT + DK + (size_t)DK * NVT) * sizeof(float);
   }
 };
 
+// acc[i][c] += sum over groups x4 = first, first + 4, .. < end of four reduction steps of row i (rows 8 apart in an image
+// [steps/4][stride][4], `rows` its row 0 of this thread) and column c (cols: [column][ld])
+template <int NC>
+__device__ __forceinline__ void tile_product(float2 (&acc)[4][NC], const float* rows, int stride, const float* cols, int ld, int first, int end) {
+#pragma unroll 1
+  for (int x4 = first; x4 < end; x4 += 4) {
+    float4 r[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r[i] = *reinterpret_cast<const float4*>(rows + ((size_t)x4 * stride + 8 * i) * 4);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const float4 v = *reinterpret_cast<const float4*>(cols + c * ld + 4 * x4);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        acc[i][c] = ffma2(make_float2(r[i].z, r[i].w), make_float2(v.z, v.w), ffma2(make_float2(r[i].x, r[i].y), make_float2(v.x, v.y), acc[i][c]));
+    }
+  }
+}
+// The sums of four columns over the four quarters of a warp (lane bits 3 and 4): a lane keeps row 2 * bit 3 + bit 4.
+template <int NC>
+__device__ __forceinline__ void tile_reduce(const float2 (&acc)[4][NC], int c0, int lane, float (&out)[4]) {
+  float v[4][4], h[2][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) v[i][c] = acc[i][c0 + c].x + acc[i][c0 + c].y;
+  }
+  const bool b3 = lane & 8, b4 = lane & 16;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) h[i][c] = (b3 ? v[2 + i][c] : v[i][c]) + __shfl_xor_sync(0xffffffffu, b3 ? v[i][c] : v[2 + i][c], 8);
+  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c) out[c] = (b4 ? h[1][c] : h[0][c]) + __shfl_xor_sync(0xffffffffu, b4 ? h[0][c] : h[1][c], 16);
+}
+
 // S tokens per batch entry, ceil(S / 64) chunks: the rows past the end are not written (the chunk-local stage has made
-// them neutral). Threads: tid & 127 = row of the W | Qg image, tid >> 7 = half of the tile's columns. The W rows' threads
-// go on to the state update (row & 63 = key channel, two of them when DK > 64), the Qg rows' threads to the output.
+// them neutral). Warp: rows 32 (wid & 3) .. + 31 of the W | Qg image, half of the tile's columns (wid >> 2) in groups of four. The
+// W rows' warps go on to the state update (32 or, when DK > 64, 64 key channels each), the Qg rows' warps to the output.
 template <typename TOut, int NVT, typename Seqs>
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(256, 2)
 scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __restrict__ o,
                  float* __restrict__ sT, float* __restrict__ hs, int S, int H, int64_t o_bs, uint32_t* status,
                  const __grid_constant__ Seqs seqs) {
-  constexpr int CT = NVT / 2;                             // columns per thread
+  constexpr int kQuads = NVT / 8, kG = kQuads < 2 ? kQuads : 2;   // groups of four columns per warp, and at a time
   const int DK = L.DK, DV = L.DV;
   const int bh = blockIdx.x, ib = bh / H, ih = bh % H;
   const int lo = blockIdx.y * NVT, nv = min(NVT, DV - lo);
   const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-  const int row = tid & 127, col0 = (tid >> 7) * CT;
-  const bool is_q = row >= kChunk;
+  const int part = lane >> 3, rl = lane & 7;              // quarter of the reduction; row of eight
+  const int rb = wid & 3, quad0 = (wid >> 2) * kQuads;
+  const bool is_q = rb >= 2;
+  const int mine = rl + 8 * (2 * (part & 1) + (part >> 1));   // row of 32 whose sums this lane keeps (tile_reduce)
   extern __shared__ __align__(128) float sm[];
   ScanTile<NVT> s(sm, DK);
   __shared__ uint64_t bar_wq, bar_ut, bar_aqk, bar_kgt;
@@ -200,7 +243,7 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
   grid_wait();
   for (int idx = tid; idx < DK * NVT; idx += 256) {
     const int c = idx / NVT, d = idx % NVT;
-    s.St[idx] = (s0 != nullptr && d < nv) ? s0[((size_t)bh * DK + c) * DV + lo + d] : 0.f;
+    s.St[d * DK + c] = (s0 != nullptr && d < nv) ? s0[((size_t)bh * DK + c) * DV + lo + d] : 0.f;
   }
   if (nv < NVT)                                            // columns past DV: no copy brings them
     for (int idx = tid; idx < kChunk * NVT; idx += 256) s.ut[idx] = 0.f;
@@ -214,7 +257,7 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
   auto wait_all = [&](uint64_t* bar, uint32_t parity, uint32_t code) {
     return tc::mbar_wait_warp(bar, parity, &abort_flag, status, code);
   };
-  float2 acc[CT / 2];
+  float qs[kQuads][4];                                     // Qg rows: this lane's row of Qg S
   int wq_ahead = 0, kgt_ahead = 0;                         // last chunk whose copies were issued
   bool ok = true;
   for (int n = 0; n < NC; ++n) {
@@ -223,31 +266,35 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
       float* hp = hs + (((size_t)ib * NC + n) * H + ih) * DK * DV + lo;
       for (int idx = tid; idx < DK * NVT; idx += 256) {
         const int c = idx / NVT, d = idx % NVT;
-        if (d < nv) hp[(size_t)c * DV + d] = s.St[idx];
+        if (d < nv) hp[(size_t)c * DV + d] = s.St[d * DK + c];
       }
     }
-    // ---- row of W S or Qg S
-#pragma unroll
-    for (int x = 0; x < CT / 2; ++x) acc[x] = make_float2(0.f, 0.f);
+    // ---- rows of W S or Qg S
     ok = ok && wait_all(&bar_wq, ph, kWaitSimtWq);
-    const float4* wrow = reinterpret_cast<const float4*>(s.wq) + row;
-#pragma unroll 4
-    for (int c4 = 0; c4 < DK / 4; ++c4) {
-      const float4 w4 = wrow[c4 * 2 * kChunk];
-      const float wv[4] = {w4.x, w4.y, w4.z, w4.w};
-#pragma unroll
-      for (int y = 0; y < 4; ++y) {
-        const float2* st = reinterpret_cast<const float2*>(&s.St[(4 * c4 + y) * NVT + col0]);
-#pragma unroll
-        for (int x = 0; x < CT / 2; ++x) acc[x] = ffma2(make_float2(wv[y], wv[y]), st[x], acc[x]);
-      }
-    }
     ok = ok && wait_all(&bar_ut, ph, kWaitSimtUt);
-    if (!is_q) {
-      const float* u = s.ut + ((row >> 2) * NVT + col0) * 4 + (row & 3);
-      float2* un = reinterpret_cast<float2*>(&s.Un[row * NVT + col0]);
 #pragma unroll
-      for (int x = 0; x < CT / 2; ++x) un[x] = make_float2(u[8 * x] - acc[x].x, u[8 * x + 4] - acc[x].y);
+    for (int j0 = 0; j0 < kQuads; j0 += kG) {
+      float2 acc[4][4 * kG];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+#pragma unroll
+        for (int c = 0; c < 4 * kG; ++c) acc[i][c] = make_float2(0.f, 0.f);
+      }
+      tile_product(acc, s.wq + (32 * rb + rl) * 4, 2 * kChunk, s.St + 4 * (quad0 + j0) * DK, DK, part, DK / 4);
+#pragma unroll
+      for (int j = 0; j < kG; ++j) {
+        float v[4];
+        tile_reduce(acc, 4 * j, lane, v);
+        const int col0 = 4 * (quad0 + j0 + j), row = 32 * rb + mine;
+        if (is_q) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) qs[j0 + j][c] = v[c];
+        } else {
+          const float* u = s.ut + ((row >> 2) * NVT + col0) * 4 + (row & 3);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) s.Un[(col0 + c) * kChunk + row] = u[4 * c] - v[c];
+        }
+      }
     }
     __syncthreads();                                       // Un complete; the state and W | Qg have been read
     if (wid == 0 && ok && n + 1 < NC) {
@@ -257,53 +304,54 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
 
     if (is_q) {
       // ---- o = Qg S + tril(Aqk) Un: source tokens up to the warp's last row (Aqk is zero above the diagonal)
-      const int r = row - kChunk;
       ok = ok && wait_all(&bar_aqk, ph, kWaitSimtAqk);
-      const float4* arow = reinterpret_cast<const float4*>(s.aqk) + r;
-      const int tq = ((r & ~31) + 32) / 4;
-#pragma unroll 4
-      for (int t4 = 0; t4 < tq; ++t4) {
-        const float4 a4 = arow[t4 * kChunk];
-        const float av[4] = {a4.x, a4.y, a4.z, a4.w};
+      const int r = 32 * (rb - 2) + mine, t = n * kChunk + r;
 #pragma unroll
-        for (int y = 0; y < 4; ++y) {
-          const float2* un = reinterpret_cast<const float2*>(&s.Un[(4 * t4 + y) * NVT + col0]);
+      for (int j0 = 0; j0 < kQuads; j0 += kG) {
+        float2 acc[4][4 * kG];
 #pragma unroll
-          for (int x = 0; x < CT / 2; ++x) acc[x] = ffma2(make_float2(av[y], av[y]), un[x], acc[x]);
+        for (int i = 0; i < 4; ++i) {
+#pragma unroll
+          for (int c = 0; c < 4 * kG; ++c) acc[i][c] = make_float2(0.f, 0.f);
         }
-      }
-      const int t = n * kChunk + r;
-      if (t < len) {
-        TOut* op = o + ((size_t)(o_row0 + t) * H + ih) * DV + lo + col0;
+        tile_product(acc, s.aqk + (32 * (rb - 2) + rl) * 4, kChunk, s.Un + 4 * (quad0 + j0) * kChunk, kChunk, part, 8 * (rb - 1));
 #pragma unroll
-        for (int x = 0; x < CT / 2; ++x) {
-          if (col0 + 2 * x < nv) {                         // nv is a multiple of 4
-            op[2 * x] = from_f32<TOut>(acc[x].x); op[2 * x + 1] = from_f32<TOut>(acc[x].y);
+        for (int j = 0; j < kG; ++j) {
+          float v[4];
+          tile_reduce(acc, 4 * j, lane, v);
+          const int col0 = 4 * (quad0 + j0 + j);
+          if (t < len && col0 < nv) {                      // nv is a multiple of 4
+            TOut* op = o + ((size_t)(o_row0 + t) * H + ih) * DV + lo + col0;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) op[c] = from_f32<TOut>(qs[j0 + j][c] + v[c]);
           }
         }
       }
     } else {
-      // ---- S <- gamma_C S + KG^T Un, this thread's channel(s)
+      // ---- S <- gamma_C S + KG^T Un, 32 channels at a time; rows past DK are formed from the record behind and dropped
       ok = ok && wait_all(&bar_kgt, ph, kWaitSimtKgt);
-      for (int c = row; c < DK; c += kChunk) {
-        float2* st = reinterpret_cast<float2*>(&s.St[c * NVT + col0]);
-        const float gm = s.gl[c];
+      for (int c0 = 32 * rb; c0 < DK; c0 += 64) {
+        const int ch = c0 + mine;
+        const float gm = ch < DK ? s.gl[ch] : 0.f;
 #pragma unroll
-        for (int x = 0; x < CT / 2; ++x) { acc[x] = st[x]; acc[x].x *= gm; acc[x].y *= gm; }
-        const float4* krow = reinterpret_cast<const float4*>(s.kgt) + c;
-#pragma unroll 4
-        for (int t4 = 0; t4 < kChunk / 4; ++t4) {
-          const float4 k4 = krow[t4 * DK];
-          const float kv[4] = {k4.x, k4.y, k4.z, k4.w};
+        for (int j0 = 0; j0 < kQuads; j0 += kG) {
+          float2 acc[4][4 * kG];
 #pragma unroll
-          for (int y = 0; y < 4; ++y) {
-            const float2* un = reinterpret_cast<const float2*>(&s.Un[(4 * t4 + y) * NVT + col0]);
+          for (int i = 0; i < 4; ++i) {
 #pragma unroll
-            for (int x = 0; x < CT / 2; ++x) acc[x] = ffma2(make_float2(kv[y], kv[y]), un[x], acc[x]);
+            for (int c = 0; c < 4 * kG; ++c) acc[i][c] = make_float2(0.f, 0.f);
+          }
+          tile_product(acc, s.kgt + (c0 + rl) * 4, DK, s.Un + 4 * (quad0 + j0) * kChunk, kChunk, part, kChunk / 4);
+#pragma unroll
+          for (int j = 0; j < kG; ++j) {
+            float v[4];
+            tile_reduce(acc, 4 * j, lane, v);
+            float* st = s.St + 4 * (quad0 + j0 + j) * DK + ch;
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              if (ch < DK) st[c * DK] = fmaf(gm, st[c * DK], v[c]);
           }
         }
-#pragma unroll
-        for (int x = 0; x < CT / 2; ++x) st[x] = acc[x];
       }
     }
     __syncthreads();                                       // the new state is complete; Un, Aqk and KG have been read
@@ -319,7 +367,7 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
   if (sT != nullptr) {
     for (int idx = tid; idx < DK * NVT; idx += 256) {
       const int c = idx / NVT, d = idx % NVT;
-      if (d < nv) sT[((size_t)bh * DK + c) * DV + lo + d] = s.St[idx];
+      if (d < nv) sT[((size_t)bh * DK + c) * DV + lo + d] = s.St[d * DK + c];
     }
   }
 }
