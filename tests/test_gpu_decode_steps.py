@@ -17,7 +17,7 @@ DEV = "cuda"
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("B,H,HK", [(24, 16, 8), (50, 3, 1)])
-@pytest.mark.parametrize("n", [2, 3, 4, 5, 6, 7, 9, 12, 13, 18])
+@pytest.mark.parametrize("n", [2, 3, 4, 5, 6, 7, 9, 12, 13, 18, 37])
 def test_steps(n, B, H, HK, dtype):
     D = 128
     q, k, _, g, b, _ = orc.make_inputs(B, n, HK, D, D, seed=n)
