@@ -254,6 +254,10 @@ class NativeKernels:
             st = self._side_streams[key] = torch.cuda.Stream(device=dev, priority=-1)
         return st
 
+    def side_stream_handle(self, dev, tokens: int) -> int:
+        """The second stream for a prefill of this length (0 where none is needed: no ragged tail)."""
+        return self._side_stream(dev).cuda_stream if dev.type == "cuda" and tokens % CHUNK else 0
+
     # -- decode ----------------------------------------------------------------------------
     def decode(self, q, k, v, g, b, w, state, scale: float, out=None) -> torch.Tensor:
         """``[B,n,H,D]`` tokens, ``state [B,H,DK,DV]`` fp32 contiguous, updated in place. Returns ``o``.
@@ -290,7 +294,7 @@ class NativeKernels:
 
     def prefill_plain(self, q, k, v, g, b, w, scale, state):
         """``gdn2_prefill_ragged`` through the host extension: ``(o, final_state)``, or ``None`` when the call is not plain."""
-        side = self._side_stream(q.device).cuda_stream if q.is_cuda and q.shape[1] % CHUNK else 0
+        side = self.side_stream_handle(q.device, q.shape[1])
         res = self.host.prefill(q, k, v, g, b, w, scale, state, self.prefill_path, side)
         if res is None:
             return None

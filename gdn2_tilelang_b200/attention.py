@@ -288,13 +288,10 @@ class GatedDeltaNet2(nn.Module):
         """``o_proj``; the head-parallel variant overrides it to add the sum over ranks."""
         return self.o_proj(normed)
 
-    def _decode_plain(self, x, cache, conv_in_place=False):
-        """The whole of ``decode`` as one native call (with ``conv_in_place`` the convolution cache is written into, too), or ``None`` where something about the layer, the cache or the input
-        needs the general path (a subclass, hooks, replaced methods, a missing or converted convolution cache, strided
-        tensors): whatever would have run when ``o_proj`` is called as a module still runs."""
-        K = _cabi.kernels()
-        host = getattr(K, "host", None)
-        call = getattr(K, "layer_step", None) if host is None else host.layer_decode
+    def _plain_call(self, cache, call, x, *rest):
+        """``call`` with the layer's tensors and sizes, or ``None`` where something about the layer or the cache needs the general
+        path (a subclass, hooks, replaced methods, a missing convolution cache): whatever would have run when ``o_proj`` is
+        called as a module still runs."""
         if call is None or type(self) is not GatedDeltaNet2 or cache.conv_state is None:
             return None
         m = self._modules
@@ -305,14 +302,36 @@ class GatedDeltaNet2(nn.Module):
             return None
         w_cat, offs, cw, cb = self._fused_tables()
         own = self._parameters
-        res = call(x, cache.recurrent_state, cache.conv_state, w_cat, cw, cb, own["A_log"], own["dt_bias"],
-                   m["o_norm"].weight, o_proj.weight, offs, self.num_heads, self.num_kv_heads, self.head_dim_k,
-                   self.head_dim_v, self.cfg.conv_size, self.erase_scale, m["o_norm"].eps, self.scale, conv_in_place)
+        return call(x, cache.recurrent_state, cache.conv_state, w_cat, cw, cb, own["A_log"], own["dt_bias"],
+                    m["o_norm"].weight, o_proj.weight, offs, self.num_heads, self.num_kv_heads, self.head_dim_k,
+                    self.head_dim_v, self.cfg.conv_size, self.erase_scale, m["o_norm"].eps, self.scale, *rest)
+
+    def _decode_plain(self, x, cache, conv_in_place=False):
+        """The whole of ``decode`` as one native call (with ``conv_in_place`` the convolution cache is written into, too), or
+        ``None`` where that does not apply."""
+        K = _cabi.kernels()
+        host = getattr(K, "host", None)
+        res = self._plain_call(cache, getattr(K, "layer_step", None) if host is None else host.layer_decode, x, conv_in_place)
         if res is None:
             return None
         out, conv, launched = res
         if not conv_in_place:
             cache.conv_state = conv
+        K.launches += launched
+        K.maybe_check_device_status(x.device)
+        return out
+
+    def _prefill_plain(self, x, cache):
+        """The whole of ``prefill`` as one native call, or ``None`` where that does not apply."""
+        K = _cabi.kernels()
+        host = getattr(K, "host", None)
+        if getattr(self, "fuse_output_norm", False) or x.dim() != 3 or not x.is_cuda:
+            return None
+        self.cfg.kernel.validate()
+        res = self._plain_call(cache, getattr(host, "layer_prefill", None), x, K.prefill_path, K.side_stream_handle(x.device, x.shape[1]))
+        if res is None:
+            return None
+        out, cache.recurrent_state, cache.conv_state, launched = res
         K.launches += launched
         K.maybe_check_device_status(x.device)
         return out
@@ -342,6 +361,9 @@ class GatedDeltaNet2(nn.Module):
         """Prefill a prompt (or a segment of one) and return ``(output, cache)`` to decode from."""
         if cache is None:
             cache = self.init_cache(hidden_states.shape[0], device=hidden_states.device)
+        out = self._prefill_plain(hidden_states, cache)
+        if out is not None:
+            return out, cache
         q, k, v, g, b, w, conv, proj = self._front(hidden_states, cache.conv_state, cached=self.q_conv is not None)
         if conv is not None:
             cache.conv_state = conv

@@ -82,20 +82,31 @@ std::optional<Tensor> decode(const Tensor& q, const Tensor& k, const Tensor& v, 
   return o;
 }
 
+// Whether a prefill of at least 64 tokens is one call of gdn2_prefill_ragged: resolves `path` and gives its workspace
+bool ragged_plan(const Problem& p, int& path, size_t& bytes) {
+  const int64_t n_full = p.S / 64 * 64;
+  if (path == GDN2_PATH_AUTO) path = p.DK == 128 && p.DV == 128 && p.dtype == GDN2_BF16 ? GDN2_PATH_TCGEN05 : GDN2_PATH_SIMT;
+  // the caller overlaps the stages of long, uncut problems segment by segment
+  if (path != GDN2_PATH_SIMT && n_full / 64 >= 32 && gdn2_prefill_scan_segments(p.B, n_full, p.H, p.DK, p.DV, p.dtype, path) <= 1)
+    return false;
+  bytes = gdn2_prefill_ragged_workspace_bytes(p.B, p.S, p.H, p.HK, p.DK, p.DV, p.dtype, path);
+  return bytes != 0;
+}
+int64_t ragged_launches(const Problem& p, int path) {
+  const int64_t n_full = p.S / 64 * 64;
+  const bool tc = path != GDN2_PATH_SIMT;
+  const int64_t scans = gdn2_prefill_scan_launches(p.B, n_full, p.H, p.DK, p.DV, p.dtype, path);
+  return (tc ? 2 : 1) + scans + (tc && p.S > n_full );
+}
+
 // gdn2_prefill_ragged. `side`: the second stream (0: none). Returns (o, final state, kernels launched) or None.
 std::optional<std::tuple<Tensor, Tensor, int64_t>> prefill(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& b, const Tensor& w,
                    std::optional<double> scale, const std::optional<Tensor>& state, int path, uint64_t side) {
   Problem p;
   if (q.dim() != 4 || !plain_tokens(q, k, v, g, b, w, p, 2)) return std::nullopt;
   if (state && !plain_state(*state, p)) return std::nullopt;
-  const int64_t n_full = p.S / 64 * 64;
-  if (n_full == 0) return std::nullopt;
-  if (path == GDN2_PATH_AUTO) path = p.DK == 128 && p.DV == 128 && p.dtype == GDN2_BF16 ? GDN2_PATH_TCGEN05 : GDN2_PATH_SIMT;
-  // the caller overlaps the stages of long, uncut problems segment by segment
-  if (path != GDN2_PATH_SIMT && n_full / 64 >= 32 && gdn2_prefill_scan_segments(p.B, n_full, p.H, p.DK, p.DV, p.dtype, path) <= 1)
-    return std::nullopt;
-  const size_t bytes = gdn2_prefill_ragged_workspace_bytes(p.B, p.S, p.H, p.HK, p.DK, p.DV, p.dtype, path);
-  if (bytes == 0) return std::nullopt;
+  size_t bytes = 0;
+  if (p.S < 64 || !ragged_plan(p, path, bytes)) return std::nullopt;
   const auto opt = v.options().requires_grad(false);
   Tensor ws = at::empty({(int64_t)bytes}, opt.dtype(at::kByte));
   Tensor o = at::empty(v.sizes(), opt);
@@ -104,40 +115,89 @@ std::optional<std::tuple<Tensor, Tensor, int64_t>> prefill(const Tensor& q, cons
   const int rc = gdn2_prefill_ragged(
       q.data_ptr(), k.data_ptr(), v.data_ptr(), static_cast<const float*>(g.data_ptr()), b.data_ptr(), w.data_ptr(),
       state ? static_cast<const float*>(state->data_ptr()) : nullptr, o.data_ptr(), static_cast<float*>(fin.data_ptr()), ws.data_ptr(),
-      bytes, p.B, p.S, p.H, p.HK, p.DK, p.DV, p.S, p.S, sc, p.dtype, path, p.S > n_full ? reinterpret_cast<void*>(side) : nullptr,
+      bytes, p.B, p.S, p.H, p.HK, p.DK, p.DV, p.S, p.S, sc, p.dtype, path, p.S % 64 ? reinterpret_cast<void*>(side) : nullptr,
       stream_of(p));
   if (rc != GDN2_OK) return std::nullopt;
-  const bool tc = path != GDN2_PATH_SIMT;
-  const int64_t launched = (tc ? 2 : 1) + gdn2_prefill_scan_launches(p.B, n_full, p.H, p.DK, p.DV, p.dtype, path) + (tc && p.S > n_full);
-  return std::make_tuple(o, fin, launched);
+  return std::make_tuple(o, fin, ragged_launches(p, path));
 }
 
 
-// GatedDeltaNet2.decode on x [B, n, hidden]: gdn2_layer_step where it applies, else projections, layer_front, decode,
-// layer_back, output projection. The recurrent state is updated in place. Returns (out [B, n, hidden], new convolution cache,
-// kernels launched) or None. `conv_in_place`: the convolution cache is updated in place too, or the call is not made.
+// What the layer's calls below share: x [B, n, hidden], the cache, the layer's tensors and sizes.
+struct Layer {
+  const Tensor &state, &w_cat, &A_log, &dt_bias, &norm_w, &o_w;
+  const std::optional<Tensor> &conv_state, &conv_w, &conv_b;
+  const std::vector<int64_t>& offs;
+  int64_t H, HK, DK, DV, K;
+  double erase_scale, eps, scale;
+  int64_t CC() const { return 2 * HK * DK + H * DV; }       // convolved channels
+};
+
+bool plain_layer(Tensor& x, const Layer& l, Problem& p) {
+  p.type = x.scalar_type();
+  p.dtype = dtype_code(p.type);
+  if (p.dtype < 0 || x.dim() != 3 || !x.is_cuda() || x.numel() == 0 || l.DK > 256 || l.DV > 256 || l.offs.size() != 7) return false;
+  p.dev = c10::cuda::current_device();
+  p.B = x.size(0); p.S = x.size(1); p.H = l.H; p.HK = l.HK; p.DK = l.DK; p.DV = l.DV;
+  for (const Tensor* t : {&l.w_cat, &l.A_log, &l.dt_bias, &l.norm_w, &l.o_w})
+    if (!plain(*t, p.type, p.dev)) return false;
+  // one token out of a prompt that lies in memory whole (x[:, t]): its rows are brought together
+  if (p.S == 1 && unwrapped(x, p.type, p.dev) && !dense(x)) x = x.clone(at::MemoryFormat::Contiguous);
+  if (!plain(x, p.type, p.dev) || !plain_state(l.state, p) || x.size(2) != l.w_cat.size(1)) return false;
+  return l.K >= 2 && l.conv_w && plain(*l.conv_w, p.type, p.dev) && (!l.conv_b || plain(*l.conv_b, p.type, p.dev)) && l.conv_state &&
+         plain(*l.conv_state, p.type, p.dev) && l.conv_state->dim() == 3 && l.conv_state->size(0) == p.B &&
+         l.conv_state->size(1) == l.CC() && l.conv_state->size(2) == l.K - 1;
+}
+
+// The layer stage by stage: projections, gdn2_layer_front, `attend` on the buffers of its inputs and output (true: done),
+// gdn2_layer_back, output projection. Returns (out, new convolution cache, kernels of the front and the back launched) or None
+// while nothing of the cache has changed, so that the general path can still take the call over.
+struct Stages { char *q, *k, *b, *v, *w, *o; float* g; };
+template <typename Attend>
+std::optional<std::tuple<Tensor, Tensor, int64_t>> layer_stages(const Tensor& x, const Layer& l, const Problem& p, Attend attend) {
+  Tensor proj = at::linear(x, l.w_cat);
+  if (proj.scalar_type() != p.type || !proj.is_contiguous()) return std::nullopt;       // an autocast region
+  const auto opt = x.options().requires_grad(false);
+  // one allocation for what lives between the stages, every part 256-byte aligned
+  const int64_t esz = p.dtype == GDN2_F32 ? 4 : 2, tokens = p.B * p.S;
+  auto part = [](int64_t bytes) { return (bytes + 255) / 256 * 256; };
+  const int64_t key = part(tokens * l.HK * l.DK * esz), decay = part(tokens * l.HK * l.DK * 4), value = part(tokens * l.H * l.DV * esz);
+  Tensor mid = at::empty({3 * key + decay + 3 * value}, opt.dtype(at::kByte)), normed = at::empty({p.B, p.S, l.H * l.DV}, opt);
+  Tensor conv = at::empty({p.B, l.CC(), l.K - 1}, opt);
+  char* at_ = static_cast<char*>(mid.data_ptr());
+  auto take = [&](int64_t bytes) { char* r = at_; at_ += bytes; return r; };
+  Stages m;
+  m.q = take(key); m.k = take(key); m.b = take(key); m.g = reinterpret_cast<float*>(take(decay));
+  m.v = take(value); m.w = take(value); m.o = take(value);
+  void* st = stream_of(p);
+  gdn2_layer_front_args a{};
+  a.proj = proj.data_ptr(); a.conv_state = l.conv_state->data_ptr(); a.conv_weight = l.conv_w->data_ptr();
+  a.conv_bias = l.conv_b ? l.conv_b->data_ptr() : nullptr;
+  a.A_log = l.A_log.data_ptr(); a.dt_bias = l.dt_bias.data_ptr();
+  a.q = m.q; a.k = m.k; a.v = m.v; a.g = m.g; a.b = m.b; a.w = m.w; a.new_conv_state = conv.data_ptr();
+  a.B = p.B; a.S = p.S; a.H = l.H; a.HK = l.HK; a.DK = l.DK; a.DV = l.DV; a.K = l.K; a.NP = proj.size(2);
+  a.off_q = l.offs[0]; a.off_k = l.offs[1]; a.off_v = l.offs[2]; a.off_b = l.offs[3]; a.off_w = l.offs[4]; a.off_f = l.offs[5];
+  a.erase_scale = (float)l.erase_scale;
+  if (gdn2_layer_front(&a, p.dtype, st) != GDN2_OK || !attend(m)) return std::nullopt;
+  const int rc = gdn2_layer_back(m.o, proj.data_ptr(), l.norm_w.data_ptr(), normed.data_ptr(), p.B * p.S, l.H, l.DV,
+                                 proj.size(2), l.offs[6], (float)l.eps, p.dtype, st);
+  if (rc != GDN2_OK) throw std::runtime_error(std::string("gdn2_layer_back: ") + gdn2_status_string(rc));
+  // the front kernel writes the new convolution cache itself in its one-token form, else a second one does
+  bool fused = p.dtype != GDN2_F32 && l.DK == 128 && l.DV == 128 && l.K == 4 && p.S < 8 && a.NP % 4 == 0;
+  for (int i = 0; i < 6; ++i) fused = fused && l.offs[i] % 4 == 0;
+  return std::make_tuple(at::linear(normed, l.o_w), conv, int64_t(fused ? 2 : 3));
+}
+
+// GatedDeltaNet2.decode on x [B, n, hidden]: gdn2_layer_step where it applies, else stage by stage. The recurrent state is updated
+// in place. Returns (out [B, n, hidden], new convolution cache, kernels launched) or None. `conv_in_place`: the convolution
+// cache is updated in place too, or the call is not made.
 std::optional<std::tuple<Tensor, Tensor, int64_t>> layer_decode(Tensor x, const Tensor& state, const std::optional<Tensor>& conv_state, const Tensor& w_cat,
                         const std::optional<Tensor>& conv_w, const std::optional<Tensor>& conv_b, const Tensor& A_log,
                         const Tensor& dt_bias, const Tensor& norm_w, const Tensor& o_w, const std::vector<int64_t>& offs, int64_t H,
                         int64_t HK, int64_t DK, int64_t DV, int64_t K, double erase_scale, double eps, double scale, bool conv_in_place) {
+  const Layer l{state, w_cat, A_log, dt_bias, norm_w, o_w, conv_state, conv_w, conv_b, offs, H, HK, DK, DV, K, erase_scale, eps, scale};
   Problem p;
-  p.type = x.scalar_type();
-  p.dtype = dtype_code(p.type);
-  if (p.dtype < 0 || x.dim() != 3 || !x.is_cuda() || x.numel() == 0 || DK > 256 || DV > 256 || offs.size() != 7) return std::nullopt;
-  p.dev = c10::cuda::current_device();
-  p.B = x.size(0); p.S = x.size(1); p.H = H; p.HK = HK; p.DK = DK; p.DV = DV;
-  for (const Tensor* t : {&w_cat, &A_log, &dt_bias, &norm_w, &o_w})
-    if (!plain(*t, p.type, p.dev)) return std::nullopt;
   at::NoGradGuard no_grad;
-  // one token out of a prompt that lies in memory whole (x[:, t]): its rows are brought together
-  if (p.S == 1 && unwrapped(x, p.type, p.dev) && !dense(x)) x = x.clone(at::MemoryFormat::Contiguous);
-  if (!plain(x, p.type, p.dev) || !plain_state(state, p) || x.size(2) != w_cat.size(1)) return std::nullopt;
-  const int64_t CC = 2 * HK * DK + H * DV;
-  if (K < 2 || !conv_w || !plain(*conv_w, p.type, p.dev) || (conv_b && !plain(*conv_b, p.type, p.dev)) || !conv_state ||
-      !plain(*conv_state, p.type, p.dev) || conv_state->dim() != 3 || conv_state->size(0) != p.B || conv_state->size(1) != CC ||
-      conv_state->size(2) != K - 1)
-    return std::nullopt;
-  const auto opt = x.options().requires_grad(false);
+  if (!plain_layer(x, l, p)) return std::nullopt;
   const int64_t hidden = x.size(2);
   // (an autocast region or a dispatch mode would have seen the two linear layers)
   const size_t step_bytes = p.S == 1 && o_w.dim() == 2 && o_w.size(0) == hidden && o_w.size(1) == H * DV &&
@@ -145,8 +205,9 @@ std::optional<std::tuple<Tensor, Tensor, int64_t>> layer_decode(Tensor x, const 
                                 ? gdn2_layer_step_workspace_bytes(p.B, hidden, H, HK, DK, DV, K, p.dtype)
                                 : 0;
   if (step_bytes > 0) {
+    const auto opt = x.options().requires_grad(false);
     Tensor ws = at::empty({(int64_t)step_bytes}, opt.dtype(at::kByte)), out = at::empty({p.B, 1, hidden}, opt);
-    Tensor conv = conv_in_place ? *conv_state : at::empty({p.B, CC, K - 1}, opt);
+    Tensor conv = conv_in_place ? *conv_state : at::empty({p.B, l.CC(), K - 1}, opt);
     gdn2_layer_step_args s{};
     s.x = x.data_ptr(); s.w_cat = w_cat.data_ptr(); s.conv_state = conv_state->data_ptr(); s.conv_weight = conv_w->data_ptr();
     s.conv_bias = conv_b ? conv_b->data_ptr() : nullptr;
@@ -162,37 +223,43 @@ std::optional<std::tuple<Tensor, Tensor, int64_t>> layer_decode(Tensor x, const 
     if (rc == GDN2_ERR_CUDA) throw std::runtime_error(std::string("gdn2_layer_step: ") + gdn2_status_string(rc));
   }
   if (conv_in_place) return std::nullopt;
-  Tensor proj = at::linear(x, w_cat);
-  if (proj.scalar_type() != p.type || !proj.is_contiguous()) return std::nullopt;       // an autocast region
-  // one allocation for what lives between the stages, every part 256-byte aligned
-  const int64_t esz = p.dtype == GDN2_F32 ? 4 : 2, tokens = p.B * p.S;
-  auto part = [](int64_t bytes) { return (bytes + 255) / 256 * 256; };
-  const int64_t key = part(tokens * HK * DK * esz), decay = part(tokens * HK * DK * 4), value = part(tokens * H * DV * esz);
-  Tensor mid = at::empty({3 * key + decay + 3 * value}, opt.dtype(at::kByte)), normed = at::empty({p.B, p.S, H * DV}, opt);
-  Tensor conv = at::empty({p.B, CC, K - 1}, opt);
-  char* at_ = static_cast<char*>(mid.data_ptr());
-  auto take = [&](int64_t bytes) { char* r = at_; at_ += bytes; return r; };
-  char *q = take(key), *k = take(key), *b = take(key), *g = take(decay), *v = take(value), *w = take(value), *o = take(value);
-  void* st = stream_of(p);
-  gdn2_layer_front_args a{};
-  a.proj = proj.data_ptr(); a.conv_state = conv_state->data_ptr(); a.conv_weight = conv_w->data_ptr();
-  a.conv_bias = conv_b ? conv_b->data_ptr() : nullptr;
-  a.A_log = A_log.data_ptr(); a.dt_bias = dt_bias.data_ptr();
-  a.q = q; a.k = k; a.v = v; a.g = reinterpret_cast<float*>(g); a.b = b; a.w = w; a.new_conv_state = conv.data_ptr();
-  a.B = p.B; a.S = p.S; a.H = H; a.HK = HK; a.DK = DK; a.DV = DV; a.K = K; a.NP = proj.size(2);
-  a.off_q = offs[0]; a.off_k = offs[1]; a.off_v = offs[2]; a.off_b = offs[3]; a.off_w = offs[4]; a.off_f = offs[5];
-  a.erase_scale = (float)erase_scale;
-  // up to the decode nothing of the cache has changed, so the general path can still take the call over
-  if (gdn2_layer_front(&a, p.dtype, st) != GDN2_OK) return std::nullopt;
-  if (gdn2_decode(q, k, v, a.g, b, w, static_cast<float*>(state.data_ptr()), o, p.B, p.S, H, HK, DK, DV, p.S, p.S, (float)scale, p.dtype, st) != GDN2_OK)
-    return std::nullopt;
-  const int rc = gdn2_layer_back(o, proj.data_ptr(), norm_w.data_ptr(), normed.data_ptr(), p.B * p.S, H, DV,
-                                 proj.size(2), offs[6], (float)eps, p.dtype, st);
-  if (rc != GDN2_OK) throw std::runtime_error(std::string("gdn2_layer_back: ") + gdn2_status_string(rc));
-  // the front kernel writes the new convolution cache itself in its one-token form, else a second one does
-  bool fused = p.dtype != GDN2_F32 && DK == 128 && DV == 128 && K == 4 && p.S < 8 && a.NP % 4 == 0;
-  for (int i = 0; i < 6; ++i) fused = fused && offs[i] % 4 == 0;
-  return std::make_tuple(at::linear(normed, o_w), conv, int64_t(fused ? 3 : 4));
+  auto res = layer_stages(x, l, p, [&](const Stages& m) {
+    return gdn2_decode(m.q, m.k, m.v, m.g, m.b, m.w, static_cast<float*>(state.data_ptr()), m.o, p.B, p.S, H, HK, DK, DV, p.S, p.S,
+                       (float)scale, p.dtype, stream_of(p)) == GDN2_OK;
+  });
+  if (res) std::get<2>(*res) += 1;
+  return res;
+}
+
+// GatedDeltaNet2.prefill on x [B, S, hidden], continuing from the cache. Returns (out [B, S, hidden], final recurrent state, new
+// convolution cache, kernels launched) or None. A prompt shorter than a chunk is decoded and updates the recurrent state in
+// place, as gdn2_prefill does.
+std::optional<std::tuple<Tensor, Tensor, Tensor, int64_t>> layer_prefill(Tensor x, const Tensor& state, const std::optional<Tensor>& conv_state, const Tensor& w_cat,
+                        const std::optional<Tensor>& conv_w, const std::optional<Tensor>& conv_b, const Tensor& A_log,
+                        const Tensor& dt_bias, const Tensor& norm_w, const Tensor& o_w, const std::vector<int64_t>& offs, int64_t H,
+                        int64_t HK, int64_t DK, int64_t DV, int64_t K, double erase_scale, double eps, double scale, int path, uint64_t side) {
+  const Layer l{state, w_cat, A_log, dt_bias, norm_w, o_w, conv_state, conv_w, conv_b, offs, H, HK, DK, DV, K, erase_scale, eps, scale};
+  Problem p;
+  at::NoGradGuard no_grad;
+  if (!plain_layer(x, l, p)) return std::nullopt;
+  size_t bytes = 0;
+  if (p.S >= 64 && !ragged_plan(p, path, bytes)) return std::nullopt;
+  Tensor fin = state;
+  const auto opt = x.options().requires_grad(false);
+  int64_t launched = 1;
+  auto res = layer_stages(x, l, p, [&](const Stages& m) {
+    if (p.S < 64)
+      return gdn2_decode_tail(m.q, m.k, m.v, m.g, m.b, m.w, static_cast<float*>(state.data_ptr()), m.o, p.B, p.S, H, HK, DK, DV, p.S, p.S,
+                              (float)scale, p.dtype, stream_of(p)) == GDN2_OK;
+    Tensor ws = at::empty({(int64_t)bytes}, opt.dtype(at::kByte));
+    fin = at::empty({p.B, H, DK, DV}, opt.dtype(at::kFloat));
+    launched = ragged_launches(p, path);
+    return gdn2_prefill_ragged(m.q, m.k, m.v, m.g, m.b, m.w, static_cast<const float*>(state.data_ptr()), m.o, static_cast<float*>(fin.data_ptr()),
+                               ws.data_ptr(), bytes, p.B, p.S, H, HK, DK, DV, p.S, p.S, (float)scale, p.dtype, path,
+                               p.S % 64 ? reinterpret_cast<void*>(side) : nullptr, stream_of(p)) == GDN2_OK;
+  });
+  if (!res) return std::nullopt;
+  return std::make_tuple(std::get<0>(*res), fin, std::get<1>(*res), std::get<2>(*res) + launched);
 }
 
 // The state of a list of parameters: where each lies, its version and its type. Equal bytes = nothing was replaced,
@@ -214,5 +281,6 @@ PYBIND11_MODULE(_gdn2_host, m) {
   m.def("decode", &decode, unlocked);
   m.def("prefill", &prefill, unlocked);
   m.def("layer_decode", &layer_decode, unlocked);
+  m.def("layer_prefill", &layer_prefill, unlocked);
   m.def("parameter_key", &parameter_key);
 }
