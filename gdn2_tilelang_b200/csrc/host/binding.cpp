@@ -96,7 +96,7 @@ int64_t ragged_launches(const Problem& p, int path) {
   const int64_t n_full = p.S / 64 * 64;
   const bool tc = path != GDN2_PATH_SIMT;
   const int64_t scans = gdn2_prefill_scan_launches(p.B, n_full, p.H, p.DK, p.DV, p.dtype, path);
-  return (tc ? 2 : 1) + scans + (tc && p.S > n_full );
+  return (tc ? 2 : 1) + scans + (tc && p.S > n_full);
 }
 
 // gdn2_prefill_ragged. `side`: the second stream (0: none). Returns (o, final state, kernels launched) or None.
@@ -121,6 +121,24 @@ std::optional<std::tuple<Tensor, Tensor, int64_t>> prefill(const Tensor& q, cons
   return std::make_tuple(o, fin, ragged_launches(p, path));
 }
 
+
+// gdn2_prefill of a prompt shorter than a chunk: the decode of its tokens, `state` updated in place and returned (none: from zero).
+// Returns (o, state) or None.
+std::optional<std::tuple<Tensor, Tensor>> prefill_short(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& b,
+                                                        const Tensor& w, std::optional<double> scale, const std::optional<Tensor>& state) {
+  Problem p;
+  if (q.dim() != 4 || !plain_tokens(q, k, v, g, b, w, p, 2) || p.S >= 64 || p.DK > 256) return std::nullopt;
+  if (state && !plain_state(*state, p)) return std::nullopt;
+  const auto opt = v.options().requires_grad(false);
+  Tensor o = at::empty(v.sizes(), opt);
+  Tensor st = state ? *state : at::zeros({p.B, p.H, p.DK, p.DV}, opt.dtype(at::kFloat));
+  const float sc = scale ? (float)*scale : (float)(1.0 / std::sqrt((double)p.DK));
+  const int rc = gdn2_decode_tail(q.data_ptr(), k.data_ptr(), v.data_ptr(), static_cast<const float*>(g.data_ptr()), b.data_ptr(), w.data_ptr(),
+                                  static_cast<float*>(st.data_ptr()), o.data_ptr(), p.B, p.S, p.H, p.HK, p.DK, p.DV, p.S, p.S, sc, p.dtype,
+                                  stream_of(p));
+  if (rc != GDN2_OK) return std::nullopt;
+  return std::make_tuple(o, st);
+}
 
 // What the layer's calls below share: x [B, n, hidden], the cache, the layer's tensors and sizes.
 struct Layer {
@@ -280,6 +298,7 @@ PYBIND11_MODULE(_gdn2_host, m) {
   const auto unlocked = py::call_guard<py::gil_scoped_release>();
   m.def("decode", &decode, unlocked);
   m.def("prefill", &prefill, unlocked);
+  m.def("prefill_short", &prefill_short, unlocked);
   m.def("layer_decode", &layer_decode, unlocked);
   m.def("layer_prefill", &layer_prefill, unlocked);
   m.def("parameter_key", &parameter_key);

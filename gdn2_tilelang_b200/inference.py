@@ -83,6 +83,17 @@ def gdn2_decode_step(q, k, v, g, b, w, state, scale=None):
     return o[:, 0]
 
 
+def _prefill_short(q, k, v, g, b, w, state, scale):
+    """A prompt shorter than a chunk in one native call, or ``None`` where the call is not plain."""
+    K = _cabi.kernels()
+    call = getattr(getattr(K, "host", None), "prefill_short", None)
+    res = None if call is None else call(q, k, v, g, b, w, scale, state)
+    if res is not None:
+        K.launches += 1
+        K.maybe_check_device_status(q.device)
+    return res
+
+
 def _prefill_plain(q, k, v, g, b, w, state, scale):
     """A prefill of at least 64 tokens in one native call, or ``None`` where the call is not plain."""
     K = _cabi.kernels()
@@ -107,7 +118,8 @@ def gdn2_prefill(q, k, v, g, b, w, state=None, scale=None, config: GDN2Config = 
     """
     config.validate()
     if gated_norm is None:
-        res = _prefill_plain(q, k, v, g, b, w, state, scale)
+        short = q.dim() == 4 and q.shape[1] < config.chunk_size
+        res = (_prefill_short if short else _prefill_plain)(q, k, v, g, b, w, state, scale)
         if res is not None:
             return res
     B, S, H, DK, DV = _check_inputs(q, k, v, g, b, w)
