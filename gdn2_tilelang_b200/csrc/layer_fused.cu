@@ -230,18 +230,32 @@ layer_front_d128_kernel(gdn2_layer_front_args a) {
   }
 }
 
-// The same for prompts, cut finer: one warp per (head-wide slot, FOUR consecutive tokens). A token's slots are its
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(*reinterpret_cast<unsigned long long*>(&d))
+      : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
+        "l"(*reinterpret_cast<unsigned long long*>(&c)));
+  return d;
+}
+
+constexpr int kPromptTokens = 8;
+
+// The same for prompts, cut finer: one warp per (head-wide slot, kPromptTokens consecutive tokens). A token's slots are its
 // HK q heads, HK k heads, H v heads (convolution kinds), HK erase-gate heads, HK decay heads and H write-gate heads
 // (element-wise kinds); the slot index runs fastest, so the warps in flight sweep whole projection rows. A
-// convolution slot reads the 7 projection rows its four outputs need once (the one-token form reads 16), every
-// warp has all of its loads in flight before the first use and holds few enough registers for 32 warps per SM.
+// convolution slot reads the 3 rows before its tokens once for all of them (the one-token form reads 4 rows a token), every
+// warp has all of its loads in flight before the first use and keeps them as they came, so that 32 warps fit on an SM.
+// 2 x 4096 tokens, hidden 2048, 16 heads (285 MB): four tokens a warp, rows converted on arrival, 102 us and 80 million warp
+// instructions, two thirds of the issue slots; eight tokens took 57 million but, with room for 20 warps, no less time; kept raw 81 us.
+// (six tokens 84, four 93.)
 // Arithmetic and summation order are those of the one-token form, so the two agree bit for bit.
 template <typename T>
-__global__ void __launch_bounds__(32 * kWarps, 6)
-layer_front_d128x4_kernel(gdn2_layer_front_args a) {
+__global__ void __launch_bounds__(32 * kWarps, 8)
+layer_front_prompt_kernel(gdn2_layer_front_args a) {
   grid_wait();
   grid_launch_dependents();
-  constexpr int D = 128, K = 4, TT = 4;
+  constexpr int D = 128, K = 4, TT = kPromptTokens;
   const int lane = threadIdx.x & 31;
   const int S = (int)a.S, NP = (int)a.NP, H = (int)a.H, HK = (int)a.HK;
   const int groups = (S + TT - 1) / TT;
@@ -258,9 +272,9 @@ layer_front_d128x4_kernel(gdn2_layer_front_args a) {
   const int nt = S - t0 < TT ? S - t0 : TT;               // tokens of this group that exist
   const size_t tok0 = (size_t)b * S + t0;
   {
-    // Pull the rows of the same slot some 4096 warps ahead (about what the GPU holds at once, a whole number of
-    // token groups of this batch row) towards L2: 4 rows x 256 B = 8 lines, one per lane 0..7.
-    const int ahead = ((4096 + nslots - 1) / nslots) * TT;
+    // Pull the rows of the same slot some thousand warps ahead (about what the GPU holds at once, a whole number of
+    // token groups of this batch row) towards L2: kPromptTokens rows x 256 B, one line per lane.
+    const int ahead = ((16384 / TT + nslots - 1) / nslots) * TT;
     const int scol = slot < HK ? (int)a.off_q + slot * D
                    : slot < 2 * HK ? (int)a.off_k + (slot - HK) * D
                    : slot < 2 * HK + H ? (int)a.off_v + (slot - 2 * HK) * D
@@ -281,34 +295,56 @@ layer_front_d128x4_kernel(gdn2_layer_front_args a) {
     const T* cs = static_cast<const T*>(a.conv_state);
     const T* cw = static_cast<const T*>(a.conv_weight);
     const T* cb = static_cast<const T*>(a.conv_bias);
-    float wt[4][4], bias[4], x[TT + K - 1][4];
+    Vec4<T> x[TT + K - 1], wr[4], br;                        // as loaded; wr: the four taps of a channel
 #pragma unroll
     for (int r = 0; r < TT + K - 1; ++r) {
       const int tt = t0 - (K - 1) + r;
       if (tt >= 0 && tt < S) {
-        load4(P + ((size_t)b * S + tt) * NP + col, x[r]);
-      } else if (tt < 0 && cs) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) x[r][i] = to_f32(cs[((size_t)b * CC + cch + i) * (K - 1) + (K - 1 + tt)]);
+        x[r] = load_raw4(P + ((size_t)b * S + tt) * NP + col);
       } else {
-        x[r][0] = x[r][1] = x[r][2] = x[r][3] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          x[r].x[i] = tt < 0 && cs ? cs[((size_t)b * CC + cch + i) * (K - 1) + (K - 1 + tt)] : from_f32<T>(0.f);
       }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) load4(cw + (size_t)(cch + i) * K, wt[i]);
-    if (cb) load4(cb + cch, bias);
-    else { bias[0] = bias[1] = bias[2] = bias[3] = 0.f; }
+    for (int i = 0; i < 4; ++i) wr[i] = load_raw4(cw + (size_t)(cch + i) * K);
+    if (cb) br = load_raw4(cb + cch);
+    float2 wt[K][2], bias[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};   // pairs of adjacent channels
+    {
+      float w4[4][4], b4[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) unpack4(wr[i], w4[i]);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int j = 0; j < K; ++j) wt[j][h] = make_float2(w4[2 * h][j], w4[2 * h + 1][j]);
+      }
+      if (cb) {
+        unpack4(br, b4);
+        bias[0] = make_float2(b4[0], b4[1]); bias[1] = make_float2(b4[2], b4[3]);
+      }
+    }
+    float2 win[K][2];                                        // the last four rows
+    auto convert = [&](int r) {
+      float y[4];
+      unpack4(x[r], y);
+      win[r % K][0] = make_float2(y[0], y[1]); win[r % K][1] = make_float2(y[2], y[3]);
+    };
+#pragma unroll
+    for (int r = 0; r < K - 1; ++r) convert(r);
     T* dst = static_cast<T*>(is_v ? a.v : slot < HK ? a.q : a.k);
     const int heads = is_v ? H : HK;
 #pragma unroll
     for (int u = 0; u < TT; ++u) {
+      convert(u + K - 1);
       float y[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float acc = bias[i];
+      for (int h = 0; h < 2; ++h) {
+        float2 acc = bias[h];
 #pragma unroll
-        for (int j = 0; j < K; ++j) acc = fmaf(wt[i][j], x[u + j][i], acc);
-        y[i] = silu(acc);
+        for (int j = 0; j < K; ++j) acc = ffma2(wt[j][h], win[(u + j) % K][h], acc);
+        y[2 * h] = silu(acc.x); y[2 * h + 1] = silu(acc.y);
       }
       if (!is_v) {
         const float ss = warp_sum(y[0] * y[0] + y[1] * y[1] + y[2] * y[2] + y[3] * y[3]);
@@ -325,30 +361,34 @@ layer_front_d128x4_kernel(gdn2_layer_front_args a) {
   const int kind = e < HK ? 0 : e < 2 * HK ? 1 : 2;
   const int head = kind == 0 ? e : kind == 1 ? e - HK : e - 2 * HK;
   const int col = (int)(kind == 0 ? a.off_b : kind == 1 ? a.off_f : a.off_w) + head * D + c;
-  float p[TT][4];
+  Vec4<T> pr[TT];
 #pragma unroll
   for (int u = 0; u < TT; ++u)
-    if (u < nt) load4(P + (tok0 + u) * NP + col, p[u]);
+    if (u < nt) pr[u] = load_raw4(P + (tok0 + u) * NP + col);
   if (kind == 1) {
     float db[4];
     load4(static_cast<const T*>(a.dt_bias) + head * D + c, db);
     const float nega = -__expf(to_f32(static_cast<const T*>(a.A_log)[head]));
 #pragma unroll
     for (int u = 0; u < TT; ++u)
-      if (u < nt)
+      if (u < nt) {
+        float p[4];
+        unpack4(pr[u], p);
         *reinterpret_cast<float4*>(a.g + ((tok0 + u) * HK + head) * D + c) =
-            make_float4(nega * softplusf_(p[u][0] + db[0]), nega * softplusf_(p[u][1] + db[1]),
-                        nega * softplusf_(p[u][2] + db[2]), nega * softplusf_(p[u][3] + db[3]));
+            make_float4(nega * softplusf_(p[0] + db[0]), nega * softplusf_(p[1] + db[1]), nega * softplusf_(p[2] + db[2]),
+                        nega * softplusf_(p[3] + db[3]));
+      }
   } else {
     T* dst = static_cast<T*>(kind == 0 ? a.b : a.w);
     const int heads = kind == 0 ? HK : H;
 #pragma unroll
     for (int u = 0; u < TT; ++u)
       if (u < nt) {
-        float y[4];
+        float p[4], y[4];
+        unpack4(pr[u], p);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          y[i] = sigmoidf_(p[u][i]);
+          y[i] = sigmoidf_(p[i]);
           if (kind == 0) y[i] = to_f32(from_f32<T>(y[i])) * a.erase_scale;
         }
         store4(dst + ((tok0 + u) * heads + head) * D + c, y);
@@ -415,9 +455,9 @@ int launch_front_typed(const gdn2_layer_front_args& a, cudaStream_t st) {
                          reinterpret_cast<uintptr_t>(a.b) | reinterpret_cast<uintptr_t>(a.w)) & 7) == 0 &&
                        (reinterpret_cast<uintptr_t>(a.g) & 15) == 0;
   if (sizeof(T) == 2 && a.DK == 128 && a.DV == 128 && a.K == 4 && aligned && a.S >= 8 &&
-      a.B * ((a.S + 3) / 4) * (4 * a.HK + 2 * a.H) < (int64_t)1 << 31) {
-    const int64_t items4 = a.B * ((a.S + 3) / 4) * (4 * a.HK + 2 * a.H);   // prompts: a slot of four tokens per warp
-    GDN2_CUDA_TRY(launch_chained(true, layer_front_d128x4_kernel<T>, dim3((unsigned)((items4 + kWarps - 1) / kWarps)), 32 * kWarps, 0, st, a));
+      a.B * ((a.S + kPromptTokens - 1) / kPromptTokens) * (4 * a.HK + 2 * a.H) < (int64_t)1 << 31) {
+    const int64_t items = a.B * ((a.S + kPromptTokens - 1) / kPromptTokens) * (4 * a.HK + 2 * a.H);   // a slot of some tokens per warp
+    GDN2_CUDA_TRY(launch_chained(true, layer_front_prompt_kernel<T>, dim3((unsigned)((items + kWarps - 1) / kWarps)), 32 * kWarps, 0, st, a));
   } else if (sizeof(T) == 2 && a.DK == 128 && a.DV == 128 && a.K == 4 && aligned) {
     GDN2_CUDA_TRY(launch_chained(true, layer_front_d128_kernel<T>, dim3((unsigned)((items + kWarps - 1) / kWarps)), 32 * kWarps, 0, st, a));
     return GDN2_OK;                                          // this form writes the new convolution cache itself

@@ -33,17 +33,32 @@ template <typename T>
 struct alignas(4 * sizeof(T)) Vec4 { T x[4]; };
 
 template <typename T>
-__device__ __forceinline__ void load4(const T* p, float (&o)[4]) {
-  const Vec4<T> v = *reinterpret_cast<const Vec4<T>*>(p);
+__device__ __forceinline__ void unpack4(const Vec4<T>& v, float (&o)[4]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) o[i] = to_f32(v.x[i]);
 }
+// (bf16 by whole words: one instruction per element, where halves taken out first are two)
+template <>
+__device__ __forceinline__ void unpack4<__nv_bfloat16>(const Vec4<__nv_bfloat16>& v, float (&o)[4]) {
+  const uint2 u = *reinterpret_cast<const uint2*>(&v);
+  o[0] = __uint_as_float(u.x << 16); o[1] = __uint_as_float(u.x & 0xffff0000u);
+  o[2] = __uint_as_float(u.y << 16); o[3] = __uint_as_float(u.y & 0xffff0000u);
+}
+template <typename T>
+__device__ __forceinline__ Vec4<T> load_raw4(const T* p) { return *reinterpret_cast<const Vec4<T>*>(p); }
+template <typename T>
+__device__ __forceinline__ void load4(const T* p, float (&o)[4]) { unpack4(load_raw4(p), o); }
 template <typename T>
 __device__ __forceinline__ void store4(T* p, const float (&o)[4]) {
   Vec4<T> v;
 #pragma unroll
   for (int i = 0; i < 4; ++i) v.x[i] = from_f32<T>(o[i]);
   *reinterpret_cast<Vec4<T>*>(p) = v;
+}
+template <>
+__device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16* p, const float (&o)[4]) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(o[0], o[1]), b = __floats2bfloat162_rn(o[2], o[3]);
+  *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
 
 }  // namespace gdn2
