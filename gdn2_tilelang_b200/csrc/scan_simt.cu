@@ -13,8 +13,9 @@
 // Inside a chunk the pace is set by what shared memory can return, 128 bytes a cycle whether lanes share an address or not. A
 // thread therefore forms 4 rows x 4 columns over a quarter of the reduction (8 loads of 16 bytes per 64 FMAs, where one row by
 // four columns took 5 for 16), and the four quarters, neighbours in a warp, meet in 12 shuffles. Two buffers per record, so that a
-// copy has a whole chunk to land, gained nothing (79 -> 84 us). Measured
-// with the chunk-local stage (prep_simt.cu), B = 2, S = 1000, 8 heads of 64, float32: 75.7 us a call, 78.9 before.
+// copy has a whole chunk to land, gained nothing (79 -> 84 us); reading U from global memory a chunk ahead, four values a lane, in
+// place of sixteen small copies a chunk did (75.6 -> 71.5). Measured
+// with the chunk-local stage (prep_simt.cu), B = 2, S = 1000, 8 heads of 64, float32: 71.5 us a call, 78.9 before.
 //
 // Output: one block per (value tile, chunk, batch*head) doing the first two lines from a stored
 // chunk state (output_kernel, gdn2/forward.py:710-725).
@@ -113,22 +114,21 @@ __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
   return d;
 }
 
-enum : uint32_t { kWaitSimtWq = 0x200000u, kWaitSimtUt = 0x400000u, kWaitSimtAqk = 0x800000u, kWaitSimtKgt = 0x1000000u };
+enum : uint32_t { kWaitSimtWq = 0x200000u, kWaitSimtAqk = 0x800000u, kWaitSimtKgt = 0x1000000u };
 
 // Shared memory of the scan: the chunk's records as stored (fp32 images), the state tile and Un, value columns outside.
 template <int NVT> struct ScanTile {
-  float *wq, *aqk, *kgt, *ut, *gl, *St, *Un;
+  float *wq, *aqk, *kgt, *gl, *St, *Un;
   __device__ ScanTile(float* base, int DK) {
     wq = base;                          // [DK/4][128 rows][4]
     kgt = wq + 2 * kChunk * DK;         // [64/4][DK][4]
     aqk = kgt + kChunk * DK;            // [64/4][64 r][4]
-    ut = aqk + kChunk * kChunk;         // [64/4][NVT][4]
-    gl = ut + kChunk * NVT;             // [DK]
+    gl = aqk + kChunk * kChunk;         // [DK]
     St = gl + DK;                       // [NVT][DK]: the state transposed
     Un = St + DK * NVT;                 // [NVT][64]
   }
   static size_t bytes(int DK) {
-    return ((size_t)3 * kChunk * DK + kChunk * kChunk + 2 * kChunk * NVT + DK + (size_t)DK * NVT) * sizeof(float);
+    return ((size_t)3 * kChunk * DK + kChunk * kChunk + kChunk * NVT + DK + (size_t)DK * NVT) * sizeof(float);
   }
 };
 
@@ -188,7 +188,7 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
   const int mine = rl + 8 * (2 * (part & 1) + (part >> 1));   // row of 32 whose sums this lane keeps (tile_reduce)
   extern __shared__ __align__(128) float sm[];
   ScanTile<NVT> s(sm, DK);
-  __shared__ uint64_t bar_wq, bar_ut, bar_aqk, bar_kgt;
+  __shared__ uint64_t bar_wq, bar_aqk, bar_kgt;
   __shared__ int abort_flag;
 
   // this block's run of chunks: how many, its records (those of its key head, and U of its value head), its first
@@ -211,19 +211,15 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
   const char* g_wq = P.wq + (size_t)ch0 * L.wq_bytes;
   const char* g_aqk = P.aqk + (size_t)ch0 * L.aqk_bytes;
   const char* g_kgt = P.kgt + (size_t)ch0 * L.kgt_bytes;
-  const char* g_ut = P.ut + (size_t)chv0 * L.ut_bytes + (size_t)lo * 16;
+  const float* g_ut = reinterpret_cast<const float*>(P.ut + (size_t)chv0 * L.ut_bytes) + (size_t)lo * 4;
   const float* g_gl = P.gl + (size_t)ch0 * DK;
 
-  // copies of chunk n, issued by the first warp (the 16 column pieces of U by its first 16 lanes)
-  auto load_wq_ut = [&](int n) {
+  // copies of chunk n, issued by one thread
+  auto load_wq = [&](int n) {
     if (lane == 0) {
       tc::mbar_expect_tx(&bar_wq, (uint32_t)L.wq_bytes);
       tc::bulk_g2s(s.wq, g_wq + (size_t)n * L.wq_bytes, (uint32_t)L.wq_bytes, &bar_wq);
-      tc::mbar_expect_tx(&bar_ut, (uint32_t)(16 * nv * 16));
     }
-    __syncwarp();
-    if (lane < 16)
-      tc::bulk_g2s(s.ut + lane * NVT * 4, g_ut + (size_t)n * L.ut_bytes + (size_t)lane * DV * 16, (uint32_t)(nv * 16), &bar_ut);
   };
   auto load_aqk_kgt = [&](int n) {
     if (lane == 0) {
@@ -236,7 +232,7 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
   };
 
   if (tid == 0) {
-    tc::mbar_init(&bar_wq, 1); tc::mbar_init(&bar_ut, 1); tc::mbar_init(&bar_aqk, 1); tc::mbar_init(&bar_kgt, 1);
+    tc::mbar_init(&bar_wq, 1); tc::mbar_init(&bar_aqk, 1); tc::mbar_init(&bar_kgt, 1);
     abort_flag = 0;
     tc::mbar_init_fence();
   }
@@ -245,11 +241,9 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
     const int c = idx / NVT, d = idx % NVT;
     s.St[d * DK + c] = (s0 != nullptr && d < nv) ? s0[((size_t)bh * DK + c) * DV + lo + d] : 0.f;
   }
-  if (nv < NVT)                                            // columns past DV: no copy brings them
-    for (int idx = tid; idx < kChunk * NVT; idx += 256) s.ut[idx] = 0.f;
   tc::fence_async_smem();
   __syncthreads();
-  if (wid == 0 && NC > 0) { load_wq_ut(0); load_aqk_kgt(0); }
+  if (wid == 0 && NC > 0) { load_wq(0); load_aqk_kgt(0); }
 
   // After a wait that ran out a warp computes on what is there (the status word says that the results are void) and keeps the
   // block's barriers; the copying warp issues nothing more. Leaving together takes a barrier that carries the result, twice
@@ -257,7 +251,18 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
   auto wait_all = [&](uint64_t* bar, uint32_t parity, uint32_t code) {
     return tc::mbar_wait_warp(bar, parity, &abort_flag, status, code);
   };
-  float qs[kQuads][4];                                     // Qg rows: this lane's row of Qg S
+  float qs[kQuads][4];                                     // Qg rows: this lane's row of Qg S; W rows: its row of U, a chunk ahead
+  auto load_u = [&](int n) {
+    const int row = 32 * rb + mine;
+    const float* u = g_ut + (size_t)n * (L.ut_bytes / sizeof(float)) + (size_t)(row >> 2) * DV * 4 + (row & 3);
+#pragma unroll
+    for (int j = 0; j < kQuads; ++j) {
+      const int col0 = 4 * (quad0 + j);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) qs[j][c] = col0 < nv ? __ldg(u + (col0 + c) * 4) : 0.f;      // nv is a multiple of 4
+    }
+  };
+  if (!is_q && NC > 0) load_u(0);
   int wq_ahead = 0, kgt_ahead = 0;                         // last chunk whose copies were issued
   bool ok = true;
   for (int n = 0; n < NC; ++n) {
@@ -271,7 +276,6 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
     }
     // ---- rows of W S or Qg S
     ok = ok && wait_all(&bar_wq, ph, kWaitSimtWq);
-    ok = ok && wait_all(&bar_ut, ph, kWaitSimtUt);
 #pragma unroll
     for (int j0 = 0; j0 < kQuads; j0 += kG) {
       float2 acc[4][4 * kG];
@@ -290,15 +294,15 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
 #pragma unroll
           for (int c = 0; c < 4; ++c) qs[j0 + j][c] = v[c];
         } else {
-          const float* u = s.ut + ((row >> 2) * NVT + col0) * 4 + (row & 3);
 #pragma unroll
-          for (int c = 0; c < 4; ++c) s.Un[(col0 + c) * kChunk + row] = u[4 * c] - v[c];
+          for (int c = 0; c < 4; ++c) s.Un[(col0 + c) * kChunk + row] = qs[j0 + j][c] - v[c];
         }
       }
     }
+    if (!is_q && n + 1 < NC) load_u(n + 1);
     __syncthreads();                                       // Un complete; the state and W | Qg have been read
     if (wid == 0 && ok && n + 1 < NC) {
-      load_wq_ut(n + 1);
+      load_wq(n + 1);
       wq_ahead = n + 1;
     }
 
@@ -361,7 +365,7 @@ scan_simt_kernel(WsLayout L, WsPtrs P, const float* __restrict__ s0, TOut* __res
     }
   }
   if (wid == 0 && NC > 0) {                                // copies that no one waited for must land before the block ends
-    tc::mbar_drain(&bar_wq, wq_ahead & 1); tc::mbar_drain(&bar_ut, wq_ahead & 1);
+    tc::mbar_drain(&bar_wq, wq_ahead & 1);
     tc::mbar_drain(&bar_kgt, kgt_ahead & 1); tc::mbar_drain(&bar_aqk, kgt_ahead & 1);
   }
   if (sT != nullptr) {
