@@ -171,7 +171,9 @@ __device__ __forceinline__ void prep_simt_chunk(const TIn* __restrict__ q, const
     return add4(*reinterpret_cast<const float4*>(&Ch[(t >> 2) * LD + c]), add4(*reinterpret_cast<const float4*>(&Cl[(t >> 2) * LD + c]), a));
   };
 
-  // The two matrices: 120 tiles below the diagonal, then the 16 on it; eight lanes per tile share its channels.
+  // The two matrices: 120 tiles below the diagonal, then the 16 on it; eight lanes per tile share its channels. The loops are a
+  // chain of shared-memory loads and exponentials: two turns at a time 36.8 us against 37.8 for one and 37.1 for four (the
+  // kernel, float32, B = 2, S = 1000, 8 heads of 64).
   const int l8 = lane & 7;
   for (int grp = wid; grp < 34; grp += 8) {
     const int p = 4 * grp + (lane >> 3);
@@ -184,6 +186,7 @@ __device__ __forceinline__ void prep_simt_chunk(const TIn* __restrict__ q, const
       if (rt * (rt - 1) / 2 > p) --rt;
       if ((rt + 1) * rt / 2 <= p) ++rt;
       st = p - rt * (rt - 1) / 2;
+#pragma unroll 2
       for (int u = l8; u < DK / 2; u += 8) {
         const int o_r = 4 * rt * LD + 2 * u, o_s = 4 * st * LD + 2 * u;
         auto at2 = [&](const float* m, int off) { return *reinterpret_cast<const float2*>(m + off); };
@@ -216,6 +219,7 @@ __device__ __forceinline__ void prep_simt_chunk(const TIn* __restrict__ q, const
       }
     } else {
       rt = st = p - 120;
+#pragma unroll 2
       for (int u = l8; u < DK / 2; u += 8) {
         const int o_r = 4 * rt * LD + 2 * u;
         float2 kk[4];                                      // k_j with the decay up to row i
