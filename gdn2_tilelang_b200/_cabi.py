@@ -540,8 +540,12 @@ class NativeKernels:
         """True when ``gdn2_layer_front`` writes the new convolution cache from the kernel that reads the old one
         (its one-token form: 16-bit storage, DK = DV = 128, four taps, fewer than 8 tokens), so that for ONE token
         the new cache may be the old cache's own memory."""
+        return proj.shape[1] < 8 and NativeKernels._layer_front_is_one_kernel(proj, offsets, DK, DV, K)
+
+    @staticmethod
+    def _layer_front_is_one_kernel(proj, offsets, DK, DV, K) -> bool:
         return (proj.dtype in (torch.bfloat16, torch.float16) and DK == 128 and DV == 128 and K == 4
-                and proj.shape[1] < 8 and proj.shape[2] % 4 == 0 and all(o % 4 == 0 for o in offsets))
+                and proj.shape[2] % 4 == 0 and all(o % 4 == 0 for o in offsets))
 
     def layer_front(self, proj, offsets, conv_state, conv_weight, conv_bias, A_log, dt_bias, H, HK, DK, DV, K,
                     erase_scale, want_conv_state, conv_out=None):
@@ -575,7 +579,7 @@ class NativeKernels:
         with _on_device(dev):
             rc = self.lib.gdn2_layer_front(ctypes.byref(a), dtype_code(dt), self._stream(proj))
         _check(self.lib, rc, "gdn2_layer_front")
-        self.launches += 2 if (new_conv is not None and not fused_tail) else 1
+        self.launches += 2 if (new_conv is not None and not self._layer_front_is_one_kernel(proj, offsets, DK, DV, K)) else 1
         return q, k, v, g, b, w, new_conv
 
     def layer_step(self, x, state, conv_state, w_cat, conv_weight, conv_bias, A_log, dt_bias, norm_weight, o_weight, offsets, H, HK,

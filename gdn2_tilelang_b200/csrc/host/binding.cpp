@@ -199,8 +199,8 @@ std::optional<std::tuple<Tensor, Tensor, int64_t>> layer_stages(const Tensor& x,
   const int rc = gdn2_layer_back(m.o, proj.data_ptr(), l.norm_w.data_ptr(), normed.data_ptr(), p.B * p.S, l.H, l.DV,
                                  proj.size(2), l.offs[6], (float)l.eps, p.dtype, st);
   if (rc != GDN2_OK) throw std::runtime_error(std::string("gdn2_layer_back: ") + gdn2_status_string(rc));
-  // the front kernel writes the new convolution cache itself in its one-token form, else a second one does
-  bool fused = p.dtype != GDN2_F32 && l.DK == 128 && l.DV == 128 && l.K == 4 && p.S < 8 && a.NP % 4 == 0;
+  // the front kernel writes the new convolution cache itself in its 16-bit forms, else a second one does
+  bool fused = p.dtype != GDN2_F32 && l.DK == 128 && l.DV == 128 && l.K == 4 && a.NP % 4 == 0;
   for (int i = 0; i < 6; ++i) fused = fused && l.offs[i] % 4 == 0;
   return std::make_tuple(at::linear(normed, l.o_w), conv, int64_t(fused ? 2 : 3));
 }

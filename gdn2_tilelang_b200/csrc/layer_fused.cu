@@ -325,6 +325,19 @@ layer_front_prompt_kernel(gdn2_layer_front_args a) {
         bias[0] = make_float2(b4[0], b4[1]); bias[1] = make_float2(b4[2], b4[3]);
       }
     }
+    // the group of the last tokens also writes the new convolution cache of its channels: copies of the last three rows, which
+    // it holds anyway (a kernel of its own took 3.2 us by ncu, and a launch)
+    if (a.new_conv_state && t0 + TT >= S) {
+      T* tails = static_cast<T*>(a.new_conv_state) + ((size_t)b * CC + cch) * (K - 1);
+#pragma unroll
+      for (int r = 0; r < TT + K - 1; ++r) {
+        const int sidx = t0 + r - S;                         // row t0 - 3 + r is number sidx of rows S - 3 .. S - 1
+        if (sidx >= 0 && sidx < K - 1) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) tails[i * (K - 1) + sidx] = x[r].x[i];
+        }
+      }
+    }
     float2 win[K][2];                                        // the last four rows
     auto convert = [&](int r) {
       float y[4];
@@ -458,9 +471,10 @@ int launch_front_typed(const gdn2_layer_front_args& a, cudaStream_t st) {
       a.B * ((a.S + kPromptTokens - 1) / kPromptTokens) * (4 * a.HK + 2 * a.H) < (int64_t)1 << 31) {
     const int64_t items = a.B * ((a.S + kPromptTokens - 1) / kPromptTokens) * (4 * a.HK + 2 * a.H);   // a slot of some tokens per warp
     GDN2_CUDA_TRY(launch_chained(true, layer_front_prompt_kernel<T>, dim3((unsigned)((items + kWarps - 1) / kWarps)), 32 * kWarps, 0, st, a));
+    return GDN2_OK;                                          // both 16-bit forms write the new convolution cache themselves
   } else if (sizeof(T) == 2 && a.DK == 128 && a.DV == 128 && a.K == 4 && aligned) {
     GDN2_CUDA_TRY(launch_chained(true, layer_front_d128_kernel<T>, dim3((unsigned)((items + kWarps - 1) / kWarps)), 32 * kWarps, 0, st, a));
-    return GDN2_OK;                                          // this form writes the new convolution cache itself
+    return GDN2_OK;
   } else
     GDN2_CUDA_TRY(launch_chained(true, layer_front_kernel<T>, dim3((unsigned)((items + kWarps - 1) / kWarps)), 32 * kWarps, 0, st, a));
   if (a.K > 1 && a.new_conv_state) {
