@@ -284,7 +284,7 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
       // references: G after the first, third sub-block; a key of block 0 seen from block 1, a key of block 1 from the chunk's end
       const float2 ref = j2 ? ref3c : ref1c;
       const float2 gam_ref = ex2(ref);
-      const float2 kg_c = ex2(g_last - ref3c);                    // >= 2^-96, and <= 1
+      const float2 kg_c = ex2(g_last - ref3c) * make_float2(kValScale, kValScale);   // 2^-96 to 1, times the record's scale
       float2 run = run0;
       uint32_t kgx[4], kgy[4];                                    // fp16 pairs of KG for 8 tokens of each channel
       auto gate4 = [&](const Raw4& r, const float2* gq, int t0, int hi) {
@@ -309,7 +309,7 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
           const float2 gam = a * gam_ref;
           e4x[u] = tf32_rn(e.x * gam.x); e4y[u] = tf32_rn(e.y * gam.y);
           qgp[u] = pack_bf16x2_rn(scale * qf.x * gam.x, scale * qf.y * gam.y);
-          kx[u] = kn.x * kg_c.x * kValScale; ky[u] = kn.y * kg_c.y * kValScale;
+          kx[u] = kn.x * kg_c.x; ky[u] = kn.y * kg_c.y;
         }
         store_group(e4x, e4y, kx, ky, qgp, kgx, kgy, t0, hi);
       };
@@ -459,25 +459,31 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
     const uint32_t t_lo = tc::tmem_addr(tm, lq * 32, 8 * i0 * (i0 + 1));
     const uint32_t t_hi = tc::tmem_addr(tm, lq * 32, 8 * (i0 + 1) * (i0 + 2));
     float* tr = s.x.sol.tm + r * TM_STRIDE;
+    const float q_mul = scale * kValScale;
     __half* ag = reinterpret_cast<__half*>(P.aqk + (size_t)ch * (BS * BS * 2));   // fp16, 256 * Aqk
 #pragma unroll 1
     for (int cg = 2 * hf; cg < 2 * hf + 2; ++cg) {
-      float lo16[16], hi16[16], row[16];
-#pragma unroll
-      for (int x = 0; x < 16; ++x) { lo16[x] = 0.f; hi16[x] = 0.f; }
+      float row[16];
       if (fine) {
+        float lo16[16], hi16[16];
+#pragma unroll
+        for (int x = 0; x < 16; ++x) { lo16[x] = 0.f; hi16[x] = 0.f; }
         if (cg <= i0) tc::tmem_ld16(t_lo + 16 * cg, lo16);          // warp-uniform conditions
         if (cg <= i0 + 1) tc::tmem_ld16(t_hi + 16 * cg, hi16);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int x = 0; x < 16; ++x) row[x] = hi ? hi16[x] : lo16[x];
       } else if (cg <= i0 + 1) {                                    // the warp's rows are one block of 32 tokens
-        tc::tmem_ld16(tc::tmem_addr(tm, lq * 32, 16 * i0 + 16 * cg), lo16);
+        tc::tmem_ld16(tc::tmem_addr(tm, lq * 32, 16 * i0 + 16 * cg), row);
+        tc::tmem_ld_wait();
+      } else {
+#pragma unroll
+        for (int x = 0; x < 16; ++x) row[x] = 0.f;
       }
-      tc::tmem_ld_wait();
 #pragma unroll
       for (int x = 0; x < 16; ++x) {
         const int sc = 16 * cg + x;
-        const float val = fine && hi ? hi16[x] : lo16[x];
-        const bool keep = is_q ? (sc <= r) : (sc < r);
-        row[x] = keep ? (is_q ? val * scale : val) : 0.f;
+        row[x] = (is_q ? sc <= r : sc < r) ? row[x] : 0.f;
       }
       if (!is_q) {
 #pragma unroll
@@ -485,8 +491,8 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
           *reinterpret_cast<float4*>(tr + 16 * cg + 4 * m4) =
               make_float4(row[4 * m4], row[4 * m4 + 1], row[4 * m4 + 2], row[4 * m4 + 3]);
       } else {
-        *reinterpret_cast<uint4*>(ag + ((2 * cg) * BS + r) * 8) = tc::pack8_f16(&row[0], kValScale);
-        *reinterpret_cast<uint4*>(ag + ((2 * cg + 1) * BS + r) * 8) = tc::pack8_f16(&row[8], kValScale);
+        *reinterpret_cast<uint4*>(ag + ((2 * cg) * BS + r) * 8) = tc::pack8_f16(&row[0], q_mul);
+        *reinterpret_cast<uint4*>(ag + ((2 * cg + 1) * BS + r) * 8) = tc::pack8_f16(&row[8], q_mul);
       }
     }
     // (w*v)^T image: the 16 tokens x 2 channels of this thread
@@ -545,13 +551,14 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
     const int g8 = lane >> 2, t4 = lane & 3;
     auto T_at = [&](int bi, int bk, int r, int cidx) { return tmm[(16 * bi + r) * TM_STRIDE + 16 * bk + cidx]; };
     auto X_at = [&](int bi, int bk, int r, int cidx) { return aim[AI(16 * bi + r, 16 * bk + cidx)]; };
-    // acc[nt][..] += A(16x16) * B(16x16); A and B are read through (row, col) accessors
+    // acc[nt][..] += A(16x16) * B(16x16); A and B are read through (row, col) accessors. D, N and X are rounded to tf32 where
+    // they are stored, once, and not by every reader (with the read-back and scale factors above as lean, four prompts
+    // of 16037 tokens 1024 -> 1013 us a call)
     auto block_mma = [&](float (&acc)[2][4], auto a_at, auto b_at) {
 #pragma unroll
       for (int kt = 0; kt < 2; ++kt) {
-        const uint32_t a[4] = {__float_as_uint(tf32_rn(a_at(g8, 8 * kt + t4))), __float_as_uint(tf32_rn(a_at(g8 + 8, 8 * kt + t4))),
-                               __float_as_uint(tf32_rn(a_at(g8, 8 * kt + t4 + 4))),
-                               __float_as_uint(tf32_rn(a_at(g8 + 8, 8 * kt + t4 + 4)))};
+        const uint32_t a[4] = {__float_as_uint(a_at(g8, 8 * kt + t4)), __float_as_uint(a_at(g8 + 8, 8 * kt + t4)),
+                               __float_as_uint(a_at(g8, 8 * kt + t4 + 4)), __float_as_uint(a_at(g8 + 8, 8 * kt + t4 + 4))};
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
           const uint32_t b0 = __float_as_uint(tf32_rn(b_at(8 * kt + t4, 8 * nt + g8)));
@@ -574,8 +581,8 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) {
         float* d0 = tmm + (16 * bi + g8) * TM_STRIDE + 16 * bk + 8 * nt + 2 * t4;
-        d0[0] = acc[nt][0]; d0[1] = acc[nt][1];
-        d0[8 * TM_STRIDE] = acc[nt][2]; d0[8 * TM_STRIDE + 1] = acc[nt][3];
+        d0[0] = tf32_rn(acc[nt][0]); d0[1] = tf32_rn(acc[nt][1]);
+        d0[8 * TM_STRIDE] = tf32_rn(acc[nt][2]); d0[8 * TM_STRIDE + 1] = tf32_rn(acc[nt][3]);
       }
     }
     __syncthreads();
@@ -587,11 +594,10 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
       auto half_mma = [&](float (&acc)[4], auto a_at, auto b_at) {
 #pragma unroll
         for (int kt = 0; kt < 2; ++kt) {
-          const uint32_t a[4] = {__float_as_uint(tf32_rn(a_at(g8, 8 * kt + t4))), __float_as_uint(tf32_rn(a_at(g8 + 8, 8 * kt + t4))),
-                                 __float_as_uint(tf32_rn(a_at(g8, 8 * kt + t4 + 4))),
-                                 __float_as_uint(tf32_rn(a_at(g8 + 8, 8 * kt + t4 + 4)))};
-          const uint32_t b0 = __float_as_uint(tf32_rn(b_at(8 * kt + t4, 8 * nh + g8)));
-          const uint32_t b1 = __float_as_uint(tf32_rn(b_at(8 * kt + t4 + 4, 8 * nh + g8)));
+          const uint32_t a[4] = {__float_as_uint(a_at(g8, 8 * kt + t4)), __float_as_uint(a_at(g8 + 8, 8 * kt + t4)),
+                                 __float_as_uint(a_at(g8, 8 * kt + t4 + 4)), __float_as_uint(a_at(g8 + 8, 8 * kt + t4 + 4))};
+          const uint32_t b0 = __float_as_uint(b_at(8 * kt + t4, 8 * nh + g8));
+          const uint32_t b1 = __float_as_uint(b_at(8 * kt + t4 + 4, 8 * nh + g8));
           asm volatile(
               "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
               : "+f"(acc[0]), "+f"(acc[1]), "+f"(acc[2]), "+f"(acc[3])
