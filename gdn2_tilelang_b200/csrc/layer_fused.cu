@@ -5,12 +5,13 @@
 //          conv_size-1 columns when decoding), L2 normalisation of q and k per head, the decay
 //          g = -exp(A_log) * softplus(f + dt_bias), the gates b = erase_scale * sigmoid(.), w = sigmoid(.),
 //          -- q, k, b, g once per key head: the attention kernels index key heads, no repeated copies;
-//   tail:  the new convolution cache (the last conv_size-1 pre-convolution columns of q | k | v);
+//   tail:  the new convolution cache (the last conv_size-1 pre-convolution columns of q | k | v), written by the 16-bit front kernels
+//          for heads of 128 themselves;
 //   back:  per-head RMSNorm of the attention output times SiLU(o_gate).
 //
 // These replace the torch operator chains of _ShortConv, F.normalize, the gate expressions and
 // _GatedRMSNorm (gdn2/attention.py:186-229, 290-297, 323-340 of the reference project): about 25 launches
-// and as many round trips through HBM per call become three. All arithmetic is fp32 with one rounding to
+// and as many round trips through HBM per call become two or three. All arithmetic is fp32 with one rounding to
 // the storage type at the end. One warp per (token, kv head) in front, per (token, value head) in back.
 #include "common.cuh"
 #include "layer_math.cuh"
