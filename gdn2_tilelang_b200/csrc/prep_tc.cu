@@ -23,12 +23,9 @@
 //     tensor-core product as long as each half of every sub-block decays by less than 2^96 (every product
 //     2^(G_r - G_s), r >= s, is then formed from two factors inside bf16 range). A chunk that decays faster
 //     is flagged in the workspace and redone exactly by the SIMT family's kernel.
-//     Most chunks decay slowly enough for the same with blocks of 32 tokens, the reference between their two sub-blocks: no 16
-//     tokens by 2^96 or more. They take 3 key rows per two keys in place of 5, and 2 products in place of 4 (four prompts of
-//     16037 tokens, 16 heads: 1115 -> 1082 us a call); the others keep the sub-blocks of 16.
 //  2. MMA1 (bf16, M = 128: rows 0..63 = b*k rows, 64..127 = q rows, all scaled by their own ref):
-//     products A * B_i^T, B_i = key rows up to the end of block i scaled to ref_i; two with N = 32, 64, or, by sub-blocks, four
-//     with N = 16(i+1). Row block i of product i gives Tm (strictly lower) and Aqk (lower incl. diagonal, * scale).
+//     four products A * B_i^T, B_i = key rows s < 16(i+1) scaled to ref_i, N = 16(i+1).
+//     Row block i of product i gives Tm (strictly lower) and Aqk (lower incl. diagonal, * scale).
 //  3. (I + Tm)^-1 by 16x16 blocks: the four diagonal blocks by forward substitution in registers,
 //     the off-diagonal blocks from 16 small products on warp-level register fragments.
 //  4. MMA2 (tf32, transposed so channels are M): W^T = E^T * Ai^T, U^T = (w*v)^T * Ai^T.
@@ -62,7 +59,7 @@ struct PrepTcSmem {
   union {
     struct {
       __nv_bfloat16 a_own[16 * A_PAD * 8];   // A of MMA1: [dk/8][129][8]
-      __nv_bfloat16 bfam[16 * B_PAD * 8];    // B of MMA1: [dk/8][161][8], rows: B_0 0..15, B_1 16..47, B_2 48..95, B_3 96..159; blocks of 32: B_0 0..31, B_1 32..95
+      __nv_bfloat16 bfam[16 * B_PAD * 8];    // B of MMA1: [dk/8][161][8], rows: B_0 0..15, B_1 16..47, B_2 48..95, B_3 96..159
     } ops;
     struct {
       float tm[BS * TM_STRIDE];              // strictly lower Tm, row-major; N_ik = D_i T_ik overwrites its blocks
@@ -80,10 +77,6 @@ struct PrepTcSmem {
   int abort_flag;
 };
 
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
-}
-
 // 2^x by the hardware approximation alone (about 2 ulp; arguments here are differences of log2 decays,
 // results that underflow flush to zero, which is the right answer for a vanished decay)
 __device__ __forceinline__ float ex2(float x) {
@@ -92,9 +85,8 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
-// Two fp32 operations in one instruction on a register pair: the gating of blocks of 32 tokens has a fifth fewer instructions with
-// them and the same bits (four prompts of 16037 tokens, 16 heads 1075 -> 1046 us a call, two heads 180.2 -> 174.8). The sub-blocks
-// of 16 keep single ones: they did not gain (0.783 against 0.779 ms for the kernel).
+// Two fp32 operations in one instruction on a register pair, with the bits of two single ones: the decay's first sum, w * v and
+// the scaling of U. The gating keeps single ones: pairs did not gain there (0.783 against 0.779 ms for the kernel).
 __device__ __forceinline__ uint64_t bits2(float2 a) { return *reinterpret_cast<uint64_t*>(&a); }
 __device__ __forceinline__ float2 from_bits2(uint64_t r) { return *reinterpret_cast<float2*>(&r); }
 __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
@@ -105,11 +97,6 @@ __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
 __device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
   uint64_t r;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits2(a)), "l"(bits2(b)));
-  return from_bits2(r);
-}
-__device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits2(a)), "l"(bits2(b)));
   return from_bits2(r);
 }
 
@@ -220,8 +207,8 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
 
   // ---- 1a. G at the first row of every sub-block and at the last token; decay-span check.
   //          Each thread sums its own sub-block (two channels); the four meet through shared memory.
-  float2 ref0, ref1, ref2, ref3, ref1c, ref3c, g_last, run0;
-  bool bad = false, coarse_bad = false;
+  float2 ref0, ref1, ref2, ref3, g_last, run0;
+  bool bad = false;
   float2 gv[16];                                         // this thread's 16 decay values: read once, used again in step 1b
   const uint32_t* qp = reinterpret_cast<const uint32_t*>(q + row0 * D + soff) + cp;
   const uint32_t* kp = reinterpret_cast<const uint32_t*>(k + row0 * D + soff) + cp;
@@ -243,9 +230,6 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
     const float2 first = make_float2(gv[0].x * kLog2e, gv[0].y * kLog2e);
     bad = !((first.x - mid.x) <= kMaxSpanLog2) || !((first.y - mid.y) <= kMaxSpanLog2) ||
           !((mid.x - run.x) <= kMaxSpanLog2) || !((mid.y - run.y) <= kMaxSpanLog2);
-    // The same for blocks of 32 tokens with the reference between their two sub-blocks: a sub-block is half a span.
-    const float2 from = (sbk & 1) ? make_float2(0.f, 0.f) : first;
-    coarse_bad = !((from.x - run.x) <= kMaxSpanLog2) || !((from.y - run.y) <= kMaxSpanLog2);
     *reinterpret_cast<float2*>(&s.pre[sbk][0][c0]) = mid;
     *reinterpret_cast<float2*>(&s.pre[sbk][1][c0]) = run;
   }
@@ -267,13 +251,11 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
     const float2 p1 = t0_, p2 = t0_ + t1_, p3 = p2 + t2_;
     ref0 = f0; ref1 = p1 + f1; ref2 = p2 + f2; ref3 = p3 + f3;
     g_last = p3 + t3_;
-    ref1c = p1; ref3c = p3;
     run0 = pick4(sbk, make_float2(0.f, 0.f), p1, p2, p3);
   }
   if (wid == 0) tc::tmem_alloc(&s.tmem_base, kTmemCols);
   tc::tc_fence_before_sync();
-  // whether the chunk decays too fast for blocks of 32 tokens (uniform over the block)
-  const bool fine = __syncthreads_or(coarse_bad ? 1 : 0) != 0;
+  __syncthreads();
   tc::tc_fence_after_sync();
   const uint32_t tm = s.tmem_base;
 
@@ -285,9 +267,49 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
     uint32_t* a_own32 = reinterpret_cast<uint32_t*>(s.x.ops.a_own) + (cp >> 2) * A_PAD * 4 + (cp & 3);
     uint32_t* bfam32 = reinterpret_cast<uint32_t*>(s.x.ops.bfam) + (cp >> 2) * B_PAD * 4 + (cp & 3);
     char* kgt_g = P.kgt + (size_t)ch * (D * BS * 2) + c0 * 16;   // fp16 image [tok/8][128 dk][8]
-    // what a group of 4 tokens leaves behind besides the operands of MMA1
-    auto store_group = [&](const float (&e4x)[4], const float (&e4y)[4], const float (&kx)[4], const float (&ky)[4], const uint32_t (&qgp)[4],
-                           uint32_t (&kgx)[4], uint32_t (&kgy)[4], int t0, int hi) {
+    const int j = sbk;                                          // warp-uniform
+    const int off_j = 8 * j * (j + 1);                          // first row of B_j: 0, 16, 48, 96
+    const int off_j1 = 8 * (j + 1) * (j + 2), off_j2 = 8 * (j + 2) * (j + 3);
+    const float2 zero2 = make_float2(0.f, 0.f);
+    const float2 ref = pick4(j, ref0, ref1, ref2, ref3);
+    const float2 refn = pick4(j, ref1, ref2, ref3, zero2);      // ref of the next sub-block (unused for j = 3)
+    const float2 gam_ref = ex2(ref);
+    const float2 nx_ref = (j < 3) ? refn : g_last;             // keys of this sub-block, seen from the next one
+    const float2 kg_c = (j < 3) ? ex2(g_last - refn) : make_float2(1.f, 1.f);
+    const float2 cc_a = ex2(pick4(j, ref2, ref3, zero2, zero2) - refn);   // B_{j+2} relative to B_{j+1}
+    const float2 cc_b = ex2(ref3 - refn);                      // B_{j+3} relative to B_{j+1} (j = 0 only)
+    float2 run = run0;
+    uint32_t kgx[4], kgy[4];                                    // fp16 pairs of KG for 8 tokens of each channel
+
+    // one group: tokens t0 .. t0 + 3 of the chunk (t0 a multiple of 4); hi = second group of an 8-token pair
+    auto gate4 = [&](const Raw4& r, const float2* gq, int t0, int hi) {
+      float e4x[4], e4y[4], kx[4], ky[4];
+      uint32_t qgp[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int t = t0 + u;
+        run.x = fmaf(gq[u].x, kLog2e, run.x); run.y = fmaf(gq[u].y, kLog2e, run.y);
+        const float2 kf = bf16x2_bits_to_f32(r.k[u]), qf = bf16x2_bits_to_f32(r.q[u]);
+        const float2 a = ex2(run - ref);                      // both bounded by the half-span check
+        const float2 co = ex2(ref - run);
+        // 2^(refn - run) (2^(g_last - run) for j = 3), <= 1. Formed from its own exponent: the step from this
+        // sub-block's reference to the next one's is not covered by the span check, so a product of
+        // 2^(refn - ref) (which may flush to zero) and 2^(ref - run) (up to 2^96) would lose keys whose true
+        // factor is still a normal number.
+        const float2 nx = ex2(nx_ref - run);
+        const float2 e = bf16x2_bits_to_f32(r.b[u]) * kf;
+        a_own32[t * 4] = pack_bf16x2_rn(e.x * a.x, e.y * a.y);
+        a_own32[(BS + t) * 4] = pack_bf16x2_rn(qf.x * a.x, qf.y * a.y);
+        bfam32[(off_j + t) * 4] = pack_bf16x2_rn(kf.x * co.x, kf.y * co.y);
+        const float2 kn = kf * nx;
+        if (j < 3) bfam32[(off_j1 + t) * 4] = pack_bf16x2_rn(kn.x, kn.y);
+        if (j < 2) bfam32[(off_j2 + t) * 4] = pack_bf16x2_rn(kn.x * cc_a.x, kn.y * cc_a.y);
+        if (j < 1) bfam32[(96 + t) * 4] = pack_bf16x2_rn(kn.x * cc_b.x, kn.y * cc_b.y);
+        const float2 gam = a * gam_ref;
+        e4x[u] = tf32_rn(e.x * gam.x); e4y[u] = tf32_rn(e.y * gam.y);
+        qgp[u] = pack_bf16x2_rn(scale * qf.x * gam.x, scale * qf.y * gam.y);
+        kx[u] = kn.x * kg_c.x * kValScale; ky[u] = kn.y * kg_c.y * kValScale;
+      }
       const int tq = t0 >> 2;                                   // token quad index
       *reinterpret_cast<float4*>(&s.y.et[(tq * D + c0) * 4]) = make_float4(e4x[0], e4x[1], e4x[2], e4x[3]);
       *reinterpret_cast<float4*>(&s.y.et[(tq * D + c0 + 1) * 4]) = make_float4(e4y[0], e4y[1], e4y[2], e4y[3]);
@@ -300,111 +322,17 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
         *reinterpret_cast<uint4*>(dst + 16) = make_uint4(kgy[0], kgy[1], kgy[2], kgy[3]);
       }
     };
-    if (!fine) {
-      const int j2 = sbk >> 1;                                    // block of 32 tokens, warp-uniform
-      // references: G after the first, third sub-block; a key of block 0 seen from block 1, a key of block 1 from the chunk's end
-      const float2 ref = j2 ? ref3c : ref1c;
-      const float2 gam_ref = ex2(ref), nref = make_float2(-ref.x, -ref.y);
-      const float2 kg_c = ex2(g_last - ref3c) * make_float2(kValScale, kValScale);   // 2^-96 to 1, times the record's scale
-      float2 run = run0;
-      uint32_t kgx[4], kgy[4];                                    // fp16 pairs of KG for 8 tokens of each channel
-      auto gate4 = [&](const Raw4& r, const float2* gq, int t0, int hi) {
-        float e4x[4], e4y[4], kx[4], ky[4];
-        uint32_t qgp[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int t = t0 + u;
-          run = ffma2(gq[u], make_float2(kLog2e, kLog2e), run);
-          const float2 kf = bf16x2_bits_to_f32(r.k[u]), qf = bf16x2_bits_to_f32(r.q[u]);
-          const float2 d = fadd2(run, nref);
-          const float2 a = ex2(d), co = ex2(make_float2(-d.x, -d.y));   // both bounded by the span check
-          const float2 e = fmul2(bf16x2_bits_to_f32(r.b[u]), kf);
-          const float2 ea = fmul2(e, a), qa = fmul2(qf, a);
-          a_own32[t * 4] = pack_bf16x2_rn(ea.x, ea.y);
-          a_own32[(BS + t) * 4] = pack_bf16x2_rn(qa.x, qa.y);
-          float2 kn = fmul2(kf, co);
-          bfam32[(32 * j2 + t) * 4] = pack_bf16x2_rn(kn.x, kn.y);
-          if (j2 == 0) {
-            kn = fmul2(kf, ex2(ffma2(run, make_float2(-1.f, -1.f), ref3c)));                           // from its own exponent, see below
-            bfam32[(32 + t) * 4] = pack_bf16x2_rn(kn.x, kn.y);
-          }
-          const float2 gam = fmul2(a, gam_ref), eg = fmul2(e, gam);
-          e4x[u] = tf32_rn(eg.x); e4y[u] = tf32_rn(eg.y);
-          const float2 qg = fmul2(fmul2(make_float2(scale, scale), qf), gam), kg = fmul2(kn, kg_c);
-          qgp[u] = pack_bf16x2_rn(qg.x, qg.y);
-          kx[u] = kg.x; ky[u] = kg.y;
-        }
-        store_group(e4x, e4y, kx, ky, qgp, kgx, kgy, t0, hi);
-      };
-      Raw4 rb;
-      {
-        const int t0 = 16 * sbk;
-        load_raw4(rb, kp + 4 * pstride, qp + 4 * pstride, bp + 4 * pstride, pstride);
-        gate4(ra, gv, t0, 0);
-        load_raw4(ra, kp + 8 * pstride, qp + 8 * pstride, bp + 8 * pstride, pstride);
-        gate4(rb, gv + 4, t0 + 4, 1);
-        load_raw4(rb, kp + 12 * pstride, qp + 12 * pstride, bp + 12 * pstride, pstride);
-        gate4(ra, gv + 8, t0 + 8, 0);
-        gate4(rb, gv + 12, t0 + 12, 1);
-      }
-    } else {
-      const int j = sbk;                                          // warp-uniform
-      const int off_j = 8 * j * (j + 1);                          // first row of B_j: 0, 16, 48, 96
-      const int off_j1 = 8 * (j + 1) * (j + 2), off_j2 = 8 * (j + 2) * (j + 3);
-      const float2 zero2 = make_float2(0.f, 0.f);
-      const float2 ref = pick4(j, ref0, ref1, ref2, ref3);
-      const float2 refn = pick4(j, ref1, ref2, ref3, zero2);      // ref of the next sub-block (unused for j = 3)
-      const float2 gam_ref = ex2(ref);
-      const float2 nx_ref = (j < 3) ? refn : g_last;             // keys of this sub-block, seen from the next one
-      const float2 kg_c = (j < 3) ? ex2(g_last - refn) : make_float2(1.f, 1.f);
-      const float2 cc_a = ex2(pick4(j, ref2, ref3, zero2, zero2) - refn);   // B_{j+2} relative to B_{j+1}
-      const float2 cc_b = ex2(ref3 - refn);                      // B_{j+3} relative to B_{j+1} (j = 0 only)
-      float2 run = run0;
-      uint32_t kgx[4], kgy[4];                                    // fp16 pairs of KG for 8 tokens of each channel
 
-      // one group: tokens t0 .. t0 + 3 of the chunk (t0 a multiple of 4); hi = second group of an 8-token pair
-      auto gate4 = [&](const Raw4& r, const float2* gq, int t0, int hi) {
-        float e4x[4], e4y[4], kx[4], ky[4];
-        uint32_t qgp[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int t = t0 + u;
-          run.x = fmaf(gq[u].x, kLog2e, run.x); run.y = fmaf(gq[u].y, kLog2e, run.y);
-          const float2 kf = bf16x2_bits_to_f32(r.k[u]), qf = bf16x2_bits_to_f32(r.q[u]);
-          const float2 a = ex2(run - ref);                      // both bounded by the half-span check
-          const float2 co = ex2(ref - run);
-          // 2^(refn - run) (2^(g_last - run) for j = 3), <= 1. Formed from its own exponent: the step from this
-          // sub-block's reference to the next one's is not covered by the span check, so a product of
-          // 2^(refn - ref) (which may flush to zero) and 2^(ref - run) (up to 2^96) would lose keys whose true
-          // factor is still a normal number.
-          const float2 nx = ex2(nx_ref - run);
-          const float2 e = bf16x2_bits_to_f32(r.b[u]) * kf;
-          a_own32[t * 4] = pack_bf16x2_rn(e.x * a.x, e.y * a.y);
-          a_own32[(BS + t) * 4] = pack_bf16x2_rn(qf.x * a.x, qf.y * a.y);
-          bfam32[(off_j + t) * 4] = pack_bf16x2_rn(kf.x * co.x, kf.y * co.y);
-          const float2 kn = kf * nx;
-          if (j < 3) bfam32[(off_j1 + t) * 4] = pack_bf16x2_rn(kn.x, kn.y);
-          if (j < 2) bfam32[(off_j2 + t) * 4] = pack_bf16x2_rn(kn.x * cc_a.x, kn.y * cc_a.y);
-          if (j < 1) bfam32[(96 + t) * 4] = pack_bf16x2_rn(kn.x * cc_b.x, kn.y * cc_b.y);
-          const float2 gam = a * gam_ref;
-          e4x[u] = tf32_rn(e.x * gam.x); e4y[u] = tf32_rn(e.y * gam.y);
-          qgp[u] = pack_bf16x2_rn(scale * qf.x * gam.x, scale * qf.y * gam.y);
-          kx[u] = kn.x * kg_c.x * kValScale; ky[u] = kn.y * kg_c.y * kValScale;
-        }
-        store_group(e4x, e4y, kx, ky, qgp, kgx, kgy, t0, hi);
-      };
-
-      Raw4 rb;
-      {
-        const int t0 = 16 * sbk;
-        load_raw4(rb, kp + 4 * pstride, qp + 4 * pstride, bp + 4 * pstride, pstride);
-        gate4(ra, gv, t0, 0);
-        load_raw4(ra, kp + 8 * pstride, qp + 8 * pstride, bp + 8 * pstride, pstride);
-        gate4(rb, gv + 4, t0 + 4, 1);
-        load_raw4(rb, kp + 12 * pstride, qp + 12 * pstride, bp + 12 * pstride, pstride);
-        gate4(ra, gv + 8, t0 + 8, 0);
-        gate4(rb, gv + 12, t0 + 12, 1);
-      }
+    Raw4 rb;
+    {
+      const int t0 = 16 * sbk;
+      load_raw4(rb, kp + 4 * pstride, qp + 4 * pstride, bp + 4 * pstride, pstride);
+      gate4(ra, gv, t0, 0);
+      load_raw4(ra, kp + 8 * pstride, qp + 8 * pstride, bp + 8 * pstride, pstride);
+      gate4(rb, gv + 4, t0 + 4, 1);
+      load_raw4(rb, kp + 12 * pstride, qp + 12 * pstride, bp + 12 * pstride, pstride);
+      gate4(ra, gv + 8, t0 + 8, 0);
+      gate4(rb, gv + 12, t0 + 12, 1);
     }
     tc::tmem_st_wait();
     if (sbk == 3) *reinterpret_cast<float2*>(&P.gl[(size_t)ch * D + c0]) = ex2(g_last);
@@ -413,17 +341,10 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
   tc::tc_fence_before_sync();
   __syncthreads();
 
-  // ---- 2. MMA1: D_i[128 x 16(i+1)] at TMEM columns 0, 16, 48, 96 (blocks of 32: D_i[128 x 32(i+1)] at 0, 32)
-  //         The products are independent: warps 0..3 (0, 1) issue one each (converged, one elected
+  // ---- 2. MMA1: D_i[128 x 16(i+1)] at TMEM columns 0, 16, 48, 96
+  //         The four products are independent: warps 0..3 issue one each (converged, one elected
   //         lane) and commit it, so no warp falls far behind the others before the value-side loads.
-  if (!fine && wid < 2) {                                  // D_i[128 x 32(i+1)] at columns 0, 32
-    tc::tc_fence_after_sync();
-    tc::mma_bf16_ktile_warp(tc::tmem_addr(tm, 0, 32 * wid), tc::smem_u32(s.x.ops.a_own), A_PAD,
-                            tc::smem_u32(s.x.ops.bfam) + 32 * wid * 16, B_PAD, D, tc::instr_desc(1, 128, 32 * (wid + 1)));
-    tc::mma_commit_warp(&s.bar_m1);
-  } else if (!fine && wid < 4) {
-    if (lane == 0) mbar_arrive(&s.bar_m1);                 // the barrier counts four products
-  } else if (wid < 4) {
+  if (wid < 4) {
     tc::tc_fence_after_sync();
     const int i = wid;
     const int off = 8 * i * (i + 1);
@@ -486,27 +407,17 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
     __half* ag = reinterpret_cast<__half*>(P.aqk + (size_t)ch * (BS * BS * 2));   // fp16, 256 * Aqk
 #pragma unroll 1
     for (int cg = 2 * hf; cg < 2 * hf + 2; ++cg) {
-      float row[16];
-      if (fine) {
-        float lo16[16], hi16[16];
+      float lo16[16], hi16[16], row[16];
 #pragma unroll
-        for (int x = 0; x < 16; ++x) { lo16[x] = 0.f; hi16[x] = 0.f; }
-        if (cg <= i0) tc::tmem_ld16(t_lo + 16 * cg, lo16);          // warp-uniform conditions
-        if (cg <= i0 + 1) tc::tmem_ld16(t_hi + 16 * cg, hi16);
-        tc::tmem_ld_wait();
-#pragma unroll
-        for (int x = 0; x < 16; ++x) row[x] = hi ? hi16[x] : lo16[x];
-      } else if (cg <= i0 + 1) {                                    // the warp's rows are one block of 32 tokens
-        tc::tmem_ld16(tc::tmem_addr(tm, lq * 32, 16 * i0 + 16 * cg), row);
-        tc::tmem_ld_wait();
-      } else {
-#pragma unroll
-        for (int x = 0; x < 16; ++x) row[x] = 0.f;
-      }
+      for (int x = 0; x < 16; ++x) { lo16[x] = 0.f; hi16[x] = 0.f; }
+      if (cg <= i0) tc::tmem_ld16(t_lo + 16 * cg, lo16);          // warp-uniform conditions
+      if (cg <= i0 + 1) tc::tmem_ld16(t_hi + 16 * cg, hi16);
+      tc::tmem_ld_wait();
 #pragma unroll
       for (int x = 0; x < 16; ++x) {
         const int sc = 16 * cg + x;
-        row[x] = (is_q ? sc <= r : sc < r) ? row[x] : 0.f;
+        const float val = hi ? hi16[x] : lo16[x];
+        row[x] = (is_q ? sc <= r : sc < r) ? val : 0.f;
       }
       if (!is_q) {
 #pragma unroll
@@ -576,8 +487,7 @@ prep_tc_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restr
     auto T_at = [&](int bi, int bk, int r, int cidx) { return tmm[(16 * bi + r) * TM_STRIDE + 16 * bk + cidx]; };
     auto X_at = [&](int bi, int bk, int r, int cidx) { return aim[AI(16 * bi + r, 16 * bk + cidx)]; };
     // acc[nt][..] += A(16x16) * B(16x16); A and B are read through (row, col) accessors. D, N and X are rounded to tf32 where
-    // they are stored, once, and not by every reader (with the read-back and scale factors above as lean, four prompts
-    // of 16037 tokens 1024 -> 1013 us a call)
+    // they are stored, once, and not by every reader (four prompts of 16037 tokens 1024 -> 1013 us a call).
     auto block_mma = [&](float (&acc)[2][4], auto a_at, auto b_at) {
 #pragma unroll
       for (int kt = 0; kt < 2; ++kt) {

@@ -1,6 +1,6 @@
-"""The chunk-local stage's two factorisations and its exact redo, on both sides of the lines between them: a chunk goes in blocks of
-32 tokens while no 16 of them decay by 2^96 in any channel, in sub-blocks of 16 while no 8 do, else to the exact kernel. One
-channel over the line is enough, and chunks of one launch take different ways."""
+"""The chunk-local stage's factorisation by sub-blocks of 16 tokens and its exact redo, on both sides of the line between them: a chunk
+goes by sub-blocks while no 8 tokens decay by 2^96 in any channel, else to the exact kernel. One channel over the line is enough, and
+chunks of one launch take different ways. The gates around -4 a token, 2^96 in 16 tokens, are well inside."""
 
 from __future__ import annotations
 
@@ -17,7 +17,7 @@ DEV = "cuda"
 
 
 @pytest.mark.parametrize("H,HK", [(2, 2), (4, 2)])
-@pytest.mark.parametrize("gate", [-3.9, -4.1, -4.3, -8.1, -8.4, -12.0])      # 2^96 lies at 66.5: -4.16 and -8.3 a token
+@pytest.mark.parametrize("gate", [-3.9, -4.1, -4.3, -8.1, -8.4, -12.0])      # 2^96 lies at 66.5: -8.3 a token over 8
 @pytest.mark.parametrize("where", ["all", "one_channel", "second_chunk", "half_block"])
 def test_decays_around_the_lines(gate, where, H, HK):
     B, S, D = 1, 192, 128
