@@ -209,14 +209,15 @@ class GatedDeltaNet2(nn.Module):
         key = (host.parameter_key(params) if host is not None
                else tuple((p.data_ptr(), p._version, p.dtype) for p in params))
         if getattr(self, "_fused_key", None) != key:
-            w_cat = torch.cat([m.weight for m in lin], 0).contiguous()
-            sizes = [m.weight.shape[0] for m in lin]
-            offs = [sum(sizes[:i]) for i in range(len(sizes))]
-            cw = cb = None
-            if convs:
-                cw = torch.cat([c.weight.reshape(c.weight.shape[0], -1) for c in convs], 0).contiguous()
-                if all(c.bias is not None for c in convs):
-                    cb = torch.cat([c.bias for c in convs], 0).contiguous()
+            with torch.no_grad():                          # kept on the module: without a graph, whoever calls first
+                w_cat = torch.cat([m.weight for m in lin], 0).contiguous()
+                sizes = [m.weight.shape[0] for m in lin]
+                offs = [sum(sizes[:i]) for i in range(len(sizes))]
+                cw = cb = None
+                if convs:
+                    cw = torch.cat([c.weight.reshape(c.weight.shape[0], -1) for c in convs], 0).contiguous()
+                    if all(c.bias is not None for c in convs):
+                        cb = torch.cat([c.bias for c in convs], 0).contiguous()
             self._fused_key, self._fused = key, (w_cat, offs, cw, cb)
         return self._fused
 
@@ -389,12 +390,13 @@ class GatedDeltaNet2(nn.Module):
     def step(self, hidden_states, cache: GDN2Cache):
         """Decode one token ``[B, hidden]``."""
         x = hidden_states.unsqueeze(1)
-        if "decode" not in self.__dict__ and type(self).decode is _DECODE:   # (what it does first, without its no-grad region)
+        if "decode" not in self.__dict__ and type(self).decode is _DECODE:   # what it does first; a native call builds no graph
             out = self._decode_plain(x, cache)
             if out is not None:
                 return out[:, 0], cache
-        out, cache = self.decode(x, cache)
-        return out[:, 0], cache
+        with torch.no_grad():                              # (a replaced decode may have no such region of its own)
+            out, cache = self.decode(x, cache)
+            return out[:, 0], cache
 
     def init_cache(self, batch_size: int, device=None, dtype=torch.float32) -> GDN2Cache:
         """Empty cache: float32 recurrent state, conv tail in the layer's parameter dtype."""
