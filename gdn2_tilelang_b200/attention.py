@@ -291,7 +291,7 @@ class GatedDeltaNet2(nn.Module):
 
     def _plain_call(self, cache, call, x, *rest):
         """``call`` with the layer's tensors and sizes, or ``None`` where something about the layer or the cache needs the general
-        path (a subclass, hooks, replaced methods, a missing convolution cache): whatever would have run when ``o_proj`` is
+        path (a subclass, hooks, replaced methods or parameters, a missing convolution cache): whatever would have run when ``o_proj`` is
         called as a module still runs."""
         if call is None or type(self) is not GatedDeltaNet2 or cache.conv_state is None:
             return None
@@ -301,9 +301,11 @@ class GatedDeltaNet2(nn.Module):
                 or "forward" in o_proj.__dict__ or _has_any_global_hook() or not _STAGES.isdisjoint(self.__dict__)
                 or any(m[n]._parameters.get("bias") is not None for n in _PROJECTIONS)):
             return None
+        A_log, dt_bias = self._parameters.get("A_log"), self._parameters.get("dt_bias")
+        if A_log is None or dt_bias is None:               # tensors set in their place: computed by the program
+            return None
         w_cat, offs, cw, cb = self._fused_tables()
-        own = self._parameters
-        return call(x, cache.recurrent_state, cache.conv_state, w_cat, cw, cb, own["A_log"], own["dt_bias"],
+        return call(x, cache.recurrent_state, cache.conv_state, w_cat, cw, cb, A_log, dt_bias,
                     m["o_norm"].weight, o_proj.weight, offs, self.num_heads, self.num_kv_heads, self.head_dim_k,
                     self.head_dim_v, self.cfg.conv_size, self.erase_scale, m["o_norm"].eps, self.scale, *rest)
 

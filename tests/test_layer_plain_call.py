@@ -79,3 +79,18 @@ def test_a_customised_output_projection_runs(layer, customise):
         undo()
     assert host.calls == 1
     torch.testing.assert_close(out, 2 * plain)
+
+
+def test_parameters_replaced_by_tensors(layer):
+    """A program that computes a decay parameter and sets the tensor in the parameter's place takes the general path."""
+    net, host = layer
+    x = torch.randn(2, 1, 32)
+    plain = net.decode(x, net.init_cache(2))[0]
+    for name in ("A_log", "dt_bias"):
+        value = getattr(net, name).detach().clone()
+        delattr(net, name)
+        setattr(net, name, value)
+        for call in (net.decode, net.prefill):
+            torch.testing.assert_close(call(x, net.init_cache(2))[0], plain)
+        torch.testing.assert_close(net.step(x[:, 0], net.init_cache(2))[0], plain[:, 0])
+    assert host.calls == 1
