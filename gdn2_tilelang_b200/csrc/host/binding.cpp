@@ -179,7 +179,7 @@ std::optional<std::tuple<Tensor, Tensor, int64_t>> layer_stages(const Tensor& x,
   const int64_t esz = p.dtype == GDN2_F32 ? 4 : 2, tokens = p.B * p.S;
   auto part = [](int64_t bytes) { return (bytes + 255) / 256 * 256; };
   const int64_t key = part(tokens * l.HK * l.DK * esz), decay = part(tokens * l.HK * l.DK * 4), value = part(tokens * l.H * l.DV * esz);
-  Tensor mid = at::empty({3 * key + decay + 3 * value}, opt.dtype(at::kByte)), normed = at::empty({p.B, p.S, l.H * l.DV}, opt);
+  Tensor mid = at::empty({3 * key + decay + 3 * value}, opt.dtype(at::kByte));
   Tensor conv = at::empty({p.B, l.CC(), l.K - 1}, opt);
   char* at_ = static_cast<char*>(mid.data_ptr());
   auto take = [&](int64_t bytes) { char* r = at_; at_ += bytes; return r; };
@@ -196,6 +196,7 @@ std::optional<std::tuple<Tensor, Tensor, int64_t>> layer_stages(const Tensor& x,
   a.off_q = l.offs[0]; a.off_k = l.offs[1]; a.off_v = l.offs[2]; a.off_b = l.offs[3]; a.off_w = l.offs[4]; a.off_f = l.offs[5];
   a.erase_scale = (float)l.erase_scale;
   if (gdn2_layer_front(&a, p.dtype, st) != GDN2_OK || !attend(m)) return std::nullopt;
+  Tensor normed = at::empty({p.B, p.S, l.H * l.DV}, opt);   // now, where the scan's workspace was
   const int rc = gdn2_layer_back(m.o, proj.data_ptr(), l.norm_w.data_ptr(), normed.data_ptr(), p.B * p.S, l.H, l.DV,
                                  proj.size(2), l.offs[6], (float)l.eps, p.dtype, st);
   if (rc != GDN2_OK) throw std::runtime_error(std::string("gdn2_layer_back: ") + gdn2_status_string(rc));
