@@ -253,12 +253,6 @@ cudaError_t ensure_dynamic_smem(const void* kernel, size_t bytes);
 int launch_decode(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
                   float* state, void* o, int B, int n, int H, int HK, int DK, int DV, int64_t in_bs, int64_t o_bs,
                   float scale, int dtype, bool chained, cudaStream_t st);
-// decode_cols.cu: a tile spread over blocks by value columns (DK = DV = 128); whether that form is taken
-bool decode_cols_wins(int64_t ntiles, int n, bool tail);
-template <typename T, typename Seqs>
-int launch_decode_cols(const T* q, const T* k, const T* v, const float* g, const T* b, const T* w, float* state, T* o,
-                       int ntiles, int n, int H, int HK, int64_t in_bs, int64_t o_bs, float scale, const Seqs& seqs, bool chained,
-                       cudaStream_t st);
 int launch_prep_simt(const void* q, const void* k, const void* v, const float* g, const void* b, const void* w,
                      const WsLayout& L, const WsPtrs& P, int B, int S, int H, int HK, int64_t in_bs, float scale,
                      int dtype, bool only_flagged, cudaStream_t st);

@@ -230,9 +230,7 @@ int launch_typed(const void* q, const void* k, const void* v, const float* g, co
   const T* tq = static_cast<const T*>(q); const T* tk = static_cast<const T*>(k);
   const T* tv = static_cast<const T*>(v); const T* tb = static_cast<const T*>(b);
   const T* tw = static_cast<const T*>(w); T* to = static_cast<T*>(o);
-  if (DK == 128 && DV == 128 && decode_cols_wins((int64_t)B * H, n, !chained)) {
-    return launch_decode_cols<T, OneLength>(tq, tk, tv, g, tb, tw, state, to, B * H, n, H, HK, in_bs, o_bs, scale, OneLength{}, chained, st);
-  } else if (DK == 128 && DV == 128 && (n >= kBlockedMinTokens || (n > 1 && B * H > device_sm_count()))) {
+  if (DK == 128 && DV == 128 && (n >= kBlockedMinTokens || (n > 1 && B * H > device_sm_count()))) {
     return launch_decode_blocked<T>(tq, tk, tv, g, tb, tw, state, to, B, n, H, HK, in_bs, o_bs, scale, chained, st);
   } else if (DK == 128 && DV == 128) {
     GDN2_CUDA_TRY(launch_chained(chained, decode_square_kernel<T, 128>, dim3(B * H), 128, 0, st, tq, tk, tv, g, tb, tw, state, to, n, H, HK, in_bs, o_bs, scale));

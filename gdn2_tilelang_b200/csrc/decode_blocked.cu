@@ -596,7 +596,7 @@ int launch_decode_blocked(const T* q, const T* k, const T* v, const float* g, co
   // token by token for n = 2 and 3): n = 2 101 -> 88 / 12.9 -> 12.8, n = 3 121 -> 90 / 14.8 -> 14.1, n = 4 113 -> 91 / 18.6 -> 14.3,
   // n = 5 114 -> 97 / 18.9 -> 16.6, n = 12 213 -> 171 / 30.1 -> 25.4; steps of 6 for n = 16 would take 251 / 34.3 in place of 214 / 30.3.
   // A prompt's ragged tail (not chained) takes steps of 8 however short it is: in a packed batch the tails of all lengths share a
-  // launch, and the others' lengths do not change the bits of one.
+  // launch, and a sequence has the same bits there and alone.
   if (!chained) return launch(decode_blocked_kernel<T, OneLength, 8>, sizeof(BlockedSmem<8>) + 128);
   if (n <= 2) return launch(decode_blocked_kernel<T, OneLength, 2>, sizeof(BlockedSmem<2>) + 128);
   if (n <= 4) return launch(decode_blocked_kernel<T, OneLength, 4>, sizeof(BlockedSmem<4>) + 128);
@@ -608,9 +608,6 @@ int launch_decode_packed_tails(const void* q, const void* k, const void* v, cons
                                float* state, void* o, const PackedSeqs& seqs, int H, int HK, float scale, cudaStream_t st) {
   using T = __nv_bfloat16;
   const size_t smem = sizeof(BlockedSmem<8>) + 128;
-  if (decode_cols_wins((int64_t)seqs.n * H, 0, true))
-    return launch_decode_cols<T, PackedSeqs>(static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v), g, static_cast<const T*>(b),
-                                             static_cast<const T*>(w), state, static_cast<T*>(o), seqs.n * H, 0, H, HK, 0, 0, scale, seqs, false, st);
   auto kern = decode_blocked_kernel<T, PackedSeqs, 8>;
   GDN2_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem));
   const int ntiles = seqs.n * H, sms = device_sm_count();
