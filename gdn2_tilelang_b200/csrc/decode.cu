@@ -21,7 +21,7 @@
 
 namespace gdn2 {
 
-// decode_blocked.cu: blocks of 2 to 8 tokens without a per-token dependent sweep (DK = DV = 128)
+// decode_blocked.cu: blocks of 4 to 8 tokens without a per-token dependent sweep (DK = DV = 128)
 template <typename T>
 int launch_decode_blocked(const T* q, const T* k, const T* v, const float* g, const T* b, const T* w, float* state,
                           T* o, int B, int n, int H, int HK, int64_t in_bs, int64_t o_bs, float scale, bool chained,
@@ -29,9 +29,11 @@ int launch_decode_blocked(const T* q, const T* k, const T* v, const float* g, co
 
 namespace {
 
-// From here on the blocked form wins over the token-by-token sweeps whatever the number of tiles; for two and three tokens it
-// wins where a block has more than one tile to walk (bf16, 16 heads, us: n = 3, 8 conversations 7.4 here and 8.3 there, 16 of
-// them 13.0 and 11.2, 256 of them 121 and 90; n = 2, 256 of them 101 and 88).
+// From here on the blocked form wins over the token-by-token sweeps whatever the number of tiles (bf16, 16 heads, n = 4, us: 8
+// conversations 7.2 here and 5.9 there, 256 of them 129 and 91). Two and three tokens stay here although steps of 2 and 4 would be
+// faster for many tiles (256 conversations: n = 2 95 and 88, n = 3 107 and 89; 8 of them 5.6 and 5.9, 7.5 and 5.9): a token then has the
+// same bits in a draft of up to three as in single steps, whatever else is decoded with it, and the state is no further from 64 bits
+// than single steps leave it (n = 2 5.5e-8 here, 6.2e-8 there).
 constexpr int kBlockedMinTokens = 4;
 constexpr int kTokBatch = 8;   // token vectors staged in shared memory per barrier round
 
@@ -230,7 +232,7 @@ int launch_typed(const void* q, const void* k, const void* v, const float* g, co
   const T* tq = static_cast<const T*>(q); const T* tk = static_cast<const T*>(k);
   const T* tv = static_cast<const T*>(v); const T* tb = static_cast<const T*>(b);
   const T* tw = static_cast<const T*>(w); T* to = static_cast<T*>(o);
-  if (DK == 128 && DV == 128 && (n >= kBlockedMinTokens || (n > 1 && B * H > device_sm_count()))) {
+  if (DK == 128 && DV == 128 && n >= kBlockedMinTokens) {
     return launch_decode_blocked<T>(tq, tk, tv, g, tb, tw, state, to, B, n, H, HK, in_bs, o_bs, scale, chained, st);
   } else if (DK == 128 && DV == 128) {
     GDN2_CUDA_TRY(launch_chained(chained, decode_square_kernel<T, 128>, dim3(B * H), 128, 0, st, tq, tk, tv, g, tb, tw, state, to, n, H, HK, in_bs, o_bs, scale));

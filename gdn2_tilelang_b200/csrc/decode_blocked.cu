@@ -1,6 +1,6 @@
 // Recurrent decode of several tokens at once, DK = DV = 128: the n-token recurrence of
-// decode_multi_kernel (gdn2/inference.py:199-303 of the reference project) evaluated in blocks of NB = 2, 4, 6
-// or 8 tokens without a per-token dependent sweep over the state.
+// decode_multi_kernel (gdn2/inference.py:199-303 of the reference project) evaluated in blocks of NB = 4, 6 or
+// 8 tokens without a per-token dependent sweep over the state.
 //
 // With A_t = exp(g_1 + .. + g_t) per key channel (A_t / A_s <= 1 for s <= t, so nothing can overflow):
 //     u_t = w_t*v_t - (b_t*k_t*A_t)^T S_0 - sum_{s<t} Akk[t,s] u_s      Akk[t,s] = sum_c b_t k_t k_s A_t/A_s
@@ -146,7 +146,7 @@ decode_blocked_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
                       float* __restrict__ state, T* __restrict__ o, int ntiles, int n, int H, int HK, int64_t in_bs,
                       int64_t o_bs, float scale, uint32_t* status, const __grid_constant__ Seqs seqs) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  static_assert(NB % 2 == 0 && NB >= 2 && NB <= 8, "products are paired, pair matrices have eight columns");
+  static_assert(NB % 2 == 0 && NB >= 4 && NB <= 8, "products are paired, pair matrices have eight columns");
   using Smem = BlockedSmem<NB>;
   Smem& s = *reinterpret_cast<Smem*>(smem_raw);
   const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
@@ -592,13 +592,13 @@ int launch_decode_blocked(const T* q, const T* k, const T* v, const float* g, co
     return GDN2_OK;
   };
   // Tokens per step: padding tokens cost what real ones do, so the fewest that n needs; in several steps 6 or 8, whichever takes
-  // less, a step of 6 being about four fifths of one of 8. bf16, 16 heads, 256 / 24 conversations, us (steps of 8 before, and
-  // token by token for n = 2 and 3): n = 2 101 -> 88 / 12.9 -> 12.8, n = 3 121 -> 90 / 14.8 -> 14.1, n = 4 113 -> 91 / 18.6 -> 14.3,
-  // n = 5 114 -> 97 / 18.9 -> 16.6, n = 12 213 -> 171 / 30.1 -> 25.4; steps of 6 for n = 16 would take 251 / 34.3 in place of 214 / 30.3.
-  // A prompt's ragged tail (not chained) takes steps of 8 however short it is: in a packed batch the tails of all lengths share a
-  // launch, and a sequence has the same bits there and alone.
+  // less, a step of 6 being about four fifths of one of 8. bf16, 16 heads, 256 / 24 conversations, us (steps of 8 before): n = 4
+  // 113 -> 91 / 18.6 -> 14.3, n = 5 114 -> 97 / 18.9 -> 16.6, n = 12 213 -> 171 / 30.1 -> 25.4; steps of 6 for n = 16 would take 251 / 34.3
+  // in place of 214 / 30.3.
+  // A prompt's ragged tail of four or more tokens (not chained) takes steps of 8 whatever its length, as the packed launch does for
+  // the tails of all lengths: a sequence has the same bits there and alone. (Tails of one to three tokens are swept token by token when
+  // alone, by this kernel when packed.)
   if (!chained) return launch(decode_blocked_kernel<T, OneLength, 8>, sizeof(BlockedSmem<8>) + 128);
-  if (n <= 2) return launch(decode_blocked_kernel<T, OneLength, 2>, sizeof(BlockedSmem<2>) + 128);
   if (n <= 4) return launch(decode_blocked_kernel<T, OneLength, 4>, sizeof(BlockedSmem<4>) + 128);
   if ((n + 5) / 6 * 4 < (n + 7) / 8 * 5) return launch(decode_blocked_kernel<T, OneLength, 6>, sizeof(BlockedSmem<6>) + 128);
   return launch(decode_blocked_kernel<T, OneLength, 8>, sizeof(BlockedSmem<8>) + 128);

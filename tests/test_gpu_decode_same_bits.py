@@ -54,3 +54,18 @@ def test_a_prompt_alone_equals_the_same_in_a_batch_and_packed():
     for i in (0, B - 1):
         o1, s1 = gdn2.gdn2_prefill(*(t[i:i + 1] for t in ins), s0[i:i + 1])
         assert torch.equal(o1, o[i:i + 1]) and torch.equal(s1, s[i:i + 1])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("call", [gdn2.gdn2_decode, gdn2.gdn2_prefill])
+@pytest.mark.parametrize("n", [2, 3])
+def test_two_and_three_tokens_equal_single_steps(n, call, dtype):
+    """Also where they are more tiles than the GPU has SMs: they are swept token by token like a single one."""
+    B, H, HK = 24, 16, 8
+    ins, s0 = _inputs(B, n, H, HK, dtype, n)
+    s, single = s0.clone(), s0.clone()
+    res = call(*ins, s)
+    o = res if call is gdn2.gdn2_decode else res[0]
+    want = torch.cat([gdn2.gdn2_decode(*(t[:, i:i + 1].contiguous() for t in ins), single) for i in range(n)], 1)
+    _cabi.kernels().check_device_status()
+    assert torch.equal(o, want) and torch.equal(s, single)

@@ -1,5 +1,5 @@
-"""The blocked decode's steps of 2, 4, 6 and 8 tokens: every number of tokens around them, full and padded last steps, with more
-(sequence, head) tiles than the GPU has SMs, so that a block walks two or three of them."""
+"""The blocked decode's steps of 4, 6 and 8 tokens: every number of tokens around them, full and padded last steps, with more (sequence,
+head) tiles than the GPU has SMs, so that a block walks two or three of them; and the token-by-token sweeps of 2 and 3 there."""
 
 from __future__ import annotations
 
