@@ -167,22 +167,20 @@ layer_step_front_kernel(gdn2_layer_step_args a, StepBuffers buf) {
   const bool conv = kind == kQ || kind == kK || kind == kV;
   const int cch = (kind == kQ ? 0 : kind == kK ? HK * D : 2 * HK * D) + head * D + c;
   float wt[4][4], bias[4] = {0.f, 0.f, 0.f, 0.f}, old[12];             // old: [channel][last three columns], contiguous
-  auto load_columns = [&](int m) {
-    const T* cs = static_cast<const T*>(a.conv_state) + ((size_t)m * CC + cch) * 3;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) load4(cs + 4 * i, *reinterpret_cast<float(*)[4]>(&old[4 * i]));
-  };
-  const int m_first = rank + 2 * wid;
-  if (conv && m_first < M) {                                           // in flight across the meeting of the two halves
+  static_assert(kMaxRows <= 2 * kWarps, "a token for every warp of the two blocks");
+  const int m = rank + 2 * wid;
+  if (conv && m < M) {                                                 // in flight across the meeting of the two halves
 #pragma unroll
     for (int i = 0; i < 4; ++i) load4(static_cast<const T*>(a.conv_weight) + (size_t)(cch + i) * 4, wt[i]);
     if (a.conv_bias) load4(static_cast<const T*>(a.conv_bias) + cch, bias);
-    load_columns(m_first);
+    const T* cs = static_cast<const T*>(a.conv_state) + ((size_t)m * CC + cch) * 3;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) load4(cs + 4 * i, *reinterpret_cast<float(*)[4]>(&old[4 * i]));
   }
   cluster.sync();
   const float* half0 = cluster.map_shared_rank(red, 0);
   const float* half1 = cluster.map_shared_rank(red, 1);
-  for (int m = m_first; m < M; m += 2 * kWarps) {
+  if (m < M) {
     float p[4];                                                        // rounded to T as a product of its own would be
     {
       const float4 x0 = *reinterpret_cast<const float4*>(half0 + m * kRedStride + c);
@@ -193,7 +191,6 @@ layer_step_front_kernel(gdn2_layer_step_args a, StepBuffers buf) {
     }
     const size_t rk = ((size_t)m * HK + head) * D + c, rv = ((size_t)m * H + head) * D + c;   // of a key / value head's row
     if (conv) {
-      if (m != m_first) load_columns(m);
       float y[4], nw[12];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
