@@ -37,24 +37,6 @@ namespace {
 constexpr int kBlockedMinTokens = 4;
 constexpr int kTokBatch = 8;   // token vectors staged in shared memory per barrier round
 
-// packed fp32 pairs (Blackwell): two FMAs / multiplies per instruction on 64-bit register pairs
-__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(*reinterpret_cast<unsigned long long*>(&d))
-      : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
-        "l"(*reinterpret_cast<unsigned long long*>(&c)));
-  return d;
-}
-__device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
-  float2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;"
-      : "=l"(*reinterpret_cast<unsigned long long*>(&d))
-      : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
-  return d;
-}
-
-
 template <typename T, int D>
 __global__ void __launch_bounds__(D, D == 128 ? 3 : 10)
 decode_square_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,

@@ -231,15 +231,6 @@ layer_front_d128_kernel(gdn2_layer_front_args a) {
   }
 }
 
-__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(*reinterpret_cast<unsigned long long*>(&d))
-      : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
-        "l"(*reinterpret_cast<unsigned long long*>(&c)));
-  return d;
-}
-
 constexpr int kPromptTokens = 8;
 
 // The same for prompts, cut finer: one warp per (head-wide slot, kPromptTokens consecutive tokens). A token's slots are its

@@ -104,16 +104,6 @@ __device__ __forceinline__ void un_and_output(OutputSmem& s, int DK, int DV, int
   }
 }
 
-// packed fp32 pairs: two FMAs per instruction
-__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(*reinterpret_cast<unsigned long long*>(&d))
-      : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
-        "l"(*reinterpret_cast<unsigned long long*>(&c)));
-  return d;
-}
-
 enum : uint32_t { kWaitSimtWq = 0x200000u, kWaitSimtAqk = 0x800000u, kWaitSimtKgt = 0x1000000u };
 
 // Shared memory of the scan: the chunk's records as stored (fp32 images), the state tile and Un, value columns outside.
