@@ -224,17 +224,22 @@ int record_cuda_error(cudaError_t e);   // stores e for gdn2_last_cuda_error(), 
     if (e__ != cudaSuccess) return gdn2::record_cuda_error(e__); \
   } while (0)
 
-// Chained launches. A launch made with launch_chained may be set up while the kernel before it in the stream is still
-// running: its blocks take their places and wait in grid_wait() until that kernel has completed and its writes are visible.
-// Every kernel launched this way calls grid_wait() first, in every thread and on every path, before it touches global
-// memory, so "the kernel before has completed" reaches back through the whole chain. The next kernel's blocks start when
-// every block of this one has exited or called grid_launch_dependents(), which comes AFTER grid_wait(): everything before
-// this kernel has then completed, and nothing that an earlier kernel read can still be cached on an SM from a time before
-// this kernel wrote it. The decode and layer kernels call it; the float32 scan does not, because blocks that take their
-// places while a kernel drains crowd onto the SMs that happen to be free first (B = 2, S = 1000, 8 heads of 64: call 103 us
-// with it, 75 without). What chaining saves is launch latency between short kernels: five
-// draft tokens for 24 conversations, f16, 18.4 -> 16.3 us; one token for 256 conversations 86.7 -> 85.3, eight 132.6 -> 129.5;
-// the float32 call above 80 -> 75 (as it was then; 79 now).
+// Chained launches. A launch made with launch_chained may be set up while the kernel before it in the stream is still running:
+// its blocks take their places and wait in grid_wait() until that kernel has completed and its writes are visible. Every
+// kernel launched this way calls grid_wait(), in every thread and on every path, before it writes global memory and before it
+// reads any that the kernel before may write, so "the kernel before has completed" reaches back through the whole chain. The
+// next kernel's blocks start when every block of this one has exited or called grid_launch_dependents(), which comes AFTER
+// grid_wait(): everything before this kernel has then completed, and nothing that an earlier kernel read can still be cached
+// on an SM from a time before this kernel wrote it. What a kernel reads BEFORE its own grid_wait() has to hold under all of
+// these: nothing in the kernel directly before it writes it; that kernel, too, is launched this way by the same host function
+// and waits before it lets the next one start, so that everything earlier has completed; and the read does not go through L1
+// (__ldcg, or .nc with no_allocate), where a line from before an earlier write could have stayed. The second and third kernel
+// of the layer step read the recurrent state and their weights so (layer_step.cu); all others wait first. The decode and layer
+// kernels call grid_launch_dependents(); the float32 scan does not, because blocks that take their places while a kernel
+// drains crowd onto the SMs that happen to be free first (B = 2, S = 1000, 8 heads of 64: call 103 us with it, 75 without).
+// What chaining saves is launch latency between short kernels: five draft tokens for 24 conversations, f16, 18.4 -> 16.3 us;
+// one token for 256 conversations 86.7 -> 85.3, eight 132.6 -> 129.5; the float32 call above 80 -> 75 (as it was then; 71
+// now).
 // The tensor-core prefill, whose calls fork to a second stream, is launched plainly (chained = false), the decode of its
 // ragged tail included, whether this library queues it or a caller that composes the stages (gdn2_decode_tail).
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
